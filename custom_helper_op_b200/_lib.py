@@ -96,6 +96,22 @@ def lib():
     return _lib
 
 
+_glue = None
+
+
+def glue():
+    """The native torch binding of the differentiable ops (cc/torch_glue.cpp); loaded once, no fallback."""
+    global _glue
+    if _glue is None:
+        try:
+            from custom_helper_op_b200 import _torch_glue
+        except ImportError as e:
+            raise ImportError("the native torch binding _torch_glue is not built for this torch and Python (%s); build "
+                              "it with `python -m custom_helper_op_b200.build`" % e) from e
+        _glue = _torch_glue
+    return _glue
+
+
 def status_string(status):
     return lib().chop_status_string(int(status)).decode()
 

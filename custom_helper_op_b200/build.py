@@ -3,20 +3,23 @@
     python -m custom_helper_op_b200.build [--force] [--verbose]
 
 Every .cu under csrc/ is compiled to an object (in parallel) and linked into
-custom_helper_op_b200/libchop_b200.so.  Objects are rebuilt only when a source or header is newer.
-No GPU is needed to build.
+custom_helper_op_b200/libchop_b200.so; cc/torch_glue.cpp, the torch binding of the differentiable ops, is
+compiled against the installed torch into custom_helper_op_b200/_torch_glue.so.  Objects are rebuilt only
+when a source or header is newer.  No GPU is needed to build.
 """
 import argparse
 import concurrent.futures
 import glob
 import os
 import subprocess
-import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libchop_b200.so")
+GLUE_SRC = os.path.join(PKG, "cc", "torch_glue.cpp")
+GLUE = os.path.join(PKG, "_torch_glue.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
@@ -35,6 +38,22 @@ def _newest_header():
     return max(os.path.getmtime(h) for h in hdrs)
 
 
+def _glue_commands():
+    """(compile, link) of the torch binding: plain C++ against torch's headers, linked to libchop_b200.so beside it."""
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    obj = os.path.join(OBJ, "torch_glue.o")
+    compile_cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden",
+                   "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] + \
+        [x for d in inc for x in ("-isystem", d)] + ["-c", GLUE_SRC, "-o", obj]
+    lib = os.path.join(root, "lib")
+    link_cmd = ["g++", "-shared", "-o", GLUE, obj, "-L" + PKG, "-l:" + os.path.basename(LIB), "-L" + lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+                "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib]
+    return obj, compile_cmd, link_cmd
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
@@ -49,6 +68,12 @@ def build(force=False, verbose=False):
             cmd = [_nvcc()] + NVCC_FLAGS + extra + (["-Xptxas", "-v"] if verbose else []) + ["-c", s, "-o", o]
             jobs.append(cmd)
 
+    glue_obj, glue_compile, glue_link = _glue_commands()
+    glue_stale = force or not os.path.exists(glue_obj) or os.path.getmtime(glue_obj) < max(
+        os.path.getmtime(GLUE_SRC), os.path.getmtime(os.path.join(PKG, "..", "include", "chop.h")))
+    if glue_stale:
+        jobs.insert(0, glue_compile)   # the longest job first
+
     def run(cmd):
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         return cmd, r.returncode, r.stdout
@@ -60,9 +85,13 @@ def build(force=False, verbose=False):
                     print(" ".join(cmd))
                     print(out)
                 if rc != 0:
-                    raise RuntimeError("nvcc failed for %s" % cmd[-3])
+                    raise RuntimeError("%s failed for %s" % (os.path.basename(cmd[0]), cmd[-3]))
+    links = []
     if jobs or force or not os.path.exists(LIB):
-        cmd = [_nvcc(), "-shared", "-o", LIB] + objs + ["-lcudart"]
+        links.append([_nvcc(), "-shared", "-o", LIB] + objs + ["-lcudart"])
+    if glue_stale or not os.path.exists(GLUE):
+        links.append(glue_link)
+    for cmd in links:
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if r.returncode != 0:
             print(r.stdout)

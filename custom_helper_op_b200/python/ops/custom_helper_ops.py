@@ -8,6 +8,10 @@ The reference wrapper feeds TensorFlow tensors to a TensorFlow op library.  Tens
 dependency here: the functions take torch CUDA tensors and call the C ABI of libchop_b200.so on the
 current CUDA stream; torch only supplies device memory, streams and autograd plumbing.  Every call
 runs the CUDA kernels - a CPU tensor or a missing library raises.
+
+The differentiable functions (the reference's names) live in native code, cc/torch_glue.cpp; the raw ops
+below them (cost_forward, sparse_conv3d_backward, ...) call the C ABI through ctypes and are what callers
+use that bring their own output buffers, depth ranges or accumulation.
 """
 import ctypes
 
@@ -160,47 +164,28 @@ def cost_backward(kind, ref_image, src_images, depth, offsets, Rs, Ts, cost_grad
     return ref_grad, src_grad, depth_grad
 
 
-class _CostFn(torch.autograd.Function):
-    """Glue between torch autograd and the two raw ops; the counterpart of the reference's
-    @tf.RegisterGradient functions."""
+_Tensor = torch.Tensor
 
-    @staticmethod
-    def forward(ctx, kind, reduce_method, groups, half_centor, ref_image, src_images, depth, offsets, Rs, Ts):
-        cost, mask = cost_forward(kind, ref_image, src_images, depth, offsets, Rs, Ts, reduce_method, groups,
-                                  half_centor)
-        ctx.save_for_backward(ref_image, src_images, depth, offsets, Rs, Ts, mask)
-        ctx.conf = (kind, reduce_method, groups, half_centor)
-        ctx.feature_dtype = ref_image.dtype
-        ctx.mark_non_differentiable(mask)
-        return cost, mask
 
-    @staticmethod
-    def backward(ctx, grad_out, grad_mask):
-        ref_image, src_images, depth, offsets, Rs, Ts, mask = ctx.saved_tensors
-        kind, reduce_method, groups, half_centor = ctx.conf
-        rg, sg, dg = cost_backward(kind, ref_image, src_images, depth, offsets, Rs, Ts, grad_out, mask,
-                                   reduce_method, groups, half_centor)
-        rg = rg.to(ctx.feature_dtype)
-        sg = sg.to(ctx.feature_dtype)
-        return None, None, None, None, rg, sg, dg.view_as(depth), None, None, None
+def _on(t, dev):
+    """t as a tensor on dev: arrays, numbers and tensors of other devices are converted, as torch.as_tensor does."""
+    return t if isinstance(t, _Tensor) and t.device == dev else torch.as_tensor(t, device=dev)
 
 
 def cost_volume(ref_image, src_images, base_plane, offsets, Rs, Ts, reduce_method="MEAN", half_centor=True,
                 name=None):
     """cost [B,H,W,D,C], cost_mask [B,H,W,D,1|C] (reference: custom_helper_ops.py:32-38)."""
     dev = ref_image.device
-    return _CostFn.apply(_lib.KIND_V1, reduce_method, None, half_centor, ref_image, src_images, base_plane,
-                         torch.as_tensor(offsets, device=dev), torch.as_tensor(Rs, device=dev),
-                         torch.as_tensor(Ts, device=dev))
+    return _lib.glue().cost_op(_lib.KIND_V1, reduce_method, 0, half_centor, ref_image, src_images, base_plane,
+                               _on(offsets, dev), _on(Rs, dev), _on(Ts, dev))
 
 
 def cost_volume_v2(ref_image, src_images, depth_grid, Rs, Ts, reduce_method="MEAN", groups=None, half_centor=True,
                    name=None):
     """cost [B,H,W,D,G], cost_mask [B,H,W,D,1|G] (reference: custom_helper_ops.py:65-71)."""
     dev = ref_image.device
-    return _CostFn.apply(_lib.KIND_V2, reduce_method, groups, half_centor, ref_image, src_images,
-                         torch.as_tensor(depth_grid, device=dev), None, torch.as_tensor(Rs, device=dev),
-                         torch.as_tensor(Ts, device=dev))
+    return _lib.glue().cost_op(_lib.KIND_V2, reduce_method, groups or 0, half_centor, ref_image, src_images,
+                               _on(depth_grid, dev), None, _on(Rs, dev), _on(Ts, dev))
 
 
 def cost_volume_v3(ref_image, src_images, base_plane, offsets, Rs, Ts, reduce_method="MEAN", groups=None,
@@ -208,9 +193,8 @@ def cost_volume_v3(ref_image, src_images, base_plane, offsets, Rs, Ts, reduce_me
     """cost [B,H,W,D,1], cost_mask [B,H,W,D,1|3]: the largest correlation between any group of the sampled
     source feature and any group of the reference feature (reference: custom_helper_ops.py:98-104)."""
     dev = ref_image.device
-    return _CostFn.apply(_lib.KIND_V3, reduce_method, groups, half_centor, ref_image, src_images, base_plane,
-                         torch.as_tensor(offsets, device=dev), torch.as_tensor(Rs, device=dev),
-                         torch.as_tensor(Ts, device=dev))
+    return _lib.glue().cost_op(_lib.KIND_V3, reduce_method, groups or 0, half_centor, ref_image, src_images, base_plane,
+                               _on(offsets, dev), _on(Rs, dev), _on(Ts, dev))
 
 
 def cost_aggregate(ref_image, src_images, base_plane, offsets, Rs, Ts, reduce_method="MEAN", half_centor=True,
@@ -218,9 +202,8 @@ def cost_aggregate(ref_image, src_images, base_plane, offsets, Rs, Ts, reduce_me
     """cost [B,H,W,D], cost_mask [B,H,W,D]: the channel-averaged form of cost_volume the reference's
     CostMapLayer uses (custom_helper_ops.py cost_aggregate)."""
     dev = ref_image.device
-    return _CostFn.apply(_lib.KIND_AGG, reduce_method, None, half_centor, ref_image, src_images, base_plane,
-                         torch.as_tensor(offsets, device=dev), torch.as_tensor(Rs, device=dev),
-                         torch.as_tensor(Ts, device=dev))
+    return _lib.glue().cost_op(_lib.KIND_AGG, reduce_method, 0, half_centor, ref_image, src_images, base_plane,
+                               _on(offsets, dev), _on(Rs, dev), _on(Ts, dev))
 
 
 # ---- manifold ("sparse") 3-D convolution --------------------------------------------------------------
@@ -249,6 +232,8 @@ def _sc_desc(images, filters, strides, dilations, dynamic_default):
 def _scalar(value, like):
     """default_value as a device scalar of the images' dtype (python floats keep full precision)."""
     if torch.is_tensor(value):
+        if value.dim() == 0 and value.dtype == like.dtype and value.device == like.device:
+            return value
         return value.to(device=like.device, dtype=like.dtype).reshape(())
     # a fill kernel on the current stream, not a synchronous host-to-device copy; float64 keeps the python float exactly
     return torch.full((), float(value), dtype=like.dtype, device=like.device)
@@ -308,31 +293,12 @@ def sparse_conv3d_backward(images, filters, default_value, base_plane, out_grad,
     return images_grad, filter_grad, default_grad
 
 
-class _SparseConvFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, images, filters, default_value, base_plane, strides, dilations, dynamic_default):
-        out = sparse_conv3d_forward(images, filters, default_value, base_plane, strides, dilations)
-        ctx.save_for_backward(images, filters, default_value, base_plane)
-        ctx.conf = (tuple(strides), tuple(dilations), bool(dynamic_default))
-        return out
-
-    @staticmethod
-    def backward(ctx, out_grad):
-        images, filters, default_value, base_plane = ctx.saved_tensors
-        strides, dilations, dynamic_default = ctx.conf
-        ig, fg, dg = sparse_conv3d_backward(images, filters, default_value, base_plane, out_grad, strides, dilations,
-                                            dynamic_default)
-        # the reference drops the default-value gradient unless dynamic_default (custom_helper_ops.py:284-286)
-        dg = dg.to(default_value.dtype) if dynamic_default else None
-        return ig, fg.to(filters.dtype), dg, None, None, None, None
-
-
 def sparse_conv3d_fast(images, filters, default_value, base_plane, data_format='NDHWC', strides=(1, 1, 1),
                        dilations=(1, 1, 1), dynamic_default=False, name=None):
     """output [B,ceil(H/s),ceil(W/s),ceil(D/s),Cout] (reference: custom_helper_ops.py:263-267)."""
     _require(data_format == 'NDHWC', "data_format must be NDHWC")
-    default_value = _scalar(default_value, images)
-    return _SparseConvFn.apply(images, filters, default_value, base_plane, strides, dilations, dynamic_default)
+    return _lib.glue().sparse_conv(images, filters, _scalar(default_value, images), base_plane, strides, dilations,
+                                   dynamic_default, None)
 
 
 # ---- transposed manifold convolution ------------------------------------------------------------------
@@ -404,31 +370,13 @@ def sparse_conv3d_transpose_backward(images, filters, default_value, base_plane,
     return images_grad, filter_grad
 
 
-class _SparseConvTransposeFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, images, filters, default_value, base_plane, output_size, strides, dilations):
-        out = sparse_conv3d_transpose_forward(images, filters, default_value, base_plane, output_size, strides, dilations)
-        ctx.save_for_backward(images, filters, default_value, base_plane)
-        ctx.conf = (tuple(int(x) for x in output_size), tuple(strides), tuple(dilations))
-        return out
-
-    @staticmethod
-    def backward(ctx, out_grad):
-        images, filters, default_value, base_plane = ctx.saved_tensors
-        output_size, strides, dilations = ctx.conf
-        ig, fg = sparse_conv3d_transpose_backward(images, filters, default_value, base_plane, output_size, out_grad,
-                                                  strides, dilations)
-        # gradients for images and filters only (reference: custom_helper_ops.py:313)
-        return ig, fg.to(filters.dtype), None, None, None, None, None
-
-
 def sparse_conv3d_transpose_fast(images, filters, default_value, base_plane, output_size, data_format='NDHWC',
                                  strides=(1, 1, 1), dilations=(1, 1, 1), dynamic_default=False, name=None):
     """output [B,*output_size,Cin] for filters [fh,fw,fd,Cin,Cout] (reference: custom_helper_ops.py:290-294)."""
     _require(data_format == 'NDHWC', "data_format must be NDHWC")
-    default_value = _scalar(default_value, images)
     output_size = [int(x) for x in (output_size.tolist() if torch.is_tensor(output_size) else output_size)]
-    return _SparseConvTransposeFn.apply(images, filters, default_value, base_plane, output_size, strides, dilations)
+    return _lib.glue().sparse_conv(images, filters, _scalar(default_value, images), base_plane, strides, dilations,
+                                   False, output_size)
 
 
 # ---- SparsePad ----------------------------------------------------------------------------------------
@@ -472,23 +420,10 @@ def sparse_pad_backward(images, base_plane, out_grad, strides=(1, 1, 1)):
     return images_grad
 
 
-class _SparsePadFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, images, base_plane, strides):
-        ctx.save_for_backward(images, base_plane)
-        ctx.strides = tuple(strides)
-        return sparse_pad_forward(images, base_plane, strides)
-
-    @staticmethod
-    def backward(ctx, out_grad):
-        images, base_plane = ctx.saved_tensors
-        return sparse_pad_backward(images, base_plane, out_grad, ctx.strides), None, None
-
-
 def sparse_pad(images, base_plane, strides=(1, 1, 1), dilations=(1, 1, 1), name=None):
     """Zero insertion of a coarse band into the fine band (reference: custom_helper_ops.py:220-234)."""
     _require(len(dilations) == 3, "dilations must be a vector have 3 element")
-    return _SparsePadFn.apply(images, base_plane, strides)
+    return _lib.glue().sparse_pad(images, base_plane, strides)
 
 
 # ---- FeatureAggregate ---------------------------------------------------------------------------------
@@ -550,28 +485,10 @@ def feature_aggregate_backward(src_images, base_plane, offsets, Rs, Ts, mapped_f
     return src_grad, base_grad
 
 
-class _FeatureAggregateFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, half_centor, src_images, base_plane, offsets, Rs, Ts):
-        mapped, mask = feature_aggregate_forward(src_images, base_plane, offsets, Rs, Ts, half_centor)
-        ctx.save_for_backward(src_images, base_plane, offsets, Rs, Ts, mask)
-        ctx.half_centor = half_centor
-        ctx.mark_non_differentiable(mask)
-        return mapped, mask
-
-    @staticmethod
-    def backward(ctx, grad_out, grad_mask):
-        src_images, base_plane, offsets, Rs, Ts, mask = ctx.saved_tensors
-        sg, bg = feature_aggregate_backward(src_images, base_plane, offsets, Rs, Ts, grad_out, mask, ctx.half_centor)
-        # gradients for src_images and base_plane only (reference: custom_helper_ops.py:192)
-        return None, sg.to(src_images.dtype), bg.to(base_plane.dtype), None, None, None
-
-
 def feature_aggregate(src_images, base_plane, offsets, Rs, Ts, half_centor=True, name=None):
     """Warped source features of every view at every voxel (reference: custom_helper_ops.py:166-171)."""
     dev = src_images.device
-    return _FeatureAggregateFn.apply(half_centor, src_images, base_plane, torch.as_tensor(offsets, device=dev),
-                                     torch.as_tensor(Rs, device=dev), torch.as_tensor(Ts, device=dev))
+    return _lib.glue().feature_aggregate(half_centor, src_images, base_plane, _on(offsets, dev), _on(Rs, dev), _on(Ts, dev))
 
 
 # ---- IndexInitializer, DecodePfm ----------------------------------------------------------------------
