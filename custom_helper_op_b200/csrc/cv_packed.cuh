@@ -299,27 +299,6 @@ __global__ void __launch_bounds__(256, CHOP_PK_FWD_BLOCKS) cv_fwd_packed(const C
 //   * the reload is one asm block that updates the eight footprint registers in place; a view that does
 //     not see the plane reads the reference pixel four times instead, which makes all differences zero.
 // ---------------------------------------------------------------------------------------------------
-// project<> without branches: every operation is executed (a non-positive z only produces values that the
-// validity test then discards), so the independent chains of several views can be interleaved by the
-// compiler.  Same unfused operations in the same order as project<float,false>: identical results.
-__device__ __forceinline__ int project_nb(const Coef<float>& c, float depth, int half_centor, int Hs, int Ws, float& dh, float& dw) {
-  const float z = xadd(xmul(c.zc, depth), c.t2);
-  const float w3 = xadd(xmul(c.wc, depth), c.t0);
-  const float h3 = xadd(xmul(c.hc, depth), c.t1);
-  float sw = xdiv(w3, z);
-  float sh = xdiv(h3, z);
-  if (half_centor) {
-    sw = xsub(sw, 0.5f);
-    sh = xsub(sh, 0.5f);
-  }
-  const bool ok = (z > 0.0f) & (sh > 0.0f) & (sw > 0.0f) & (sh < (float)(Hs - 1)) & (sw < (float)(Ws - 1));
-  const int fh = ok ? (int)sh : 0;
-  const int fw = ok ? (int)sw : 0;
-  dh = ok ? xsub(sh, (float)fh) : 0.0f;
-  dw = ok ? xsub(sw, (float)fw) : 0.0f;
-  return ok ? fw + Ws * (fh + c.row0) : -1;
-}
-
 // Shared memory per warp of the plane-major forward: one 16-byte record and one texel index per (view, lane),
 // three ballot words per view / block.
 __host__ __device__ inline size_t pm_fwd_smem_per_warp(int NV) {
@@ -425,11 +404,14 @@ __global__ void __launch_bounds__(32 * CHOP_PM_FWD_WARPS, CHOP_PM_FWD_BLOCKS) cv
       int tt[NV];
       float dhh[NV], dww[NV];
 #pragma unroll
-      for (int n = 0; n < NV; ++n) tt[n] = project_nb(cf[n], depth, a.half_centor, a.Hs, a.Ws, dhh[n], dww[n]);
+      for (int n = 0; n < NV; ++n) {
+        float gh, gw;
+        tt[n] = project<float, false>(cf[n], depth, a.half_centor, a.Hs, a.Ws, dhh[n], dww[n], gh, gw);
+      }
 #pragma unroll
       for (int n = 0; n < NV; ++n) {
         const int t = dv ? tt[n] : -1;
-        const float dh = dv ? dhh[n] : 0.0f, dw = dv ? dww[n] : 0.0f;
+        const float dh = t >= 0 ? dhh[n] : 0.0f, dw = t >= 0 ? dww[n] : 0.0f;
         used += t >= 0;
         rec[n * 32 + lane] = make_float4(dw, dw, dh, dh);
         tex[n * 32 + lane] = t;

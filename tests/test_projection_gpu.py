@@ -1,0 +1,35 @@
+"""The forward kernels' projection (one reciprocal for both quotients) against the oracle where its fast range ends:
+depths around 1e-12 and 1e18 in camera units, where the plain division takes over."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from custom_helper_op_b200.python.ops import custom_helper_ops as ops
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", [1, 2, 3])
+@pytest.mark.parametrize("half_centor", [True, False])
+@pytest.mark.parametrize("scale", [1.0, 3e-14, 4e-14, 5e-14, 3e16, 4e16, 5e16, 1e25])
+def test_depth_scale_does_not_change_the_samples(kind, half_centor, scale):
+    c = helpers.make_case(kind, 91, 1, 2, 11, 13, 8, 9, "random", np.float32)
+    s = np.float32(scale)   # depth and translation scale together: the sample points stay
+    for k in ("depth", "offsets", "Ts"):
+        if c[k] is not None:
+            c[k] = c[k] * s
+    groups = 4 if kind == 2 else 1
+    want, mask = oracle.cost_fwd(kind, c["ref"], c["src"], c["depth"], c["offsets"], c["Rs"], c["Ts"], "MEAN", groups,
+                                 half_centor, np.float32)
+    t = {k: None if v is None else torch.from_numpy(v).cuda() for k, v in c.items()}
+    for reduce in ("MEAN", "MIN"):
+        got, m = ops.cost_forward(kind, t["ref"], t["src"], t["depth"], t["offsets"], t["Rs"], t["Ts"], reduce, groups,
+                                  half_centor)
+        if reduce == "MIN":
+            want, mask = oracle.cost_fwd(kind, c["ref"], c["src"], c["depth"], c["offsets"], c["Rs"], c["Ts"], "MIN",
+                                         groups, half_centor, np.float32)
+            assert helpers.bits_equal(got.cpu().numpy().reshape(want.shape), want)
+        assert np.array_equal(m.cpu().numpy().reshape(mask.shape), mask)
+        assert helpers.rel_err(got.cpu().numpy().reshape(want.shape), want) <= 1e-5
