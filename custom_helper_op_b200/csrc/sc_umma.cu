@@ -102,27 +102,19 @@ __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, uint32_t* r) {
   tmem_ld<16>(taddr + 16, r + 16);
 }
 
-// ---- tap geometry (3x3x3, dilation 1, any strides) -------------------------------------------------------
-// TG = false, "forward form": the tile's voxels are OUTPUT voxels of the (strided) convolution, grid
-//   [B,oH,oW,oD]; a tap reads the input grid [B,H,W,D] (sc_tap in sc_common.cuh).
-// TG = true, "transposed form": the tile's voxels are voxels of the fine grid [B,H,W,D]; a tap reads the
-//   coarse grid [B,oH,oW,oD] and exists only where row, column and absolute depth are multiples of the
-//   strides (sc_tap_t).  At stride 1 the two forms coincide.
+// ---- tap geometry (3x3x3, dilation 1) -----------------------------------------------------------------------
+// The tile's voxels are OUTPUT voxels of the (strided) convolution, grid [B,oH,oW,oD]; a tap reads the input grid
+// [B,H,W,D] (sc_tap in sc_common.cuh).  At stride 1 the same geometry serves the image gradient and the transposed
+// convolution (S1: no multiplications by strides); with strides those run in sc_umma_class_kernel below.
 struct VoxPos {
-  int b, r, c;      // batch, row and column in the fine grid (forward form: of the voxel's centre tap)
+  int b, r, c;      // batch, row and column in the fine grid (of the voxel's centre tap)
   int depth_abs;    // absolute fine depth plane of the voxel
 };
 
-// SM (stride mode): 0 = any strides (runtime divisions), 1 = all strides are 1 (no divisions in the gather),
-// 2 = all strides are powers of two (the transposed form tests and divides with masks and shifts; it performs
-// about a hundred such operations per voxel, which otherwise dominate the kernel).
-__device__ __forceinline__ int div_pow2_trunc(int t, int l) { return t >= 0 ? (t >> l) : -((-t) >> l); }
-
-template <bool TG, int SM>
+template <bool S1>
 __device__ __forceinline__ VoxPos vox_pos(const ScArgs& a, long long v) {
   VoxPos p;
-  constexpr bool S1 = SM == 1;
-  const int d1 = (TG || S1) ? a.D : a.oD, d2 = (TG || S1) ? a.W : a.oW, d3 = (TG || S1) ? a.H : a.oH;
+  const int d1 = S1 ? a.D : a.oD, d2 = S1 ? a.W : a.oW, d3 = S1 ? a.H : a.oH;
   int dz, cc, rr;
   if (v <= 0x7fffffffLL) {   // 64-bit divisions cost several times the rest of this function
     unsigned u = (unsigned)v;
@@ -136,50 +128,26 @@ __device__ __forceinline__ VoxPos vox_pos(const ScArgs& a, long long v) {
     rr = (int)(v % d3);
     p.b = (int)(v / d3);
   }
-  p.r = (TG || S1) ? rr : rr * a.sr;
-  p.c = (TG || S1) ? cc : cc * a.sc;
+  p.r = S1 ? rr : rr * a.sr;
+  p.c = S1 ? cc : cc * a.sc;
   const int bp = __ldg(a.base_plane + (p.b * a.H + p.r) * a.W + p.c);
-  p.depth_abs = (TG || S1) ? dz + bp : (dz + (bp + a.sd - 1) / a.sd) * a.sd;
+  p.depth_abs = S1 ? dz + bp : (dz + (bp + a.sd - 1) / a.sd) * a.sd;
   return p;
 }
 
 // One (fr, fc) column of taps: false if the whole column is padding; otherwise base = index of the source
 // pixel's first voxel and shift = what to subtract from the tap's absolute depth.
-template <bool TG, int SM>
 __device__ __forceinline__ bool tap_column(const ScArgs& a, const VoxPos& p, int fr, int fc, long long& base, int& shift) {
   const int orow = p.r - 1 + fr, ocol = p.c - 1 + fc;
   if (oob(orow, a.H) || oob(ocol, a.W)) return false;
-  const int bp = __ldg(a.base_plane + (p.b * a.H + orow) * a.W + ocol);
-  if (TG && SM == 2) {
-    if ((orow & (a.sr - 1)) != 0 || (ocol & (a.sc - 1)) != 0) return false;   // orow, ocol >= 0 here
-    base = (((long long)p.b * a.oH + (orow >> a.ls_r)) * a.oW + (ocol >> a.ls_c)) * a.oD;
-    shift = div_pow2_trunc(bp + a.sd - 1, a.ls_d);
-  } else if (TG && SM == 0) {
-    if ((orow % a.sr) != 0 || (ocol % a.sc) != 0) return false;
-    base = (((long long)p.b * a.oH + orow / a.sr) * a.oW + ocol / a.sc) * a.oD;
-    shift = (bp + a.sd - 1) / a.sd;
-  } else {
-    base = ((long long)(p.b * a.H + orow) * a.W + ocol) * a.D;
-    shift = bp;
-  }
+  shift = __ldg(a.base_plane + (p.b * a.H + orow) * a.W + ocol);
+  base = ((long long)(p.b * a.H + orow) * a.W + ocol) * a.D;
   return true;
 }
 
 // Source voxel of tap fz in a column, or -1.
-template <bool TG, int SM>
 __device__ __forceinline__ long long tap_voxel(const ScArgs& a, const VoxPos& p, long long base, int shift, int fz) {
-  const int od = p.depth_abs - 1 + fz;
-  if (TG && SM == 2) {
-    if ((od & (a.sd - 1)) != 0) return -1;           // two's complement: also right for negative od
-    const int cd = (od >> a.ls_d) - shift;            // od is a multiple of sd: the shift divides exactly
-    return oob(cd, a.oD) ? -1 : base + cd;
-  }
-  if (TG && SM == 0) {
-    if ((od % a.sd) != 0) return -1;
-    const int cd = od / a.sd - shift;
-    return oob(cd, a.oD) ? -1 : base + cd;
-  }
-  const int ind = od - shift;
+  const int ind = p.depth_abs - 1 + fz - shift;
   return oob(ind, a.D) ? -1 : base + ind;
 }
 
@@ -208,7 +176,7 @@ __device__ __forceinline__ void stage_filter_tiles(const unsigned short* flt, un
 }
 
 // CIN: channels of the gathered tensor (K per tap), COUT: channels produced (N).
-template <int CIN, int COUT, bool DGRAD, int SM>
+template <int CIN, int COUT, bool DGRAD, bool S1>
 __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long long nvox, const int ntiles) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar_s;
@@ -260,7 +228,7 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
     const long long v = (long long)tile * 128 + tid;
     const bool vvalid = v < nvox;
     VoxPos pos = {0, 0, 0, 0};
-    if (vvalid) pos = vox_pos<DGRAD, SM>(a, v);
+    if (vvalid) pos = vox_pos<S1>(a, v);
     unsigned char* a_row = sA + (tid / 8) * SBO + (tid % 8) * 16;
 
     for (int fr = 0; fr < 3; ++fr) {
@@ -269,10 +237,10 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
       for (int fc = 0; fc < 3; ++fc) {
         long long base = 0;
         int shift = 0;
-        const bool inb = vvalid && tap_column<DGRAD, SM>(a, pos, fr, fc, base, shift);
+        const bool inb = vvalid && tap_column(a, pos, fr, fc, base, shift);
 #pragma unroll
         for (int fz = 0; fz < 3; ++fz) {
-          const long long sv = inb ? tap_voxel<DGRAD, SM>(a, pos, base, shift, fz) : -1;
+          const long long sv = inb ? tap_voxel(a, pos, base, shift, fz) : -1;
           const bool ok = sv >= 0;
           const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)(ok ? sv : 0) * CIN);
           unsigned char* dstA = a_row + (fc * 3 + fz) * A_TAP_BYTES;
@@ -333,6 +301,263 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t ncols = 32;
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+  }
+}
+
+
+// ---------------------------------------------------------------------------------------------------------
+// Strided image gradient and transposed convolution: every FINE voxel [B,H,W,D] sums the coarse voxels that lie under
+// its taps.  A tap exists only where row, column and absolute depth are multiples of the strides - at strides (2,2,2)
+// 3.4 of the 27 on average - and which filter columns exist depends on (row mod sr, column mod sc) alone.  So a tile
+// takes 128 voxels of pixels of ONE such class: all its rows share the class's columns (1, 2 or 4 of the nine at
+// stride 2) and only those are gathered and multiplied.
+// Depth is not classed (its parity depends on the base planes): a depth tap that is not aligned is a row of zeros.
+//
+// Padded taps read default_value.  The op's own layer fixes it to zero, then they contribute nothing; for any other
+// value the tile walks all nine columns with the padding rows filled in.
+// ---------------------------------------------------------------------------------------------------------
+// The class a CTA is in.  A CTA's tiles ascend, so the divisions of a class are done when it moves on to the next one, not
+// per tile (they were half of the kernel's instructions).
+struct TileClass {
+  int k;               // pr * sc + pc
+  int pr, pc;          // row and column residue
+  int hc, wc;          // rows and columns of the class
+  int begin, end;      // its tiles
+  unsigned real;       // bit fr*3 + fc: the class has this filter column
+};
+__device__ __forceinline__ void class_open(const ScArgs& a, TileClass& c) {
+  c.pr = c.k / a.sc;
+  c.pc = c.k - c.pr * a.sc;
+  c.hc = (a.H - c.pr + a.sr - 1) / a.sr;
+  c.wc = (a.W - c.pc + a.sc - 1) / a.sc;
+  c.end = c.begin + (int)(((unsigned)a.B * c.hc * c.wc * a.D + 127u) / 128u);   // voxel counts fit 31 bits
+  c.real = 0;
+  for (int f = 0; f < 9; ++f)   // the tap's row and column must be multiples of the strides
+    if ((c.pr - 1 + f / 3 + a.sr) % a.sr == 0 && (c.pc - 1 + f % 3 + a.sc) % a.sc == 0) c.real |= 1u << f;
+}
+
+constexpr int CLS_COLS = 2;   // filter columns staged per round
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, const int ntiles) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ __align__(8) uint64_t mbar_s;
+  __shared__ uint32_t tmem_base_s;
+  constexpr int KC = CIN / 8;
+  constexpr uint32_t LBO = 128, SBO = KC * 128;
+  constexpr int A_TAP_BYTES = 128 * CIN * 2;
+  constexpr int B_TAP_BYTES = COUT * CIN * 2;
+  unsigned char* sB = smem;                       // 27 taps
+  unsigned char* sA = smem + 27 * B_TAP_BYTES;    // CLS_COLS columns of three depth taps
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.out_grad);
+  __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.images_grad);
+
+  stage_filter_tiles<CIN, COUT, true>(static_cast<const unsigned short*>(a.filters), sB, tid, LBO, SBO, B_TAP_BYTES);
+  if (warp == 0) {
+    uint32_t slot = smem_u32(&tmem_base_s), ncols = 32;
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&mbar_s)), "r"(1) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  const uint32_t mbar = smem_u32(&mbar_s);
+  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COUT >> 3) << 17) | ((128u >> 4) << 24);
+
+  unsigned d16 = 0;
+  if (!a.pad_zero) d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
+  const bool padded = (d16 & 0x7fffu) != 0;       // a non-zero default: every tap of every voxel contributes
+  const unsigned d32 = d16 | (d16 << 16);
+  const uint4 padv = make_uint4(d32, d32, d32, d32);
+
+  unsigned char* const a_row = sA + (tid / 8) * SBO + (tid % 8) * 16;
+
+  // the round that is being loaded: this thread's voxel, the class's filter columns still to do
+  int tile = blockIdx.x;
+  TileClass cl;
+  cl.k = 0;
+  cl.begin = 0;
+  class_open(a, cl);
+  unsigned todo = 0;                              // bit fr*3 + fc: filter column still to do
+  bool vvalid = false;
+  int b = 0, r = 0, c = 0, cr = 0, cc = 0;
+  int cdz[3];                                     // absolute coarse plane under depth tap fz
+  unsigned dok = 0;                               // bit fz: the depth tap is aligned
+  long long out_vox = -1;                         // fine voxel of this thread, -1: none
+  auto open_tile = [&]() {
+    while (tile >= cl.end) {
+      ++cl.k;
+      cl.begin = cl.end;
+      class_open(a, cl);
+    }
+    todo = padded ? 0x1ffu : cl.real;
+    const unsigned v = (unsigned)(tile - cl.begin) * 128u + tid;
+    vvalid = v < (unsigned)a.B * cl.hc * cl.wc * a.D;
+    out_vox = -1;
+    dok = 0;
+    if (vvalid) {
+      unsigned u = v;
+      const int dz = (int)(u % (unsigned)a.D); u /= (unsigned)a.D;
+      cc = (int)(u % (unsigned)cl.wc); u /= (unsigned)cl.wc;
+      cr = (int)(u % (unsigned)cl.hc);
+      b = (int)(u / (unsigned)cl.hc);
+      r = cr * a.sr + cl.pr;
+      c = cc * a.sc + cl.pc;
+      const int pix = (b * a.H + r) * a.W + c;
+      out_vox = (long long)pix * a.D + dz;
+      const int d = dz + __ldg(a.base_plane + pix);
+      int q = d / a.sd, rem = d - q * a.sd;       // floor division: one for the three depth taps
+      if (rem < 0) { rem += a.sd; --q; }
+      cdz[0] = a.sd == 1 ? q - 1 : q;
+      cdz[1] = q;
+      cdz[2] = q + 1;
+      dok = (a.sd == 1 || rem == 1 ? 1u : 0u) | (rem == 0 ? 2u : 0u) | (rem + 1 == a.sd ? 4u : 0u);
+    }
+  };
+  int cols[CLS_COLS], ncols = 0;
+  uint4 pre[CLS_COLS * 3 * KC];
+  auto request = [&]() {   // the next CLS_COLS filter columns of the open tile into registers
+    ncols = 0;
+#pragma unroll
+    for (int i = 0; i < CLS_COLS; ++i) {
+      cols[i] = todo ? __ffs(todo) - 1 : 0;
+      if (todo) {
+        ++ncols;
+        todo &= todo - 1;
+      }
+    }
+    int base[CLS_COLS], shift[CLS_COLS];
+    bool ok[CLS_COLS];
+#pragma unroll
+    for (int i = 0; i < CLS_COLS; ++i) {
+      const int fr = cols[i] / 3, fc = cols[i] - fr * 3;
+      const int orow = r - 1 + fr, ocol = c - 1 + fc;
+      ok[i] = i < ncols && vvalid && ((cl.real >> cols[i]) & 1u) && !oob(orow, a.H) && !oob(ocol, a.W);
+      base[i] = shift[i] = 0;
+      if (ok[i]) {
+        // (pr - 1 + fr) / sr of an aligned tap: -1, 0 or 1
+            const int er = cl.pr - 1 + fr, ec = cl.pc - 1 + fc;
+            base[i] = ((b * a.oH + cr + (er > 0) - (er < 0)) * a.oW + cc + (ec > 0) - (ec < 0)) * a.oD;
+        shift[i] = (__ldg(a.base_plane + (b * a.H + orow) * a.W + ocol) + a.sd - 1) / a.sd;   // as in sc_tap_t
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < CLS_COLS; ++i) {
+#pragma unroll
+      for (int fz = 0; fz < 3; ++fz) {
+        const int cd = cdz[fz] - shift[i];
+        const bool in = ok[i] && ((dok >> fz) & 1u) && !oob(cd, a.oD);
+        const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)(in ? base[i] + cd : 0) * CIN);
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc) {
+          uint4 x = vvalid ? padv : make_uint4(0, 0, 0, 0);
+          if (in) x = __ldg(p + kc);
+          pre[(i * 3 + fz) * KC + kc] = x;
+        }
+      }
+    }
+  };
+  cdz[0] = cdz[1] = cdz[2] = 0;
+  open_tile();
+  request();
+
+  uint32_t phase = 0;
+  bool started = false;                           // the tile in the tensor core has accumulated something
+  while (true) {
+    // ---- the requested rows -> staging buffer; MMAs ------------------------------------------------------------
+    const int n_now = ncols;
+    int cols_now[CLS_COLS];
+#pragma unroll
+    for (int i = 0; i < CLS_COLS; ++i) cols_now[i] = cols[i];
+    const bool last = todo == 0;                  // last round of its tile
+    const long long out_now = out_vox;
+    const int KT = CLS_COLS * 3;
+#pragma unroll
+    for (int q = 0; q < KT; ++q) {
+      if (q < n_now * 3) {
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc) *reinterpret_cast<uint4*>(a_row + q * A_TAP_BYTES + kc * LBO) = pre[q * KC + kc];
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int i = 0; i < n_now; ++i) {
+#pragma unroll
+        for (int fz = 0; fz < 3; ++fz) {
+#pragma unroll
+          for (int k16 = 0; k16 < CIN / 16; ++k16) {
+            const uint64_t da = umma_desc(smem_u32(sA + (i * 3 + fz) * A_TAP_BYTES + k16 * 2 * LBO), LBO, SBO);
+            const uint64_t db = umma_desc(smem_u32(sB + (cols_now[i] * 3 + fz) * B_TAP_BYTES + k16 * 2 * LBO), LBO, SBO);
+            umma_bf16(tmem, da, db, IDESC, (started || i > 0 || fz > 0 || k16 > 0) ? 1u : 0u);
+          }
+        }
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+    }
+    started = started || n_now > 0;
+
+    // ---- while they run: the next round's lookups and rows -------------------------------------------------------
+    bool more = true;
+    if (last) {
+      tile += gridDim.x;
+      more = tile < ntiles;
+      if (more) open_tile();
+    }
+    if (more) request();
+
+    bool done = true;
+    if (warp == 0) done = mbar_wait(mbar, phase);
+    phase ^= 1;
+    if (!__syncthreads_and(done)) {
+      if (tid == 0) note_timeout();
+      break;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    if (last) {
+      // ---- epilogue: accumulator rows -> bf16 -> global; a class without taps (strides above 3) is zero --------
+      uint32_t acc[COUT];
+      if (started) {
+        tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16), acc);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      } else {
+#pragma unroll
+        for (int n = 0; n < COUT; ++n) acc[n] = 0u;
+      }
+      if (out_now >= 0) {
+        uint4* o = reinterpret_cast<uint4*>(dst + (size_t)out_now * COUT);
+#pragma unroll
+        for (int q = 0; q < COUT / 8; ++q) {
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(acc[q * 8 + 2 * i]), __uint_as_float(acc[q * 8 + 2 * i + 1]));
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+          o[q] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      started = false;
+    }
+    if (!more) break;
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -575,11 +800,15 @@ __global__ void __launch_bounds__(128, CIN <= 16 ? 4 : 2) sc_umma_rows_kernel(co
 // fixed-order reduction kernel as the generic path sums over the CTAs.
 // d(default_value) (dynamic_default only) is accumulated on the CUDA cores while gathering.
 // ---------------------------------------------------------------------------------------------------------
-// TG = true is the filter gradient of the TRANSPOSED convolution: the voxels are those of the fine grid, the
-// gathered tensor (CIN channels) is the op's coarse input under every tap (default_value where there is
-// none) and G (COUT channels) its upstream gradient; the slab is written [tap][coarse ch][fine ch] and the
-// reduction kernel moves it to filter_grad[flipped tap][fine ch][coarse ch].
-template <int CIN, int COUT, bool TG, int SM>
+// TS = true is the filter gradient of the TRANSPOSED convolution with the roles swapped: a coarse voxel lies under tap t
+// of exactly one fine voxel, which is the voxel that tap 26 - t of the STRIDED convolution reads.  So the same kernel runs
+// over the coarse voxels with a.images = the fine upstream gradient and a.out_grad = the op's coarse input, padding
+// nothing - instead of walking the fine grid (8x the voxels at strides (2,2,2)) whose taps are mostly empty: 133 -> 27 us
+// at the c4 band, 16 -> 16 channels.  What a
+// non-zero default_value adds at the empty taps is linear: default * (sum of the fine gradient over all voxels - over the
+// voxels with a coarse voxel under the tap).  The op's own layer fixes the default to zero, so the two sums are added up in
+// a plain loop, and only if it is not.
+template <int CIN, int COUT, bool TS, bool S1>
 __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, const long long nvox, const int ntiles) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar_s;
@@ -599,7 +828,7 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
   const __nv_bfloat16* img = static_cast<const __nv_bfloat16*>(a.images);
   const __nv_bfloat16* og = static_cast<const __nv_bfloat16*>(a.out_grad);
 
-  const bool dyn = !TG && a.dynamic_default;
+  const bool dyn = !TS && a.dynamic_default;
   if (dyn) {
     const __nv_bfloat16* flt = static_cast<const __nv_bfloat16*>(a.filters);
     for (int e = tid; e < 27 * COUT; e += 128) {
@@ -628,7 +857,7 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
                              ((128u >> 4) << 24);
   const unsigned d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
   const unsigned d32 = d16 | (d16 << 16);
-  const uint4 padv = make_uint4(d32, d32, d32, d32);
+  const uint4 padv = TS ? make_uint4(0, 0, 0, 0) : make_uint4(d32, d32, d32, d32);
   const uint4 zero4 = make_uint4(0, 0, 0, 0);
 
   uint32_t phase = 0;
@@ -645,7 +874,7 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
     float gf[COUT];
 #pragma unroll
     for (int n = 0; n < COUT; ++n) gf[n] = 0.f;
-    if (vvalid) pos = vox_pos<TG, SM>(a, v);
+    if (vvalid) pos = vox_pos<S1>(a, v);
     // out_grad row of this voxel -> G tile (previous tile's MMAs have completed: every round waits)
 #pragma unroll
     for (int nc = 0; nc < COUT / 8; ++nc) {
@@ -662,26 +891,29 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
       }
     }
 
-    for (int rd = 0; rd < NT; ++rd) {
-      // ---- gather the taps of M group rd ---------------------------------------------------------------------
+    // the nine filter columns' source pixels, their base-plane lookups all in flight at once
+    int cbase[9], cshift[9];
+#pragma unroll
+    for (int col = 0; col < 9; ++col) {
+      long long base = 0;
+      int shift = 0;
+      cbase[col] = vvalid && tap_column(a, pos, col / 3, col % 3, base, shift) ? (int)base : -1;
+      cshift[col] = pos.depth_abs - 1 - shift;
+    }
+    // rows of M group rd: requested while the previous group's MMAs run, so only the first group's latency is exposed
+    uint4 pre[TPR * KC];
+    auto request = [&](int rd) {
 #pragma unroll
       for (int tt = 0; tt < TPR; ++tt) {
         const int t = rd * TPR + tt;
+        const bool real_tap = t < 27;
         bool ok = false;
-        bool real_tap = t < 27;
         size_t off = 0;
-        if (real_tap && vvalid) {
-          const int fz = t % 3, fc = (t / 3) % 3, fr = t / 9;
-          long long base = 0;
-          int shift = 0;
-          if (tap_column<TG, SM>(a, pos, fr, fc, base, shift)) {
-            const long long sv = tap_voxel<TG, SM>(a, pos, base, shift, fz);
-            if (sv >= 0) {
-              ok = true;
-              off = (size_t)sv * CIN;
-            }
-          }
-          if (!ok && dyn) {
+        if (real_tap) {
+          const int col = t / 3, ind = cshift[t < 27 ? col : 0] + t % 3;
+          ok = cbase[t < 27 ? col : 0] >= 0 && !oob(ind, a.D);
+          if (ok) off = (size_t)(cbase[t < 27 ? col : 0] + ind) * CIN;
+          if (!ok && dyn && vvalid) {
             // fixed_param_op_gpu.cu.cc:273-277: d(default) += sum_n (sum_ci filter[t][ci][n]) * out_grad[m][n]
             const float* ws = wsum + t * COUT;
 #pragma unroll
@@ -692,9 +924,15 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
         for (int kc = 0; kc < KC; ++kc) {
           uint4 x = (real_tap && vvalid) ? padv : zero4;
           if (ok) x = __ldg(reinterpret_cast<const uint4*>(img + off) + kc);
-          *reinterpret_cast<uint4*>(a_row + (tt * KC + kc) * SBO) = x;
+          pre[tt * KC + kc] = x;
         }
       }
+    };
+    request(0);
+#pragma unroll
+    for (int rd = 0; rd < NT; ++rd) {
+#pragma unroll
+      for (int q = 0; q < TPR * KC; ++q) *reinterpret_cast<uint4*>(a_row + q * SBO) = pre[q];
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncthreads();
@@ -708,6 +946,7 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
       }
+      if (rd + 1 < NT) request(rd + 1);
       // one warp polls the mbarrier (every poll is a shared-memory access); the others wait at the hardware barrier
       bool done = true;
       if (warp == 0) done = mbar_wait(mbar, phase);
@@ -725,6 +964,33 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
   // ---- accumulators -> this CTA's partial slab -----------------------------------------------------------------
   constexpr int K = 27 * CIN;
   float* part = static_cast<float*>(a.workspace) + (size_t)blockIdx.x * ((size_t)K * COUT + 1);
+  float dval = 0.f;
+  if constexpr (TS) {
+    if ((d16 & 0x7fffu) != 0) {   // this CTA's share of the channel sums of the fine gradient, in a fixed order
+      dval = __uint_as_float(d16 << 16);
+      float fs[CIN];
+#pragma unroll
+      for (int ci = 0; ci < CIN; ++ci) fs[ci] = 0.f;
+      for (long long v = (long long)blockIdx.x * 128 + tid; v < a.nvox_in; v += (long long)gridDim.x * 128) {
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc) {
+          const uint4 x = __ldg(reinterpret_cast<const uint4*>(img + (size_t)v * CIN) + kc);
+          const unsigned w4[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            fs[kc * 8 + 2 * i] += __uint_as_float(w4[i] << 16);
+            fs[kc * 8 + 2 * i + 1] += __uint_as_float(w4[i] & 0xffff0000u);
+          }
+        }
+      }
+#pragma unroll
+      for (int ci = 0; ci < CIN; ++ci) {
+        for (int o = 16; o > 0; o >>= 1) fs[ci] += __shfl_xor_sync(0xffffffffu, fs[ci], o);
+        if ((tid & 31) == 0) red_s[warp * CIN + ci] = fs[ci];
+      }
+    }
+    __syncthreads();
+  }
   if (alive) {
 #pragma unroll
     for (int rd = 0; rd < NT; ++rd) {
@@ -734,12 +1000,35 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
       const int k = rd * 128 + tid;
-      if (k < K) {
-#pragma unroll
-        for (int n = 0; n < COUT; ++n) part[(size_t)k * COUT + n] = first ? 0.f : __uint_as_float(acc[n]);
+      float add = 0.f;
+      if constexpr (TS) {
+        if (dval != 0.f) {
+          const int t = k / CIN, ci = k - t * CIN;
+          float seen = 0.f;
+          for (int tile = blockIdx.x; tile < ntiles && k < K; tile += gridDim.x) {
+            for (int m = 0; m < 128 && (long long)tile * 128 + m < nvox; ++m) {
+              const VoxPos p = vox_pos<S1>(a, (long long)tile * 128 + m);
+              long long base;
+              int shift;
+              if (!tap_column(a, p, t / 9, (t / 3) % 3, base, shift)) continue;
+              const long long sv = tap_voxel(a, p, base, shift, t % 3);
+              if (sv >= 0) seen += __bfloat162float(img[(size_t)sv * CIN + ci]);
+            }
+          }
+          add = dval * ((((red_s[ci] + red_s[CIN + ci]) + red_s[2 * CIN + ci]) + red_s[3 * CIN + ci]) - seen);
+        }
       }
+      // through shared memory, so that the stores are consecutive (the staging buffer is free; rows of COUT + 1 floats)
+      float* rows = reinterpret_cast<float*>(sA);
+      __syncthreads();
+#pragma unroll
+      for (int n = 0; n < COUT; ++n) rows[tid * (COUT + 1) + n] = (first ? 0.f : __uint_as_float(acc[n])) + add;
+      __syncthreads();
+      for (int e = tid; e < 128 * COUT; e += 128)
+        if (rd * 128 + e / COUT < K) part[(size_t)rd * 128 * COUT + e] = rows[(e / COUT) * (COUT + 1) + e % COUT];
     }
   }
+  __syncthreads();
   red_s[tid] = dacc;
   __syncthreads();
   for (int o = 64; o > 0; o >>= 1) {
@@ -986,10 +1275,16 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
         // Block 0 supplies columns 0..7, block 1 only column 8 (its rows 112..127).
         const int q = 2 * blk + tid / 8;
         const int col = q / KC, ci = (q % KC) * 8 + (tid % 8);
-        if (blk == 0 || col == 8) {
-          const int k = (col * 3 + fz) * CIN + ci;
+        // Through shared memory (the column buffers are free), so that the stores are consecutive: the CIN rows of
+        // (column, tap) are one stretch of the slab.
+        float* rows = reinterpret_cast<float*>(sX);
+        __syncthreads();
 #pragma unroll
-          for (int n = 0; n < COUT; ++n) part[(size_t)k * COUT + n] = first ? 0.f : __uint_as_float(acc[n]);
+        for (int n = 0; n < COUT; ++n) rows[(col * CIN + ci) * (COUT + 1) + n] = first ? 0.f : __uint_as_float(acc[n]);
+        __syncthreads();
+        for (int e = tid; e < (blk == 0 ? 8 : 1) * CIN * COUT; e += 128) {
+          const int cc = (blk == 0 ? 0 : 8) + e / (CIN * COUT), w = e % (CIN * COUT);
+          part[(size_t)(cc * 3 + fz) * CIN * COUT + w] = rows[(cc * CIN + w / COUT) * (COUT + 1) + w % COUT];
         }
       }
     }
@@ -1010,26 +1305,28 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
   }
 }
 
-// Sum of element e over the slabs warp, warp + 8, warp + 16, ... in a fixed order, four loads in flight (the
-// slabs are 27*CIN*COUT*4 bytes apart, so every load is a separate DRAM/L2 access and one at a time is latency-bound).
+// Sum of element e over the slabs warp, warp + RED_WARPS, ... in a fixed order, four loads in flight (the slabs are
+// 27*CIN*COUT*4 bytes apart, so every load is a separate DRAM/L2 access and one at a time is latency-bound: 592 slabs took
+// 9 us with 8 warps per block).
+constexpr int RED_WARPS = 32;
 __device__ __forceinline__ float slab_column_sum(const float* col, size_t stride, int first, int nparts) {
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   int p = first;
-  for (; p + 24 < nparts; p += 32) {
-    const float a0 = col[(size_t)p * stride], a1 = col[(size_t)(p + 8) * stride], a2 = col[(size_t)(p + 16) * stride],
-                a3 = col[(size_t)(p + 24) * stride];
+  for (; p + 3 * RED_WARPS < nparts; p += 4 * RED_WARPS) {
+    const float a0 = col[(size_t)p * stride], a1 = col[(size_t)(p + RED_WARPS) * stride],
+                a2 = col[(size_t)(p + 2 * RED_WARPS) * stride], a3 = col[(size_t)(p + 3 * RED_WARPS) * stride];
     s0 += a0; s1 += a1; s2 += a2; s3 += a3;
   }
-  for (; p < nparts; p += 8) s0 += col[(size_t)p * stride];
+  for (; p < nparts; p += RED_WARPS) s0 += col[(size_t)p * stride];
   return (s0 + s1) + (s2 + s3);
 }
 
 // Sum of the per-CTA partial slabs in a fixed order (deterministic).  A block owns 32 consecutive
-// elements; its 8 warps each add every 8th slab with coalesced 128-byte reads, then the 8 warp sums are
-// added in warp order.  Element n_el is the default-value gradient.
-__global__ void __launch_bounds__(256) sc_umma_wgrad_reduce(const float* part, int nparts, long long n_el, float* filter_grad,
+// elements; its warps each add every RED_WARPS-th slab with coalesced 128-byte reads, then the warp sums are
+// added in warp order.  Element n_el is the default-value gradient (null: not wanted).
+__global__ void __launch_bounds__(32 * RED_WARPS) sc_umma_wgrad_reduce(const float* part, int nparts, long long n_el, float* filter_grad,
                                                             float* default_grad) {
-  __shared__ float sm[8][32];
+  __shared__ float sm[RED_WARPS][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long e = (long long)blockIdx.x * 32 + lane;
   float s = 0.f;
@@ -1039,16 +1336,16 @@ __global__ void __launch_bounds__(256) sc_umma_wgrad_reduce(const float* part, i
   if (warp == 0 && e <= n_el) {
     float t = sm[0][lane];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) t += sm[w][lane];
+    for (int w = 1; w < RED_WARPS; ++w) t += sm[w][lane];
     if (e < n_el) filter_grad[e] = t;
-    else *default_grad = t;
+    else if (default_grad) *default_grad = t;
   }
 }
 
 // Transposed convolution: slab element [tap][kc][n] (kc: coarse channel of KC, n: fine channel of NC) ->
 // filter_grad[26 - tap][n][kc]; same fixed summation order.
-__global__ void __launch_bounds__(256) sc_umma_wgrad_reduce_t(const float* part, int nparts, int KC, int NC, float* filter_grad) {
-  __shared__ float sm[8][32];
+__global__ void __launch_bounds__(32 * RED_WARPS) sc_umma_wgrad_reduce_t(const float* part, int nparts, int KC, int NC, float* filter_grad) {
+  __shared__ float sm[RED_WARPS][32];
   const long long n_el = (long long)27 * KC * NC;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long e = (long long)blockIdx.x * 32 + lane;
@@ -1059,7 +1356,7 @@ __global__ void __launch_bounds__(256) sc_umma_wgrad_reduce_t(const float* part,
   if (warp == 0 && e < n_el) {
     float t = sm[0][lane];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) t += sm[w][lane];
+    for (int w = 1; w < RED_WARPS; ++w) t += sm[w][lane];
     const int n = (int)(e % NC), kc = (int)((e / NC) % KC), tap = (int)(e / ((long long)NC * KC));
     filter_grad[((long long)(26 - tap) * NC + n) * KC + kc] = t;
   }
@@ -1079,39 +1376,33 @@ int launch_wgrad_rows(const ScArgs& a, int nparts, cudaStream_t st) {
   if (e != cudaSuccess) return (int)e;
   const long long n_el = (long long)27 * 16 * COUT;
   if (TG)
-    sc_umma_wgrad_reduce_t<<<(unsigned)((n_el + 31) / 32), 256, 0, st>>>(static_cast<const float*>(a.workspace), nparts, 16, COUT,
+    sc_umma_wgrad_reduce_t<<<(unsigned)((n_el + 31) / 32), 32 * RED_WARPS, 0, st>>>(static_cast<const float*>(a.workspace), nparts, 16, COUT,
                                                                           static_cast<float*>(a.filter_grad));
   else
-    sc_umma_wgrad_reduce<<<(unsigned)((n_el + 1 + 31) / 32), 256, 0, st>>>(static_cast<const float*>(a.workspace), nparts, n_el,
+    sc_umma_wgrad_reduce<<<(unsigned)((n_el + 1 + 31) / 32), 32 * RED_WARPS, 0, st>>>(static_cast<const float*>(a.workspace), nparts, n_el,
                                                                              static_cast<float*>(a.filter_grad),
                                                                              static_cast<float*>(a.default_grad));
   return (int)cudaGetLastError();
 }
 
-template <int CIN, int COUT, bool TG>
+template <int CIN, int COUT, bool TS>
 int launch_wgrad(const ScArgs& a, int nparts, cudaStream_t st) {
   const bool s1 = a.sr == 1 && a.sc == 1 && a.sd == 1;
-  if constexpr (CIN == 16) {
-    if (s1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_wgrad_rows<COUT, TG>(a, nparts, st);
+  if constexpr (CIN == 16 && !TS) {
+    if (s1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_wgrad_rows<COUT, false>(a, nparts, st);
   }
-  auto k = s1 ? sc_umma_wgrad_kernel<CIN, COUT, TG, 1>
-              : ((TG && a.ls_r >= 0) ? sc_umma_wgrad_kernel<CIN, COUT, TG, TG ? 2 : 0> : sc_umma_wgrad_kernel<CIN, COUT, TG, 0>);
+  auto k = s1 ? sc_umma_wgrad_kernel<CIN, COUT, TS, true> : sc_umma_wgrad_kernel<CIN, COUT, TS, false>;
   const size_t smem = (size_t)16 * 2048 + (size_t)16 * (COUT / 8) * 128 + (size_t)27 * COUT * 4 + 1024;
   if (int e = grant_smem(k, smem)) return e;
-  const long long nvox = TG ? a.nvox_in : a.nvox_out;
-  const int ntiles = (int)((nvox + 127) / 128);
+  const int ntiles = (int)((a.nvox_out + 127) / 128);
   if (nparts > ntiles) nparts = ntiles;  // a persistent CTA per slab: more CTAs than tiles would leave slabs unwritten
-  k<<<nparts, 128, smem, st>>>(a, nvox, ntiles);
+  k<<<nparts, 128, smem, st>>>(a, a.nvox_out, ntiles);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   const long long n_el = (long long)27 * CIN * COUT;
-  if (TG)
-    sc_umma_wgrad_reduce_t<<<(unsigned)((n_el + 31) / 32), 256, 0, st>>>(static_cast<const float*>(a.workspace), nparts, CIN,
-                                                                          COUT, static_cast<float*>(a.filter_grad));
-  else
-    sc_umma_wgrad_reduce<<<(unsigned)((n_el + 1 + 31) / 32), 256, 0, st>>>(static_cast<const float*>(a.workspace), nparts, n_el,
-                                                                             static_cast<float*>(a.filter_grad),
-                                                                             static_cast<float*>(a.default_grad));
+  sc_umma_wgrad_reduce<<<(unsigned)((n_el + 1 + 31) / 32), 32 * RED_WARPS, 0, st>>>(static_cast<const float*>(a.workspace), nparts, n_el,
+                                                                           static_cast<float*>(a.filter_grad),
+                                                                           TS ? nullptr : static_cast<float*>(a.default_grad));
   return (int)cudaGetLastError();
 }
 
@@ -1133,13 +1424,36 @@ int launch_rows(const ScArgs& a, cudaStream_t st) {
 }
 
 
+// Strided image gradient / transposed convolution (c4 band 256x320x9, 16 -> 16, strides (2,2,2): 38 us,
+// against 75 us with all 27 taps gathered per voxel; bound by the index arithmetic of the gather).
+template <int CIN, int COUT>
+int launch_class(const ScArgs& a, cudaStream_t st) {
+  auto k = sc_umma_class_kernel<CIN, COUT>;
+  const size_t smem = (size_t)27 * COUT * CIN * 2 + (size_t)CLS_COLS * 3 * 128 * CIN * 2 + 1024;
+  if (int e = grant_smem(k, smem)) return e;
+  long long ntiles = 0;
+  for (int pr = 0; pr < a.sr; ++pr)
+    for (int pc = 0; pc < a.sc; ++pc) {
+      const long long hc = (a.H - pr + a.sr - 1) / a.sr, wc = (a.W - pc + a.sc - 1) / a.sc;
+      ntiles += (a.B * hc * wc * a.D + 127) / 128;
+    }
+  int per_sm = (int)((size_t)220 * 1024 / (smem + 2048));
+  if (per_sm > 8) per_sm = 8;
+  if (per_sm < 1) per_sm = 1;
+  const long long grid = ntiles < 148LL * per_sm ? ntiles : 148LL * per_sm;
+  k<<<(unsigned)grid, 128, smem, st>>>(a, (int)ntiles);
+  return (int)cudaGetLastError();
+}
+
 template <int CIN, int COUT, bool DGRAD>
 int launch(const ScArgs& a, long long nvox, cudaStream_t st) {
-  // stride 1 and a band of at most 126 planes: the shifted-row kernel
-  if (a.sr == 1 && a.sc == 1 && a.sd == 1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_rows<CIN, COUT, DGRAD>(a, st);
   const bool s1 = a.sr == 1 && a.sc == 1 && a.sd == 1;
-  auto k = s1 ? sc_umma_kernel<CIN, COUT, DGRAD, 1>
-              : ((DGRAD && a.ls_r >= 0) ? sc_umma_kernel<CIN, COUT, DGRAD, DGRAD ? 2 : 0> : sc_umma_kernel<CIN, COUT, DGRAD, 0>);
+  // stride 1 and a band of at most 126 planes: the shifted-row kernel
+  if (s1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_rows<CIN, COUT, DGRAD>(a, st);
+  if constexpr (DGRAD) {
+    if (!s1) return launch_class<CIN, COUT>(a, st);
+  }
+  auto k = s1 ? sc_umma_kernel<CIN, COUT, DGRAD, true> : sc_umma_kernel<CIN, COUT, DGRAD, DGRAD>;
   const size_t smem = (size_t)27 * COUT * CIN * 2 + (size_t)9 * 128 * CIN * 2 + 1024;
   if (int e = grant_smem(k, smem)) return e;
   const int ntiles = (int)((nvox + 127) / 128);
@@ -1182,13 +1496,19 @@ int sc_umma_wgrad_launch(const ScArgs& a, int nparts, cudaStream_t st) {
   return launch_wgrad<32, 32, false>(a, nparts, st);
 }
 
-// Filter gradient of the transposed convolution: gathers a.images (coarse, Cout channels) under the taps of
-// every fine voxel, G = a.out_grad (fine, Cin channels).
+// Filter gradient of the transposed convolution; a.images = its coarse input (Cout channels), a.out_grad = the fine
+// upstream gradient (Cin channels), nparts slabs of 27*Cin*Cout + 1 floats in the workspace.  Stride 1 with 16 coarse
+// channels: the shifted-row kernel over the fine grid; otherwise the swapped roles (see sc_umma_wgrad_kernel).
 int sc_umma_twgrad_launch(const ScArgs& a, int nparts, cudaStream_t st) {
-  if (a.Cin == 16 && a.Cout == 16) return launch_wgrad<16, 16, true>(a, nparts, st);
-  if (a.Cin == 16 && a.Cout == 32) return launch_wgrad<32, 16, true>(a, nparts, st);
-  if (a.Cin == 32 && a.Cout == 16) return launch_wgrad<16, 32, true>(a, nparts, st);
-  return launch_wgrad<32, 32, true>(a, nparts, st);
+  if (a.Cout == 16 && a.sr == 1 && a.sc == 1 && a.sd == 1 && a.D + 2 <= 128 && g_umma_rows.load())
+    return a.Cin == 16 ? launch_wgrad_rows<16, true>(a, nparts, st) : launch_wgrad_rows<32, true>(a, nparts, st);
+  ScArgs w = a;
+  w.images = a.out_grad;
+  w.out_grad = a.images;
+  if (a.Cin == 16 && a.Cout == 16) return launch_wgrad<16, 16, true>(w, nparts, st);
+  if (a.Cin == 16 && a.Cout == 32) return launch_wgrad<16, 32, true>(w, nparts, st);
+  if (a.Cin == 32 && a.Cout == 16) return launch_wgrad<32, 16, true>(w, nparts, st);
+  return launch_wgrad<32, 32, true>(w, nparts, st);
 }
 
 void sc_umma_set_rows(int on) { g_umma_rows = on; }
