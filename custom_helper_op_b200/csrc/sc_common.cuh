@@ -78,4 +78,37 @@ __device__ __forceinline__ long long sc_tap_t(const ScArgs& a, int b, int r, int
   return (((long long)b * a.oH + orow / a.sr) * a.oW + ocol / a.sc) * a.oD + od;
 }
 
+// ---- (row, column) residue classes of the fine grid ------------------------------------------------------------
+// Which filter columns of the gather form exist at a fine voxel depends on (row mod sr, column mod sc) alone, so the
+// strided kernels take their tiles from one class at a time.  A CTA's tiles ascend: the divisions of a class are done
+// when it moves on to the next one, not per tile.
+struct TileClass {
+  int k;               // pr * sc + pc
+  int pr, pc;          // row and column residue
+  int hc, wc;          // rows and columns of the class
+  int begin, end;      // its tiles
+  unsigned real;       // bit fr*3 + fc: a 3x3 filter has this column here (dilation 1)
+};
+template <int TILE>
+__device__ __forceinline__ void class_open(const ScArgs& a, TileClass& c) {
+  c.pr = c.k / a.sc;
+  c.pc = c.k - c.pr * a.sc;
+  c.hc = (a.H - c.pr + a.sr - 1) / a.sr;
+  c.wc = (a.W - c.pc + a.sc - 1) / a.sc;
+  c.end = c.begin + (int)(((unsigned)a.B * c.hc * c.wc * a.D + (unsigned)(TILE - 1)) / (unsigned)TILE);   // 31-bit voxel counts
+  c.real = 0;
+  for (int f = 0; f < 9; ++f)   // the tap's row and column must be multiples of the strides
+    if ((c.pr - 1 + f / 3 + a.sr) % a.sr == 0 && (c.pc - 1 + f % 3 + a.sc) % a.sc == 0) c.real |= 1u << f;
+}
+inline long long class_tiles(const ScArgs& a, int tile) {   // all classes' tiles, for the host
+  long long n = 0;
+  for (int pr = 0; pr < a.sr; ++pr)
+    for (int pc = 0; pc < a.sc; ++pc) {
+      if (pr >= a.H || pc >= a.W) continue;
+      const long long hc = (a.H - pr + a.sr - 1) / a.sr, wc = (a.W - pc + a.sc - 1) / a.sc;
+      n += (a.B * hc * wc * a.D + tile - 1) / tile;
+    }
+  return n;
+}
+
 }  // namespace chop

@@ -26,6 +26,9 @@ bool sc_tile_wgrad_supported(int dtype, const ScArgs& a, bool transposed);
 int sc_tile_wgrad_launch(int dtype, const ScArgs& a, int nparts, cudaStream_t st);
 int sc_tile_twgrad_launch(int dtype, const ScArgs& a, int nparts, cudaStream_t st);
 int sc_tile_gather_launch(int dtype, const ScArgs& a, cudaStream_t st);
+// sums nparts slabs of taps*KC*NC + 1 floats; default_grad may be null
+int sc_slab_reduce(const float* part, int nparts, int taps, int KC, int NC, bool transposed, float* filter_grad,
+                   float* default_grad, cudaStream_t st);
 int sc_umma_timeouts();
 int sc_umma_watch();
 int sc_umma_note_timeout_for_test(int on);

@@ -43,13 +43,15 @@ __global__ void __launch_bounds__(256) sc_fwd_simt(const ScArgs a) {
       for (int fz = 0; fz < a.fd; ++fz) {
         const long long at = sc_tap(a, b, ro, co, dz, fr, fc, fz);
         const T* w = flt + ((long long)(fr * a.fw + fc) * a.fd + fz) * a.Cin * a.Cout + oc;
+        ACC tap = 0;   // per tap first: a two-level sum rounds less than one chain over taps x channels
         if (at < 0) {
-          for (int ci = 0; ci < a.Cin; ++ci) acc += (ACC)ScIo<T>::ld(w + (long long)ci * a.Cout) * defv;
+          for (int ci = 0; ci < a.Cin; ++ci) tap += (ACC)ScIo<T>::ld(w + (long long)ci * a.Cout) * defv;
         } else {
           const T* x = img + at * a.Cin;
           for (int ci = 0; ci < a.Cin; ++ci)
-            acc += (ACC)ScIo<T>::ld(w + (long long)ci * a.Cout) * (ACC)ScIo<T>::ld(x + ci);
+            tap += (ACC)ScIo<T>::ld(w + (long long)ci * a.Cout) * (ACC)ScIo<T>::ld(x + ci);
         }
+        acc += tap;
       }
   ScIo<T>::st(static_cast<T*>(a.output) + idx, acc);
 }
@@ -98,7 +100,9 @@ __global__ void __launch_bounds__(256) sc_dgrad_simt(const ScArgs a) {
         }
         const T* g = og + at * a.Cout;
         const T* w = flt + ((long long)(taps - 1 - t) * a.Cin + ci) * a.Cout;
-        for (int o = 0; o < a.Cout; ++o) acc += (ACC)ScIo<T>::ld(w + o) * (ACC)ScIo<T>::ld(g + o);
+        ACC tap = 0;
+        for (int o = 0; o < a.Cout; ++o) tap += (ACC)ScIo<T>::ld(w + o) * (ACC)ScIo<T>::ld(g + o);
+        acc += tap;
       }
   if (PADDED) acc += pad * (ACC)ScIo<T>::ld(static_cast<const T*>(a.default_value));
   ScIo<T>::st(static_cast<T*>(a.images_grad) + idx, acc);

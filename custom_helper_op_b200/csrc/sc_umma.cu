@@ -323,26 +323,6 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
 // Padded taps read default_value.  The op's own layer fixes it to zero, then they contribute nothing; for any other
 // value the tile walks all nine columns with the padding rows filled in.
 // ---------------------------------------------------------------------------------------------------------
-// The class a CTA is in.  A CTA's tiles ascend, so the divisions of a class are done when it moves on to the next one, not
-// per tile (they were half of the kernel's instructions).
-struct TileClass {
-  int k;               // pr * sc + pc
-  int pr, pc;          // row and column residue
-  int hc, wc;          // rows and columns of the class
-  int begin, end;      // its tiles
-  unsigned real;       // bit fr*3 + fc: the class has this filter column
-};
-__device__ __forceinline__ void class_open(const ScArgs& a, TileClass& c) {
-  c.pr = c.k / a.sc;
-  c.pc = c.k - c.pr * a.sc;
-  c.hc = (a.H - c.pr + a.sr - 1) / a.sr;
-  c.wc = (a.W - c.pc + a.sc - 1) / a.sc;
-  c.end = c.begin + (int)(((unsigned)a.B * c.hc * c.wc * a.D + 127u) / 128u);   // voxel counts fit 31 bits
-  c.real = 0;
-  for (int f = 0; f < 9; ++f)   // the tap's row and column must be multiples of the strides
-    if ((c.pr - 1 + f / 3 + a.sr) % a.sr == 0 && (c.pc - 1 + f % 3 + a.sc) % a.sc == 0) c.real |= 1u << f;
-}
-
 constexpr int CLS_COLS = 2;   // filter columns staged per round
 
 template <int CIN, int COUT>
@@ -391,7 +371,7 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
   TileClass cl;
   cl.k = 0;
   cl.begin = 0;
-  class_open(a, cl);
+  class_open<128>(a, cl);
   unsigned todo = 0;                              // bit fr*3 + fc: filter column still to do
   bool vvalid = false;
   int b = 0, r = 0, c = 0, cr = 0, cc = 0;
@@ -402,7 +382,7 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
     while (tile >= cl.end) {
       ++cl.k;
       cl.begin = cl.end;
-      class_open(a, cl);
+      class_open<128>(a, cl);
     }
     todo = padded ? 0x1ffu : cl.real;
     const unsigned v = (unsigned)(tile - cl.begin) * 128u + tid;
@@ -1305,63 +1285,6 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
   }
 }
 
-// Sum of element e over the slabs warp, warp + RED_WARPS, ... in a fixed order, four loads in flight (the slabs are
-// 27*CIN*COUT*4 bytes apart, so every load is a separate DRAM/L2 access and one at a time is latency-bound: 592 slabs took
-// 9 us with 8 warps per block).
-constexpr int RED_WARPS = 32;
-__device__ __forceinline__ float slab_column_sum(const float* col, size_t stride, int first, int nparts) {
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  int p = first;
-  for (; p + 3 * RED_WARPS < nparts; p += 4 * RED_WARPS) {
-    const float a0 = col[(size_t)p * stride], a1 = col[(size_t)(p + RED_WARPS) * stride],
-                a2 = col[(size_t)(p + 2 * RED_WARPS) * stride], a3 = col[(size_t)(p + 3 * RED_WARPS) * stride];
-    s0 += a0; s1 += a1; s2 += a2; s3 += a3;
-  }
-  for (; p < nparts; p += RED_WARPS) s0 += col[(size_t)p * stride];
-  return (s0 + s1) + (s2 + s3);
-}
-
-// Sum of the per-CTA partial slabs in a fixed order (deterministic).  A block owns 32 consecutive
-// elements; its warps each add every RED_WARPS-th slab with coalesced 128-byte reads, then the warp sums are
-// added in warp order.  Element n_el is the default-value gradient (null: not wanted).
-__global__ void __launch_bounds__(32 * RED_WARPS) sc_umma_wgrad_reduce(const float* part, int nparts, long long n_el, float* filter_grad,
-                                                            float* default_grad) {
-  __shared__ float sm[RED_WARPS][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long e = (long long)blockIdx.x * 32 + lane;
-  float s = 0.f;
-  if (e <= n_el) s = slab_column_sum(part + e, (size_t)(n_el + 1), warp, nparts);
-  sm[warp][lane] = s;
-  __syncthreads();
-  if (warp == 0 && e <= n_el) {
-    float t = sm[0][lane];
-#pragma unroll
-    for (int w = 1; w < RED_WARPS; ++w) t += sm[w][lane];
-    if (e < n_el) filter_grad[e] = t;
-    else if (default_grad) *default_grad = t;
-  }
-}
-
-// Transposed convolution: slab element [tap][kc][n] (kc: coarse channel of KC, n: fine channel of NC) ->
-// filter_grad[26 - tap][n][kc]; same fixed summation order.
-__global__ void __launch_bounds__(32 * RED_WARPS) sc_umma_wgrad_reduce_t(const float* part, int nparts, int KC, int NC, float* filter_grad) {
-  __shared__ float sm[RED_WARPS][32];
-  const long long n_el = (long long)27 * KC * NC;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long e = (long long)blockIdx.x * 32 + lane;
-  float s = 0.f;
-  if (e < n_el) s = slab_column_sum(part + e, (size_t)(n_el + 1), warp, nparts);
-  sm[warp][lane] = s;
-  __syncthreads();
-  if (warp == 0 && e < n_el) {
-    float t = sm[0][lane];
-#pragma unroll
-    for (int w = 1; w < RED_WARPS; ++w) t += sm[w][lane];
-    const int n = (int)(e % NC), kc = (int)((e / NC) % KC), tap = (int)(e / ((long long)NC * KC));
-    filter_grad[((long long)(26 - tap) * NC + n) * KC + kc] = t;
-  }
-}
-
 template <int COUT, bool TG>
 int launch_wgrad_rows(const ScArgs& a, int nparts, cudaStream_t st) {
   auto k = sc_umma_wgrad_rows_kernel<COUT, TG>;
@@ -1374,15 +1297,8 @@ int launch_wgrad_rows(const ScArgs& a, int nparts, cudaStream_t st) {
   k<<<nparts, 128, smem, st>>>(a, (int)ntiles, PT);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  const long long n_el = (long long)27 * 16 * COUT;
-  if (TG)
-    sc_umma_wgrad_reduce_t<<<(unsigned)((n_el + 31) / 32), 32 * RED_WARPS, 0, st>>>(static_cast<const float*>(a.workspace), nparts, 16, COUT,
-                                                                          static_cast<float*>(a.filter_grad));
-  else
-    sc_umma_wgrad_reduce<<<(unsigned)((n_el + 1 + 31) / 32), 32 * RED_WARPS, 0, st>>>(static_cast<const float*>(a.workspace), nparts, n_el,
-                                                                             static_cast<float*>(a.filter_grad),
-                                                                             static_cast<float*>(a.default_grad));
-  return (int)cudaGetLastError();
+  return sc_slab_reduce(static_cast<const float*>(a.workspace), nparts, 27, 16, COUT, TG, static_cast<float*>(a.filter_grad),
+                        TG ? nullptr : static_cast<float*>(a.default_grad), st);
 }
 
 template <int CIN, int COUT, bool TS>
@@ -1399,11 +1315,8 @@ int launch_wgrad(const ScArgs& a, int nparts, cudaStream_t st) {
   k<<<nparts, 128, smem, st>>>(a, a.nvox_out, ntiles);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  const long long n_el = (long long)27 * CIN * COUT;
-  sc_umma_wgrad_reduce<<<(unsigned)((n_el + 1 + 31) / 32), 32 * RED_WARPS, 0, st>>>(static_cast<const float*>(a.workspace), nparts, n_el,
-                                                                           static_cast<float*>(a.filter_grad),
-                                                                           TS ? nullptr : static_cast<float*>(a.default_grad));
-  return (int)cudaGetLastError();
+  return sc_slab_reduce(static_cast<const float*>(a.workspace), nparts, 27, CIN, COUT, false, static_cast<float*>(a.filter_grad),
+                        TS ? nullptr : static_cast<float*>(a.default_grad), st);
 }
 
 template <int CIN, int COUT, bool DGRAD>
@@ -1431,12 +1344,7 @@ int launch_class(const ScArgs& a, cudaStream_t st) {
   auto k = sc_umma_class_kernel<CIN, COUT>;
   const size_t smem = (size_t)27 * COUT * CIN * 2 + (size_t)CLS_COLS * 3 * 128 * CIN * 2 + 1024;
   if (int e = grant_smem(k, smem)) return e;
-  long long ntiles = 0;
-  for (int pr = 0; pr < a.sr; ++pr)
-    for (int pc = 0; pc < a.sc; ++pc) {
-      const long long hc = (a.H - pr + a.sr - 1) / a.sr, wc = (a.W - pc + a.sc - 1) / a.sc;
-      ntiles += (a.B * hc * wc * a.D + 127) / 128;
-    }
+  const long long ntiles = class_tiles(a, 128);
   int per_sm = (int)((size_t)220 * 1024 / (smem + 2048));
   if (per_sm > 8) per_sm = 8;
   if (per_sm < 1) per_sm = 1;

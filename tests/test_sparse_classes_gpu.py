@@ -58,3 +58,27 @@ def test_image_gradient_of_the_strided_convolution(strides, chans):
     ig, _, _ = ops.sparse_conv3d_backward(_t(images, bf), _t(filters, bf), float(defv), _t(bp), _t(og, bf), strides)
     assert helpers.rel_err(ig.float().cpu().numpy(), ig_w) <= 1e-2
     assert _lib.lib().chop_umma_timeouts() == 0
+
+
+@pytest.mark.parametrize("strides", [(1, 1, 1), (2, 2, 2), (3, 1, 2)])
+@pytest.mark.parametrize("chans", [(8, 32), (32, 8), (8, 8), (32, 32)])
+@pytest.mark.parametrize("ksize", [(3, 3, 3), (1, 3, 5)])
+def test_register_tiled_kernels_at_every_channel_pair(strides, chans, ksize):
+    """float32 on the lane-split CUDA-core kernels: every number of lanes per voxel, ragged last tiles, residue classes."""
+    Cin, Cout = chans
+    B, H, W, D = 2, 7, 9, 5
+    images, filters, defv, bp, _ = make_case(55, B, H, W, D, Cin, Cout, ksize, 20, np.float32)
+    want = oracle.sparse_conv3d_fwd(images, filters, defv, bp, strides=strides, dtype=np.float32)
+    og = np.random.default_rng(56).uniform(-1, 1, want.shape).astype(np.float32)
+    ig_w, fg_w, dg_w = oracle.sparse_conv3d_bwd(images, filters, defv, bp, og, strides=strides, dynamic_default=True,
+                                                dtype=np.float32)
+    out = ops.sparse_conv3d_forward(_t(images), _t(filters), float(defv), _t(bp), strides)
+    ig, fg, dg = ops.sparse_conv3d_backward(_t(images), _t(filters), float(defv), _t(bp), _t(og), strides, dynamic_default=True)
+    assert helpers.rel_err(out.cpu().numpy(), want) <= 1e-5
+    assert helpers.rel_err(ig.cpu().numpy(), ig_w) <= 1e-5
+    assert helpers.rel_err(fg.cpu().numpy(), fg_w) <= 1e-5
+    assert abs(float(dg) - float(dg_w)) <= 2e-4 * max(1.0, abs(float(dg_w)))   # a cancelling sum over all padded taps
+    images, filters, defv, bp = make_transpose_case(57, B, H, W, D, Cin, Cout, ksize, strides, dtype=np.float32)
+    want = oracle.sparse_conv3d_transpose_fwd(images, filters, defv, bp, (H, W, D), strides, (1, 1, 1), np.float32)
+    out = ops.sparse_conv3d_transpose_forward(_t(images), _t(filters), float(defv), _t(bp), (H, W, D), strides)
+    assert helpers.rel_err(out.cpu().numpy(), want) <= 1e-5
