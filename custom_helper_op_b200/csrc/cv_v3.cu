@@ -17,7 +17,7 @@
 // smallest reference group.  The shuffle reduction applies exactly that order, and sample and dot product
 // are evaluated with unfused operations in the reference's order, so cost, mask and winner indices are
 // bit-identical to the reference compiled without contraction.
-#include "cv_project.cuh"
+#include "cv_packed.cuh"
 #include "cv_v3_entry.h"
 #include "smem_grant.h"
 
@@ -408,6 +408,407 @@ __global__ void __launch_bounds__(256) cv3_bwd_kernel(const CvArgs a, const int 
   if (pvalid && li == 0) atomicAdd(static_cast<R*>(a.depth_grad) + pix, dsum);   // :505
 }
 
+// ---- MEAN, single precision, groups and channels per group known at compile time ------------------------------
+// The kernels above take their arithmetic one operation at a time and fetch the corners and the reference groups for every
+// plane.  Here
+//   * the reference pixel stays in registers as pairs of reference groups {ref[2p][k], ref[2p+1][k]}, so a dot product with
+//     two groups is SUB paired multiplications and SUB-1 paired additions (each rounded like the scalar operation,
+//     nothing is fused: values stay bit-identical);
+//   * the source group's four corners stay in registers until the footprint moves;
+//   * MEAN needs the largest VALUE in the forward pass, not its indices: one max per candidate and a butterfly of maxima.
+// The gradient finds the winner from the same values (largest; on ties the smallest source group, then the smallest
+// reference group - the order of the sequential search) and collects the moments of the upstream gradient while lane,
+// footprint and reference group stay the same, so a plane costs the winning lane a dozen operations and the corner
+// reductions are made once per run instead of once per plane.
+// Bound: issue of the unfused multiplications and additions.  128x160x192, two views, C = 32, eight groups: forward 595 -> 320
+// us, gradient 916 -> 630 us.
+template <int G>
+struct V3Cfg {
+  static constexpr int PX = 32 / G;      // pixels per warp, G lanes each
+  static constexpr int PB = 8;           // planes per block
+  static constexpr int PL = PB / G;      // planes that a lane projects
+};
+template <int G>
+__host__ __device__ constexpr size_t v3_mean_smem(int N, int C, bool bwd) {
+  typedef V3Cfg<G> Cf;
+  return (size_t)N * Cf::PX * sizeof(Coef<float>) + (size_t)Cf::PB * Cf::PX * (32 + 4 + (bwd ? 32 : 0)) +
+         (bwd ? (size_t)2 * Cf::PX * C * 4 : 0);
+}
+
+// a source group's corners: SUB channels as pairs
+template <typename T, int SUB>
+struct V3Corner {
+  pk2 v[SUB / 2];
+  __device__ __forceinline__ void load(const T* p) {
+#pragma unroll
+    for (int q = 0; q < SUB / 4; ++q) PkLoad<T>::ld(p + 4 * q, v[2 * q], v[2 * q + 1]);
+  }
+};
+
+// The assembler contracts a paired multiplication and a paired addition into one fused operation although both carry .rn
+// (measured; it leaves the scalar ones alone).  An addition written as x*1 + y with a 1 that it cannot see through rounds
+// once, like the addition, and cannot take the product in.
+__device__ __forceinline__ pk2 opaque_ones(const CvArgs& a) {
+  const float one = a.B > 0 ? 1.0f : 2.0f;   // B >= 1 always; only the host knows
+  return pk_make(one, one);
+}
+__device__ __forceinline__ pk2 pk_add_unfused(pk2 x, pk2 y, pk2 ones) { return pk_fma(x, ones, y); }
+
+// dot products of this lane's sampled group with every reference group: val[p] = pair of groups 2p, 2p+1
+template <typename T, int SUB, int G>
+__device__ __forceinline__ void v3_dots(const V3Corner<T, SUB>& c00, const V3Corner<T, SUB>& c01, const V3Corner<T, SUB>& c10,
+                                        const V3Corner<T, SUB>& c11, const ulonglong2 wA, const ulonglong2 wB,
+                                        const pk2 (&ref)[SUB][G / 2], pk2 ones, pk2 (&val)[G / 2]) {
+#pragma unroll
+  for (int q = 0; q < SUB / 2; ++q) {
+    // operand order of cost_volume_kernels_gpu_v3.cu.cc:114-115
+    pk2 s2 = pk_add_unfused(pk_mul(wA.y, c01.v[q]), pk_mul(wA.x, c00.v[q]), ones);
+    s2 = pk_add_unfused(pk_mul(wB.y, c11.v[q]), s2, ones);
+    s2 = pk_add_unfused(pk_mul(wB.x, c10.v[q]), s2, ones);
+    float s[2];
+    pk_split(s2, s[0], s[1]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const pk2 ss = pk_make(s[i], s[i]);
+#pragma unroll
+      for (int p = 0; p < G / 2; ++p) {
+        const pk2 m = pk_mul(ss, ref[2 * q + i][p]);
+        val[p] = q == 0 && i == 0 ? m : pk_add_unfused(m, val[p], ones);   // :118-126
+      }
+    }
+  }
+}
+
+template <typename T, int SUB, int G>
+__global__ void __launch_bounds__(128, 5) cv3_fwd_mean(const CvArgs a, const int smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef V3Cfg<G> Cf;
+  constexpr int C = SUB * G, PX = Cf::PX, PB = Cf::PB, PL = Cf::PL;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int li = lane & (G - 1), g = lane / G;
+  const long long item = (long long)blockIdx.x * 4 + wib;
+  if (item >= (long long)a.npb * a.nchunks) return;
+  const int chunk_id = (int)(item / a.npb);
+  const long long pix0 = (item - (long long)chunk_id * a.npb) * PX;
+  const bool pvalid = pix0 + g < a.npix;
+  const long long pix = pvalid ? pix0 + g : a.npix - 1;
+  const int dlo = a.d_begin + chunk_id * a.chunk, dhi = min(a.d_end, dlo + a.chunk);
+  const int N = a.N, D = a.D;
+  unsigned char* mine = smem_raw + (size_t)wib * smem_per_warp;
+  Coef<float>* coef = reinterpret_cast<Coef<float>*>(mine);                       // [N][PX]
+  float4* wgt = reinterpret_cast<float4*>(coef + N * PX);                         // [PB][PX][2] {w00,w00,w01,w01} {w10,w10,w11,w11}
+  int* tex = reinterpret_cast<int*>(wgt + 2 * PB * PX);                           // [PB][PX] texel or -1
+  stage_coefs<float>(a, coef, lane, PX, pix0);
+  pk2 ref[SUB][G / 2];
+  {
+    const T* rp = static_cast<const T*>(a.ref) + pix * C;
+#pragma unroll
+    for (int k = 0; k < SUB; ++k)
+#pragma unroll
+      for (int p = 0; p < G / 2; ++p)
+        ref[k][p] = pk_make(ld1<T, float>(rp + 2 * p * SUB + k), ld1<T, float>(rp + (2 * p + 1) * SUB + k));
+  }
+  const int b = (int)(pix / ((long long)a.H * a.W));
+  const float base = static_cast<const float*>(a.depth)[pix];
+  const float* offs = static_cast<const float*>(a.offsets) + (long long)b * D;
+  const T* src_lane = static_cast<const T*>(a.src) + li * SUB;
+  const size_t row = (size_t)a.Ws * C;
+  const pk2 ones = opaque_ones(a);
+  __syncwarp();
+
+  for (int dblk = dlo; dblk < dhi; dblk += PB) {
+    float acc[PB];
+    int used[PL];
+    float depth[PL];
+#pragma unroll
+    for (int j = 0; j < PB; ++j) acc[j] = 0.0f;
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      used[p] = 0;
+      depth[p] = xadd(base, offs[min(dblk + p * G + li, dhi - 1)]);
+    }
+    for (int n = 0; n < N; ++n) {
+      const Coef<float> cf = coef[n * PX + g];
+#pragma unroll
+      for (int p = 0; p < PL; ++p) {
+        float dh, dw, gh, gw, w00, w01, w11, w10;
+        const int t = project<float, false>(cf, depth[p], a.half_centor, a.Hs, a.Ws, dh, dw, gh, gw);
+        bilinear_weights(dh, dw, w00, w01, w11, w10);
+        used[p] += t >= 0;
+        const int slot = (p * G + li) * PX + g;
+        wgt[2 * slot] = make_float4(w00, w00, w01, w01);
+        wgt[2 * slot + 1] = make_float4(w10, w10, w11, w11);
+        tex[slot] = t;
+      }
+      __syncwarp();
+      int cur = -1;
+      V3Corner<T, SUB> c00, c01, c10, c11;
+#pragma unroll
+      for (int q = 0; q < SUB / 2; ++q) c00.v[q] = c01.v[q] = c10.v[q] = c11.v[q] = 0ull;
+#pragma unroll
+      for (int j = 0; j < PB; ++j) {
+        const int t = tex[j * PX + g];
+        if (t >= 0 && t != cur) {
+          cur = t;
+          const T* p = src_lane + (size_t)t * C;
+          c00.load(p);
+          c01.load(p + C);
+          c10.load(p + row);
+          c11.load(p + row + C);
+        }
+        const ulonglong2 wA = *reinterpret_cast<const ulonglong2*>(wgt + 2 * (j * PX + g));
+        const ulonglong2 wB = *reinterpret_cast<const ulonglong2*>(wgt + 2 * (j * PX + g) + 1);
+        pk2 val[G / 2];
+        v3_dots<T, SUB, G>(c00, c01, c10, c11, wA, wB, ref, ones, val);
+        float m = Lim<float>::min_pos();   // :110
+#pragma unroll
+        for (int p = 0; p < G / 2; ++p) {
+          float x, y;
+          pk_split(val[p], x, y);
+          m = fmaxf(m, fmaxf(x, y));
+        }
+#pragma unroll
+        for (int o = G >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (t >= 0) acc[j] = xadd(acc[j], m);   // :130
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      float v = 0.0f;
+#pragma unroll
+      for (int i = 0; i < G; ++i)
+        if (li == i) v = acc[p * G + i];
+      const int d = dblk + p * G + li;
+      if (pvalid && d < dhi) {
+        static_cast<float*>(a.cost)[pix * D + d] = used[p] > 0 ? xdiv(v, (float)used[p]) : 0.0f;   // :136-141
+        a.mask[pix * D + d] = used[p];
+      }
+    }
+  }
+}
+
+template <typename T, int SUB, int G>
+__global__ void __launch_bounds__(128, 4) cv3_bwd_mean(const CvArgs a, const int smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef V3Cfg<G> Cf;
+  constexpr int C = SUB * G, PX = Cf::PX, PB = Cf::PB, PL = Cf::PL;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int li = lane & (G - 1), g = lane / G;
+  const long long item = (long long)blockIdx.x * 4 + wib;
+  if (item >= (long long)a.npb * a.nchunks) return;
+  const int chunk_id = (int)(item / a.npb);
+  const long long pix0 = (item - (long long)chunk_id * a.npb) * PX;
+  const bool pvalid = pix0 + g < a.npix;
+  const long long pix = pvalid ? pix0 + g : a.npix - 1;
+  const int dlo = a.d_begin + chunk_id * a.chunk, dhi = min(a.d_end, dlo + a.chunk);
+  const int N = a.N, D = a.D;
+  unsigned char* mine = smem_raw + (size_t)wib * smem_per_warp;
+  Coef<float>* coef = reinterpret_cast<Coef<float>*>(mine);                       // [N][PX]
+  float4* wgt = reinterpret_cast<float4*>(coef + N * PX);                         // [PB][PX][2], as in the forward pass
+  float4* aux = wgt + 2 * PB * PX;                                                // [PB][PX][2] {dw, dh, cg, -} {gh*cg, gw*cg, -, -}
+  float* refs = reinterpret_cast<float*>(aux + 2 * PB * PX);                      // [PX][C]
+  float* rgacc = refs + PX * C;                                                   // [PX][C] d(ref) of this work item
+  int* tex = reinterpret_cast<int*>(rgacc + PX * C);                              // [PB][PX]
+  stage_coefs<float>(a, coef, lane, PX, pix0);
+  for (int e = lane; e < PX * C; e += 32) {
+    long long p = pix0 + e / C;
+    if (p >= a.npix) p = a.npix - 1;
+    refs[e] = ld1<T, float>(static_cast<const T*>(a.ref) + p * C + (e % C));
+    rgacc[e] = 0.0f;
+  }
+  __syncwarp();
+  const float* refp = refs + g * C;
+  float* rgp = rgacc + g * C;
+  pk2 ref[SUB][G / 2];
+#pragma unroll
+  for (int k = 0; k < SUB; ++k)
+#pragma unroll
+    for (int p = 0; p < G / 2; ++p) ref[k][p] = pk_make(refp[2 * p * SUB + k], refp[(2 * p + 1) * SUB + k]);
+  const int b = (int)(pix / ((long long)a.H * a.W));
+  const float base = static_cast<const float*>(a.depth)[pix];
+  const float* offs = static_cast<const float*>(a.offsets) + (long long)b * D;
+  const T* src_lane = static_cast<const T*>(a.src) + li * SUB;
+  float* sg_lane = static_cast<float*>(a.src_grad) + li * SUB;
+  const size_t row = (size_t)a.Ws * C;
+  const pk2 ones = opaque_ones(a);
+  float dsum = 0.0f;
+
+  // the lane's validity counts and upstream values of the next block stream in while this block is worked on
+  int m_next[PL];
+  float cg_next[PL];
+  auto stream = [&](int d0) {
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      const int d = d0 + p * G + li;
+      m_next[p] = 0;
+      cg_next[p] = 0.0f;
+      if (pvalid && d < dhi) {
+        m_next[p] = __ldg(a.mask + pix * D + d);
+        cg_next[p] = __ldg(static_cast<const float*>(a.cost_grad) + pix * D + d);
+      }
+    }
+  };
+  stream(dlo);
+  for (int dblk = dlo; dblk < dhi; dblk += PB) {
+    int m_cur[PL];
+    float cg[PL], depth[PL];
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      m_cur[p] = m_next[p];
+      cg[p] = m_cur[p] > 0 ? cg_next[p] / (float)m_cur[p] : 0.0f;   // :393, :426
+      depth[p] = xadd(base, offs[min(dblk + p * G + li, dhi - 1)]);
+    }
+    stream(dblk + PB);
+    for (int n = 0; n < N; ++n) {
+      const Coef<float> cf = coef[n * PX + g];
+#pragma unroll
+      for (int p = 0; p < PL; ++p) {
+        float dh = 0.0f, dw = 0.0f, gh = 0.0f, gw = 0.0f, w00, w01, w11, w10;
+        int t = -1;
+        if (m_cur[p] > 0) t = project<float, true>(cf, depth[p], a.half_centor, a.Hs, a.Ws, dh, dw, gh, gw);
+        if (t < 0) dh = dw = gh = gw = 0.0f;
+        bilinear_weights(dh, dw, w00, w01, w11, w10);
+        const int slot = (p * G + li) * PX + g;
+        wgt[2 * slot] = make_float4(w00, w00, w01, w01);
+        wgt[2 * slot + 1] = make_float4(w10, w10, w11, w11);
+        aux[2 * slot] = make_float4(dw, dh, cg[p], 0.0f);
+        aux[2 * slot + 1] = make_float4(gh * cg[p], gw * cg[p], 0.0f, 0.0f);
+        tex[slot] = t;
+      }
+      __syncwarp();
+
+      int cur = -1, gi_run = -1;
+      V3Corner<T, SUB> c00, c01, c10, c11;
+#pragma unroll
+      for (int q = 0; q < SUB / 2; ++q) c00.v[q] = c01.v[q] = c10.v[q] = c11.v[q] = 0ull;
+      // moments of the upstream gradient over the run, and d(correlation)/d(sample position) of the run's group pair
+      float m0 = 0.0f, m1 = 0.0f, m2 = 0.0f, m3 = 0.0f, P = 0.0f, Q = 0.0f, S = 0.0f;
+      auto flush = [&]() {
+        const float k01 = m1 - m3, k10 = m2 - m3, k00 = (m0 - m1) - k10;
+        float* g00 = sg_lane + (size_t)cur * C;
+#pragma unroll
+        for (int q = 0; q < SUB / 4; ++q) {
+          const float4 rv = *reinterpret_cast<const float4*>(refp + gi_run * SUB + 4 * q);
+          const float r4[4] = {rv.x, rv.y, rv.z, rv.w};
+          float e00[4], e01[4], e10[4], e11[4], o[4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            pk_split(c00.v[2 * q + h], e00[2 * h], e00[2 * h + 1]);
+            pk_split(c01.v[2 * q + h], e01[2 * h], e01[2 * h + 1]);
+            pk_split(c10.v[2 * q + h], e10[2 * h], e10[2 * h + 1]);
+            pk_split(c11.v[2 * q + h], e11[2 * h], e11[2 * h + 1]);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k)   // :490; lanes of a pixel may share the reference group
+            atomicAdd(rgp + gi_run * SUB + 4 * q + k, fmaf(k00, e00[k], fmaf(k01, e01[k], fmaf(k10, e10[k], m3 * e11[k]))));
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = k00 * r4[k];   // :491-495
+          red_add<float, 4>(g00 + 4 * q, o);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = k01 * r4[k];
+          red_add<float, 4>(g00 + C + 4 * q, o);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = k10 * r4[k];
+          red_add<float, 4>(g00 + row + 4 * q, o);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = m3 * r4[k];
+          red_add<float, 4>(g00 + row + C + 4 * q, o);
+        }
+      };
+#pragma unroll 1
+      for (int j = 0; j < PB; ++j) {
+        const int t = tex[j * PX + g];
+        if (t >= 0 && t != cur) {
+          if (gi_run >= 0) flush();
+          gi_run = -1;
+          cur = t;
+          const T* p = src_lane + (size_t)t * C;
+          c00.load(p);
+          c01.load(p + C);
+          c10.load(p + row);
+          c11.load(p + row + C);
+        }
+        const ulonglong2 wA = *reinterpret_cast<const ulonglong2*>(wgt + 2 * (j * PX + g));
+        const ulonglong2 wB = *reinterpret_cast<const ulonglong2*>(wgt + 2 * (j * PX + g) + 1);
+        pk2 val[G / 2];
+        v3_dots<T, SUB, G>(c00, c01, c10, c11, wA, wB, ref, ones, val);
+        // this view's winner, found as the forward pass does (:470-489)
+        float v[G], best = Lim<float>::min_pos();
+#pragma unroll
+        for (int p = 0; p < G / 2; ++p) {
+          pk_split(val[p], v[2 * p], v[2 * p + 1]);
+          best = fmaxf(best, fmaxf(v[2 * p], v[2 * p + 1]));
+        }
+        float m = best;
+#pragma unroll
+        for (int o = G >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const unsigned won = (__ballot_sync(0xffffffffu, best == m) >> (g * G)) & ((1u << G) - 1u);
+        // a view without a winner (no dot product above the start value) contributes nothing
+        if (t >= 0 && m > Lim<float>::min_pos() && li == __ffs(won) - 1) {
+          int gi = 0;
+#pragma unroll
+          for (int i = G - 1; i >= 0; --i)
+            if (v[i] == m) gi = i;
+          if (gi != gi_run) {
+            if (gi_run >= 0) flush();
+            gi_run = gi;
+            m0 = m1 = m2 = m3 = 0.0f;
+            P = Q = S = 0.0f;
+#pragma unroll
+            for (int q = 0; q < SUB / 2; ++q) {
+              float x00, y00, x01, y01, x10, y10, x11, y11;
+              pk_split(c00.v[q], x00, y00);
+              pk_split(c01.v[q], x01, y01);
+              pk_split(c10.v[q], x10, y10);
+              pk_split(c11.v[q], x11, y11);
+              const float ra = refp[gi * SUB + 2 * q], rb = refp[gi * SUB + 2 * q + 1];
+              P = fmaf(ra, (x11 - x10) - (x01 - x00), fmaf(rb, (y11 - y10) - (y01 - y00), P));   // :498
+              Q = fmaf(ra, x10 - x00, fmaf(rb, y10 - y00, Q));
+              S = fmaf(ra, x01 - x00, fmaf(rb, y01 - y00, S));
+            }
+          }
+          const float4 x = aux[2 * (j * PX + g)];
+          const float2 y = *reinterpret_cast<const float2*>(aux + 2 * (j * PX + g) + 1);
+          const float cd = x.z * x.x;
+          m0 += x.z;
+          m1 += cd;
+          m2 = fmaf(x.z, x.y, m2);
+          m3 = fmaf(cd, x.y, m3);
+          dsum = fmaf(y.x, fmaf(x.x, P, Q), fmaf(y.y, fmaf(x.y, P, S), dsum));   // :502
+        }
+      }
+      if (gi_run >= 0) flush();
+      __syncwarp();
+    }
+  }
+  __syncwarp();
+  if (pvalid)
+    for (int c = li; c < C; c += G) {
+      const float v = rgp[c];
+      if (v != 0.0f) atomicAdd(static_cast<float*>(a.ref_grad) + pix * C + c, v);
+    }
+#pragma unroll
+  for (int o = G >> 1; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+  if (pvalid && li == 0) atomicAdd(static_cast<float*>(a.depth_grad) + pix, dsum);   // :505
+}
+
+template <typename T, bool BWD, int SUB, int G>
+int launch_mean(const CvArgs& a0, cudaStream_t st) {
+  typedef V3Cfg<G> Cf;
+  CvArgs a = a0;
+  a.chunk = (a.chunk + Cf::PB - 1) / Cf::PB * Cf::PB;   // whole blocks of planes
+  a.nchunks = (a.d_end - a.d_begin + a.chunk - 1) / a.chunk;
+  const size_t spw = (v3_mean_smem<G>(a.N, SUB * G, BWD) + 15) & ~(size_t)15;
+  if (spw * 4 > 200 * 1024) return -4;
+  const long long blocks = ((long long)a.npb * a.nchunks + 3) / 4;
+  if (blocks > 0x7fffffffLL) return -2;   // CHOP_ERR_SHAPE
+  auto k = BWD ? cv3_bwd_mean<T, SUB, G> : cv3_fwd_mean<T, SUB, G>;
+  if (int e = grant_smem(k, spw * 4)) return e;
+  k<<<(unsigned)blocks, 128, spw * 4, st>>>(a, (int)spw);
+  return (int)cudaGetLastError();
+}
+
 template <typename T, typename R, bool BWD, bool RMIN, int SUBT>
 int launch_sub(const CvArgs& a, cudaStream_t st) {
   const int LG = 1 << a.lg_log2, G = 32 / LG;
@@ -429,6 +830,15 @@ template <typename T, typename R, bool BWD, bool RMIN>
 int launch(const CvArgs& a, cudaStream_t st) {
   if constexpr (sizeof(R) == 4) {
     const int sub = a.C / a.G;
+    if constexpr (!RMIN) {   // the group counts whose reference pixel fits the registers; many views do not fit the records
+      int r = -4;
+      if (sub == 4 && a.G == 2) r = launch_mean<T, BWD, 4, 2>(a, st);
+      if (sub == 4 && a.G == 4) r = launch_mean<T, BWD, 4, 4>(a, st);
+      if (sub == 4 && a.G == 8) r = launch_mean<T, BWD, 4, 8>(a, st);
+      if (sub == 8 && a.G == 2) r = launch_mean<T, BWD, 8, 2>(a, st);
+      if (sub == 8 && a.G == 4) r = launch_mean<T, BWD, 8, 4>(a, st);
+      if (r != -4) return r;
+    }
     if (sub == 4) return launch_sub<T, R, BWD, RMIN, 4>(a, st);
     if (sub == 8) return launch_sub<T, R, BWD, RMIN, 8>(a, st);
   }
