@@ -1,5 +1,6 @@
 // bfloat16 features with float32 arithmetic and outputs: channel slices of 1 or 8 per lane in the
 // generic kernels, 4 per lane in the compile-time-C CostVolume MEAN kernels.
+#include "cv2_wide.cuh"
 #include "cv_launch.cuh"
 #include "cv_entry.h"
 
@@ -23,6 +24,10 @@ int cv_fwd_bf16(const CvArgs& a, const CvPlan& p, cudaStream_t st) {
       case 64: return fwd_tuned_go<__nv_bfloat16, 64, 4, true>(a, st);
       default: break;
     }
+  }
+  if (p.use_tuned && p.use_packed && p.kind == 2 && p.mode == 0 && p.cpl == 4) {
+    const int r = v2_wide_fwd(a, st);   // eight channels per lane where that is the better kernel
+    if (r != -4) return r;
   }
   if (p.use_tuned && p.kind == 2 && p.mode != 1 && p.cpl == 4) {
     const int r = tuned2_dispatch<__nv_bfloat16>(false, p.mode == 2, a, st);
