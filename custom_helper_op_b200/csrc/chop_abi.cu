@@ -87,6 +87,7 @@ int validate(const chop_cv_desc* d, CvArgs* a, Typed* ty) {
   a->d_begin = (int)d->d_begin;
   a->d_end = (int)d_end;
   a->half_centor = d->half_centor ? 1 : 0;
+  a->lim = chop::proj_lim(a->half_centor, a->Hs, a->Ws);
   a->npix = d->B * d->H * d->W;
   return 0;
 }
@@ -419,6 +420,7 @@ int fa_prepare(const chop_cv_desc* d, CvArgs* a, Typed* ty, int* cpl) {
   a->N = (int)d->N; a->Hs = (int)d->Hs; a->Ws = (int)d->Ws; a->G = 1;
   a->d_begin = (int)d->d_begin; a->d_end = (int)d_end;
   a->half_centor = d->half_centor ? 1 : 0;
+  a->lim = chop::proj_lim(a->half_centor, a->Hs, a->Ws);
   a->npix = d->B * d->H * d->W;
   int c = 1;
   if (d->dtype == CHOP_F64) { if (a->C % 2 == 0) c = 2; }

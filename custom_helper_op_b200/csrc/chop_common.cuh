@@ -167,6 +167,15 @@ __device__ __forceinline__ void red_add(R* p, const R* v) {
   }
 }
 
+// Limits of the single-precision projection (project_rcp), filled by the host.
+struct ProjLim {
+  float half, Hm1, Wm1;   // 0.5 or 0; last row, last column
+  float zmax;             // depths from here on take the plain path
+};
+inline ProjLim proj_lim(int half_centor, int Hs, int Ws) {
+  return {half_centor ? 0.5f : 0.0f, (float)(Hs - 1), (float)(Ws - 1), (Hs | Ws) >> 22 ? 0.0f : 1e18f};
+}
+
 // Arguments shared by the forward and backward cost-volume kernels (device pointers, validated and
 // narrowed on the host).
 struct CvArgs {
@@ -190,6 +199,7 @@ struct CvArgs {
   int nchunks;
   int npb;         // pixel blocks = ceil(B*H*W / pixels per warp)
   long long npix;  // B*H*W
+  ProjLim lim;
 };
 
 }  // namespace chop

@@ -73,7 +73,6 @@ __global__ void __launch_bounds__(128, V2Wide<C, SUB>::BLOCKS) cv2_fwd_wide(cons
     x = xadd(x, 0.5f);
     y = xadd(y, 0.5f);
   }
-  const ProjLim lim = proj_lim(a.half_centor, a.Hs, a.Ws);
   const T* src_lane = static_cast<const T*>(a.src) + li * 8;
   pk2 ref[4];
   {
@@ -120,7 +119,7 @@ __global__ void __launch_bounds__(128, V2Wide<C, SUB>::BLOCKS) cv2_fwd_wide(cons
       for (int p = 0; p < PL; ++p) {
         int fh, fw;
         float gh, gw;
-        const bool seen = project_rcp<false>(cf, depth[p], lim, fh, fw, dh[p], dw[p], gh, gw);
+        const bool seen = project_rcp<false>(cf, depth[p], a, fh, fw, dh[p], dw[p], gh, gw);
         tex[p] = seen ? (fh - FLOOR_BIAS + cf.row0) * a.Ws + (fw - FLOOR_BIAS) : -1;
         used[p] += seen;
         all_seen &= seen;

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) cv_bwd_kernel(const CvArgs a, const BwdCf
           pr.aux = scale;
           const int n = n0 + v;
           if (live && n < a.N)
-            pr.texel = project<R, true>(coef[n * G + g], depth, a.half_centor, a.Hs, Ws, pr.dh, pr.dw, pr.gh, pr.gw);
+            pr.texel = project<R, true>(coef[n * G + g], depth, a, pr.dh, pr.dw, pr.gh, pr.gw);
           proj[v * 32 + lane] = pr;
         }
       }

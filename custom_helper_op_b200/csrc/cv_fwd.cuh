@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256) cv_fwd_kernel(const CvArgs a, const FwdCf
         pr.dh = pr.dw = pr.aux = (R)0;
         if (dv) {
           R gh, gw;
-          pr.texel = project<R, false>(coef[n * G + g], depth, a.half_centor, a.Hs, Ws, pr.dh, pr.dw, gh, gw);
+          pr.texel = project<R, false>(coef[n * G + g], depth, a, pr.dh, pr.dw, gh, gw);
           used += pr.texel >= 0;
         }
         proj[n * 32 + lane] = pr;

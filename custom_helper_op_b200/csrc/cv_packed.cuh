@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(256, CHOP_PK_FWD_BLOCKS) cv_fwd_packed(const C
         float dh = 0.0f, dw = 0.0f;
         if (dv) {
           float gh, gw;
-          t = project<float, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, dh, dw, gh, gw);
+          t = project<float, false>(coef[n * G + g], depth, a, dh, dw, gh, gw);
           used += t >= 0;
         }
         rec[n * 32 + lane] = make_float4(dw, dw, dh, dh);
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(32 * CHOP_PM_FWD_WARPS, CHOP_PM_FWD_BLOCKS) cv
 #pragma unroll
       for (int n = 0; n < NV; ++n) {
         float gh, gw;
-        tt[n] = project<float, false>(cf[n], depth, a.half_centor, a.Hs, a.Ws, dhh[n], dww[n], gh, gw);
+        tt[n] = project<float, false>(cf[n], depth, a, dhh[n], dww[n], gh, gw);
       }
 #pragma unroll
       for (int n = 0; n < NV; ++n) {

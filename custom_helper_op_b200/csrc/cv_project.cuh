@@ -76,19 +76,19 @@ __device__ __forceinline__ void stage_coefs(const CvArgs& a, Coef<R>* coef, int 
 
 // One voxel into one view (cost_volume_kernels_gpu.cu.cc:84-104).  Returns the texel index or -1.
 template <typename R, bool BWD>
-__device__ __forceinline__ int project(const Coef<R>& c, R depth, int half_centor, int Hs, int Ws, R& dh,
-                                       R& dw, R& gh, R& gw) {
+__device__ __forceinline__ int project_div(const Coef<R>& c, R depth, const CvArgs& a, R& dh, R& dw, R& gh,
+                                       R& gw) {
   const R z = xadd(xmul(c.zc, depth), c.t2);
   if (!(z > (R)0)) return -1;
   const R w3 = xadd(xmul(c.wc, depth), c.t0);
   R sw = xdiv(w3, z);
   const R h3 = xadd(xmul(c.hc, depth), c.t1);
   R sh = xdiv(h3, z);
-  if (half_centor) {
+  if (a.half_centor) {
     sw = xsub(sw, (R)0.5);
     sh = xsub(sh, (R)0.5);
   }
-  if (sh > (R)0 && sw > (R)0 && sh < (R)(Hs - 1) && sw < (R)(Ws - 1)) {
+  if (sh > (R)0 && sw > (R)0 && sh < (R)(a.Hs - 1) && sw < (R)(a.Ws - 1)) {
     const int fh = (int)sh;
     const int fw = (int)sw;
     dh = xsub(sh, (R)fh);
@@ -100,7 +100,7 @@ __device__ __forceinline__ int project(const Coef<R>& c, R depth, int half_cento
       gh = (c.hc * z - c.zc * h3) * izz;
       gw = (c.wc * z - c.zc * w3) * izz;
     }
-    return fw + Ws * (fh + c.row0);
+    return fw + a.Ws * (fh + c.row0);
   }
   return -1;
 }
@@ -113,22 +113,17 @@ __device__ __forceinline__ int project(const Coef<R>& c, R depth, int half_cento
 // Functions", 2000, ch. 8; the remainder a - z*q is exact in a fused multiply-add).  Checked against __fdiv_rn on every
 // pair of significands whose quotient lies within 8 units of the hardest distance to a rounding boundary (36 million
 // pairs, exhaustive) and on 7e10 random pairs: no difference.  Outside 1e-12 < z < 1e18 the plain division runs.
-// 24 -> 9 instructions per voxel and view, and two branches (the range checks of the divisions) fewer.  The forward
-// kernels use it; the gradient kernels sit at their register limit and ran slower with it (cv_bwd_tuned<float, 32> 257 ->
-// 272 us at 128x160x192, two views), so they keep project<>.
+// 24 -> 9 instructions per voxel and view, and two branches (the range checks of the divisions) fewer.  cv_bwd_tuned
+// for CostVolume sits at its register limit (with this form ptxas recomputes addresses in its plane loop: 256 -> 270 us at
+// 128x160x192, two views, C = 32), so it alone keeps project_div.
 //
 // Floor: for 0 < s < 2^23, s + 2^23 rounded towards zero holds floor(s) in its low bits; subtracting 2^23 gives it back as
 // a float, exactly.  Larger images take the plain path as well.
 constexpr int FLOOR_BIAS = 0x4b000000;   // what project_rcp adds to the row and column that it returns (the bits of 2^23)
-struct ProjLim {
-  float half, Hm1, Wm1;   // 0.5 or 0; last row, last column
-  float zmax;             // depths from here on take the plain path
-};
-__device__ __forceinline__ ProjLim proj_lim(int half_centor, int Hs, int Ws) {
-  return {half_centor ? 0.5f : 0.0f, (float)(Hs - 1), (float)(Ws - 1), (Hs | Ws) >> 22 ? 0.0f : 1e18f};
-}
+// The limits are kernel arguments (CvArgs::lim): constant-bank operands, where computed ones would each hold a register
+// through the whole plane loop.
 template <bool BWD>
-__device__ __forceinline__ bool project_rcp(const Coef<float>& c, float depth, const ProjLim& l, int& fh, int& fw, float& dh,
+__device__ __forceinline__ bool project_rcp(const Coef<float>& c, float depth, const CvArgs& a, int& fh, int& fw, float& dh,
                                             float& dw, float& gh, float& gw) {
   const float z = xadd(xmul(c.zc, depth), c.t2);
   const float w3 = xadd(xmul(c.wc, depth), c.t0);
@@ -139,20 +134,20 @@ __device__ __forceinline__ bool project_rcp(const Coef<float>& c, float depth, c
   float sw = __fmul_rn(w3, y), sh = __fmul_rn(h3, y);
   sw = __fmaf_rn(__fmaf_rn(-z, sw, w3), y, sw);
   sh = __fmaf_rn(__fmaf_rn(-z, sh, h3), y, sh);
-  sw = xsub(sw, l.half);
-  sh = xsub(sh, l.half);
-  bool seen = (sh > 0.0f) & (sw > 0.0f) & (sh < l.Hm1) & (sw < l.Wm1);
+  sw = xsub(sw, a.lim.half);
+  sh = xsub(sh, a.lim.half);
+  bool seen = (sh > 0.0f) & (sw > 0.0f) & (sh < a.lim.Hm1) & (sw < a.lim.Wm1);
   const float th = __fadd_rz(sh, 8388608.0f), tw = __fadd_rz(sw, 8388608.0f);
   dh = xsub(sh, xsub(th, 8388608.0f));
   dw = xsub(sw, xsub(tw, 8388608.0f));
   fh = __float_as_int(th);   // + FLOOR_BIAS
   fw = __float_as_int(tw);
-  if (!(z > 1e-12f && z < l.zmax)) {
+  if (!(z > 1e-12f && z < a.lim.zmax)) {
     seen = false;
     if (z > 0.0f) {
-      sw = xsub(xdiv(w3, z), l.half);
-      sh = xsub(xdiv(h3, z), l.half);
-      seen = (sh > 0.0f) & (sw > 0.0f) & (sh < l.Hm1) & (sw < l.Wm1);
+      sw = xsub(xdiv(w3, z), a.lim.half);
+      sh = xsub(xdiv(h3, z), a.lim.half);
+      seen = (sh > 0.0f) & (sw > 0.0f) & (sh < a.lim.Hm1) & (sw < a.lim.Wm1);
       if (seen) {
         fh = (int)sh;
         fw = (int)sw;
@@ -172,14 +167,19 @@ __device__ __forceinline__ bool project_rcp(const Coef<float>& c, float depth, c
   return seen;
 }
 
-template <>
-__device__ __forceinline__ int project<float, false>(const Coef<float>& c, float depth, int half_centor, int Hs, int Ws, float& dh,
-                                                     float& dw, float& gh, float& gw) {
-  int fh, fw;
-  const bool seen = project_rcp<false>(c, depth, proj_lim(half_centor, Hs, Ws), fh, fw, dh, dw, gh, gw);
-  if (!seen) dh = dw = 0.0f;
-  return seen ? (fw - FLOOR_BIAS) + Ws * (fh - FLOOR_BIAS + c.row0) : -1;
+// The projection in the form that its type has: project_rcp for float, project_div otherwise.
+template <typename R, bool BWD>
+__device__ __forceinline__ int project(const Coef<R>& c, R depth, const CvArgs& a, R& dh, R& dw, R& gh, R& gw) {
+  if constexpr (sizeof(R) == 4) {
+    int fh, fw;
+    const bool seen = project_rcp<BWD>(c, depth, a, fh, fw, dh, dw, gh, gw);
+    if (!seen) dh = dw = gh = gw = 0.0f;
+    return seen ? (fw - FLOOR_BIAS) + a.Ws * (fh - FLOOR_BIAS + c.row0) : -1;
+  } else {
+    return project_div<R, BWD>(c, depth, a, dh, dw, gh, gw);
+  }
 }
+
 // Bilinear weights, reference naming in brackets (:105-108): w00 [coef_cc] for texel (fh,fw), w01
 // [coef_cf] for (fh,fw+1), w11 [coef_ff] for (fh+1,fw+1), w10 [coef_fc] for (fh+1,fw).
 // The same weights with 4 operations instead of 6 (differs from the reference in the last bit; used

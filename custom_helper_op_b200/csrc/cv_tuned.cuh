@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256, CHOP_FWD_MIN_BLOCKS) cv_fwd_tuned(const C
         r.dh = r.dw = r.aux = 0.0f;
         if (dv) {
           float gh, gw;
-          r.texel = project<float, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, gh, gw);
+          r.texel = project<float, false>(coef[n * G + g], depth, a, r.dh, r.dw, gh, gw);
           used += r.texel >= 0;
         }
         proj[n * 32 + lane] = r;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256, 2) cv_fwd_min_tuned(const CvArgs a, const
         r.dh = r.dw = r.aux = 0.0f;
         if (dv) {
           float gh, gw;
-          r.texel = project<float, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, gh, gw);
+          r.texel = project<float, false>(coef[n * G + g], depth, a, r.dh, r.dw, gh, gw);
         }
         proj[n * 32 + lane] = r;
       }
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(256, 2) cv_agg_min_fwd_tuned(const CvArgs a, c
         r.dh = r.dw = r.aux = 0.0f;
         if (dv) {
           float gh, gw;
-          r.texel = project<float, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, gh, gw);
+          r.texel = project<float, false>(coef[n * G + g], depth, a, r.dh, r.dw, gh, gw);
         }
         proj[n * 32 + lane] = r;
       }
@@ -619,7 +619,8 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
         q.gh = q.gw = 0.0f;
         // aggregate MIN: only the winning view of the voxel is differentiated
         if (live && (!(RMIN && AGG) || m0 == n))
-          r.texel = project<float, true>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, q.gh, q.gw);
+          r.texel = AGG ? project<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw)
+                        : project_div<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw);
         recA[n * 32 + lane] = r;
         recG[n * 32 + lane] = q;
       }
@@ -795,7 +796,7 @@ __global__ void __launch_bounds__(256, 3) cv2_fwd_tuned(const CvArgs a, const in
         r.dh = r.dw = r.aux = 0.0f;
         if (dv) {
           float gh, gw;
-          r.texel = project<float, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, gh, gw);
+          r.texel = project<float, false>(coef[n * G + g], depth, a, r.dh, r.dw, gh, gw);
           used += r.texel >= 0;
         }
         proj[n * 32 + lane] = r;
@@ -934,7 +935,7 @@ __global__ void __launch_bounds__(256, 2) cv2_fwd_min_tuned(const CvArgs a, cons
         r.dh = r.dw = r.aux = 0.0f;
         if (dv) {
           float gh, gw;
-          r.texel = project<float, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, gh, gw);
+          r.texel = project<float, false>(coef[n * G + g], depth, a, r.dh, r.dw, gh, gw);
         }
         proj[n * 32 + lane] = r;
       }
@@ -1124,7 +1125,7 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
         r.dh = r.dw = 0.0f;
         r.aux = scale;
         q.gh = q.gw = 0.0f;
-        if (live) r.texel = project<float, true>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, q.gh, q.gw);
+        if (live) r.texel = project<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw);
         recA[n * 32 + lane] = r;
         recG[n * 32 + lane] = q;
       }

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256) cv3_fwd_kernel(const CvArgs a, const int 
         r.texel = -1;
         r.dh = r.dw = r.aux = (R)0;
         R gh, gw;
-        if (dv) r.texel = project<R, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, gh, gw);
+        if (dv) r.texel = project<R, false>(coef[n * G + g], depth, a, r.dh, r.dw, gh, gw);
         rec[n * 32 + lane] = r;
       }
     }
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256) cv3_bwd_kernel(const CvArgs a, const int 
         r.cg = cg;
         r.gi = m1; r.gs = m2;
         if (live && (!RMIN || n == m0))
-          r.texel = project<R, true>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, r.gh, r.gw);
+          r.texel = project<R, true>(coef[n * G + g], depth, a, r.dh, r.dw, r.gh, r.gw);
         rec[n * 32 + lane] = r;
       }
     }
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(128, 5) cv3_fwd_mean(const CvArgs a, const int
 #pragma unroll
       for (int p = 0; p < PL; ++p) {
         float dh, dw, gh, gw, w00, w01, w11, w10;
-        const int t = project<float, false>(cf, depth[p], a.half_centor, a.Hs, a.Ws, dh, dw, gh, gw);
+        const int t = project<float, false>(cf, depth[p], a, dh, dw, gh, gw);
         bilinear_weights(dh, dw, w00, w01, w11, w10);
         used[p] += t >= 0;
         const int slot = (p * G + li) * PX + g;
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(128, 4) cv3_bwd_mean(const CvArgs a, const int
       for (int p = 0; p < PL; ++p) {
         float dh = 0.0f, dw = 0.0f, gh = 0.0f, gw = 0.0f, w00, w01, w11, w10;
         int t = -1;
-        if (m_cur[p] > 0) t = project<float, true>(cf, depth[p], a.half_centor, a.Hs, a.Ws, dh, dw, gh, gw);
+        if (m_cur[p] > 0) t = project<float, true>(cf, depth[p], a, dh, dw, gh, gw);
         if (t < 0) dh = dw = gh = gw = 0.0f;
         bilinear_weights(dh, dw, w00, w01, w11, w10);
         const int slot = (p * G + li) * PX + g;

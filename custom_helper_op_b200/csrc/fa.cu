@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) fa_fwd_kernel(const CvArgs a, const int w
         r.dh = r.dw = r.aux = (R)0;
         R gh, gw;
         if (dv) {
-          r.texel = project<R, false>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, gh, gw);
+          r.texel = project<R, false>(coef[n * G + g], depth, a, r.dh, r.dw, gh, gw);
           __stcs(a.mask + (pix * D + d) * N + n, r.texel >= 0 ? 1 : 0);   // :108 / :118
         }
         rec[n * 32 + lane] = r;
@@ -150,7 +150,7 @@ __device__ __forceinline__ void fa_flush(R* gp, size_t row, int C, R (&m)[4][CPL
 // compile-time constants; the plane loops unroll and the index arithmetic folds (a third of the generic kernel's
 // instructions were integer address and loop work).  LGC = 0 keeps them run-time values.
 template <typename T, typename R, int CPL, bool STAGED, int LGC = 0>
-__global__ void __launch_bounds__(256) fa_bwd_kernel(const CvArgs a, const int warps, const size_t smem_per_warp) {
+__global__ void __launch_bounds__(256, 3) fa_bwd_kernel(const CvArgs a, const int warps, const size_t smem_per_warp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int LG = LGC > 0 ? LGC : 1 << a.lg_log2, G = 32 / LG;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256) fa_bwd_kernel(const CvArgs a, const int w
         r.dh = r.dw = r.aux = (R)0;
         q.gh = q.gw = (R)0;
         if (dv && __ldg(a.mask + (pix * D + d) * N + n) != 0)   // :262-264
-          r.texel = project<R, true>(coef[n * G + g], depth, a.half_centor, a.Hs, a.Ws, r.dh, r.dw, q.gh, q.gw);
+          r.texel = project<R, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw);
         rec[n * 32 + lane] = r;
         recg[n * 32 + lane] = q;
       }
