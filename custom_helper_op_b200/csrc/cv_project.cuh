@@ -113,9 +113,7 @@ __device__ __forceinline__ int project_div(const Coef<R>& c, R depth, const CvAr
 // Functions", 2000, ch. 8; the remainder a - z*q is exact in a fused multiply-add).  Checked against __fdiv_rn on every
 // pair of significands whose quotient lies within 8 units of the hardest distance to a rounding boundary (36 million
 // pairs, exhaustive) and on 7e10 random pairs: no difference.  Outside 1e-12 < z < 1e18 the plain division runs.
-// 24 -> 9 instructions per voxel and view, and two branches (the range checks of the divisions) fewer.  cv_bwd_tuned
-// for CostVolume sits at its register limit (with this form ptxas recomputes addresses in its plane loop: 256 -> 270 us at
-// 128x160x192, two views, C = 32), so it alone keeps project_div.
+// 24 -> 9 instructions per voxel and view, and two branches (the range checks of the divisions) fewer.
 //
 // Floor: for 0 < s < 2^23, s + 2^23 rounded towards zero holds floor(s) in its low bits; subtracting 2^23 gives it back as
 // a float, exactly.  Larger images take the plain path as well.

@@ -610,6 +610,7 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
             scale = 2.0f * ag0 / (float)(m0 * C);
         }
       }
+#pragma unroll 2   // two views at a time: 250 us at c1, 257 one at a time (and 260 with four, which costs registers)
       for (int n = 0; n < N; ++n) {
         ProjF<float> r;
         RecG q;
@@ -619,8 +620,7 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
         q.gh = q.gw = 0.0f;
         // aggregate MIN: only the winning view of the voxel is differentiated
         if (live && (!(RMIN && AGG) || m0 == n))
-          r.texel = AGG ? project<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw)
-                        : project_div<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw);
+          r.texel = project<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw);
         recA[n * 32 + lane] = r;
         recG[n * 32 + lane] = q;
       }
