@@ -89,13 +89,12 @@ struct TileClass {
   int begin, end;      // its tiles
   unsigned real;       // bit fr*3 + fc: a 3x3 filter has this column here (dilation 1)
 };
-template <int TILE>
-__device__ __forceinline__ void class_open(const ScArgs& a, TileClass& c) {
+__device__ __forceinline__ void class_open(const ScArgs& a, TileClass& c, int tile) {
   c.pr = c.k / a.sc;
   c.pc = c.k - c.pr * a.sc;
   c.hc = (a.H - c.pr + a.sr - 1) / a.sr;
   c.wc = (a.W - c.pc + a.sc - 1) / a.sc;
-  c.end = c.begin + (int)(((unsigned)a.B * c.hc * c.wc * a.D + (unsigned)(TILE - 1)) / (unsigned)TILE);   // 31-bit voxel counts
+  c.end = c.begin + (int)(((unsigned)a.B * c.hc * c.wc * a.D + (unsigned)(tile - 1)) / (unsigned)tile);   // 31-bit voxel counts
   c.real = 0;
   for (int f = 0; f < 9; ++f)   // the tap's row and column must be multiples of the strides
     if ((c.pr - 1 + f / 3 + a.sr) % a.sr == 0 && (c.pc - 1 + f % 3 + a.sc) % a.sc == 0) c.real |= 1u << f;

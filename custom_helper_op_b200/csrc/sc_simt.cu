@@ -385,7 +385,7 @@ int sc_wgrad_simt_launch_parts(int dtype, const ScArgs& a, int nparts, cudaStrea
 }
 
 int sc_wgrad_parts(long long nvox_out) {
-  long long p = (nvox_out + 511) / 512;  // at least 512 voxels per CTA
+  long long p = (nvox_out + 127) / 128;  // a tensor-core tile of voxels per CTA at least: 512 left most SMs idle below 75 000 voxels
   if (p > 148 * 4) p = 148 * 4;
   if (p < 1) p = 1;
   return (int)p;

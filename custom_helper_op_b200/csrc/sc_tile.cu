@@ -38,6 +38,7 @@ template <> struct TileIo<__nv_bfloat16> {
 // FORM 0: forward - voxels of the output grid gather the input grid (sc_tap); weights w[t][ci][co].
 // FORM 1: gather form - voxels of the fine grid gather the coarse grid (sc_tap_t); the gathered tensor has Cout
 //         channels, the produced one Cin, weights flipped: w'[t][co][ci] = filter[taps-1-t][ci][co].
+// FORM 2: the gather form by residue class, for row or column strides.
 //
 // The gathered channels are split over lanes: LK = KCH/4 neighbouring lanes share a voxel, each holding four of its
 // channels, and a thread accumulates RT voxels x all NCH produced channels over its quarter of the reduction; the lanes'
@@ -46,76 +47,137 @@ template <> struct TileIo<__nv_bfloat16> {
 // 16-byte weight load (LK addresses per warp, padded to different banks) feeds 4*RT multiply-adds, issued two at a time
 // (fma.rn.f32x2).  Which voxel a tap reads is worked out once per CTA and tile into a shared table, and the next tap's
 // values are requested before the present tap's arithmetic.
+// A CTA has as many warps as it takes for 16 of them to be resident beside the staged weights (32 -> 32 channels: 114 KB,
+// one CTA of 16 warps; with four warps a CTA the SM held four: 1290 us against 740 at 180x230x9, 3x3x3, float32).
+// Strided gather form: tiles of one residue class, and only the filter columns that exist there are looked up and
+// multiplied (2.25 of 9 on average at strides 2: 136 -> 81 us for 16 -> 16 channels), unless the padding value is not zero.
 // Bound: the FMA pipe.  189x251x7, 16 -> 16 channels, 3x3x3, float32: 142 us forward (235
 // before), 147 us image gradient (287); the FMA pipe is 55 % busy, the rest is splatting the gathered values and latency.
-template <int KCH, int NCH>
+constexpr int tile_warps(int kch, int nch) { return kch * nch <= 256 ? 4 : kch * nch <= 512 ? 8 : 16; }
+template <int KCH, int NCH, int NW>
 struct TileCfg {
   static constexpr int LK = KCH / 4;                  // lanes per voxel
   static constexpr int RPW = 32 / LK;                 // voxels per warp-wide load
   static constexpr int RT = NCH <= 16 ? 4 : 2;        // loads (voxels per thread) in flight: 4*RT*NCH/4 accumulators
-  static constexpr int VPC = 4 * RPW * RT;            // voxels per CTA (four warps)
+  static constexpr int VPC = NW * RPW * RT;           // voxels per CTA
   static constexpr int WROW = 4 * NCH + 4;            // floats of a lane's four weight rows, padded by 16 bytes
+  static size_t smem(int taps, int ncols) {
+    return (size_t)taps * LK * WROW * 4 + (size_t)VPC * (sizeof(int4) + 4 + (size_t)taps * 4) + (size_t)(ncols + 1) * 4;
+  }
 };
 
-// Source voxels of the taps of filter column (fr, fc) for voxel (b, r, c, dz): tab[fz*step] = voxel index or -1.
+// Source voxels of the taps of filter column (fr, fc) for voxel (b, r, c, dz): tab[fz*step] = voxel index or -1
+// (sc_tap / sc_tap_t with the column's share of the work done once and no division where the stride is 1).
 template <int FORM>
 __device__ __forceinline__ void tile_column(const ScArgs& a, const int4 vx, int fr, int fc, int* tab, int step) {
-  const bool s1 = a.sr == 1 && a.sc == 1 && a.sd == 1;
-  if (!s1) {   // strides: the plain index functions
-    for (int fz = 0; fz < a.fd; ++fz)
-      tab[fz * step] = (int)(FORM == 0 ? sc_tap(a, vx.x, vx.y, vx.z, vx.w, fr, fc, fz) : sc_tap_t(a, vx.x, vx.y, vx.z, vx.w, fr, fc, fz));
+  if (a.sr == 1 && a.sc == 1 && a.sd == 1) {
+    const int pr = FORM == 0 ? a.pr : (a.fh - 1) * a.dr - a.pr, pc = FORM == 0 ? a.pc : (a.fw - 1) * a.dc - a.pc;
+    const int pd = FORM == 0 ? a.pd : (a.fd - 1) * a.dd - a.pd;
+    const int orow = vx.y - pr + fr * a.dr, ocol = vx.z - pc + fc * a.dc;
+    const bool in = !oob(orow, a.H) && !oob(ocol, a.W);
+    const int pix = in ? (vx.x * a.H + orow) * a.W + ocol : 0;
+    const int d = vx.w + __ldg(a.base_plane + (vx.x * a.H + vx.y) * a.W + vx.z) - __ldg(a.base_plane + pix) - pd;
+    for (int fz = 0; fz < a.fd; ++fz) {
+      const int ind = d + fz * a.dd;
+      tab[fz * step] = in && !oob(ind, a.D) ? pix * a.D + ind : -1;
+    }
     return;
   }
-  const int pr = FORM == 0 ? a.pr : (a.fh - 1) * a.dr - a.pr, pc = FORM == 0 ? a.pc : (a.fw - 1) * a.dc - a.pc;
-  const int pd = FORM == 0 ? a.pd : (a.fd - 1) * a.dd - a.pd;
-  const int orow = vx.y - pr + fr * a.dr, ocol = vx.z - pc + fc * a.dc;
-  const bool in = !oob(orow, a.H) && !oob(ocol, a.W);
-  const int pix = in ? (vx.x * a.H + orow) * a.W + ocol : 0;
-  const int d = vx.w + __ldg(a.base_plane + (vx.x * a.H + vx.y) * a.W + vx.z) - __ldg(a.base_plane + pix) - pd;
-  for (int fz = 0; fz < a.fd; ++fz) {
-    const int ind = d + fz * a.dd;
-    tab[fz * step] = in && !oob(ind, a.D) ? pix * a.D + ind : -1;
+  if (FORM == 0) {
+    const int row = vx.y * a.sr, col = vx.z * a.sc;
+    const int orow = row - a.pr + fr * a.dr, ocol = col - a.pc + fc * a.dc;
+    const bool in = !oob(orow, a.H) && !oob(ocol, a.W);
+    const int pix = in ? (vx.x * a.H + orow) * a.W + ocol : 0;
+    const int bp = __ldg(a.base_plane + (vx.x * a.H + row) * a.W + col);
+    const int depth = a.sd == 1 ? vx.w + bp : (vx.w + (bp + a.sd - 1) / a.sd) * a.sd;
+    const int d = depth - a.pd - __ldg(a.base_plane + pix);
+    for (int fz = 0; fz < a.fd; ++fz) {
+      const int ind = d + fz * a.dd;
+      tab[fz * step] = in && !oob(ind, a.D) ? pix * a.D + ind : -1;
+    }
+    return;
+  }
+  const int orow = vx.y - ((a.fh - 1) * a.dr - a.pr) + fr * a.dr, ocol = vx.z - ((a.fw - 1) * a.dc - a.pc) + fc * a.dc;
+  bool in = !oob(orow, a.H) && !oob(ocol, a.W);
+  int crow = orow, ccol = ocol;
+  if (a.sr > 1) { crow = orow / a.sr; in &= crow * a.sr == orow; }
+  if (a.sc > 1) { ccol = ocol / a.sc; in &= ccol * a.sc == ocol; }
+  const int cpix = in ? ((vx.x * a.oH + crow) * a.oW + ccol) * a.oD : 0;
+  const int under = __ldg(a.base_plane + (in ? (vx.x * a.H + orow) * a.W + ocol : 0));
+  const int d = vx.w + __ldg(a.base_plane + (vx.x * a.H + vx.y) * a.W + vx.z) - ((a.fd - 1) * a.dd - a.pd);
+  if (a.sd == 1) {
+    for (int fz = 0; fz < a.fd; ++fz) {
+      const int ind = d - under + fz * a.dd;
+      tab[fz * step] = in && !oob(ind, a.oD) ? cpix + ind : -1;
+    }
+  } else {
+    int q = d / a.sd, rem = d - q * a.sd;   // d = q*sd + rem, 0 <= rem < sd
+    if (rem < 0) { rem += a.sd; --q; }
+    q -= (under + a.sd - 1) / a.sd;
+    for (int fz = 0; fz < a.fd; ++fz) {
+      tab[fz * step] = in && rem == 0 && !oob(q, a.oD) ? cpix + q : -1;
+      rem += a.dd;
+      while (rem >= a.sd) { rem -= a.sd; ++q; }
+    }
   }
 }
 
-template <typename T, int KCH, int NCH, int FORM>
-__global__ void __launch_bounds__(128, 4) sc_tile_kernel(const ScArgs a, const int nvox, const int ntiles) {
+// Moves on to the residue class that holds the tile and lists the filter columns that exist in it (one thread).
+__device__ __noinline__ void next_class(const ScArgs& a, TileClass& cl, int tile, int vpc, bool first, bool padded, int* live) {
+  if (!first && tile < cl.end) return;
+  if (first) {
+    cl.k = 0;
+    cl.begin = 0;
+    class_open(a, cl, vpc);
+  }
+  while (tile >= cl.end) {
+    ++cl.k;
+    cl.begin = cl.end;
+    class_open(a, cl, vpc);
+  }
+  int n = 0;
+  for (int c = 0; c < a.fh * a.fw; ++c) {
+    const int orow = cl.pr - ((a.fh - 1) * a.dr - a.pr) + c / a.fw * a.dr;
+    const int ocol = cl.pc - ((a.fw - 1) * a.dc - a.pc) + c % a.fw * a.dc;
+    if (padded || (orow % a.sr == 0 && ocol % a.sc == 0)) live[1 + n++] = c;
+  }
+  live[0] = n;
+}
+
+template <typename T, int KCH, int NCH, int FORM, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW) sc_tile_kernel(const __grid_constant__ ScArgs a, const int nvox, const int ntiles) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  typedef TileCfg<KCH, NCH> Cf;
-  constexpr int LK = Cf::LK, RPW = Cf::RPW, RT = Cf::RT, VPC = Cf::VPC, WROW = Cf::WROW;
-  const int taps = a.fh * a.fw * a.fd;
+  typedef TileCfg<KCH, NCH, NW> Cf;
+  constexpr int LK = Cf::LK, RPW = Cf::RPW, RT = Cf::RT, WROW = Cf::WROW, VPC = Cf::VPC, NTHR = 32 * NW;
+  const int taps = a.fh * a.fw * a.fd, ncols = a.fh * a.fw;
   float* ws = reinterpret_cast<float*>(smem_raw);                         // [taps][LK][WROW]
   int4* vox = reinterpret_cast<int4*>(ws + (size_t)taps * LK * WROW);      // [VPC] batch (-1: none), row, column, depth
   int* outv = reinterpret_cast<int*>(vox + VPC);                           // [VPC] produced voxel
-  int* tab = outv + VPC;                                                   // [taps][VPC] gathered voxel, -1 padding, -2 none
+  int* tab = outv + VPC;                                                   // [live taps][VPC] gathered voxel, -1 padding, -2 none
+  int* live = tab + (size_t)taps * VPC;                                    // [1 + ncols] number of live filter columns, columns
   const T* flt = static_cast<const T*>(a.filters);
-  for (int e = threadIdx.x; e < taps * KCH * NCH; e += 128) {
-    const int n = e % NCH, k = (e / NCH) % KCH, t = e / (NCH * KCH);
-    ws[((size_t)t * LK + k / 4) * WROW + (k % 4) * NCH + n] =
-        FORM == 0 ? TileIo<T>::ld1(flt + e) : TileIo<T>::ld1(flt + ((size_t)(taps - 1 - t) * NCH + n) * KCH + k);
+  for (int e = threadIdx.x; e < taps * KCH * NCH; e += NTHR) {             // filter order: consecutive reads
+    const int n = FORM == 0 ? e % NCH : (e / KCH) % NCH, k = FORM == 0 ? (e / NCH) % KCH : e % KCH;
+    const int t = FORM == 0 ? e / (NCH * KCH) : taps - 1 - e / (NCH * KCH);
+    ws[((size_t)t * LK + k / 4) * WROW + (k % 4) * NCH + n] = TileIo<T>::ld1(flt + e);
   }
   const T* src = static_cast<const T*>(FORM == 0 ? a.images : a.out_grad);
   T* dst = static_cast<T*>(FORM == 0 ? a.output : a.images_grad);
   const float pad = a.pad_zero ? 0.f : TileIo<T>::ld1(static_cast<const T*>(a.default_value));
   const float4 pad4 = make_float4(pad, pad, pad, pad);
-  const bool classes = FORM == 1 && (a.sr > 1 || a.sc > 1);
-  TileClass cl;
-  cl.k = 0;
-  cl.begin = 0;
-  if (classes) class_open<VPC>(a, cl);
+  constexpr bool classes = FORM == 2;
+  __shared__ TileClass cl;   // the present class (strided gather form)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q = lane % LK, row0 = warp * RPW * RT + lane / LK;   // this thread's voxels: row0 + i*RPW
   const T* src_lane = src + q * 4;
 
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    if (classes)
-      while (tile >= cl.end) {
-        ++cl.k;
-        cl.begin = cl.end;
-        class_open<VPC>(a, cl);
-      }
     __syncthreads();   // the previous tile's tables have been read
-    for (int e = threadIdx.x; e < VPC; e += 128) {
+    if (classes) {
+      if (threadIdx.x == 0) next_class(a, cl, tile, VPC, tile == blockIdx.x, pad != 0.f, live);
+      __syncthreads();
+    }
+    for (int e = threadIdx.x; e < VPC; e += NTHR) {
       int4 x = make_int4(-1, 0, 0, 0);
       int o = -1;
       if (classes) {   // voxels of one (row, column) residue class: whole taps of a tile are empty and skipped
@@ -142,11 +204,12 @@ __global__ void __launch_bounds__(128, 4) sc_tile_kernel(const ScArgs a, const i
       outv[e] = o;
     }
     __syncthreads();
-    const int ncols = a.fh * a.fw;
-    for (int e = threadIdx.x; e < VPC * ncols; e += 128) {
-      const int col = e / VPC, v = e % VPC;
+    const int nlive = classes ? live[0] : ncols;
+    for (int e = threadIdx.x; e < VPC * nlive; e += NTHR) {
+      const int i = e / VPC, v = e % VPC;
+      const int col = classes ? live[1 + i] : i;
       const int4 x = vox[v];
-      int* t = tab + col * a.fd * VPC + v;
+      int* t = tab + i * a.fd * VPC + v;
       if (x.x < 0) {
         for (int fz = 0; fz < a.fd; ++fz) t[fz * VPC] = -2;
       } else {
@@ -154,6 +217,7 @@ __global__ void __launch_bounds__(128, 4) sc_tile_kernel(const ScArgs a, const i
       }
     }
     __syncthreads();
+    const int ntaps = classes ? nlive * a.fd : taps;
 
     pk2 acc[RT][NCH / 2];
 #pragma unroll
@@ -172,7 +236,8 @@ __global__ void __launch_bounds__(128, 4) sc_tile_kernel(const ScArgs a, const i
       }
       return __any_sync(0xffffffffu, live);
     };
-    auto multiply = [&](const float4 (&x)[RT], int t) {
+    auto multiply = [&](const float4 (&x)[RT], int i) {
+      const int t = classes ? live[1 + i / a.fd] * a.fd + i % a.fd : i;
       const float* wt = ws + (t * LK + q) * WROW;
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
@@ -194,12 +259,12 @@ __global__ void __launch_bounds__(128, 4) sc_tile_kernel(const ScArgs a, const i
       }
     };
     float4 xa[RT], xb[RT];
-    bool la = request(xa, 0), lb = false;
-    for (int t = 0; t < taps; t += 2) {
-      if (t + 1 < taps) lb = request(xb, t + 1);
+    bool la = ntaps > 0 && request(xa, 0), lb = false;
+    for (int t = 0; t < ntaps; t += 2) {
+      if (t + 1 < ntaps) lb = request(xb, t + 1);
       if (la) multiply(xa, t);
-      if (t + 1 >= taps) break;
-      if (t + 2 < taps) la = request(xa, t + 2);
+      if (t + 1 >= ntaps) break;
+      if (t + 2 < ntaps) la = request(xa, t + 2);
       if (lb) multiply(xb, t + 1);
     }
 
@@ -232,54 +297,98 @@ __global__ void __launch_bounds__(128, 4) sc_tile_kernel(const ScArgs a, const i
   }
 }
 
-// Filter gradient, float32: dW[tap][k][n] = sum over voxels of gathered(voxel, tap)[k] * upstream(voxel)[n].
-// A CTA owns a contiguous slice of the voxels and the whole [taps*KCH][NCH] result: thread q holds four consecutive
-// gathered channels of one tap times NT upstream channels in registers (4*NT accumulators in pairs), so a voxel costs one
-// 16-byte load of the gathered values, NT/4 warp-uniform 16-byte loads of the upstream row from shared memory and
-// 2*NT paired FMAs.  Tap indices and upstream rows of WT voxels are staged per step.  Per-CTA slabs are summed in a fixed
-// order by sc_slab_reduce (deterministic).  TR = transposed convolution: the voxels are those of the fine grid,
-// the gathered tensor is the coarse input (Cout channels), the upstream one has Cin channels, and the reduction
-// writes element [tap][co][ci] to filter_grad[taps-1-tap][ci][co].
-constexpr int WT = 32;   // voxels per staging step
+// Filter gradient: dW[tap][k][n] = sum over output voxels of gathered(voxel, tap)[k] * upstream(voxel)[n].
+// A CTA owns a contiguous slice of the voxels.  A thread holds four consecutive gathered channels of one tap times NT
+// upstream channels in registers (4*NT accumulators in pairs), so a voxel costs it one 16-byte load of the gathered values,
+// NT/4 warp-uniform 16-byte loads of the upstream row from shared memory and 2*NT paired FMAs.  Where taps*KCH/4 such
+// threads do not fill 256, that many groups of them share the CTA and take every other (fourth) four voxels; larger filters
+// are swept in rows of 256 threads.  Tap indices and upstream rows of WT voxels are staged per step.  The groups' sums are
+// added in shared memory in a fixed order and the CTA's slab is written with consecutive stores; sc_slab_reduce sums the
+// slabs in a fixed order (deterministic).
+//
+// TS = filter gradient of the TRANSPOSED convolution with the roles swapped, as in sc_umma_wgrad_kernel: the voxels are those of
+// the coarse grid, a.images is the fine upstream gradient (padding nothing) and a.out_grad the op's coarse input; what
+// a non-zero default_value adds at the empty taps is default * (sum of the fine gradient - the part under a coarse voxel).
+// Bound: FMA issue, and the gathers' latency at 16 warps an SM.  float32, 3x3x3: 189x251x7 16 -> 16 215 -> 189 us; 180x230x9
+// 8 -> 8 134 -> 86; strides (2,2,2) 16 -> 16 114 -> 37 (slabs of 128 voxels, not 512, keep every SM busy there); transposed
+// at strides (2,2,2) 286 -> 33 for 16 -> 16, 868 -> 106 for 32 -> 32.
+constexpr int WT = 64;   // voxels per staging step
 
-template <typename T, int KCH, int NCH, bool TR>
-__global__ void __launch_bounds__(256) sc_wgrad_tile_kernel(const ScArgs a, const int vox_per_cta) {
+template <int KCH, int NCH>
+struct WgradCfg {
+  static constexpr int NT = NCH < 16 ? NCH : 16;     // upstream channels per sweep
+  static constexpr int OCC = NT < 16 ? 3 : 2;        // resident CTAs per SM (registers)
+  static int kthreads(int taps) {                    // threads of a group, a power of two
+    int n = 64;
+    while (n < taps * KCH / 4 && n < 256) n <<= 1;
+    return n;
+  }
+  static size_t stage_bytes(int taps) { return (size_t)WT * (NCH * 4 + sizeof(int4) + (size_t)taps * 4); }
+  static size_t area_bytes(int taps) {               // staging, reused for a group's sums
+    const size_t a = stage_bytes(taps), b = (size_t)4 * NT * (kthreads(taps) + 1) * 4;
+    return ((a > b ? a : b) + 15) / 16 * 16;
+  }
+};
+
+template <typename T, int KCH, int NCH, bool TS>
+__global__ void __launch_bounds__(256, WgradCfg<KCH, NCH>::OCC)
+sc_wgrad_tile_kernel(const ScArgs a, const int vox_per_cta, const int kthreads, const int area) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int NT = NCH < 16 ? NCH : 16;                   // upstream channels per sweep
+  constexpr int NT = WgradCfg<KCH, NCH>::NT;
   const int taps = a.fh * a.fw * a.fd;
-  const int K4 = taps * KCH / 4;                            // threads with work
+  const int K4 = taps * KCH / 4;
   float* gt = reinterpret_cast<float*>(smem_raw);                         // [WT][NCH]
   int4* vox = reinterpret_cast<int4*>(gt + WT * NCH);                     // [WT]: b, row, column, depth of a staged voxel
   int* tapidx = reinterpret_cast<int*>(vox + WT);                         // [taps][WT] gathered voxel or -1
-  float* wsum = reinterpret_cast<float*>(tapidx + (size_t)WT * taps);      // [taps][NCH], dynamic_default only
-  float* red = wsum + (size_t)taps * NCH;                                 // [blockDim]
+  float* sums = reinterpret_cast<float*>(smem_raw);                       // [4*NT][kthreads + 1], after the voxels
+  float4* red4 = reinterpret_cast<float4*>(smem_raw + area);              // [256]
+  float* red = reinterpret_cast<float*>(red4 + 256);                      // [256]
+  float* wsum = red + 256;                                                // [taps][NCH] (dynamic_default) / [KCH] (TS)
   const T* img = static_cast<const T*>(a.images);
   const T* og = static_cast<const T*>(a.out_grad);
-  const bool dyn = !TR && a.dynamic_default;
+  const bool dyn = !TS && a.dynamic_default;
+  const float defv = TileIo<T>::ld1(static_cast<const T*>(a.default_value));
   if (dyn) {
     const T* flt = static_cast<const T*>(a.filters);
-    for (int e = threadIdx.x; e < taps * NCH; e += blockDim.x) {
+    for (int e = threadIdx.x; e < taps * NCH; e += 256) {
       const int n = e % NCH, t = e / NCH;
       float s = 0.f;
       for (int k = 0; k < KCH; ++k) s += TileIo<T>::ld1(flt + ((size_t)t * KCH + k) * NCH + n);
       wsum[e] = s;
     }
   }
-  const float defv = TileIo<T>::ld1(static_cast<const T*>(a.default_value));
-  const float4 pad4 = make_float4(defv, defv, defv, defv);
-  const long long nvox = TR ? a.nvox_in : a.nvox_out;
-  const int d1 = TR ? a.D : a.oD, d2 = TR ? a.W : a.oW, d3 = TR ? a.H : a.oH;
+  if (TS && defv != 0.f) {   // this CTA's share of the channel sums of the fine gradient
+    constexpr int L = KCH / 4, R = 256 / L;
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long long v = (long long)blockIdx.x * R + threadIdx.x / L; v < a.nvox_in; v += (long long)gridDim.x * R) {
+      const float4 x = TileIo<T>::ld4(img + (size_t)v * KCH + threadIdx.x % L * 4);
+      f.x += x.x; f.y += x.y; f.z += x.z; f.w += x.w;
+    }
+    red4[threadIdx.x] = f;
+    __syncthreads();
+    if (threadIdx.x < KCH) {
+      float s = 0.f;
+      for (int r = 0; r < R; ++r) s += reinterpret_cast<const float*>(red4 + r * L)[threadIdx.x];
+      wsum[threadIdx.x] = s;
+    }
+    __syncthreads();
+  }
+  const float padv = TS ? 0.f : defv;
+  const float4 pad4 = make_float4(padv, padv, padv, padv);
   const long long v0 = (long long)blockIdx.x * vox_per_cta;
-  const long long v1 = min(nvox, v0 + vox_per_cta);
-  const int q = threadIdx.x;
-  const bool active = q < K4;
-  const int my_tap = active ? (q * 4) / KCH : 0;
-  const int my_k = active ? (q * 4) % KCH : 0;
+  const long long v1 = min(a.nvox_out, v0 + vox_per_cta);
+  const int group = threadIdx.x / kthreads, ngroups = 256 / kthreads, qt = threadIdx.x % kthreads;
   const size_t slab = (size_t)taps * KCH * NCH + 1;
   float* part = static_cast<float*>(a.workspace) + (size_t)blockIdx.x * slab;
   float dacc = 0.f;
 
-  for (int n0 = 0; n0 < NCH; n0 += NT) {
+  for (int sweep = 0; sweep < (K4 + kthreads - 1) / kthreads * (NCH / NT); ++sweep) {
+    const int q0 = sweep / (NCH / NT) * kthreads, n0 = sweep % (NCH / NT) * NT;
+    const int q = q0 + qt;
+    const bool active = q < K4;
+    const int my_tap = active ? (q * 4) / KCH : 0;
+    const int my_k = active ? (q * 4) % KCH : 0;
+    float4 seen = make_float4(0.f, 0.f, 0.f, 0.f);
     pk2 acc[4][NT / 2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -288,23 +397,22 @@ __global__ void __launch_bounds__(256) sc_wgrad_tile_kernel(const ScArgs a, cons
     for (long long vt = v0; vt < v1; vt += WT) {
       const int tm = (int)min((long long)WT, v1 - vt);
       __syncthreads();
-      // voxel coordinates once per voxel (the 64-bit divisions are the expensive part), then the tap table
       if (threadIdx.x < tm) {
         unsigned v = (unsigned)(vt + threadIdx.x);   // 31-bit voxel counts
-        const int dz = (int)(v % (unsigned)d1); v /= (unsigned)d1;
-        const int cc = (int)(v % (unsigned)d2); v /= (unsigned)d2;
-        vox[threadIdx.x] = make_int4((int)(v / (unsigned)d3), (int)(v % (unsigned)d3), cc, dz);
+        const int dz = (int)(v % (unsigned)a.oD); v /= (unsigned)a.oD;
+        const int cc = (int)(v % (unsigned)a.oW); v /= (unsigned)a.oW;
+        vox[threadIdx.x] = make_int4((int)(v / (unsigned)a.oH), (int)(v % (unsigned)a.oH), cc, dz);
       }
-      for (int e = threadIdx.x; e < tm * NCH; e += blockDim.x) gt[e] = TileIo<T>::ld1(og + vt * NCH + e);
+      for (int e = threadIdx.x; e < tm * NCH; e += 256) gt[e] = TileIo<T>::ld1(og + vt * NCH + e);
       __syncthreads();
-      for (int e = threadIdx.x; e < WT * a.fh * a.fw; e += blockDim.x) {
+      for (int e = threadIdx.x; e < WT * a.fh * a.fw; e += 256) {
         const int col = e / WT, m = e % WT;
-        if (m < tm) tile_column<TR ? 1 : 0>(a, vox[m], col / a.fw, col % a.fw, tapidx + col * a.fd * WT + m, WT);
+        if (m < tm) tile_column<0>(a, vox[m], col / a.fw, col % a.fw, tapidx + col * a.fd * WT + m, WT);
       }
       __syncthreads();
       if (active) {
         // four voxels per step: their gathered loads are issued together, then 4 x 4 x NT FMAs
-        for (int m0 = 0; m0 < tm; m0 += 4) {
+        for (int m0 = group * 4; m0 < tm; m0 += ngroups * 4) {
           int at[4];
           float4 x[4];
           *reinterpret_cast<int4*>(at) = *reinterpret_cast<const int4*>(tapidx + my_tap * WT + m0);
@@ -329,6 +437,7 @@ __global__ void __launch_bounds__(256) sc_wgrad_tile_kernel(const ScArgs a, cons
                 pk_fma_to(acc[i][n4 * 2 + 1], xs[i], g.y);
               }
             }
+            if (TS) { seen.x += x[u].x; seen.y += x[u].y; seen.z += x[u].z; seen.w += x[u].w; }
             if (dyn && at[u] == -1 && my_k == 0) {
               // d(default) collects (sum over input channels of the filter) . out_grad over the padded taps
               // (sparse_conv3d_fast_fixed_param_op_gpu.cu.cc:273-277); one thread per tap does it
@@ -341,73 +450,91 @@ __global__ void __launch_bounds__(256) sc_wgrad_tile_kernel(const ScArgs a, cons
         }
       }
     }
-    if (active) {
+    if (TS) red4[threadIdx.x] = seen;
+    for (int g = ngroups - 1; g >= 0; --g) {   // the groups' sums, last group first
+      __syncthreads();
+      if (group == g && active) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float* o = part + ((size_t)my_tap * KCH + my_k + i) * NCH + n0;
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int n = 0; n < NT / 2; ++n) pk_split(acc[i][n], o[2 * n], o[2 * n + 1]);
+          for (int n = 0; n < NT / 2; ++n) {
+            float lo, hi;
+            pk_split(acc[i][n], lo, hi);
+            float* o = sums + (i * NT + 2 * n) * (kthreads + 1) + qt;
+            o[0] = g == ngroups - 1 ? lo : lo + o[0];
+            o[kthreads + 1] = g == ngroups - 1 ? hi : hi + o[kthreads + 1];
+          }
       }
     }
+    __syncthreads();
+    for (int e = threadIdx.x; e < min(kthreads, K4 - q0) * 4 * NT; e += 256) {
+      const int n = e % NT, k = e / NT;   // k: row of the sweep
+      float v = sums[(k % 4 * NT + n) * (kthreads + 1) + k / 4];
+      if (TS && defv != 0.f) {
+        float s = wsum[(q0 * 4 + k) % KCH];
+        for (int g = 0; g < ngroups; ++g) s -= reinterpret_cast<const float*>(red4 + g * kthreads + k / 4)[k % 4];
+        v = fmaf(defv, s, v);
+      }
+      part[((size_t)q0 * 4 + k) * NCH + n0 + n] = v;
+    }
   }
-  __syncthreads();
   red[threadIdx.x] = dacc;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+  for (int o = 128; o > 0; o >>= 1) {
     if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
   }
   if (threadIdx.x == 0) part[slab - 1] = red[0];
 }
 
-template <typename T, int KCH, int NCH, bool TR>
+template <typename T, int KCH, int NCH, bool TS>
 int launch_wgrad(const ScArgs& a, int nparts, cudaStream_t st) {
+  typedef WgradCfg<KCH, NCH> Cf;
   const int taps = a.fh * a.fw * a.fd;
-  const int K4 = taps * KCH / 4;
-  int threads = 64;   // a power of two (the block sum of the default-value gradient halves the block repeatedly)
-  while (threads < K4) threads <<= 1;
-  if (threads > 256) return -4;
-  const long long nvox = TR ? a.nvox_in : a.nvox_out;
-  if (nparts > (nvox + WT - 1) / WT) nparts = (int)((nvox + WT - 1) / WT);
-  const int vox_per_cta = (int)((nvox + nparts - 1) / nparts);
-  nparts = (int)((nvox + vox_per_cta - 1) / vox_per_cta);   // every launched CTA owns at least one voxel and writes its slab
-  const size_t smem = (size_t)WT * NCH * 4 + WT * sizeof(int4) + (size_t)WT * taps * 4 + ((size_t)taps * NCH + threads) * 4;
-  auto k = sc_wgrad_tile_kernel<T, KCH, NCH, TR>;
+  if (nparts > 148 * Cf::OCC) nparts = 148 * Cf::OCC;   // equal slices, all resident
+  if (nparts > (a.nvox_out + WT - 1) / WT) nparts = (int)((a.nvox_out + WT - 1) / WT);
+  const int vox_per_cta = (int)((a.nvox_out + nparts - 1) / nparts);
+  nparts = (int)((a.nvox_out + vox_per_cta - 1) / vox_per_cta);   // every launched CTA owns at least one voxel and writes its slab
+  const size_t area = Cf::area_bytes(taps);
+  const size_t smem = area + 256 * sizeof(float4) + 256 * 4 + (size_t)(taps * NCH > KCH ? taps * NCH : KCH) * 4;
+  auto k = sc_wgrad_tile_kernel<T, KCH, NCH, TS>;
   if (int e = grant_smem(k, smem)) return e;
-  k<<<nparts, threads, smem, st>>>(a, vox_per_cta);
+  k<<<nparts, 256, smem, st>>>(a, vox_per_cta, Cf::kthreads(taps), (int)area);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  return sc_slab_reduce(static_cast<const float*>(a.workspace), nparts, taps, KCH, NCH, TR, static_cast<float*>(a.filter_grad),
-                        TR ? nullptr : static_cast<float*>(a.default_grad), st);
+  return sc_slab_reduce(static_cast<const float*>(a.workspace), nparts, taps, KCH, NCH, false, static_cast<float*>(a.filter_grad),
+                        TS ? nullptr : static_cast<float*>(a.default_grad), st);
 }
 
-template <typename T, bool TR>
+template <typename T, bool TS>
 int dispatch_wgrad(const ScArgs& a, int nparts, cudaStream_t st) {
-  const int kch = TR ? a.Cout : a.Cin, nch = TR ? a.Cin : a.Cout;
 #define CHOP_TILE_CASE(K, N) \
-  if (kch == K && nch == N) return launch_wgrad<T, K, N, TR>(a, nparts, st);
+  if (a.Cin == K && a.Cout == N) return launch_wgrad<T, K, N, TS>(a, nparts, st);
   CHOP_TILE_CASE(8, 8) CHOP_TILE_CASE(8, 16) CHOP_TILE_CASE(8, 32) CHOP_TILE_CASE(16, 8) CHOP_TILE_CASE(16, 16)
   CHOP_TILE_CASE(16, 32) CHOP_TILE_CASE(32, 8) CHOP_TILE_CASE(32, 16) CHOP_TILE_CASE(32, 32)
 #undef CHOP_TILE_CASE
   return -4;
 }
 
-template <typename T, int KCH, int NCH, int FORM>
+template <typename T, int KCH, int NCH, int FORM, int NW>
 int launch(const ScArgs& a, cudaStream_t st) {
-  typedef TileCfg<KCH, NCH> Cf;
+  typedef TileCfg<KCH, NCH, NW> Cf;
   const int taps = a.fh * a.fw * a.fd;
-  const size_t smem = (size_t)taps * Cf::LK * Cf::WROW * 4 + (size_t)Cf::VPC * (sizeof(int4) + 4) + (size_t)Cf::VPC * taps * 4;
-  auto k = sc_tile_kernel<T, KCH, NCH, FORM>;
+  const size_t smem = Cf::smem(taps, a.fh * a.fw);
+  // a filter so large that the tables of many warps do not fit beside its weights
+  if constexpr (NW > 4)
+    if (smem > 220 * 1024) return launch<T, KCH, NCH, FORM, 4>(a, st);
+  auto k = sc_tile_kernel<T, KCH, NCH, FORM, NW>;
   if (int e = grant_smem(k, smem)) return e;
   const long long nvox = FORM == 0 ? a.nvox_out : a.nvox_in;
   long long ntiles = (nvox + Cf::VPC - 1) / Cf::VPC;
-  if (FORM == 1 && (a.sr > 1 || a.sc > 1)) ntiles = class_tiles(a, Cf::VPC);
+  if (FORM == 2) ntiles = class_tiles(a, Cf::VPC);
   // weights are staged per CTA: as many CTAs as are resident, each walking its tiles
-  int per_sm = (int)((size_t)220 * 1024 / (smem + 1024));
-  if (per_sm > 4) per_sm = 4;
+  int per_sm = (int)((size_t)224 * 1024 / (smem + 1024));
+  if (per_sm > 16 / NW) per_sm = 16 / NW;
   if (per_sm < 1) per_sm = 1;
   const long long blocks = ntiles < 148LL * per_sm ? ntiles : 148LL * per_sm;
-  k<<<(unsigned)blocks, 128, smem, st>>>(a, (int)nvox, (int)ntiles);
+  k<<<(unsigned)blocks, 32 * NW, smem, st>>>(a, (int)nvox, (int)ntiles);
   return (int)cudaGetLastError();
 }
 
@@ -415,7 +542,7 @@ template <typename T, int FORM>
 int dispatch(const ScArgs& a, cudaStream_t st) {
   const int kch = FORM == 0 ? a.Cin : a.Cout, nch = FORM == 0 ? a.Cout : a.Cin;
 #define CHOP_TILE_CASE(K, N) \
-  if (kch == K && nch == N) return launch<T, K, N, FORM>(a, st);
+  if (kch == K && nch == N) return launch<T, K, N, FORM, tile_warps(K, N)>(a, st);
   CHOP_TILE_CASE(8, 8) CHOP_TILE_CASE(8, 16) CHOP_TILE_CASE(8, 32) CHOP_TILE_CASE(16, 8) CHOP_TILE_CASE(16, 16)
   CHOP_TILE_CASE(16, 32) CHOP_TILE_CASE(32, 8) CHOP_TILE_CASE(32, 16) CHOP_TILE_CASE(32, 32)
 #undef CHOP_TILE_CASE
@@ -439,15 +566,13 @@ bool sc_tile_supported(int dtype, const ScArgs& a) {
   return a.nvox_in < (1LL << 31) - 4096 && a.nvox_out < (1LL << 31) - 4096;
 }
 
-// the filter gradient additionally needs taps * (gathered channels) / 4 <= 256 threads
-bool sc_tile_wgrad_supported(int dtype, const ScArgs& a, bool transposed) {
-  if (!sc_tile_supported(dtype, a)) return false;
-  return (long long)a.fh * a.fw * a.fd * (transposed ? a.Cout : a.Cin) / 4 <= 256;
-}
 int sc_tile_wgrad_launch(int dtype, const ScArgs& a, int nparts, cudaStream_t st) {
   return dtype == 0 ? dispatch_wgrad<float, false>(a, nparts, st) : dispatch_wgrad<__nv_bfloat16, false>(a, nparts, st);
 }
-int sc_tile_twgrad_launch(int dtype, const ScArgs& a, int nparts, cudaStream_t st) {
+int sc_tile_twgrad_launch(int dtype, const ScArgs& in, int nparts, cudaStream_t st) {
+  ScArgs a = in;
+  a.images = in.out_grad;   // see TS above
+  a.out_grad = in.images;
   return dtype == 0 ? dispatch_wgrad<float, true>(a, nparts, st) : dispatch_wgrad<__nv_bfloat16, true>(a, nparts, st);
 }
 
@@ -457,6 +582,7 @@ int sc_tile_fwd_launch(int dtype, const ScArgs& a, cudaStream_t st) {
 // gather form: a.out_grad = the coarse tensor (Cout channels), a.images_grad = the fine result (Cin channels);
 // a.pad_zero selects the image gradient (1) or the transposed forward (0)
 int sc_tile_gather_launch(int dtype, const ScArgs& a, cudaStream_t st) {
+  if (a.sr > 1 || a.sc > 1) return dtype == 0 ? dispatch<float, 2>(a, st) : dispatch<__nv_bfloat16, 2>(a, st);
   return dtype == 0 ? dispatch<float, 1>(a, st) : dispatch<__nv_bfloat16, 1>(a, st);
 }
 

@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
   TileClass cl;
   cl.k = 0;
   cl.begin = 0;
-  class_open<128>(a, cl);
+  class_open(a, cl, 128);
   unsigned todo = 0;                              // bit fr*3 + fc: filter column still to do
   bool vvalid = false;
   int b = 0, r = 0, c = 0, cr = 0, cc = 0;
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
     while (tile >= cl.end) {
       ++cl.k;
       cl.begin = cl.end;
-      class_open<128>(a, cl);
+      class_open(a, cl, 128);
     }
     todo = padded ? 0x1ffu : cl.real;
     const unsigned v = (unsigned)(tile - cl.begin) * 128u + tid;

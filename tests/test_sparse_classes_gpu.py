@@ -82,3 +82,26 @@ def test_register_tiled_kernels_at_every_channel_pair(strides, chans, ksize):
     want = oracle.sparse_conv3d_transpose_fwd(images, filters, defv, bp, (H, W, D), strides, (1, 1, 1), np.float32)
     out = ops.sparse_conv3d_transpose_forward(_t(images), _t(filters), float(defv), _t(bp), (H, W, D), strides)
     assert helpers.rel_err(out.cpu().numpy(), want) <= 1e-5
+
+
+@pytest.mark.parametrize("default", [0.0, None])
+@pytest.mark.parametrize("chans,ksize,strides", [((8, 8), (3, 3, 3), (2, 2, 2)), ((8, 32), (3, 3, 3), (2, 2, 1)),
+                                                 ((32, 8), (3, 3, 3), (1, 1, 1)), ((16, 16), (3, 3, 3), (3, 1, 2)),
+                                                 ((32, 32), (3, 3, 3), (2, 2, 2)), ((16, 32), (5, 5, 3), (2, 3, 2)),
+                                                 ((32, 16), (5, 5, 3), (1, 2, 2)), ((32, 32), (7, 7, 1), (2, 2, 1)),
+                                                 ((16, 8), (1, 1, 5), (1, 2, 3))])
+def test_register_tiled_transposed_gradients(chans, ksize, strides, default):
+    """Operands swapped over the coarse voxels: one, two and four groups per block, several sweeps of a large filter, weights
+    that leave room for few warps only, ragged last steps, the default value's share."""
+    Cin, Cout = chans
+    B, H, W, D = 2, 9, 11, 7
+    images, filters, defv, bp = make_transpose_case(58, B, H, W, D, Cin, Cout, ksize, strides, dtype=np.float32, default=default)
+    want = oracle.sparse_conv3d_transpose_fwd(images, filters, defv, bp, (H, W, D), strides, (1, 1, 1), np.float32)
+    og = np.random.default_rng(59).uniform(-1, 1, want.shape).astype(np.float32)
+    ig_w, fg_w = oracle.sparse_conv3d_transpose_bwd(images, filters, defv, bp, (H, W, D), og, strides, (1, 1, 1), False,
+                                                    np.float32)
+    out = ops.sparse_conv3d_transpose_forward(_t(images), _t(filters), float(defv), _t(bp), (H, W, D), strides)
+    ig, fg = ops.sparse_conv3d_transpose_backward(_t(images), _t(filters), float(defv), _t(bp), (H, W, D), _t(og), strides)
+    assert helpers.rel_err(out.cpu().numpy(), want) <= 1e-5
+    assert helpers.rel_err(ig.cpu().numpy(), ig_w) <= 1e-5
+    assert helpers.rel_err(fg.cpu().numpy(), fg_w) <= 1e-5
