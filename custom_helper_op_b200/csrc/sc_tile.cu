@@ -1,5 +1,5 @@
 // Register-tiled CUDA-core manifold convolution for float32 data (the reference's own dtype) and for bfloat16 storage
-// with float32 accumulation where the tensor-core kernels do not apply (8 channels, other filter sizes, dilation):
+// with float32 accumulation where the tensor-core kernels do not apply (other filter sizes, dilation):
 // forward, gather-form image gradient, transposed forward and filter gradient, any filter size / stride / dilation,
 // 8, 16 or 32 channels on either side.
 //

@@ -1,6 +1,6 @@
 // Manifold 3-D convolution as an implicit GEMM on the 5th-generation tensor cores (tcgen05), for the
 // case the depth-band networks actually run: 3x3x3 filter, stride 1, dilation 1, bfloat16 storage,
-// float32 accumulation, 16 or 32 channels.
+// float32 accumulation, 8, 16 or 32 channels.
 //
 //   D[m][n] = sum_k A[m][k] * B[n][k]     m: 128 output voxels of a tile (one per thread)
 //                                          n: output channels (16 / 32)
@@ -97,6 +97,13 @@ __device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, uint32_t* r) {
                : "memory");
 }
 template <>
+__device__ __forceinline__ void tmem_ld<8>(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+template <>
 __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, uint32_t* r) {
   tmem_ld<16>(taddr, r);
   tmem_ld<16>(taddr + 16, r + 16);
@@ -155,33 +162,39 @@ __device__ __forceinline__ long long tap_voxel(const ScArgs& a, const VoxPos& p,
 // (forward: n = output channel, k = input channel; DGRAD: the flipped tap with the channels swapped, whose rows are
 // contiguous in the filter tensor).  One 16-byte chunk (eight k of one n) per thread and step, its loads independent of
 // each other: every CTA repeats this, so it must not be a chain of dependent scalar loads.
-template <int CIN, int COUT, bool DGRAD>
+// CR, NR: the channels the tensors have.  Eight are padded to 16 (the K of an MMA, the least N at M = 128) with zeros.
+// The tensor pipe is idle most of the time anyway: 180x230x9, 3x3x3, bf16 forward / image gradient / filter gradient took
+// 91 / 110 / 127 us for 8 -> 16 channels on the CUDA cores and take 30 / 31 / 21 here, 32 -> 8 191 / 159 / 236 and 68 / 35 / 120.
+__host__ __device__ constexpr int pad16(int c) { return c < 16 ? 16 : c; }
+template <int CR, int NR, bool DGRAD>
 __device__ __forceinline__ void stage_filter_tiles(const unsigned short* flt, unsigned char* sB, int tid, uint32_t lbo,
                                                    uint32_t sbo, int tap_bytes) {
-  constexpr int KC = CIN / 8;
+  constexpr int COUT = pad16(NR), KC = pad16(CR) / 8;
 #pragma unroll 2
   for (int e = tid; e < 27 * COUT * KC; e += 128) {
     const int kg = e % KC, n = (e / KC) % COUT, t = e / (KC * COUT);
-    uint4 w;
-    if (DGRAD) {
-      w = __ldg(reinterpret_cast<const uint4*>(flt + ((size_t)(26 - t) * COUT + n) * CIN + kg * 8));  // f[flip t][ci = n][oc = k]
+    uint4 w = make_uint4(0, 0, 0, 0);
+    if (kg * 8 >= CR || n >= NR) {
+    } else if (DGRAD) {
+      w = __ldg(reinterpret_cast<const uint4*>(flt + ((size_t)(26 - t) * NR + n) * CR + kg * 8));  // f[flip t][ci = n][oc = k]
     } else {
       unsigned h[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) h[i] = __ldg(flt + ((size_t)t * CIN + kg * 8 + i) * COUT + n);        // f[t][ci = k][oc = n]
+      for (int i = 0; i < 8; ++i) h[i] = __ldg(flt + ((size_t)t * CR + kg * 8 + i) * NR + n);        // f[t][ci = k][oc = n]
       w = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
     }
     *reinterpret_cast<uint4*>(sB + t * tap_bytes + (n / 8) * sbo + kg * lbo + (n % 8) * 16) = w;
   }
 }
 
-// CIN: channels of the gathered tensor (K per tap), COUT: channels produced (N).
-template <int CIN, int COUT, bool DGRAD, bool S1>
+// CR: channels of the gathered tensor (K per tap), NR: channels produced (N).
+template <int CR, int NR, bool DGRAD, bool S1>
 __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long long nvox, const int ntiles) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar_s;
   __shared__ uint32_t tmem_base_s;
-  constexpr int KC = CIN / 8;                     // 16-byte k-chunks per tap
+  constexpr int CIN = pad16(CR), COUT = pad16(NR);
+  constexpr int KC = CIN / 8, KR = CR / 8;        // 16-byte k-chunks per tap, those that are channels
   constexpr uint32_t LBO = 128, SBO = KC * 128;   // core-matrix strides in K and in M/N
   constexpr int A_TAP_BYTES = 128 * CIN * 2;
   constexpr int B_TAP_BYTES = COUT * CIN * 2;
@@ -194,7 +207,10 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
 
   // ---- filter -> canonical K-major B tiles: B[n][k] of tap t at sB + t*B_TAP_BYTES -----------------------
   {
-    stage_filter_tiles<CIN, COUT, DGRAD>(static_cast<const unsigned short*>(a.filters), sB, tid, LBO, SBO, B_TAP_BYTES);
+    stage_filter_tiles<CR, NR, DGRAD>(static_cast<const unsigned short*>(a.filters), sB, tid, LBO, SBO, B_TAP_BYTES);
+    if (KR < KC)   // the padding channels of the staging rows stay zero
+      for (int e = tid; e < 9 * 128; e += 128)
+        *reinterpret_cast<uint4*>(sA + e / 128 * A_TAP_BYTES + (e % 128 / 8) * SBO + e % 8 * 16 + LBO) = make_uint4(0, 0, 0, 0);
   }
   if (warp == 0) {
     uint32_t slot = smem_u32(&tmem_base_s), ncols = 32;
@@ -242,10 +258,10 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
         for (int fz = 0; fz < 3; ++fz) {
           const long long sv = inb ? tap_voxel(a, pos, base, shift, fz) : -1;
           const bool ok = sv >= 0;
-          const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)(ok ? sv : 0) * CIN);
+          const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)(ok ? sv : 0) * CR);
           unsigned char* dstA = a_row + (fc * 3 + fz) * A_TAP_BYTES;
 #pragma unroll
-          for (int kc = 0; kc < KC; ++kc) {
+          for (int kc = 0; kc < KR; ++kc) {
             uint4 x = vvalid ? padv : make_uint4(0, 0, 0, 0);
             if (ok) x = __ldg(p + kc);
             *reinterpret_cast<uint4*>(dstA + kc * LBO) = x;
@@ -288,9 +304,9 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
     tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16), acc);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     if (vvalid) {
-      uint4* o = reinterpret_cast<uint4*>(dst + (size_t)v * COUT);
+      uint4* o = reinterpret_cast<uint4*>(dst + (size_t)v * NR);
 #pragma unroll
-      for (int q = 0; q < COUT / 8; ++q) {
+      for (int q = 0; q < NR / 8; ++q) {
         uint32_t w[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -325,12 +341,12 @@ __global__ void __launch_bounds__(128) sc_umma_kernel(const ScArgs a, const long
 // ---------------------------------------------------------------------------------------------------------
 constexpr int CLS_COLS = 2;   // filter columns staged per round
 
-template <int CIN, int COUT>
+template <int CR, int NR>
 __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, const int ntiles) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar_s;
   __shared__ uint32_t tmem_base_s;
-  constexpr int KC = CIN / 8;
+  constexpr int CIN = pad16(CR), COUT = pad16(NR), KC = CIN / 8, KR = CR / 8;
   constexpr uint32_t LBO = 128, SBO = KC * 128;
   constexpr int A_TAP_BYTES = 128 * CIN * 2;
   constexpr int B_TAP_BYTES = COUT * CIN * 2;
@@ -340,7 +356,10 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
   const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.out_grad);
   __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.images_grad);
 
-  stage_filter_tiles<CIN, COUT, true>(static_cast<const unsigned short*>(a.filters), sB, tid, LBO, SBO, B_TAP_BYTES);
+  stage_filter_tiles<CR, NR, true>(static_cast<const unsigned short*>(a.filters), sB, tid, LBO, SBO, B_TAP_BYTES);
+  if (KR < KC)   // the padding channels of the staging rows stay zero
+    for (int e = tid; e < CLS_COLS * 3 * 128; e += 128)
+      *reinterpret_cast<uint4*>(sA + e / 128 * A_TAP_BYTES + (e % 128 / 8) * SBO + e % 8 * 16 + LBO) = make_uint4(0, 0, 0, 0);
   if (warp == 0) {
     uint32_t slot = smem_u32(&tmem_base_s), ncols = 32;
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(ncols) : "memory");
@@ -409,7 +428,7 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
     }
   };
   int cols[CLS_COLS], ncols = 0;
-  uint4 pre[CLS_COLS * 3 * KC];
+  uint4 pre[CLS_COLS * 3 * KR];
   auto request = [&]() {   // the next CLS_COLS filter columns of the open tile into registers
     ncols = 0;
 #pragma unroll
@@ -441,12 +460,12 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
       for (int fz = 0; fz < 3; ++fz) {
         const int cd = cdz[fz] - shift[i];
         const bool in = ok[i] && ((dok >> fz) & 1u) && !oob(cd, a.oD);
-        const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)(in ? base[i] + cd : 0) * CIN);
+        const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)(in ? base[i] + cd : 0) * CR);
 #pragma unroll
-        for (int kc = 0; kc < KC; ++kc) {
+        for (int kc = 0; kc < KR; ++kc) {
           uint4 x = vvalid ? padv : make_uint4(0, 0, 0, 0);
           if (in) x = __ldg(p + kc);
-          pre[(i * 3 + fz) * KC + kc] = x;
+          pre[(i * 3 + fz) * KR + kc] = x;
         }
       }
     }
@@ -470,7 +489,7 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
     for (int q = 0; q < KT; ++q) {
       if (q < n_now * 3) {
 #pragma unroll
-        for (int kc = 0; kc < KC; ++kc) *reinterpret_cast<uint4*>(a_row + q * A_TAP_BYTES + kc * LBO) = pre[q * KC + kc];
+        for (int kc = 0; kc < KR; ++kc) *reinterpret_cast<uint4*>(a_row + q * A_TAP_BYTES + kc * LBO) = pre[q * KR + kc];
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -522,9 +541,9 @@ __global__ void __launch_bounds__(128) sc_umma_class_kernel(const ScArgs a, cons
         for (int n = 0; n < COUT; ++n) acc[n] = 0u;
       }
       if (out_now >= 0) {
-        uint4* o = reinterpret_cast<uint4*>(dst + (size_t)out_now * COUT);
+        uint4* o = reinterpret_cast<uint4*>(dst + (size_t)out_now * NR);
 #pragma unroll
-        for (int q = 0; q < COUT / 8; ++q) {
+        for (int q = 0; q < NR / 8; ++q) {
           uint32_t w[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -602,13 +621,13 @@ __device__ __forceinline__ void rows_tab_read(const int2* tab, int q, int j, int
 // Against the per-tap gather this stages 9 instead of 27 rows per voxel, issues all 27 taps of a tile
 // behind one barrier (one commit, one wait) and reads every neighbour plane once.
 // ---------------------------------------------------------------------------------------------------------
-template <int CIN, int COUT, bool DGRAD>
-__global__ void __launch_bounds__(128, CIN <= 16 ? 4 : 2) sc_umma_rows_kernel(const ScArgs a, const int ntiles, const int PT) {
+template <int CR, int NR, bool DGRAD>
+__global__ void __launch_bounds__(128, CR <= 16 ? 4 : 2) sc_umma_rows_kernel(const ScArgs a, const int ntiles, const int PT) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar_s;
   __shared__ uint32_t tmem_base_s;
   __shared__ int2 tab_s[ROWS_TAB];
-  constexpr int KC = CIN / 8;
+  constexpr int CIN = pad16(CR), COUT = pad16(NR), KC = CIN / 8, KR = CR / 8;
   // rows per column buffer: 128 + the two shifted reads; 132 rows make the K-chunk stride 64 bytes off a multiple
   // of 128, so the KC lanes that store the chunks of one row hit different banks
   constexpr int NRB = 132;
@@ -624,12 +643,15 @@ __global__ void __launch_bounds__(128, CIN <= 16 ? 4 : 2) sc_umma_rows_kernel(co
   __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(DGRAD ? a.images_grad : a.output);
 
   {
-    stage_filter_tiles<CIN, COUT, DGRAD>(static_cast<const unsigned short*>(a.filters), sB, tid, B_LBO, B_SBO, B_TAP_BYTES);
+    stage_filter_tiles<CR, NR, DGRAD>(static_cast<const unsigned short*>(a.filters), sB, tid, B_LBO, B_SBO, B_TAP_BYTES);
     // rows 128..135 of every column buffer are only ever read into discarded output rows; keep them defined
     for (int e = tid; e < 9 * KC * (NRB - 128); e += 128) {
       const int rr = e % (NRB - 128), kc = (e / (NRB - 128)) % KC, col = e / ((NRB - 128) * KC);
       *reinterpret_cast<uint4*>(sX + col * COL_BYTES + kc * A_LBO + (128 + rr) * 16) = make_uint4(0, 0, 0, 0);
     }
+    if (KR < KC)   // the padding channels stay zero
+      for (int e = tid; e < 9 * 128; e += 128)
+        *reinterpret_cast<uint4*>(sX + e / 128 * COL_BYTES + A_LBO + e % 128 * 16) = make_uint4(0, 0, 0, 0);
   }
   if (warp == 0) {
     uint32_t slot = smem_u32(&tmem_base_s), ncols = 32;
@@ -672,20 +694,20 @@ __global__ void __launch_bounds__(128, CIN <= 16 ? 4 : 2) sc_umma_rows_kernel(co
     rvalid = row_used && tile < ntiles && pix < npix;
     rows_tab_read(tab_s, p_in_tile, j, D, row_used, sv);
   };
-  // The KC 16-byte chunks of a row are fetched by KC neighbouring lanes (the row's owner hands its source voxel
+  // The KR 16-byte chunks of a row are fetched by KR neighbouring lanes (the row's owner hands its source voxel
   // over by shuffle), so a warp-wide load covers whole rows - contiguous 32*16 bytes where the rows are
   // consecutive planes of one pixel - instead of every other 16 bytes of twice the span: half the L1 wavefronts.
-  // Pass i of lane l: row 32*warp + l/KC + i*(32/KC), chunk l%KC.
-  uint4 val[9][KC];
-  const int lane = tid & 31, chunk = lane % KC, lrow = lane / KC;
+  // Pass i of lane l: row 32*warp + l/KR + i*(32/KR), chunk l%KR.
+  uint4 val[9][KR];
+  const int lane = tid & 31, chunk = lane % KR, lrow = lane / KR;
   auto request = [&]() {
 #pragma unroll
     for (int col = 0; col < 9; ++col) {
 #pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        const int sr = __shfl_sync(0xffffffffu, sv[col], lrow + i * (32 / KC));
+      for (int i = 0; i < KR; ++i) {
+        const int sr = KR == 1 ? sv[col] : __shfl_sync(0xffffffffu, sv[col], lrow + i * (32 / KR));
         val[col][i] = sr == -2 ? make_uint4(0, 0, 0, 0) : padv;
-        if (sr >= 0) val[col][i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)sr * CIN) + chunk);
+        if (sr >= 0) val[col][i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)sr * CR) + chunk);
       }
     }
   };
@@ -706,7 +728,7 @@ __global__ void __launch_bounds__(128, CIN <= 16 ? 4 : 2) sc_umma_rows_kernel(co
     for (int col = 0; col < 9; ++col) {
       unsigned char* dx = sX + col * COL_BYTES + chunk * A_LBO + (warp * 32 + lrow) * 16;
 #pragma unroll
-      for (int i = 0; i < KC; ++i) *reinterpret_cast<uint4*>(dx + i * (32 / KC) * 16) = val[col][i];
+      for (int i = 0; i < KR; ++i) *reinterpret_cast<uint4*>(dx + i * (32 / KR) * 16) = val[col][i];
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -745,9 +767,9 @@ __global__ void __launch_bounds__(128, CIN <= 16 ? 4 : 2) sc_umma_rows_kernel(co
     tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16), acc);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     if (rvalid_out && j < D) {
-      uint4* o = reinterpret_cast<uint4*>(dst + ((size_t)pix_out * D + j) * COUT);
+      uint4* o = reinterpret_cast<uint4*>(dst + ((size_t)pix_out * D + j) * NR);
 #pragma unroll
-      for (int q = 0; q < COUT / 8; ++q) {
+      for (int q = 0; q < NR / 8; ++q) {
         uint32_t w[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -795,12 +817,13 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
   __shared__ uint32_t tmem_base_s;
   __shared__ float red_s[128];
   constexpr int KC = CIN / 8;            // 16-byte channel chunks per tap
+  constexpr int NP = pad16(COUT);        // N of an MMA; what the padding columns hold is not used
   constexpr int TPR = 128 / CIN;         // taps per round (one 128-row M group)
   constexpr int NT = (27 + TPR - 1) / TPR;
-  constexpr int TMEM_COLS = NT * COUT <= 32 ? 32 : (NT * COUT <= 64 ? 64 : (NT * COUT <= 128 ? 128 : 256));
+  constexpr int TMEM_COLS = NT * NP <= 32 ? 32 : (NT * NP <= 64 ? 64 : (NT * NP <= 128 ? 128 : 256));
   constexpr uint32_t SBO = 128;                    // between 8-channel groups (M / N direction)
   constexpr uint32_t LBO_A = 16 * 128;             // between 8-voxel groups of the A staging tile
-  constexpr uint32_t LBO_G = (COUT / 8) * 128;     // between 8-voxel groups of the G tile
+  constexpr uint32_t LBO_G = (NP / 8) * 128;       // between 8-voxel groups of the G tile
   unsigned char* sA = smem;                        // 16 voxel groups x 2048 B
   unsigned char* sG = smem + 16 * LBO_A;           // 16 voxel groups x LBO_G
   float* wsum = reinterpret_cast<float*>(sG + 16 * LBO_G);  // [27][COUT], dynamic_default only
@@ -833,7 +856,7 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
   const uint32_t tmem = tmem_base_s;
   const uint32_t mbar = smem_u32(&mbar_s);
   // D f32, A/B bf16, both operands MN-major (bits 15, 16), N = COUT, M = 128
-  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(COUT >> 3) << 17) |
+  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(NP >> 3) << 17) |
                              ((128u >> 4) << 24);
   const unsigned d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
   const unsigned d32 = d16 | (d16 << 16);
@@ -922,7 +945,7 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
         for (int ks = 0; ks < 8; ++ks) {  // 16 voxels (two 8-voxel groups) per MMA
           const uint64_t da = umma_desc(smem_u32(sA + ks * 2 * LBO_A), LBO_A, SBO);
           const uint64_t db = umma_desc(smem_u32(sG + ks * 2 * LBO_G), LBO_G, SBO);
-          umma_bf16(tmem + rd * COUT, da, db, IDESC, (first && ks == 0) ? 0u : 1u);
+          umma_bf16(tmem + rd * NP, da, db, IDESC, (first && ks == 0) ? 0u : 1u);
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
       }
@@ -974,9 +997,9 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
   if (alive) {
 #pragma unroll
     for (int rd = 0; rd < NT; ++rd) {
-      uint32_t acc[COUT];
+      uint32_t acc[NP];
       if (!first) {
-        tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + rd * COUT, acc);
+        tmem_ld<NP>(tmem + ((uint32_t)(warp * 32) << 16) + rd * NP, acc);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
       const int k = rd * 128 + tid;
@@ -1038,22 +1061,24 @@ __global__ void __launch_bounds__(128) sc_umma_wgrad_kernel(const ScArgs a, cons
 // all tiles of the CTA.  One barrier per tile instead of four, 9 staged rows per voxel instead of 27.
 // TG (transposed convolution) only changes the operand roles, exactly as in sc_umma_wgrad_kernel.
 // ---------------------------------------------------------------------------------------------------------
-template <int COUT, bool TG>
+template <int CIN, int COUT, bool TG>
 __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs a, const int ntiles, const int PT) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar_s;
   __shared__ uint32_t tmem_base_s;
   __shared__ float red_s[128];
-  constexpr int CIN = 16, KC = 2;
+  constexpr int KC = CIN / 8;                      // 1 or 2
+  constexpr int NBLK = KC;                         // eight channels: one block holds all nine columns
   constexpr int NRB = 132;                         // as in sc_umma_rows_kernel
   constexpr uint32_t X_SBO = NRB * 16;             // chunk stride (M direction)
   constexpr uint32_t X_LBO = 128;                  // eight voxels further (reduction direction): rows are linear
   // out_grad tile with the three depth taps side by side in N: chunk fz*(COUT/8) + nc of voxel group m'/8 holds
   // channels nc*8.. of out_grad row m' - fz, so ONE MMA with N = 3*COUT per 16 tile rows serves the three taps
   // (an N = 16 MMA costs the issuing thread as much as an N = 48 one, and that thread is the tile's critical path)
-  constexpr int NCH = 3 * (COUT / 8);              // 16-byte chunks per row of the widened tile
+  constexpr int NCH = (3 * (COUT / 8) + 1) / 2 * 2;   // 16-byte chunks per row of the widened tile (N a multiple of 16)
+  constexpr int NP = NCH * 8;                      // tensor-memory columns of a block
   constexpr uint32_t G_SBO = 128, G_LBO = NCH * 128;
-  constexpr int TMEM_COLS = 6 * COUT <= 128 ? 128 : 256;
+  constexpr int TMEM_COLS = NBLK * NP <= 32 ? 32 : (NBLK * NP <= 64 ? 64 : (NBLK * NP <= 128 ? 128 : 256));
   unsigned char* sX = smem;                        // 18 chunks x NRB rows x 16 B
   unsigned char* sG = smem + 18 * X_SBO;           // 16 voxel groups x G_LBO
   float* wsum = reinterpret_cast<float*>(sG + 16 * G_LBO);   // [27][COUT], dynamic_default only
@@ -1094,7 +1119,7 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
   const uint32_t tmem = tmem_base_s;
   const uint32_t mbar = smem_u32(&mbar_s);
   // D f32, A/B bf16, both operands MN-major (bits 15, 16), N = COUT, M = 128
-  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)((3 * COUT) >> 3) << 17) |
+  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)NCH << 17) |
                              ((128u >> 4) << 24);
   const unsigned d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
   const unsigned d32 = d16 | (d16 << 16);
@@ -1169,7 +1194,7 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
     for (int col = 0; col < 9; ++col) {
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
-        const int sr = __shfl_sync(0xffffffffu, sv[col], lrow + i * (32 / KC));
+        const int sr = KC == 1 ? sv[col] : __shfl_sync(0xffffffffu, sv[col], lrow + i * (32 / KC));
         val[col][i] = sr == -2 ? zero4 : padv;
         if (sr >= 0) val[col][i] = __ldg(reinterpret_cast<const uint4*>(img + (size_t)sr * CIN) + chunk);
       }
@@ -1188,12 +1213,12 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-      for (int blk = 0; blk < 2; ++blk) {
+      for (int blk = 0; blk < NBLK; ++blk) {
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {   // 16 tile rows (two 8-row groups) per MMA
           const uint64_t da = umma_desc_advance(da0, blk * 2 * X_SBO + ks * 2 * X_LBO);
           const uint64_t db = umma_desc_advance(db0, ks * 2 * G_LBO);
-          umma_bf16(tmem + blk * 3 * COUT, da, db, IDESC, (first && ks == 0) ? 0u : 1u);
+          umma_bf16(tmem + blk * NP, da, db, IDESC, (first && ks == 0) ? 0u : 1u);
         }
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
@@ -1245,14 +1270,14 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
 #pragma unroll
     for (int fz = 0; fz < 3; ++fz) {
 #pragma unroll
-      for (int blk = 0; blk < 2; ++blk) {
+      for (int blk = 0; blk < NBLK; ++blk) {
         uint32_t acc[COUT];
         if (!first) {
-          tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + (blk * 3 + fz) * COUT, acc);
+          tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + blk * NP + fz * COUT, acc);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         }
         // MMA row tid of block blk is chunk q = 2*blk + tid/8, element tid%8: column q/2, channel (q%2)*8 + tid%8.
-        // Block 0 supplies columns 0..7, block 1 only column 8 (its rows 112..127).
+        // Block 0 supplies columns 0..7, block 1 only column 8 (its rows 112..127); with eight channels block 0 holds all nine.
         const int q = 2 * blk + tid / 8;
         const int col = q / KC, ci = (q % KC) * 8 + (tid % 8);
         // Through shared memory (the column buffers are free), so that the stores are consecutive: the CIN rows of
@@ -1260,9 +1285,10 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
         float* rows = reinterpret_cast<float*>(sX);
         __syncthreads();
 #pragma unroll
-        for (int n = 0; n < COUT; ++n) rows[(col * CIN + ci) * (COUT + 1) + n] = first ? 0.f : __uint_as_float(acc[n]);
+        for (int n = 0; n < COUT; ++n)
+          if (col < 9) rows[(col * CIN + ci) * (COUT + 1) + n] = first ? 0.f : __uint_as_float(acc[n]);
         __syncthreads();
-        for (int e = tid; e < (blk == 0 ? 8 : 1) * CIN * COUT; e += 128) {
+        for (int e = tid; e < (blk == 0 ? 10 - NBLK : 1) * CIN * COUT; e += 128) {
           const int cc = (blk == 0 ? 0 : 8) + e / (CIN * COUT), w = e % (CIN * COUT);
           part[(size_t)(cc * 3 + fz) * CIN * COUT + w] = rows[(cc * CIN + w / COUT) * (COUT + 1) + w % COUT];
         }
@@ -1285,10 +1311,10 @@ __global__ void __launch_bounds__(128, 4) sc_umma_wgrad_rows_kernel(const ScArgs
   }
 }
 
-template <int COUT, bool TG>
+template <int CIN, int COUT, bool TG>
 int launch_wgrad_rows(const ScArgs& a, int nparts, cudaStream_t st) {
-  auto k = sc_umma_wgrad_rows_kernel<COUT, TG>;
-  const size_t smem = (size_t)18 * 132 * 16 + (size_t)16 * 3 * (COUT / 8) * 128 + (size_t)27 * COUT * 4 + 1024;
+  auto k = sc_umma_wgrad_rows_kernel<CIN, COUT, TG>;
+  const size_t smem = (size_t)18 * 132 * 16 + (size_t)16 * ((3 * (COUT / 8) + 1) / 2 * 2) * 128 + (size_t)27 * COUT * 4 + 1024;
   if (int e = grant_smem(k, smem)) return e;
   const int PT = 128 / (a.D + 2);
   const long long npix = (long long)a.B * a.H * a.W;
@@ -1297,18 +1323,18 @@ int launch_wgrad_rows(const ScArgs& a, int nparts, cudaStream_t st) {
   k<<<nparts, 128, smem, st>>>(a, (int)ntiles, PT);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  return sc_slab_reduce(static_cast<const float*>(a.workspace), nparts, 27, 16, COUT, TG, static_cast<float*>(a.filter_grad),
+  return sc_slab_reduce(static_cast<const float*>(a.workspace), nparts, 27, CIN, COUT, TG, static_cast<float*>(a.filter_grad),
                         TG ? nullptr : static_cast<float*>(a.default_grad), st);
 }
 
 template <int CIN, int COUT, bool TS>
 int launch_wgrad(const ScArgs& a, int nparts, cudaStream_t st) {
   const bool s1 = a.sr == 1 && a.sc == 1 && a.sd == 1;
-  if constexpr (CIN == 16 && !TS) {
-    if (s1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_wgrad_rows<COUT, false>(a, nparts, st);
+  if constexpr (CIN <= 16 && !TS) {
+    if (s1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_wgrad_rows<CIN, COUT, false>(a, nparts, st);
   }
   auto k = s1 ? sc_umma_wgrad_kernel<CIN, COUT, TS, true> : sc_umma_wgrad_kernel<CIN, COUT, TS, false>;
-  const size_t smem = (size_t)16 * 2048 + (size_t)16 * (COUT / 8) * 128 + (size_t)27 * COUT * 4 + 1024;
+  const size_t smem = (size_t)16 * 2048 + (size_t)16 * (pad16(COUT) / 8) * 128 + (size_t)27 * COUT * 4 + 1024;
   if (int e = grant_smem(k, smem)) return e;
   const int ntiles = (int)((a.nvox_out + 127) / 128);
   if (nparts > ntiles) nparts = ntiles;  // a persistent CTA per slab: more CTAs than tiles would leave slabs unwritten
@@ -1322,7 +1348,7 @@ int launch_wgrad(const ScArgs& a, int nparts, cudaStream_t st) {
 template <int CIN, int COUT, bool DGRAD>
 int launch_rows(const ScArgs& a, cudaStream_t st) {
   auto k = sc_umma_rows_kernel<CIN, COUT, DGRAD>;
-  const size_t smem = (size_t)27 * COUT * CIN * 2 + (size_t)9 * (CIN / 8) * 132 * 16 + 1024;
+  const size_t smem = (size_t)27 * pad16(COUT) * pad16(CIN) * 2 + (size_t)9 * (pad16(CIN) / 8) * 132 * 16 + 1024;
   if (int e = grant_smem(k, smem)) return e;
   const int PT = 128 / (a.D + 2);
   const long long npix = (long long)a.B * a.H * a.W;
@@ -1342,7 +1368,7 @@ int launch_rows(const ScArgs& a, cudaStream_t st) {
 template <int CIN, int COUT>
 int launch_class(const ScArgs& a, cudaStream_t st) {
   auto k = sc_umma_class_kernel<CIN, COUT>;
-  const size_t smem = (size_t)27 * COUT * CIN * 2 + (size_t)CLS_COLS * 3 * 128 * CIN * 2 + 1024;
+  const size_t smem = (size_t)27 * pad16(COUT) * pad16(CIN) * 2 + (size_t)CLS_COLS * 3 * 128 * pad16(CIN) * 2 + 1024;
   if (int e = grant_smem(k, smem)) return e;
   const long long ntiles = class_tiles(a, 128);
   int per_sm = (int)((size_t)220 * 1024 / (smem + 2048));
@@ -1362,7 +1388,7 @@ int launch(const ScArgs& a, long long nvox, cudaStream_t st) {
     if (!s1) return launch_class<CIN, COUT>(a, st);
   }
   auto k = s1 ? sc_umma_kernel<CIN, COUT, DGRAD, true> : sc_umma_kernel<CIN, COUT, DGRAD, DGRAD>;
-  const size_t smem = (size_t)27 * COUT * CIN * 2 + (size_t)9 * 128 * CIN * 2 + 1024;
+  const size_t smem = (size_t)27 * pad16(COUT) * pad16(CIN) * 2 + (size_t)9 * 128 * pad16(CIN) * 2 + 1024;
   if (int e = grant_smem(k, smem)) return e;
   const int ntiles = (int)((nvox + 127) / 128);
   int per_sm = (int)((size_t)220 * 1024 / (smem + 2048));
@@ -1378,45 +1404,51 @@ int launch(const ScArgs& a, long long nvox, cudaStream_t st) {
 
 bool sc_umma_supported(int dtype, const ScArgs& a) {
   return dtype == 2 && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 &&
-         (a.Cin == 16 || a.Cin == 32) && (a.Cout == 16 || a.Cout == 32) && a.nvox_in < ((long long)1 << 31) - 128;
+         (a.Cin == 8 || a.Cin == 16 || a.Cin == 32) && (a.Cout == 8 || a.Cout == 16 || a.Cout == 32) && a.nvox_in < ((long long)1 << 31) - 128;
 }
 
+#define CHOP_UMMA_PAIRS(CASE) \
+  CASE(8, 8) CASE(8, 16) CASE(8, 32) CASE(16, 8) CASE(16, 16) CASE(16, 32) CASE(32, 8) CASE(32, 16) CASE(32, 32)
+
 int sc_umma_fwd_launch(const ScArgs& a, cudaStream_t st) {
-  if (a.Cin == 16 && a.Cout == 16) return launch<16, 16, false>(a, a.nvox_out, st);
-  if (a.Cin == 16 && a.Cout == 32) return launch<16, 32, false>(a, a.nvox_out, st);
-  if (a.Cin == 32 && a.Cout == 16) return launch<32, 16, false>(a, a.nvox_out, st);
-  return launch<32, 32, false>(a, a.nvox_out, st);
+#define CHOP_CASE(I, O) if (a.Cin == I && a.Cout == O) return launch<I, O, false>(a, a.nvox_out, st);
+  CHOP_UMMA_PAIRS(CHOP_CASE)
+#undef CHOP_CASE
+  return -4;
 }
 
 // gathers out_grad (Cout channels) and produces images_grad (Cin channels)
 int sc_umma_dgrad_launch(const ScArgs& a, cudaStream_t st) {
-  if (a.Cin == 16 && a.Cout == 16) return launch<16, 16, true>(a, a.nvox_in, st);
-  if (a.Cin == 16 && a.Cout == 32) return launch<32, 16, true>(a, a.nvox_in, st);
-  if (a.Cin == 32 && a.Cout == 16) return launch<16, 32, true>(a, a.nvox_in, st);
-  return launch<32, 32, true>(a, a.nvox_in, st);
+#define CHOP_CASE(I, O) if (a.Cin == I && a.Cout == O) return launch<O, I, true>(a, a.nvox_in, st);
+  CHOP_UMMA_PAIRS(CHOP_CASE)
+#undef CHOP_CASE
+  return -4;
 }
 
 // nparts partial slabs of (27*Cin*Cout + 1) floats must fit in the workspace; every CTA writes one.
 int sc_umma_wgrad_launch(const ScArgs& a, int nparts, cudaStream_t st) {
-  if (a.Cin == 16 && a.Cout == 16) return launch_wgrad<16, 16, false>(a, nparts, st);
-  if (a.Cin == 16 && a.Cout == 32) return launch_wgrad<16, 32, false>(a, nparts, st);
-  if (a.Cin == 32 && a.Cout == 16) return launch_wgrad<32, 16, false>(a, nparts, st);
-  return launch_wgrad<32, 32, false>(a, nparts, st);
+#define CHOP_CASE(I, O) if (a.Cin == I && a.Cout == O) return launch_wgrad<I, O, false>(a, nparts, st);
+  CHOP_UMMA_PAIRS(CHOP_CASE)
+#undef CHOP_CASE
+  return -4;
 }
 
 // Filter gradient of the transposed convolution; a.images = its coarse input (Cout channels), a.out_grad = the fine
-// upstream gradient (Cin channels), nparts slabs of 27*Cin*Cout + 1 floats in the workspace.  Stride 1 with 16 coarse
+// upstream gradient (Cin channels), nparts slabs of 27*Cin*Cout + 1 floats in the workspace.  Stride 1 with 8 or 16 coarse
 // channels: the shifted-row kernel over the fine grid; otherwise the swapped roles (see sc_umma_wgrad_kernel).
 int sc_umma_twgrad_launch(const ScArgs& a, int nparts, cudaStream_t st) {
-  if (a.Cout == 16 && a.sr == 1 && a.sc == 1 && a.sd == 1 && a.D + 2 <= 128 && g_umma_rows.load())
-    return a.Cin == 16 ? launch_wgrad_rows<16, true>(a, nparts, st) : launch_wgrad_rows<32, true>(a, nparts, st);
+  if (a.Cout <= 16 && a.sr == 1 && a.sc == 1 && a.sd == 1 && a.D + 2 <= 128 && g_umma_rows.load()) {
+#define CHOP_CASE(I, O) if (a.Cin == I && a.Cout == O) return launch_wgrad_rows<O, I, true>(a, nparts, st);
+    CHOP_CASE(8, 8) CHOP_CASE(16, 8) CHOP_CASE(32, 8) CHOP_CASE(8, 16) CHOP_CASE(16, 16) CHOP_CASE(32, 16)
+#undef CHOP_CASE
+  }
   ScArgs w = a;
   w.images = a.out_grad;
   w.out_grad = a.images;
-  if (a.Cin == 16 && a.Cout == 16) return launch_wgrad<16, 16, true>(w, nparts, st);
-  if (a.Cin == 16 && a.Cout == 32) return launch_wgrad<16, 32, true>(w, nparts, st);
-  if (a.Cin == 32 && a.Cout == 16) return launch_wgrad<32, 16, true>(w, nparts, st);
-  return launch_wgrad<32, 32, true>(w, nparts, st);
+#define CHOP_CASE(I, O) if (a.Cin == I && a.Cout == O) return launch_wgrad<I, O, true>(w, nparts, st);
+  CHOP_UMMA_PAIRS(CHOP_CASE)
+#undef CHOP_CASE
+  return -4;
 }
 
 void sc_umma_set_rows(int on) { g_umma_rows = on; }

@@ -105,3 +105,42 @@ def test_register_tiled_transposed_gradients(chans, ksize, strides, default):
     assert helpers.rel_err(out.cpu().numpy(), want) <= 1e-5
     assert helpers.rel_err(ig.cpu().numpy(), ig_w) <= 1e-5
     assert helpers.rel_err(fg.cpu().numpy(), fg_w) <= 1e-5
+
+
+@pytest.mark.parametrize("strides", [(1, 1, 1), (2, 2, 2), (2, 1, 3)])
+@pytest.mark.parametrize("chans", [(8, 8), (8, 16), (8, 32), (16, 8), (32, 8)])
+@pytest.mark.parametrize("rows", [1, 0])
+def test_eight_channels_on_the_tensor_cores(chans, strides, rows):
+    """Eight channels are padded to sixteen on chip: every kernel, both directions, the transposed op, a default value."""
+    Cin, Cout = chans
+    B, H, W, D = 2, 11, 13, 7
+    images, filters, defv, bp, _ = make_case(60, B, H, W, D, Cin, Cout, (3, 3, 3), 24, np.float32)
+    images, filters, defv = _round(images), _round(filters * 0.3), float(_round(np.array([defv]))[0])
+    want = oracle.sparse_conv3d_fwd(images, filters, defv, bp, strides=strides, dtype=np.float32)
+    og = _round(np.random.default_rng(61).uniform(-1, 1, want.shape))
+    ig_w, fg_w, dg_w = oracle.sparse_conv3d_bwd(images, filters, defv, bp, og, strides=strides, dynamic_default=True,
+                                                dtype=np.float32)
+    _lib.set_tuning("umma_rows", rows)
+    try:
+        out = ops.sparse_conv3d_forward(_t(images, bf), _t(filters, bf), defv, _t(bp), strides)
+        ig, fg, dg = ops.sparse_conv3d_backward(_t(images, bf), _t(filters, bf), defv, _t(bp), _t(og, bf), strides,
+                                                dynamic_default=True)
+        assert helpers.rel_err(out.float().cpu().numpy(), want) <= 1e-2
+        assert helpers.rel_err(ig.float().cpu().numpy(), ig_w) <= 1e-2
+        assert helpers.rel_err(fg.cpu().numpy(), fg_w) <= 1e-5
+        assert abs(float(dg) - float(dg_w)) <= 2e-4 * max(1.0, abs(float(dg_w)))
+        images, filters, defv, bp = make_transpose_case(62, B, H, W, D, Cin, Cout, (3, 3, 3), strides, dtype=np.float32)
+        images, filters, defv = _round(images), _round(filters * 0.3), float(_round(np.array([defv]))[0])
+        want = oracle.sparse_conv3d_transpose_fwd(images, filters, defv, bp, (H, W, D), strides, (1, 1, 1), np.float32)
+        og = _round(np.random.default_rng(63).uniform(-1, 1, want.shape))
+        ig_w, fg_w = oracle.sparse_conv3d_transpose_bwd(images, filters, defv, bp, (H, W, D), og, strides, (1, 1, 1), False,
+                                                        np.float32)
+        out = ops.sparse_conv3d_transpose_forward(_t(images, bf), _t(filters, bf), defv, _t(bp), (H, W, D), strides)
+        ig, fg = ops.sparse_conv3d_transpose_backward(_t(images, bf), _t(filters, bf), defv, _t(bp), (H, W, D), _t(og, bf),
+                                                      strides)
+        assert helpers.rel_err(out.float().cpu().numpy(), want) <= 1e-2
+        assert helpers.rel_err(ig.float().cpu().numpy(), ig_w) <= 1e-2
+        assert helpers.rel_err(fg.cpu().numpy(), fg_w) <= 1e-5
+    finally:
+        _lib.set_tuning("umma_rows", 1)
+    assert _lib.lib().chop_umma_timeouts() == 0
