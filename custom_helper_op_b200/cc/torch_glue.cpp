@@ -83,6 +83,22 @@ void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 void* cuda_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 bool has_shape(const Tensor& t, std::initializer_list<int64_t> s) { return t.sizes() == at::IntArrayRef(s.begin(), s.size()); }
 
+// float32 gradients as the features' type: bfloat16 ones in one launch, otherwise what the tensor library does
+void as_features(const Tensor& g0, const Tensor* g1, at::ScalarType ft, Tensor* out0, Tensor* out1) {
+  if (g0.scalar_type() == at::kFloat && ft == at::kBFloat16) {
+    const at::Device dev = g0.device();
+    if (out0) *out0 = fresh(g0.sizes(), ft, dev);
+    if (out1) *out1 = fresh(g1->sizes(), ft, dev);
+    check(chop_narrow_bf16(out0 ? g0.const_data_ptr<float>() : nullptr, out0 ? ptr(*out0) : nullptr, out0 ? g0.numel() : 0,
+                           out1 ? g1->const_data_ptr<float>() : nullptr, out1 ? ptr(*out1) : nullptr, out1 ? g1->numel() : 0,
+                           cuda_stream()),
+          "chop_narrow_bf16");
+    return;
+  }
+  if (out0) *out0 = g0.scalar_type() == ft ? g0 : g0.to(ft);
+  if (out1) *out1 = g1->scalar_type() == ft ? *g1 : g1->to(ft);
+}
+
 // A node with the inputs that its gradient needs.
 struct SavingNode : public Node {
   std::vector<SavedVariable> saved;
@@ -190,9 +206,7 @@ struct CvNode : public SavingNode {
     check(chop_cost_volume_bwd(&a.d, ptr(a.ref), ptr(a.src), ptr(a.depth), ptr(a.offsets), ptr(a.Rs), ptr(a.Ts), ptr(cg),
                                static_cast<const int32_t*>(ptr(mask)), ptr(rg), ptr(sg), ptr(dg), cuda_stream()),
           "chop_cost_volume_bwd");
-    const at::ScalarType ft = a.ref.scalar_type();
-    if (wanted(0)) out[0] = ft == a.real ? rg : rg.to(ft);
-    if (wanted(1)) out[1] = ft == a.real ? sg : sg.to(ft);
+    as_features(rg, &sg, a.ref.scalar_type(), wanted(0) ? &out[0] : nullptr, wanted(1) ? &out[1] : nullptr);
     out[2] = dg.sizes() == t[2].sizes() ? dg : dg.view_as(t[2]);
     return out;
   }
@@ -285,7 +299,7 @@ struct FaNode : public SavingNode {
           "chop_feature_aggregate_bwd");
     // gradients for src_images and base_plane only (reference: custom_helper_ops.py:192)
     const at::ScalarType ft = t[0].scalar_type(), bt = t[1].scalar_type();
-    if (wanted(0)) out[0] = ft == a.real ? sg : sg.to(ft);
+    if (wanted(0)) as_features(sg, nullptr, ft, &out[0], nullptr);
     if (wanted(1)) out[1] = bt == a.real ? bg : bg.to(bt);
     return out;
   }
@@ -415,7 +429,7 @@ struct ScNode : public SavingNode {
       if (conf.dynamic_default && wanted(2)) out[2] = dg.to(t[2].scalar_type());
     }
     if (wanted(0)) out[0] = ig;
-    if (wanted(1)) out[1] = fg.to(t[1].scalar_type());
+    if (wanted(1)) as_features(fg, nullptr, t[1].scalar_type(), &out[1], nullptr);
     return out;
   }
 };

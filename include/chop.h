@@ -255,6 +255,10 @@ CHOP_API int chop_umma_watch(void);
 CHOP_API int chop_copy_2d_async(void *dst, size_t dst_pitch, const void *src, size_t src_pitch, size_t width_bytes,
                                 size_t rows, void *stream);
 
+/* float32 -> bfloat16 (round to nearest even) of up to two buffers in one launch; n1 may be 0. */
+CHOP_API int chop_narrow_bf16(const float *src0, void *dst0, int64_t n0, const float *src1, void *dst1, int64_t n1,
+                              void *stream);
+
 /* Text for a status returned by any entry point (negative: chop_status, positive: CUDA). */
 CHOP_API const char *chop_status_string(int status);
 
