@@ -203,8 +203,9 @@ struct CvNode : public SavingNode {
     Tensor rg = fresh(a.ref.sizes(), a.real, a.ref.device());
     Tensor sg = fresh(a.src.sizes(), a.real, a.ref.device());
     Tensor dg = fresh(a.depth.sizes(), a.real, a.ref.device());
-    check(chop_cost_volume_bwd(&a.d, ptr(a.ref), ptr(a.src), ptr(a.depth), ptr(a.offsets), ptr(a.Rs), ptr(a.Ts), ptr(cg),
-                               static_cast<const int32_t*>(ptr(mask)), ptr(rg), ptr(sg), ptr(dg), cuda_stream()),
+    check(chop_cost_volume_bwd_saved(&a.d, ptr(a.ref), ptr(a.src), ptr(a.depth), ptr(a.offsets), ptr(a.Rs), ptr(a.Ts),
+                                     ptr(cg), static_cast<const int32_t*>(ptr(mask)), ptr(t[7]), ptr(rg), ptr(sg), ptr(dg),
+                                     cuda_stream()),
           "chop_cost_volume_bwd");
     as_features(rg, &sg, a.ref.scalar_type(), wanted(0) ? &out[0] : nullptr, wanted(1) ? &out[1] : nullptr);
     out[2] = dg.sizes() == t[2].sizes() ? dg : dg.view_as(t[2]);
@@ -221,7 +222,8 @@ std::tuple<Tensor, Tensor> cost_op(int kind, const std::string& reduce, int64_t 
       throw std::invalid_argument("Invalid reduce method " + reduce + ". Supported types: MEAN, MIN");
     const CvConf conf{kind, reduce == "MIN" ? CHOP_REDUCE_MIN : CHOP_REDUCE_MEAN, groups, half_centor};
     const Tensor offs = offsets ? *offsets : Tensor();
-    Tensor cost, mask;
+    const bool train = torch::autograd::compute_requires_grad(ref, src, depth, offs, Rs, Ts);
+    Tensor cost, mask, saved;   // saved: for the gradient only
     {
       at::AutoDispatchBelowADInplaceOrView below;
       const CvArgs a = cv_prepare(conf, ref, src, depth, offs, Rs, Ts);
@@ -235,14 +237,16 @@ std::tuple<Tensor, Tensor> cost_op(int kind, const std::string& reduce, int64_t 
         cost = fresh({d.B, d.H, d.W, d.D, cv_channels(a)}, a.real, dev);
         mask = fresh({d.B, d.H, d.W, d.D, cv_mask_channels(a)}, at::kInt, dev);
       }
-      check(chop_cost_volume_fwd(&d, ptr(a.ref), ptr(a.src), ptr(a.depth), ptr(a.offsets), ptr(a.Rs), ptr(a.Ts), ptr(cost),
-                                 static_cast<int32_t*>(ptr(mask)), cuda_stream()),
+      if (train && kind == CHOP_COST_VOLUME_V3)
+        if (const size_t n = chop_cost_volume_saved_bytes(&d)) saved = fresh({(int64_t)n}, at::kByte, dev);
+      check(chop_cost_volume_fwd_save(&d, ptr(a.ref), ptr(a.src), ptr(a.depth), ptr(a.offsets), ptr(a.Rs), ptr(a.Ts),
+                                      ptr(cost), static_cast<int32_t*>(ptr(mask)), ptr(saved), cuda_stream()),
             "chop_cost_volume_fwd");
     }
-    if (torch::autograd::compute_requires_grad(ref, src, depth, offs, Rs, Ts)) {
+    if (train) {
       auto node = make_node<CvNode>(ref, src, depth, offs, Rs, Ts);
       node->conf = conf;
-      node->save({ref, src, depth, offs, Rs, Ts, mask});
+      node->save({ref, src, depth, offs, Rs, Ts, mask, saved});
       torch::autograd::set_history(cost, node);
     }
     return std::make_tuple(cost, mask);

@@ -253,9 +253,23 @@ int chop_narrow_bf16(const float* src0, void* dst0, int64_t n0, const float* src
   return (int)cudaGetLastError();
 }
 
+size_t chop_cost_volume_saved_bytes(const chop_cv_desc* d) {
+  CvArgs a;
+  std::memset(&a, 0, sizeof(a));
+  Typed ty;
+  if (validate(d, &a, &ty) || d->kind != CHOP_COST_VOLUME_V3 || a.d_begin != 0 || a.d_end != a.D) return 0;
+  return chop::cv3_winner_bytes(d->dtype, d->reduce == CHOP_REDUCE_MIN, a);
+}
+
 int chop_cost_volume_fwd(const chop_cv_desc* d, const void* ref, const void* src, const void* depth,
                          const void* offsets, const void* Rs, const void* Ts, void* cost, int32_t* mask,
                          void* stream) {
+  return chop_cost_volume_fwd_save(d, ref, src, depth, offsets, Rs, Ts, cost, mask, nullptr, stream);
+}
+
+int chop_cost_volume_fwd_save(const chop_cv_desc* d, const void* ref, const void* src, const void* depth,
+                              const void* offsets, const void* Rs, const void* Ts, void* cost, int32_t* mask, void* saved,
+                              void* stream) {
   CvArgs a;
   std::memset(&a, 0, sizeof(a));
   Typed ty;
@@ -273,6 +287,7 @@ int chop_cost_volume_fwd(const chop_cv_desc* d, const void* ref, const void* src
     plan_chunks(&a, 1 << a.lg_log2, 148 * 64, 16, g_fwd_chunk.load());
     a.ref = ref; a.src = src; a.depth = depth; a.offsets = offsets; a.Rs = Rs; a.Ts = Ts;
     a.cost = cost; a.mask = mask;
+    if (saved && chop_cost_volume_saved_bytes(d)) a.winners = static_cast<unsigned char*>(saved);
     return chop::cv3_fwd_launch(d->dtype, d->reduce == CHOP_REDUCE_MIN, a, static_cast<cudaStream_t>(stream));
   }
   int cpl, lgl;
@@ -350,6 +365,14 @@ int chop_cost_volume_fwd(const chop_cv_desc* d, const void* ref, const void* src
 int chop_cost_volume_bwd(const chop_cv_desc* d, const void* ref, const void* src, const void* depth,
                          const void* offsets, const void* Rs, const void* Ts, const void* cost_grad,
                          const int32_t* mask, void* ref_grad, void* src_grad, void* depth_grad, void* stream) {
+  return chop_cost_volume_bwd_saved(d, ref, src, depth, offsets, Rs, Ts, cost_grad, mask, nullptr, ref_grad, src_grad,
+                                    depth_grad, stream);
+}
+
+int chop_cost_volume_bwd_saved(const chop_cv_desc* d, const void* ref, const void* src, const void* depth,
+                               const void* offsets, const void* Rs, const void* Ts, const void* cost_grad,
+                               const int32_t* mask, const void* saved, void* ref_grad, void* src_grad, void* depth_grad,
+                               void* stream) {
   CvArgs a;
   std::memset(&a, 0, sizeof(a));
   Typed ty;
@@ -375,6 +398,9 @@ int chop_cost_volume_bwd(const chop_cv_desc* d, const void* ref, const void* src
     a.ref = ref; a.src = src; a.depth = depth; a.offsets = offsets; a.Rs = Rs; a.Ts = Ts;
     a.cost_grad = cost_grad; a.mask = const_cast<int32_t*>(mask);
     a.ref_grad = ref_grad; a.src_grad = src_grad; a.depth_grad = depth_grad;
+    // the gradient by winners adds to ref_grad with 16-byte reductions
+    if (saved && aligned(ref_grad, 16) && chop_cost_volume_saved_bytes(d))
+      a.winners = static_cast<unsigned char*>(const_cast<void*>(saved));
     return chop::cv3_bwd_launch(d->dtype, d->reduce == CHOP_REDUCE_MIN, a, st3);
   }
   int cpl, lgl;

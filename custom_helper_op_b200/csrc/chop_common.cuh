@@ -191,6 +191,7 @@ struct CvArgs {
   void* ref_grad;
   void* src_grad;
   void* depth_grad;
+  unsigned char* winners;   // CostVolumeV3 MEAN: a byte per (pixel, view, plane), or null
   int B, H, W, C, D, N, Hs, Ws, G;
   int d_begin, d_end;
   int half_centor;

@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(256) cv3_bwd_kernel(const CvArgs a, const int 
 // footprint and reference group stay the same, so a plane costs the winning lane a dozen operations and the corner
 // reductions are made once per run instead of once per plane.
 // Bound: issue of the unfused multiplications and additions.  128x160x192, two views, C = 32, eight groups: forward 595 -> 320
-// us, gradient 916 -> 630 us.
+// us (353 when it records winners), gradient 916 -> 600 us; with recorded winners cv3_bwd_won takes the gradient.
 template <int G>
 struct V3Cfg {
   static constexpr int PX = 32 / G;      // pixels per warp, G lanes each
@@ -479,8 +479,10 @@ __device__ __forceinline__ void v3_dots(const V3Corner<T, SUB>& c00, const V3Cor
   }
 }
 
-template <typename T, int SUB, int G>
-__global__ void __launch_bounds__(128, 5) cv3_fwd_mean(const CvArgs a, const int smem_per_warp) {
+// WIN = true also records every (voxel, view)'s winner, a byte gs*G + gi at winners[pixel][view][plane] (255: none), for
+// cv3_bwd_won: the gradient then needs none of the G*G dot products.
+template <typename T, int SUB, int G, bool WIN>
+__global__ void __launch_bounds__(128, WIN ? 4 : 5) cv3_fwd_mean(const CvArgs a, const int smem_per_warp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typedef V3Cfg<G> Cf;
   constexpr int C = SUB * G, PX = Cf::PX, PB = Cf::PB, PL = Cf::PL;
@@ -517,23 +519,23 @@ __global__ void __launch_bounds__(128, 5) cv3_fwd_mean(const CvArgs a, const int
   __syncwarp();
 
   for (int dblk = dlo; dblk < dhi; dblk += PB) {
-    float acc[PB];
+    float acc[PL], depth[PL];   // of the planes p*G + li that this lane projects and finishes
     int used[PL];
-    float depth[PL];
-#pragma unroll
-    for (int j = 0; j < PB; ++j) acc[j] = 0.0f;
 #pragma unroll
     for (int p = 0; p < PL; ++p) {
+      acc[p] = 0.0f;
       used[p] = 0;
       depth[p] = xadd(base, offs[min(dblk + p * G + li, dhi - 1)]);
     }
     for (int n = 0; n < N; ++n) {
       const Coef<float> cf = coef[n * PX + g];
+      bool sees[PL];
 #pragma unroll
       for (int p = 0; p < PL; ++p) {
         float dh, dw, gh, gw, w00, w01, w11, w10;
         const int t = project<float, false>(cf, depth[p], a, dh, dw, gh, gw);
         bilinear_weights(dh, dw, w00, w01, w11, w10);
+        sees[p] = t >= 0;
         used[p] += t >= 0;
         const int slot = (p * G + li) * PX + g;
         wgt[2 * slot] = make_float4(w00, w00, w01, w01);
@@ -541,6 +543,8 @@ __global__ void __launch_bounds__(128, 5) cv3_fwd_mean(const CvArgs a, const int
         tex[slot] = t;
       }
       __syncwarp();
+      float best[PB];   // this source group's largest dot product, and with which reference group
+      int code[PB];
       int cur = -1;
       V3Corner<T, SUB> c00, c01, c10, c11;
 #pragma unroll
@@ -560,28 +564,57 @@ __global__ void __launch_bounds__(128, 5) cv3_fwd_mean(const CvArgs a, const int
         const ulonglong2 wB = *reinterpret_cast<const ulonglong2*>(wgt + 2 * (j * PX + g) + 1);
         pk2 val[G / 2];
         v3_dots<T, SUB, G>(c00, c01, c10, c11, wA, wB, ref, ones, val);
-        float m = Lim<float>::min_pos();   // :110
+        best[j] = Lim<float>::min_pos();   // :110
+        int gi = 0;
 #pragma unroll
         for (int p = 0; p < G / 2; ++p) {
           float x, y;
           pk_split(val[p], x, y);
-          m = fmaxf(m, fmaxf(x, y));
+          if (WIN) {   // the smallest reference group on ties
+            if (x > best[j]) { best[j] = x; gi = 2 * p; }
+            if (y > best[j]) { best[j] = y; gi = 2 * p + 1; }
+          } else {
+            best[j] = fmaxf(best[j], fmaxf(x, y));
+          }
         }
+        if (WIN) code[j] = li * G + gi;
+      }
+      // The lanes' maxima, reduced and scattered in one go for the block's planes: lane li ends up with planes p*G + li.
+      // (A butterfly per plane took three times the shuffles and left their latency in the plane loop.)  On ties the
+      // smaller code is the smaller source group's.
 #pragma unroll
-        for (int o = G >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (t >= 0) acc[j] = xadd(acc[j], m);   // :130
+      for (int o = G >> 1; o > 0; o >>= 1) {
+        const bool hi = (li & o) != 0;
+#pragma unroll
+        for (int p = 0; p < PL; ++p)
+#pragma unroll
+          for (int e = 0; e < G / 2; ++e) {
+            if (e >= o) continue;
+            const int x = p * G + e, y = x + o;
+            const float mine = hi ? best[y] : best[x], other = __shfl_xor_sync(0xffffffffu, hi ? best[x] : best[y], o);
+            if (WIN) {
+              const int cm = hi ? code[y] : code[x], co = __shfl_xor_sync(0xffffffffu, hi ? code[x] : code[y], o);
+              code[x] = other > mine || (other == mine && co < cm) ? co : cm;
+            }
+            best[x] = fmaxf(mine, other);
+          }
+      }
+#pragma unroll
+      for (int p = 0; p < PL; ++p) {
+        if (sees[p]) acc[p] = xadd(acc[p], best[p * G]);   // :130
+        if (WIN) {
+          const int d = dblk + p * G + li;
+          if (pvalid && d < dhi)
+            a.winners[(pix * N + n) * D + d] = (unsigned char)(sees[p] && best[p * G] > Lim<float>::min_pos() ? code[p * G] : 255);
+        }
       }
       __syncwarp();
     }
 #pragma unroll
     for (int p = 0; p < PL; ++p) {
-      float v = 0.0f;
-#pragma unroll
-      for (int i = 0; i < G; ++i)
-        if (li == i) v = acc[p * G + i];
       const int d = dblk + p * G + li;
       if (pvalid && d < dhi) {
-        static_cast<float*>(a.cost)[pix * D + d] = used[p] > 0 ? xdiv(v, (float)used[p]) : 0.0f;   // :136-141
+        static_cast<float*>(a.cost)[pix * D + d] = used[p] > 0 ? xdiv(acc[p], (float)used[p]) : 0.0f;   // :136-141
         a.mask[pix * D + d] = used[p];
       }
     }
@@ -793,17 +826,198 @@ __global__ void __launch_bounds__(128, 4) cv3_bwd_mean(const CvArgs a, const int
   if (pvalid && li == 0) atomicAdd(static_cast<float*>(a.depth_grad) + pix, dsum);   // :505
 }
 
+// Gradient with the winners that the forward pass recorded.  Lane (pixel g, source group li) takes the planes of the block
+// that its group won, in order, as a bit mask: corners are loaded only where a won plane's footprint differs from the last
+// one's, and a run of planes with the same footprint and reference group costs a plane a dozen operations.  Without the dot
+// products the reference pixel leaves the registers and twice as many warps are resident.
+// Bound: the load-store pipe (divergent corner loads and reductions).  128x160x192, two views, C = 32, eight groups: 600 us in
+// cv3_bwd_mean, 237 here (276 with d(ref) summed by shared-memory atomics instead of 16-byte reductions).
+template <int G>
+__host__ __device__ constexpr size_t v3_won_smem(int N, int C) {
+  typedef V3Cfg<G> Cf;
+  return (size_t)N * Cf::PX * sizeof(Coef<float>) + (size_t)Cf::PB * Cf::PX * (32 + 4 + 1) + (size_t)Cf::PX * C * 4;
+}
+template <typename T, int SUB, int G>
+__global__ void __launch_bounds__(128, SUB == 8 ? 5 : G == 8 ? 8 : 6) cv3_bwd_won(const CvArgs a, const int smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef V3Cfg<G> Cf;
+  constexpr int C = SUB * G, PX = Cf::PX, PB = Cf::PB, PL = Cf::PL;
+  constexpr int GB = G == 2 ? 1 : G == 4 ? 2 : 3;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int li = lane & (G - 1), g = lane / G;
+  const long long item = (long long)blockIdx.x * 4 + wib;
+  if (item >= (long long)a.npb * a.nchunks) return;
+  const int chunk_id = (int)(item / a.npb);
+  const long long pix0 = (item - (long long)chunk_id * a.npb) * PX;
+  const bool pvalid = pix0 + g < a.npix;
+  const long long pix = pvalid ? pix0 + g : a.npix - 1;
+  const int dlo = a.d_begin + chunk_id * a.chunk, dhi = min(a.d_end, dlo + a.chunk);
+  const int N = a.N, D = a.D;
+  unsigned char* mine = smem_raw + (size_t)wib * smem_per_warp;
+  Coef<float>* coef = reinterpret_cast<Coef<float>*>(mine);                       // [N][PX]
+  float4* aux = reinterpret_cast<float4*>(coef + N * PX);                         // [PB][PX][2] {dw, dh, cg, -} {gh*cg, gw*cg, -, -}
+  float* refs = reinterpret_cast<float*>(aux + 2 * PB * PX);                      // [PX][C]
+  int* tex = reinterpret_cast<int*>(refs + PX * C);                               // [PB][PX]
+  unsigned char* winb = reinterpret_cast<unsigned char*>(tex + PB * PX);          // [PX][PB]
+  stage_coefs<float>(a, coef, lane, PX, pix0);
+  for (int e = lane; e < PX * C; e += 32) {
+    long long p = pix0 + e / C;
+    if (p >= a.npix) p = a.npix - 1;
+    refs[e] = ld1<T, float>(static_cast<const T*>(a.ref) + p * C + (e % C));
+  }
+  __syncwarp();
+  const float* refp = refs + g * C;
+  float* rgp = static_cast<float*>(a.ref_grad) + pix * C;
+  const int b = (int)(pix / ((long long)a.H * a.W));
+  const float base = static_cast<const float*>(a.depth)[pix];
+  const float* offs = static_cast<const float*>(a.offsets) + (long long)b * D;
+  const T* src_lane = static_cast<const T*>(a.src) + li * SUB;
+  float* sg_lane = static_cast<float*>(a.src_grad) + li * SUB;
+  const size_t row = (size_t)a.Ws * C;
+  float dsum = 0.0f;
+
+  int m_next[PL];
+  float cg_next[PL];
+  auto stream = [&](int d0) {   // the next block's validity counts and upstream values
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      const int d = d0 + p * G + li;
+      m_next[p] = 0;
+      cg_next[p] = 0.0f;
+      if (pvalid && d < dhi) {
+        m_next[p] = __ldg(a.mask + pix * D + d);
+        cg_next[p] = __ldg(static_cast<const float*>(a.cost_grad) + pix * D + d);
+      }
+    }
+  };
+  stream(dlo);
+  for (int dblk = dlo; dblk < dhi; dblk += PB) {
+    int m_cur[PL];
+    float cg[PL], depth[PL];
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      m_cur[p] = m_next[p];
+      cg[p] = m_cur[p] > 0 ? cg_next[p] / (float)m_cur[p] : 0.0f;   // :393, :426
+      depth[p] = xadd(base, offs[min(dblk + p * G + li, dhi - 1)]);
+    }
+    stream(dblk + PB);
+    for (int n = 0; n < N; ++n) {
+      const Coef<float> cf = coef[n * PX + g];
+      int wv[PL];
+#pragma unroll
+      for (int p = 0; p < PL; ++p) {
+        const int d = dblk + p * G + li;
+        wv[p] = pvalid && d < dhi ? __ldg(a.winners + (pix * N + n) * D + d) : 255;
+      }
+#pragma unroll
+      for (int p = 0; p < PL; ++p) {
+        float dh = 0.0f, dw = 0.0f, gh = 0.0f, gw = 0.0f;
+        int t = -1;
+        if (m_cur[p] > 0) t = project<float, true>(cf, depth[p], a, dh, dw, gh, gw);
+        const int slot = (p * G + li) * PX + g;
+        aux[2 * slot] = make_float4(dw, dh, cg[p], 0.0f);
+        *reinterpret_cast<float2*>(aux + 2 * slot + 1) = make_float2(gh * cg[p], gw * cg[p]);
+        tex[slot] = t;
+        winb[g * PB + p * G + li] = t >= 0 ? (unsigned char)wv[p] : (unsigned char)255;
+      }
+      __syncwarp();
+
+      unsigned todo = 0;   // planes that this lane's source group won
+      const uint2 w8 = *reinterpret_cast<const uint2*>(winb + g * PB);
+#pragma unroll
+      for (int j = 0; j < PB; ++j) {
+        const unsigned w = ((j < 4 ? w8.x : w8.y) >> (8 * (j & 3))) & 0xffu;
+        todo |= (w >> GB) == (unsigned)li ? 1u << j : 0u;
+      }
+      int cur = -1, gi_run = -1;
+      float e00[SUB], e01[SUB], e10[SUB], e11[SUB];
+      // moments of the upstream gradient over the run, and d(correlation)/d(sample position) of the run's group pair
+      float m0 = 0.0f, m1 = 0.0f, m2 = 0.0f, m3 = 0.0f, P = 0.0f, Q = 0.0f, S = 0.0f;
+      auto flush = [&]() {
+        const float k01 = m1 - m3, k10 = m2 - m3, k00 = (m0 - m1) - k10;
+        float* g00 = sg_lane + (size_t)cur * C;
+#pragma unroll
+        for (int q = 0; q < SUB; q += 4) {
+          const float4 rv = *reinterpret_cast<const float4*>(refp + gi_run * SUB + q);
+          const float r4[4] = {rv.x, rv.y, rv.z, rv.w};
+          float o[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)   // :490
+            o[k] = fmaf(k00, e00[q + k], fmaf(k01, e01[q + k], fmaf(k10, e10[q + k], m3 * e11[q + k])));
+          red_add<float, 4>(rgp + gi_run * SUB + q, o);   // lanes of a pixel may share the reference group
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = k00 * r4[k];   // :491-495
+          red_add<float, 4>(g00 + q, o);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = k01 * r4[k];
+          red_add<float, 4>(g00 + C + q, o);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = k10 * r4[k];
+          red_add<float, 4>(g00 + row + q, o);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = m3 * r4[k];
+          red_add<float, 4>(g00 + row + C + q, o);
+        }
+      };
+      while (todo) {
+        const int j = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int t = tex[j * PX + g], gi = winb[g * PB + j] & (G - 1);
+        if (t != cur || gi != gi_run) {
+          if (gi_run >= 0) flush();
+          if (t != cur) {
+            cur = t;
+            const T* p = src_lane + (size_t)t * C;
+#pragma unroll
+            for (int q = 0; q < SUB; q += 4) {
+              Vec<T, float, 4>::load(p + q, e00 + q);
+              Vec<T, float, 4>::load(p + C + q, e01 + q);
+              Vec<T, float, 4>::load(p + row + q, e10 + q);
+              Vec<T, float, 4>::load(p + row + C + q, e11 + q);
+            }
+          }
+          gi_run = gi;
+          m0 = m1 = m2 = m3 = 0.0f;
+          P = Q = S = 0.0f;
+#pragma unroll
+          for (int k = 0; k < SUB; ++k) {
+            const float r = refp[gi * SUB + k];
+            P = fmaf(r, (e11[k] - e10[k]) - (e01[k] - e00[k]), P);   // :498
+            Q = fmaf(r, e10[k] - e00[k], Q);
+            S = fmaf(r, e01[k] - e00[k], S);
+          }
+        }
+        const float4 x = aux[2 * (j * PX + g)];
+        const float2 y = *reinterpret_cast<const float2*>(aux + 2 * (j * PX + g) + 1);
+        const float cd = x.z * x.x;
+        m0 += x.z;
+        m1 += cd;
+        m2 = fmaf(x.z, x.y, m2);
+        m3 = fmaf(cd, x.y, m3);
+        dsum = fmaf(y.x, fmaf(x.x, P, Q), fmaf(y.y, fmaf(x.y, P, S), dsum));   // :502
+      }
+      if (gi_run >= 0) flush();
+      __syncwarp();
+    }
+  }
+#pragma unroll
+  for (int o = G >> 1; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+  if (pvalid && li == 0) atomicAdd(static_cast<float*>(a.depth_grad) + pix, dsum);   // :505
+}
+
 template <typename T, bool BWD, int SUB, int G>
 int launch_mean(const CvArgs& a0, cudaStream_t st) {
   typedef V3Cfg<G> Cf;
   CvArgs a = a0;
   a.chunk = (a.chunk + Cf::PB - 1) / Cf::PB * Cf::PB;   // whole blocks of planes
   a.nchunks = (a.d_end - a.d_begin + a.chunk - 1) / a.chunk;
-  const size_t spw = (v3_mean_smem<G>(a.N, SUB * G, BWD) + 15) & ~(size_t)15;
+  const bool won = a.winners != nullptr;
+  const size_t spw = ((BWD && won ? v3_won_smem<G>(a.N, SUB * G) : v3_mean_smem<G>(a.N, SUB * G, BWD)) + 15) & ~(size_t)15;
   if (spw * 4 > 200 * 1024) return -4;
   const long long blocks = ((long long)a.npb * a.nchunks + 3) / 4;
   if (blocks > 0x7fffffffLL) return -2;   // CHOP_ERR_SHAPE
-  auto k = BWD ? cv3_bwd_mean<T, SUB, G> : cv3_fwd_mean<T, SUB, G>;
+  auto k = BWD ? (won ? cv3_bwd_won<T, SUB, G> : cv3_bwd_mean<T, SUB, G>)
+               : (won ? cv3_fwd_mean<T, SUB, G, true> : cv3_fwd_mean<T, SUB, G, false>);
   if (int e = grant_smem(k, spw * 4)) return e;
   k<<<(unsigned)blocks, 128, spw * 4, st>>>(a, (int)spw);
   return (int)cudaGetLastError();
@@ -855,6 +1069,15 @@ int dispatch(int dtype, bool rmin, const CvArgs& a, cudaStream_t st) {
 }
 
 }  // namespace
+
+// one byte per (voxel, view) where launch_mean takes the forward pass and the gradient
+size_t cv3_winner_bytes(int dtype, bool rmin, const CvArgs& a) {
+  const int sub = a.C / a.G;
+  if (rmin || dtype == 1 || !((sub == 4 && (a.G == 2 || a.G == 4 || a.G == 8)) || (sub == 8 && (a.G == 2 || a.G == 4)))) return 0;
+  const size_t most = 4 * (a.G == 2 ? v3_mean_smem<2>(a.N, a.C, true) : a.G == 4 ? v3_mean_smem<4>(a.N, a.C, true)
+                                                                                 : v3_mean_smem<8>(a.N, a.C, true));
+  return most + 64 > 200 * 1024 ? 0 : (size_t)a.npix * a.N * a.D;
+}
 
 int cv3_fwd_launch(int dtype, bool rmin, const CvArgs& a, cudaStream_t st) { return dispatch<false>(dtype, rmin, a, st); }
 int cv3_bwd_launch(int dtype, bool rmin, const CvArgs& a, cudaStream_t st) { return dispatch<true>(dtype, rmin, a, st); }

@@ -119,6 +119,19 @@ CHOP_API int chop_cost_volume_bwd(const chop_cv_desc *desc, const void *ref, con
                          const int32_t *mask, void *ref_grad, void *src_grad, void *depth_grad,
                          void *stream);
 
+/* A training step's forward pass and gradient may hand over what the gradient would otherwise work out again: a device
+ * buffer of chop_cost_volume_saved_bytes(desc) bytes that _fwd_save fills and _bwd_saved reads with the same desc and
+ * inputs (CostVolumeV3 MEAN: each (voxel, view)'s winning pair of groups, one byte).  0: this call saves nothing.
+ * `saved` may be NULL; the calls then are chop_cost_volume_fwd / _bwd. */
+CHOP_API size_t chop_cost_volume_saved_bytes(const chop_cv_desc *desc);
+CHOP_API int chop_cost_volume_fwd_save(const chop_cv_desc *desc, const void *ref, const void *src, const void *depth,
+                         const void *offsets, const void *Rs, const void *Ts, void *cost, int32_t *mask, void *saved,
+                         void *stream);
+CHOP_API int chop_cost_volume_bwd_saved(const chop_cv_desc *desc, const void *ref, const void *src, const void *depth,
+                         const void *offsets, const void *Rs, const void *Ts, const void *cost_grad,
+                         const int32_t *mask, const void *saved, void *ref_grad, void *src_grad, void *depth_grad,
+                         void *stream);
+
 /* Describes one manifold ("sparse") 3-D convolution call.  Replaces the reference's SparseConv3DFastParams
  * (custom_helper_op/cc/kernels/sparse_conv3d_fast_op.h:26-49); output extents are ceil(input/stride) and
  * the left padding is (filter/2)*dilation as in sparse_conv3d_fast_op.cc:104-109.
