@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(256) cv3_bwd_kernel(const CvArgs a, const int 
 // footprint and reference group stay the same, so a plane costs the winning lane a dozen operations and the corner
 // reductions are made once per run instead of once per plane.
 // Bound: issue of the unfused multiplications and additions.  128x160x192, two views, C = 32, eight groups: forward 595 -> 320
-// us (353 when it records winners), gradient 916 -> 600 us; with recorded winners cv3_bwd_won takes the gradient.
+// us (340 when it records winners), gradient 916 -> 600 us; with recorded winners cv3_bwd_won takes the gradient.
 template <int G>
 struct V3Cfg {
   static constexpr int PX = 32 / G;      // pixels per warp, G lanes each
@@ -482,7 +482,7 @@ __device__ __forceinline__ void v3_dots(const V3Corner<T, SUB>& c00, const V3Cor
 // WIN = true also records every (voxel, view)'s winner, a byte gs*G + gi at winners[pixel][view][plane] (255: none), for
 // cv3_bwd_won: the gradient then needs none of the G*G dot products.
 template <typename T, int SUB, int G, bool WIN>
-__global__ void __launch_bounds__(128, WIN ? 4 : 5) cv3_fwd_mean(const CvArgs a, const int smem_per_warp) {
+__global__ void __launch_bounds__(128, 4) cv3_fwd_mean(const CvArgs a, const int smem_per_warp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typedef V3Cfg<G> Cf;
   constexpr int C = SUB * G, PX = Cf::PX, PB = Cf::PB, PL = Cf::PL;
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(128, WIN ? 4 : 5) cv3_fwd_mean(const CvArgs a,
       }
       __syncwarp();
       float best[PB];   // this source group's largest dot product, and with which reference group
-      int code[PB];
+      unsigned gis = 0;   // 4 bits a plane
       int cur = -1;
       V3Corner<T, SUB> c00, c01, c10, c11;
 #pragma unroll
@@ -564,24 +564,26 @@ __global__ void __launch_bounds__(128, WIN ? 4 : 5) cv3_fwd_mean(const CvArgs a,
         const ulonglong2 wB = *reinterpret_cast<const ulonglong2*>(wgt + 2 * (j * PX + g) + 1);
         pk2 val[G / 2];
         v3_dots<T, SUB, G>(c00, c01, c10, c11, wA, wB, ref, ones, val);
-        best[j] = Lim<float>::min_pos();   // :110
-        int gi = 0;
+        float v[G];
 #pragma unroll
-        for (int p = 0; p < G / 2; ++p) {
-          float x, y;
-          pk_split(val[p], x, y);
-          if (WIN) {   // the smallest reference group on ties
-            if (x > best[j]) { best[j] = x; gi = 2 * p; }
-            if (y > best[j]) { best[j] = y; gi = 2 * p + 1; }
-          } else {
-            best[j] = fmaxf(best[j], fmaxf(x, y));
-          }
+        for (int p = 0; p < G / 2; ++p) pk_split(val[p], v[2 * p], v[2 * p + 1]);
+        best[j] = Lim<float>::min_pos();   // :110
+#pragma unroll
+        for (int p = 0; p < G; p += 2) best[j] = fmaxf(best[j], fmaxf(v[p], v[p + 1]));
+        if (WIN) {   // the smallest reference group that has it; compares that wait for nothing but the maximum
+          unsigned gi = (G - 1u) << (4 * j);
+#pragma unroll
+          for (int p = G - 2; p >= 0; --p) gi = v[p] == best[j] ? (unsigned)p << (4 * j) : gi;
+          gis |= gi;
         }
-        if (WIN) code[j] = li * G + gi;
       }
       // The lanes' maxima, reduced and scattered in one go for the block's planes: lane li ends up with planes p*G + li.
-      // (A butterfly per plane took three times the shuffles and left their latency in the plane loop.)  On ties the
-      // smaller code is the smaller source group's.
+      // (A butterfly per plane took three times the shuffles and left their latency in the plane loop.)  `from` is the lane,
+      // i.e. the source group, that has the maximum: the smaller one on ties.  Its reference group is fetched at the end.
+      int from[PB];
+      if (WIN)
+#pragma unroll
+        for (int j = 0; j < PB; ++j) from[j] = li;
 #pragma unroll
       for (int o = G >> 1; o > 0; o >>= 1) {
         const bool hi = (li & o) != 0;
@@ -593,8 +595,9 @@ __global__ void __launch_bounds__(128, WIN ? 4 : 5) cv3_fwd_mean(const CvArgs a,
             const int x = p * G + e, y = x + o;
             const float mine = hi ? best[y] : best[x], other = __shfl_xor_sync(0xffffffffu, hi ? best[x] : best[y], o);
             if (WIN) {
-              const int cm = hi ? code[y] : code[x], co = __shfl_xor_sync(0xffffffffu, hi ? code[x] : code[y], o);
-              code[x] = other > mine || (other == mine && co < cm) ? co : cm;
+              const int fm = hi ? from[y] : from[x];
+              const int fo = o == G >> 1 ? li ^ o : __shfl_xor_sync(0xffffffffu, hi ? from[x] : from[y], o);
+              from[x] = other > mine || (other == mine && fo < fm) ? fo : fm;
             }
             best[x] = fmaxf(mine, other);
           }
@@ -603,9 +606,10 @@ __global__ void __launch_bounds__(128, WIN ? 4 : 5) cv3_fwd_mean(const CvArgs a,
       for (int p = 0; p < PL; ++p) {
         if (sees[p]) acc[p] = xadd(acc[p], best[p * G]);   // :130
         if (WIN) {
-          const int d = dblk + p * G + li;
+          const unsigned w = __shfl_sync(0xffffffffu, gis, lane - li + from[p * G]);
+          const int d = dblk + p * G + li, code = from[p * G] * G + (int)((w >> (4 * (p * G + li))) & 15u);
           if (pvalid && d < dhi)
-            a.winners[(pix * N + n) * D + d] = (unsigned char)(sees[p] && best[p * G] > Lim<float>::min_pos() ? code[p * G] : 255);
+            a.winners[(pix * N + n) * D + d] = (unsigned char)(sees[p] && best[p * G] > Lim<float>::min_pos() ? code : 255);
         }
       }
       __syncwarp();
