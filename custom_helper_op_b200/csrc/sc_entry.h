@@ -28,6 +28,12 @@ int sc_tile_gather_launch(int dtype, const ScArgs& a, cudaStream_t st);
 // sums nparts slabs of taps*KC*NC + 1 floats; default_grad may be null
 int sc_slab_reduce(const float* part, int nparts, int taps, int KC, int NC, bool transposed, float* filter_grad,
                    float* default_grad, cudaStream_t st);
+// stride 1 with every voxel staged once per tile (sc_band.cu); cin: gathered channels, cout: produced ones
+bool sc_band_better(const ScArgs& a, int cin, int cout);
+int sc_band_launch(const ScArgs& a, bool dgrad, cudaStream_t st);
+int sc_band_timeouts();
+int sc_band_publish_mirror(int* dptr);
+int sc_band_clear_timeouts();
 int sc_umma_timeouts();
 int sc_umma_watch();
 int sc_umma_note_timeout_for_test(int on);

@@ -1,4 +1,4 @@
-// Opt-in to more than 48 KB of dynamic shared memory is a per-(device, kernel) attribute.  grant_smem sets it
+// Opt-in to more than 48 KB of shared memory, static and dynamic together, is a per-(device, kernel) attribute.  grant_smem sets it
 // the first time a launch of that kernel on that device needs that much, not on every call; the table of what
 // has been granted is the only state it keeps (process-wide, guarded by a mutex, a few entries).
 #pragma once
@@ -12,7 +12,7 @@ namespace chop {
 
 template <typename K>
 inline int grant_smem(K kernel, size_t smem) {
-  if (smem <= 48 * 1024) return 0;
+  if (smem <= 40 * 1024) return 0;   // no kernel here has more than 8 KB of static shared memory
   static std::mutex mu;
   static std::map<std::pair<int, const void*>, size_t> granted;
   int dev = 0;
