@@ -13,7 +13,7 @@
 
 namespace chop {
 std::atomic<int> g_use_umma{1};  // tuning knob "umma": 0 forces the generic kernels
-std::atomic<int> g_use_tile{1};  // tuning knob "tile": 0 = never the register-tiled float32 kernels
+std::atomic<int> g_use_tile{1};  // tuning knob "tile": 0 = never the register-tiled float32 kernels, 2 = never those of sc_run.cu and sc_band.cu
 }
 
 namespace {
@@ -27,6 +27,8 @@ inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) =
 int run_fwd(int dtype, const ScArgs& a, cudaStream_t st) {
   if (chop::g_use_umma.load() && chop::sc_umma_supported(dtype, a) && al16(a.images) && al16(a.output) && al16(a.filters))
     return chop::sc_umma_fwd_launch(a, st);
+  if (chop::g_use_tile.load() == 1 && chop::sc_run_supported(dtype, a, a.Cin) && al16(a.images) && al16(a.output))
+    return chop::sc_run_launch(a, false, st);
   if (chop::g_use_tile.load() && chop::sc_tile_supported(dtype, a) && al16(a.images) && al16(a.output) && al16(a.filters))
     return chop::sc_tile_fwd_launch(dtype, a, st);
   return chop::sc_fwd_simt_launch(dtype, a, st);
@@ -48,6 +50,8 @@ int run_dgrad(int dtype, const ScArgs& in, cudaStream_t st) {
   a.pad_zero = 1;  // a padded tap contributes nothing to the image gradient (sparse_conv3d_fast_op.cc:306,321)
   if (chop::g_use_umma.load() && chop::sc_umma_supported(dtype, a) && al16(a.out_grad) && al16(a.images_grad) && al16(a.filters))
     return chop::sc_umma_dgrad_launch(a, st);
+  if (chop::g_use_tile.load() == 1 && chop::sc_run_supported(dtype, a, a.Cout) && al16(a.out_grad) && al16(a.images_grad))
+    return chop::sc_run_launch(a, true, st);
   if (chop::g_use_tile.load() && chop::sc_tile_supported(dtype, a) && al16(a.out_grad) && al16(a.images_grad) && al16(a.filters))
     return chop::sc_tile_gather_launch(dtype, a, st);
   return chop::sc_dgrad_simt_launch(dtype, a, st);
@@ -175,6 +179,8 @@ int chop_sparse_conv3d_transpose_fwd(const chop_sc_desc* d, const void* images, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (chop::g_use_umma.load() && chop::sc_umma_supported(d->dtype, a) && al16(a.out_grad) && al16(a.images_grad) && al16(a.filters))
     return chop::sc_umma_dgrad_launch(a, st);
+  if (chop::g_use_tile.load() == 1 && chop::sc_run_supported(d->dtype, a, a.Cout) && al16(a.out_grad) && al16(a.images_grad))
+    return chop::sc_run_launch(a, true, st);
   if (chop::g_use_tile.load() && chop::sc_tile_supported(d->dtype, a) && al16(a.out_grad) && al16(a.images_grad) && al16(a.filters))
     return chop::sc_tile_gather_launch(d->dtype, a, st);
   return chop::sc_tconv_simt_launch(d->dtype, a, st);

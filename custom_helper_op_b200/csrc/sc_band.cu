@@ -1,5 +1,5 @@
-// Stride-1 manifold convolution on the tensor cores with every voxel staged ONCE per tile: 3x3x3, dilation 1, bfloat16
-// storage, float32 accumulation, 8, 16 or 32 channels, bands of up to 24 planes.
+// Stride-1 manifold convolution on the tensor cores with every voxel staged ONCE per tile: 3x3x3, dilation 1, bands of up to 24
+// planes; bfloat16 with 8, 16 or 32 channels, and float32 (in three bfloat16 pieces, below) where that pays; float32 accumulation.
 //
 // sc_umma_rows_kernel (sc_umma.cu) stages each neighbour pixel nine times, once per filter column, because a column's rows
 // have to be shifted by base_plane[pixel] - base_plane[neighbour].  In ABSOLUTE depth there is no shift: here a tile is
@@ -20,6 +20,13 @@
 // MMA operands) and, with four CTAs an SM, a tile's chain of staging, MMAs and epilogue.  256x320x9, 3x3x3, bfloat16, us:
 // 16 -> 16 channels 59 -> 41, 8 -> 8 51 -> 33, 32 -> 32 213 -> 100, 32 -> 16 129 -> 74; at 17 planes 97 -> 72, 344 -> 182.
 // Tiles of four rows with 256 threads: 45; of one row: 49; windows that do not divide 32 rows (25 for 17 planes): 108.
+//
+// float32: a value is the exact sum of three bfloat16 pieces, x = x1 + x2 + x3, and x*w the sum of the six products
+// x1w1, x1w2, x2w1, x1w3, x2w2, x3w1 (what is left out is below 2^-24 of it).  Steps whose values are not finite or all tiny are
+// computed by plain multiply-adds (band_plain).  189x251x7, 16 -> 16 channels: 150 us with a thread per four voxels (sc_tile.cu),
+// 127 in runs of planes (sc_run.cu), 88 here; 16 -> 32 334, 238, 166.  Bound: 79 % of the shared-memory data pipe (operands 38,
+// load-store 41) at eight warps an SM; with a quarter of the MMAs 72 us, without the loads 90, without splitting 85.  Three
+// groups of four warps around one filter 92 us, a thread per four channels instead of eight 99.
 #include "sc_entry.h"
 #include "sc_umma_common.cuh"
 #include "smem_grant.h"
@@ -28,46 +35,144 @@ namespace chop {
 namespace {
 
 // RP: rows of a pixel's window.  R: image rows of a tile.
-// One where two would leave room for two CTAs only (tensor memory: R*3*channels of 512 columns): 16 -> 32 channels 64 us
-// with one, 74 with two; 32 -> 32, where shared memory allows two CTAs anyway, 131 and 100.
-constexpr int band_tile_rows(int cr, int nr) { return nr > 16 && cr <= 16 ? 1 : 2; }
-template <int CR, int NR, int RP> struct BandGeo {
+// bfloat16: one where two would leave room for two CTAs only (tensor memory: R*3*channels of 512 columns): 16 -> 32 channels
+// 64 us with one, 74 with two; 32 -> 32, where shared memory allows two CTAs anyway, 131 and 100.  float32: one (three pieces).
+template <typename T> struct BandType;
+template <> struct BandType<__nv_bfloat16> {
+  static constexpr int P = 1;
+  static constexpr int rows(int cr, int nr) { return nr > 16 && cr <= 16 ? 1 : 2; }
+};
+template <> struct BandType<float> {
+  static constexpr int P = 3;
+  static constexpr int rows(int, int) { return 1; }
+};
+template <typename T, int CR, int NR, int RP> struct BandGeo {
+  static constexpr int P = BandType<T>::P;            // bfloat16 pieces of a value
   static constexpr int PT = 128 / RP;                 // pixels of an image row that make one MMA block
-  static constexpr int R = band_tile_rows(CR, NR);        // MMA blocks of a tile
-  static constexpr int NTHR = 128;                     // one thread per accumulator row
+  static constexpr int R = BandType<T>::rows(CR, NR); // MMA blocks of a tile
   static constexpr int PW = PT + 2, NPIX = (R + 2) * PW;
   static constexpr int ROWS = NPIX * RP;              // staged rows
   static constexpr int NRB = ROWS + 4;                // K-chunk stride 64 bytes off a multiple of 128 (bank conflicts)
   static constexpr int CG = ROWS / 128;               // filter columns per step of a rough tile
   static constexpr int GROUPS = (9 + CG - 1) / CG;
-  static constexpr size_t SMEM = (size_t)27 * pad16(NR) * pad16(CR) * 2 + (size_t)(pad16(CR) / 8) * NRB * 16 + 1024;
-  static constexpr uint32_t TMEM = R * 3 * pad16(NR) <= 64 ? 64 : R * 3 * pad16(NR) <= 128 ? 128 : 256;
-  static constexpr int BY_SMEM = (int)((size_t)220 * 1024 / (SMEM + 2048)), BY_TMEM = 512 / TMEM;
-  static constexpr int CTAS = BY_SMEM < BY_TMEM ? BY_SMEM : BY_TMEM;
-  static_assert(PT * RP == 128 && 32 % RP == 0 && ROWS % 8 == 0 && NPIX <= NTHR && R * PT <= 32 && R * 3 * pad16(NR) <= 256, "tile");
+  static constexpr int FILTER = P * 27 * pad16(NR) * pad16(CR) * 2;
+  static constexpr size_t SMEM = (size_t)FILTER + (size_t)P * (pad16(CR) / 8) * NRB * 16 + 1024;
+  static constexpr int COLS = R * P * 3 * pad16(NR);  // accumulators
+  static constexpr uint32_t TMEM = COLS <= 64 ? 64 : COLS <= 128 ? 128 : 256;
+  static constexpr int BY_SMEM = (int)((size_t)224 * 1024 / (SMEM + 2048)), BY_TMEM = 512 / TMEM;
+  static constexpr int CTAS = BY_SMEM < 1 ? 1 : BY_SMEM < BY_TMEM ? BY_SMEM : BY_TMEM;
+  static_assert(PT * RP == 128 && 32 % RP == 0 && ROWS % 8 == 0 && NPIX <= 128 && R * PT <= 32 && COLS <= 256 && (P == 1 || R == 1), "tile");
 };
 
-template <int CR, int NR, bool DGRAD, int RP>
-__global__ void __launch_bounds__(BandGeo<CR, NR, RP>::NTHR, BandGeo<CR, NR, RP>::CTAS)
+// Eight float32 values as three bfloat16 pieces each, by truncation: x = x1 + x2 + x3 exactly (8 + 8 + 8 significant bits).
+__device__ __forceinline__ void split3(const float (&v)[8], unsigned (&p)[3][4]) {
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    unsigned hi[3][2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float r = v[i + j];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        hi[q][j] = __float_as_uint(r) & 0xffff0000u;
+        if (q < 2) r = __fsub_rn(r, __uint_as_float(hi[q][j]));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) p[q][i / 2] = __byte_perm(hi[q][0], hi[q][1], 0x7632);
+  }
+}
+// Largest magnitude, as bits.  Values of which it is not finite, or not zero and below 2^-50, are not for the pieces: an
+// infinity times a zero piece is not a number, and products of low pieces would fall below the normal range.
+__device__ __forceinline__ unsigned top_bits(const float (&v)[8]) {
+  unsigned m = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
+  return m;
+}
+__device__ __forceinline__ bool not_for_pieces(unsigned top) { return top >= 0x7f800000u || (top != 0 && top < 0x26800000u); }
+
+// The filter in three pieces: tile [filter column][filter row][piece][depth tap], each as in stage_filter_tiles; channels n0 ..
+// n0 + NR - 1 of NF produced ones.  Returns the largest magnitude that this thread has seen.
+template <int CR, int NR, int NF, bool DGRAD>
+__device__ __forceinline__ unsigned stage_filter_pieces(const float* flt, int n0, unsigned char* sB, int tid, uint32_t lbo, uint32_t sbo, int tap_bytes) {
+  constexpr int COUT = pad16(NR), KC = pad16(CR) / 8;
+  unsigned top = 0;
+#pragma unroll 1
+  for (int e = tid; e < 27 * COUT * KC; e += 128) {
+    const int kg = e % KC, n = (e / KC) % COUT, t = e / (KC * COUT);
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = kg * 8 + i;
+      v[i] = kg * 8 >= CR || n >= NR ? 0.f
+             : __ldg(DGRAD ? flt + ((size_t)(26 - t) * NF + n0 + n) * CR + k : flt + ((size_t)t * CR + k) * NF + n0 + n);
+    }
+    top = max(top, top_bits(v));
+    unsigned p[3][4];
+    split3(v, p);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int slot = ((t / 3 % 3 * 3 + t / 9) * 3 + q) * 3 + t % 3;
+      *reinterpret_cast<uint4*>(sB + slot * tap_bytes + (n / 8) * sbo + kg * lbo + (n % 8) * 16) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+    }
+  }
+  return top;
+}
+
+// The same sums by plain multiply-adds, for a step whose values are not for the pieces: output pixels `todo` of image row r.
+template <int CR, int NR, int NF, bool DGRAD>
+__device__ __noinline__ void band_plain(const ScArgs& a, const int2* tab, int pw, int r, unsigned todo, int n0, float pad) {
+  const float* src = static_cast<const float*>(DGRAD ? a.out_grad : a.images);
+  const float* flt = static_cast<const float*>(a.filters);
+  float* dst = static_cast<float*>(DGRAD ? a.images_grad : a.output);
+  const int D = a.D;
+  for (; todo; todo &= todo - 1) {
+    const int q = __ffs(todo) - 1;
+    const int2 o = tab[(r + 1) * pw + q + 1];
+    for (int e = threadIdx.x & 127; e < D * NR; e += 128) {
+      const int n = n0 + e % NR, d = e / NR;
+      float s = 0.f;
+      for (int t = 0; t < 27; ++t) {
+        const int2 nb = tab[(r + t / 9) * pw + q + t / 3 % 3];
+        const int plane = d + o.y - nb.y - 1 + t % 3;
+        const bool in = nb.x >= 0 && !oob(plane, D);
+        if (!in && pad == 0.f) continue;
+        for (int k = 0; k < CR; ++k) {
+          const float x = in ? __ldg(src + ((size_t)nb.x + plane) * CR + k) : pad;
+          s = fmaf(x, __ldg(DGRAD ? flt + ((size_t)(26 - t) * NF + n) * CR + k : flt + ((size_t)t * CR + k) * NF + n), s);
+        }
+      }
+      dst[((size_t)o.x + d) * NF + n] = s;
+    }
+  }
+}
+
+// NR: produced channels of a CTA, NF: of the convolution (float32: 32 are produced by two CTAs, blockIdx.y).
+template <typename T, int CR, int NF, bool DGRAD, int RP, int NR>
+__global__ void __launch_bounds__(128, (BandGeo<T, CR, NR, RP>::CTAS))
 sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int tiles_h) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  typedef BandGeo<CR, NR, RP> G;
-  constexpr int PT = G::PT, R = G::R, PW = G::PW, NPIX = G::NPIX, NRB = G::NRB, CG = G::CG, NTHR = G::NTHR;
+  typedef BandGeo<T, CR, NR, RP> G;
+  constexpr int PT = G::PT, R = G::R, PW = G::PW, NPIX = G::NPIX, NRB = G::NRB, CG = G::CG, P = G::P;
   __shared__ __align__(8) uint64_t mbar_s;
   __shared__ uint32_t tmem_base_s;
   __shared__ int2 tab_s[3][NPIX];                       // per pixel around the tile: first voxel (-1: outside the image), base plane
+  __shared__ unsigned top_s[4];                         // float32: largest magnitude of a step, three steps in turn
   constexpr int CIN = pad16(CR), COUT = pad16(NR), KC = CIN / 8, KR = CR / 8, N3 = 3 * COUT;
   constexpr uint32_t B_LBO = 128, B_SBO = KC * 128;     // filter tiles: K-chunks adjacent, then 8-row groups, taps behind each other
   constexpr uint32_t A_LBO = NRB * 16, A_SBO = 128;     // stage: rows linear, K-chunks NRB rows apart
   constexpr int B_TAP_BYTES = COUT * CIN * 2;
   unsigned char* sB = smem;                             // 27 taps
-  unsigned char* sX = smem + 27 * B_TAP_BYTES;
+  unsigned char* sX = smem + G::FILTER;      // [piece][K-chunk][row]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(DGRAD ? a.out_grad : a.images);
-  __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(DGRAD ? a.images_grad : a.output);
+  const int n0 = NF > NR ? (int)blockIdx.y * NR : 0;
+  const T* src = static_cast<const T*>(DGRAD ? a.out_grad : a.images);
+  T* dst = static_cast<T*>(DGRAD ? a.images_grad : a.output) + n0;
 
   if (KR < KC)   // the padding channels stay zero
-    for (int e = tid; e < G::ROWS; e += NTHR) *reinterpret_cast<uint4*>(sX + A_LBO + e * 16) = make_uint4(0, 0, 0, 0);
+    for (int e = tid; e < P * G::ROWS; e += 128)
+      *reinterpret_cast<uint4*>(sX + (e / G::ROWS * KC + 1) * A_LBO + e % G::ROWS * 16) = make_uint4(0, 0, 0, 0);
   constexpr uint32_t TCOLS = G::TMEM;
   if (warp == 0) {
     uint32_t slot = smem_u32(&tmem_base_s), ncols = TCOLS;
@@ -80,10 +185,15 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
   }
 
   const int H = a.H, W = a.W, D = a.D;
-  uint4 padv = make_uint4(0, 0, 0, 0);
+  uint4 padv = make_uint4(0, 0, 0, 0);                  // 16 bytes of padding values
   if (!a.pad_zero) {
-    const unsigned d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
-    const unsigned d32 = d16 | (d16 << 16);
+    unsigned d32;
+    if constexpr (P == 1) {
+      const unsigned d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
+      d32 = d16 | (d16 << 16);
+    } else {
+      d32 = __ldg(static_cast<const unsigned*>(a.default_value));
+    }
     padv = make_uint4(d32, d32, d32, d32);
   }
   auto entry = [&](int tile) {   // this thread's entry of a tile's table
@@ -134,10 +244,11 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
   };
   auto more = [&](const Step& s) { return s.sub >= 0 ? s.sub + 1 < R * G::GROUPS : s.left != 0; };
 
-  constexpr int NI = (G::ROWS * KR + NTHR - 1) / NTHR;  // 16-byte chunks a thread stages per step
-  constexpr int RSTEP = NTHR / KR;                      // rows between them
+  constexpr int NI = (G::ROWS * KR + 127) / 128;        // chunks of eight channels that a thread stages per step
+  constexpr int RSTEP = 128 / KR;                       // rows between them
+  constexpr int VEC = (int)sizeof(T) / 2;               // 16-byte words of a chunk
   const int chunk = tid % KR, row0 = tid / KR;
-  uint4 val[NI];
+  uint4 val[NI][VEC];
   // The chunks of a row are fetched by neighbouring lanes, a pixel's planes by the lanes behind: consecutive addresses.
   auto request = [&](const Step& s, const int2* tab) {
 #pragma unroll
@@ -157,8 +268,12 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
           plane = row % RP - 1 + o.y - e.y;
         }
       }
-      val[i] = padv;
-      if (e.x >= 0 && !oob(plane, D)) val[i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(e.x + plane) * CR) + chunk);
+      const bool in = e.x >= 0 && !oob(plane, D);
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) {
+        val[i][k] = padv;
+        if (in) val[i][k] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(e.x + plane) * CR) + chunk * VEC + k);
+      }
     }
   };
 
@@ -170,7 +285,17 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
   open(cur, tab_s[0]);
   request(cur, tab_s[0]);
   ahead = entry(cur.tile + (int)gridDim.x);             // of the tile after the present one
-  stage_filter_tiles<CR, NR, DGRAD, true, NTHR>(static_cast<const unsigned short*>(a.filters), sB, tid, B_LBO, B_SBO, B_TAP_BYTES);
+  bool plain_filter = false;
+  if constexpr (P == 1) {
+    stage_filter_tiles<CR, NR, DGRAD, true>(static_cast<const unsigned short*>(a.filters), sB, tid, B_LBO, B_SBO, B_TAP_BYTES);
+  } else {
+    const unsigned top = __reduce_max_sync(0xffffffffu, stage_filter_pieces<CR, NR, NF, DGRAD>(static_cast<const float*>(a.filters), n0, sB, tid, B_LBO, B_SBO, B_TAP_BYTES));
+    if (lane == 0) top_s[warp] = top;
+    __syncthreads();
+    plain_filter = not_for_pieces(max(max(top_s[0], top_s[1]), max(top_s[2], top_s[3])));
+    __syncthreads();
+    if (tid < 3) top_s[tid] = 0;
+  }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -184,17 +309,47 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
   int buf = 0;
   auto next = [](int b) { return b == 2 ? 0 : b + 1; };
 
+  unsigned top = 0;
+  bool plain = false;                                   // float32: this step's values are not for the pieces
+  auto store = [&](int i) {
+    unsigned char* o = sX + chunk * A_LBO + (row0 + i * RSTEP) * 16;
+    if constexpr (P == 1) {
+      *reinterpret_cast<uint4*>(o) = val[i][0];
+    } else {
+      const uint4 lo = val[i][0], hi = val[i][VEC - 1];
+      const float v[8] = {__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(lo.w),
+                          __uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z), __uint_as_float(hi.w)};
+      top = max(top, top_bits(v));
+      unsigned p[3][4];
+      split3(v, p);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(o + q * KC * A_LBO) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+    }
+  };
+  // Piece p of the gathered values meets pieces 0 .. P-1-p of the weights, side by side in N: accumulators [piece sum][depth tap],
+  // the products x1*w1 | x1*w2, x2*w1 | x1*w3, x2*w2, x3*w1.  Apart from one another the small ones cost the large ones no bits: a
+  // chain of 9*CIN/16 additions in tensor memory each, against 27*CIN/4 in registers before.
   while (true) {
     const bool again = more(cur);
     // the table of the next step; its buffer was last read two steps ago, before the barrier behind the last staging
     if (tid < NPIX) tab_s[next(buf)][tid] = again ? tab_s[buf][tid] : ahead;
+    top = 0;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if ((i + 1) * RSTEP <= G::ROWS || row0 + i * RSTEP < G::ROWS)
-        *reinterpret_cast<uint4*>(sX + chunk * A_LBO + (row0 + i * RSTEP) * 16) = val[i];
+        store(i);
+    if constexpr (P > 1) {
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0) atomicMax(&top_s[buf], top);
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (P > 1) {
+      if (cur.sub < 0 || cur.sub % G::GROUPS == 0) plain = plain_filter;
+      plain = plain || not_for_pieces(top_s[buf]);
+      if (tid == 0) top_s[next(next(buf))] = 0;         // read in the last step, written two steps on
+    }
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (cur.sub < 0) {
@@ -206,7 +361,14 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
 #pragma unroll
             for (int k16 = 0; k16 < CIN / 16; ++k16) {
               const uint64_t da = umma_desc_advance(da0, (hr * PW + fc) * RP * 16 + k16 * 2 * A_LBO);
-              const uint64_t db = umma_desc_advance(db0, fc * 9 * B_TAP_BYTES + k16 * 2 * B_LBO);
+              const uint64_t db = umma_desc_advance(db0, fc * 9 * P * B_TAP_BYTES + k16 * 2 * B_LBO);
+              if constexpr (P > 1) {                    // R == 1: staged row hr is filter row hr
+#pragma unroll
+                for (int p = 0; p < P; ++p)
+                  umma_bf16(tmem + p * N3, umma_desc_advance(da, p * KC * A_LBO), umma_desc_advance(db, hr * P * 3 * B_TAP_BYTES),
+                            idesc(P - p), (hr | fc | k16 | p) != 0 ? 1u : 0u);
+                continue;
+              }
               const bool fresh = lo == 0 && fc == 0 && k16 == 0;   // the first sums of output row hr
               const int from = fresh ? 1 : lo;
               if (fresh) umma_bf16(tmem + (R - 1 - hr) * N3, da, db, idesc(1), 0u);
@@ -221,8 +383,11 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
           for (int k16 = 0; k16 < CIN / 16; ++k16) {
             const uint64_t da = umma_desc_advance(da0, i * 128 * 16 + k16 * 2 * A_LBO);
             const int col = first + i;
-            const uint64_t db = umma_desc_advance(db0, (col % 3 * 3 + col / 3) * 3 * B_TAP_BYTES + k16 * 2 * B_LBO);
-            umma_bf16(tmem + (R - 1 - blk) * N3, da, db, idesc(1), (first | i | k16) != 0 ? 1u : 0u);
+            const uint64_t db = umma_desc_advance(db0, (col % 3 * 3 + col / 3) * P * 3 * B_TAP_BYTES + k16 * 2 * B_LBO);
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+              umma_bf16(tmem + (R - 1 - blk) * N3 + p * N3, umma_desc_advance(da, p * KC * A_LBO), db, idesc(P - p),
+                        (first | i | k16 | p) != 0 ? 1u : 0u);
           }
         }
       }
@@ -256,48 +421,71 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     // ---- epilogue: accumulator row = (pixel q, window row w); taps fz of rows w-1, w, w+1 make output row w -----------
-    constexpr int NE = NR < 16 ? NR : 16;               // channels at a time
+    constexpr int NE = P > 1 || NR < 16 ? 8 : 16;       // channels at a time
     const int q = tid / RP, w = tid % RP;
 #pragma unroll 1
     for (int r = 0; r < R; ++r) {
       const int2 e = tab_s[buf][(r + 1) * PW + q + 1];
       bool mine;
       int d;
+      unsigned todo = (cur.now >> (r * PT)) & ((1u << PT) - 1u);
       if (cur.sub < 0) {
-        mine = (cur.now >> (r * PT + q)) & 1u;
+        mine = (todo >> q) & 1u;
         d = w + cur.z0 - e.y;
-        if (((cur.now >> (r * PT)) & ((1u << PT) - 1u)) == 0) continue;
       } else {
-        if (cur.sub != r * G::GROUPS + G::GROUPS - 1) continue;   // the row's last group of filter columns
+        todo = __ballot_sync(0xffffffffu, lane < PT && tab_s[buf][(r + 1) * PW + lane % PT + 1].x >= 0);
+        if (cur.sub != r * G::GROUPS + G::GROUPS - 1) todo = 0;   // not the row's last group of filter columns
         mine = e.x >= 0;
         d = w - 1;
       }
+      if (todo == 0) continue;
+      if constexpr (P > 1) {
+        if (plain) {
+          band_plain<CR, NR, NF, DGRAD>(a, tab_s[buf], PW, r, todo, n0, __uint_as_float(padv.x));
+          continue;
+        }
+      }
       mine = mine && !oob(d, D);
-      uint4* o = reinterpret_cast<uint4*>(dst + (size_t)(mine ? e.x + d : 0) * NR);
+      T* o = dst + (size_t)(mine ? e.x + d : 0) * NF;
 #pragma unroll 1
-      for (int n0 = 0; n0 < NR; n0 += NE) {
-        uint32_t t0[NE], t1[NE], t2[NE];
-        const uint32_t col = tmem + ((uint32_t)(warp * 32) << 16) + (R - 1 - r) * N3 + n0;
-        tmem_ld<NE>(col, t0);
-        tmem_ld<NE>(col + COUT, t1);
-        tmem_ld<NE>(col + 2 * COUT, t2);
+      for (int c = 0; c < NR; c += NE) {
+        uint32_t t[P][3][NE];
+        const uint32_t col = tmem + ((uint32_t)(warp * 32) << 16) + (R - 1 - r) * N3 + c;
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+#pragma unroll
+          for (int fz = 0; fz < 3; ++fz) tmem_ld<NE>(col + p * N3 + fz * COUT, t[p][fz]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        uint32_t h[NE / 2];
+        float s[NE];
 #pragma unroll
-        for (int k = 0; k < NE; k += 2) {
-          float s[2];
+        for (int k = 0; k < NE; ++k) {
+          float f[3];
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const float below = __uint_as_float(__shfl_up_sync(0xffffffffu, t0[k + i], 1));
-            const float above = __uint_as_float(__shfl_down_sync(0xffffffffu, t2[k + i], 1));
-            s[i] = below + __uint_as_float(t1[k + i]) + above;
+          for (int fz = 0; fz < 3; ++fz) {
+            f[fz] = __uint_as_float(t[P - 1][fz][k]);   // the small products first
+#pragma unroll
+            for (int p = P - 2; p >= 0; --p) f[fz] += __uint_as_float(t[p][fz][k]);
           }
-          const __nv_bfloat162 p = __floats2bfloat162_rn(s[0], s[1]);
-          h[k / 2] = *reinterpret_cast<const uint32_t*>(&p);
+          const float below = __shfl_up_sync(0xffffffffu, f[0], 1);
+          const float above = __shfl_down_sync(0xffffffffu, f[2], 1);
+          s[k] = below + f[1] + above;
         }
         if (mine) {
+          if constexpr (P == 1) {
 #pragma unroll
-          for (int k = 0; k < NE / 8; ++k) o[n0 / 8 + k] = make_uint4(h[4 * k], h[4 * k + 1], h[4 * k + 2], h[4 * k + 3]);
+            for (int k = 0; k < NE; k += 8) {
+              uint32_t h[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const __nv_bfloat162 b = __floats2bfloat162_rn(s[k + 2 * i], s[k + 2 * i + 1]);
+                h[i] = *reinterpret_cast<const uint32_t*>(&b);
+              }
+              *reinterpret_cast<uint4*>(o + c + k) = make_uint4(h[0], h[1], h[2], h[3]);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < NE; k += 4) *reinterpret_cast<float4*>(o + c + k) = make_float4(s[k], s[k + 1], s[k + 2], s[k + 3]);
+          }
         }
       }
     }
@@ -316,22 +504,26 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
 }
 
 // Windows of 16 rows for bands of up to 10 planes, of 32 rows for up to 24: base_plane may vary by four planes at least.
-template <int CIN, int COUT, bool DGRAD, int RP>
+template <typename T, int CIN, int COUT, bool DGRAD, int RP>
 int launch_rp(const ScArgs& a, cudaStream_t st) {
-  typedef BandGeo<CIN, COUT, RP> G;
-  auto k = sc_band_kernel<CIN, COUT, DGRAD, RP>;
+  constexpr int NR = BandType<T>::P > 1 && COUT > 16 ? 16 : COUT;
+  typedef BandGeo<T, CIN, NR, RP> G;
+  auto k = sc_band_kernel<T, CIN, COUT, DGRAD, RP, NR>;
   if (int e = grant_smem(k, G::SMEM)) return e;
   const int tw = (a.W + G::PT - 1) / G::PT, th = (a.H + G::R - 1) / G::R;
   const long long ntiles = (long long)a.B * tw * th;    // at most as many as pixels: 31 bits
-  constexpr long long slots = 148LL * G::CTAS;
-  k<<<(unsigned)(ntiles < slots ? ntiles : slots), G::NTHR, G::SMEM, st>>>(a, (int)ntiles, tw, th);
+  constexpr long long slots = 148LL * G::CTAS / (COUT / NR);
+  k<<<dim3((unsigned)(ntiles < slots ? ntiles : slots), COUT / NR), 128, G::SMEM, st>>>(a, (int)ntiles, tw, th);
   return (int)cudaGetLastError();
 }
-template <int CIN, int COUT, bool DGRAD>
+template <typename T, int CIN, int COUT, bool DGRAD>
 int launch_band(const ScArgs& a, cudaStream_t st) {
-  if (a.D <= 10) return launch_rp<CIN, COUT, DGRAD, 16>(a, st);
-  return launch_rp<CIN, COUT, DGRAD, 32>(a, st);
+  if (a.D <= 10) return launch_rp<T, CIN, COUT, DGRAD, 16>(a, st);
+  return launch_rp<T, CIN, COUT, DGRAD, 32>(a, st);
 }
+#define CHOP_CASE(T, I, O)                                                            \
+  if (!dgrad && a.Cin == I && a.Cout == O) return launch_band<T, I, O, false>(a, st); \
+  if (dgrad && a.Cout == I && a.Cin == O) return launch_band<T, I, O, true>(a, st);
 
 }  // namespace
 
@@ -343,19 +535,30 @@ int launch_band(const ScArgs& a, cudaStream_t st) {
 bool sc_band_better(const ScArgs& a, int cin, int cout) {
   if (a.D > 24) return false;
   const int rp = a.D <= 10 ? 16 : 32;
-  if (band_tile_rows(cin, cout) == 1 && 16 * (a.D + 2) < 9 * rp) return false;
+  if (BandType<__nv_bfloat16>::rows(cin, cout) == 1 && 16 * (a.D + 2) < 9 * rp) return false;
   return rp == 32 || (long long)a.B * a.H * a.W >= 16000;
 }
 
+// float32, where this beats sc_run_kernel and is no less exact.  189x251x7, us there and here: 16 -> 16 127, 88; 16 -> 32 238, 166;
+// 16 -> 8 79, 84; 8 -> 8 49, 70; 8 -> 16 73, 74; 256x320x9 254, 140; 493, 268; 155, 134; 87, 112; 134, 117; 60x75x9, 16 -> 16 29, 30.
+// 2-norm of the error against float64 over that of the result: 16 gathered channels 1.77e-7 here, 1.80 to 1.92e-7 there; 32, whose
+// chains are twice as long, 3.0e-7, so they stay there.
+bool sc_band_f32_better(const ScArgs& a, int cin, int cout) { return cin == 16 && cout >= 16 && a.D >= 5 && a.D <= 24; }
+
 int sc_band_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {
-#define CHOP_CASE(I, O)                                                            \
-  if (!dgrad && a.Cin == I && a.Cout == O) return launch_band<I, O, false>(a, st); \
-  if (dgrad && a.Cout == I && a.Cin == O) return launch_band<I, O, true>(a, st);
-  CHOP_CASE(8, 8) CHOP_CASE(8, 16) CHOP_CASE(8, 32) CHOP_CASE(16, 8) CHOP_CASE(16, 16) CHOP_CASE(16, 32) CHOP_CASE(32, 8)
-  CHOP_CASE(32, 16) CHOP_CASE(32, 32)
-#undef CHOP_CASE
+  typedef __nv_bfloat16 bf;
+  CHOP_CASE(bf, 8, 8) CHOP_CASE(bf, 8, 16) CHOP_CASE(bf, 8, 32) CHOP_CASE(bf, 16, 8) CHOP_CASE(bf, 16, 16) CHOP_CASE(bf, 16, 32)
+  CHOP_CASE(bf, 32, 8) CHOP_CASE(bf, 32, 16) CHOP_CASE(bf, 32, 32)
   return -4;
 }
+int sc_band_f32_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {
+  if (!dgrad && a.Cin == 16 && a.Cout == 16) return launch_band<float, 16, 16, false>(a, st);
+  if (!dgrad && a.Cin == 16 && a.Cout == 32) return launch_band<float, 16, 32, false>(a, st);
+  if (dgrad && a.Cout == 16 && a.Cin == 16) return launch_band<float, 16, 16, true>(a, st);
+  if (dgrad && a.Cout == 16 && a.Cin == 32) return launch_band<float, 16, 32, true>(a, st);
+  return -4;
+}
+#undef CHOP_CASE
 
 int sc_band_timeouts() { return timeouts_here(); }
 int sc_band_publish_mirror(int* dptr) { return (int)publish_mirror_here(dptr); }

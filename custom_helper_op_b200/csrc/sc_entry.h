@@ -25,12 +25,17 @@ int sc_tile_fwd_launch(int dtype, const ScArgs& a, cudaStream_t st);
 int sc_tile_wgrad_launch(int dtype, const ScArgs& a, int nparts, cudaStream_t st);
 int sc_tile_twgrad_launch(int dtype, const ScArgs& a, int nparts, cudaStream_t st);
 int sc_tile_gather_launch(int dtype, const ScArgs& a, cudaStream_t st);
+// float32, 3x3x3, stride 1, by runs of planes (sc_run.cu) or on the tensor cores (sc_band.cu); the filter may lie at any address
+bool sc_run_supported(int dtype, const ScArgs& a, int gathered);
+int sc_run_launch(const ScArgs& a, bool dgrad, cudaStream_t st);
 // sums nparts slabs of taps*KC*NC + 1 floats; default_grad may be null
 int sc_slab_reduce(const float* part, int nparts, int taps, int KC, int NC, bool transposed, float* filter_grad,
                    float* default_grad, cudaStream_t st);
 // stride 1 with every voxel staged once per tile (sc_band.cu); cin: gathered channels, cout: produced ones
 bool sc_band_better(const ScArgs& a, int cin, int cout);
 int sc_band_launch(const ScArgs& a, bool dgrad, cudaStream_t st);
+bool sc_band_f32_better(const ScArgs& a, int cin, int cout);
+int sc_band_f32_launch(const ScArgs& a, bool dgrad, cudaStream_t st);   // float32, in three bfloat16 pieces
 int sc_band_timeouts();
 int sc_band_publish_mirror(int* dptr);
 int sc_band_clear_timeouts();

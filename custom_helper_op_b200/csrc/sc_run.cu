@@ -1,0 +1,210 @@
+// Stride-1 3x3x3 manifold convolution of float32 data on the CUDA cores, in runs of planes: forward, image gradient and
+// transposed forward, 8, 16 or 32 channels on either side.
+//
+// As in sc_tile.cu the gathered channels are split over lanes - LK = KCH/4 neighbouring lanes share an item, each holding
+// four channels of it, and their sums are added once at the end - but an item is a RUN of TZ consecutive planes of one pixel,
+// not a voxel.  The three depth taps of a filter column read the same neighbour pixel at consecutive planes, so a run loads
+// TZ + 2 rows per column where single voxels load 3*TZ, and every row then feeds up to three planes from its registers.
+// Nothing is looked up per tap: one (first voxel, shift) pair per item and column, in a table that each warp fills for
+// itself, so that after the weights are staged no warp waits for another.
+// Bound: shared memory returns 128 bytes a cycle, so a 16-byte weight load occupies it for the four cycles that its eight paired
+// multiply-adds take (load-store data pipe 75 % busy, FMA pipe 63).  189x251x7, float32, us before (sc_tile.cu) and now:
+// 8 -> 8 channels 66, 49; 8 -> 16 104, 73; 16 -> 8 99, 78; 16 -> 16 150, 127; 32 -> 32 683, 447; scalar instead of paired 156.
+#include "cv_packed.cuh"
+#include "sc_common.cuh"
+#include "sc_entry.h"
+#include "smem_grant.h"
+
+namespace chop {
+namespace {
+
+constexpr int RUN_WARPS = 4, RUN_OCC = 3;   // 168 registers: two columns' rows and 64 sums (four CTAs of 128: 127 -> 158 us)
+template <int KCH, int NCH, int TZ>
+struct RunCfg {
+  static constexpr int LK = KCH / 4;                  // lanes per item
+  static constexpr int IPW = 32 / LK;                 // items per warp
+  static constexpr int NT = NCH < 16 ? NCH : 16;      // produced channels per thread; 32 are produced by two CTAs
+  static constexpr int WROW = 4 * NT + 4;             // floats of a lane's four weight rows, padded by 16 bytes
+  static constexpr size_t WBYTES = (size_t)27 * LK * WROW * 4;
+  static constexpr size_t SMEM = WBYTES + (size_t)RUN_WARPS * IPW * 9 * sizeof(int2);
+};
+
+// FWD: weights w[t][ci][co], otherwise flipped and swapped, w'[t][co][ci] = filter[26 - t][ci][co], over a.out_grad.
+template <int KCH, int NCH, int TZ, bool FWD>
+__global__ void __launch_bounds__(32 * RUN_WARPS, RUN_OCC) sc_run_kernel(const __grid_constant__ ScArgs a, const int nz, const unsigned nitems) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef RunCfg<KCH, NCH, TZ> Cf;
+  constexpr int LK = Cf::LK, IPW = Cf::IPW, NT = Cf::NT, WROW = Cf::WROW;
+  float* ws = reinterpret_cast<float*>(smem_raw);                          // [27][LK][WROW]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int2* tab = reinterpret_cast<int2*>(smem_raw + Cf::WBYTES) + warp * IPW * 9;   // [9][IPW] first voxel (-1: padding), shift
+  const int n0 = NCH > NT ? blockIdx.y * NT : 0;
+  const float* flt = static_cast<const float*>(a.filters);
+  for (int e = threadIdx.x; e < 27 * KCH * NT; e += 32 * RUN_WARPS) {
+    int t, k, n;
+    if (FWD) {
+      n = e % NT; k = e / NT % KCH; t = e / (NT * KCH);
+    } else {
+      k = e % KCH; n = e / KCH % NT; t = e / (NT * KCH);
+    }
+    ws[(size_t)(t * LK + k / 4) * WROW + (k % 4) * NT + n] =
+        __ldg(FWD ? flt + ((size_t)t * KCH + k) * NCH + n0 + n : flt + ((size_t)(26 - t) * NCH + n0 + n) * KCH + k);
+  }
+  __syncthreads();
+  const float pad = a.pad_zero ? 0.f : __ldg(static_cast<const float*>(a.default_value));
+  const float4 pad4 = make_float4(pad, pad, pad, pad);
+  const int q = lane % LK, it = lane / LK;
+  const float* src = static_cast<const float*>(FWD ? a.images : a.out_grad) + q * 4;
+  float* dst = static_cast<float*>(FWD ? a.output : a.images_grad) + n0;
+  const int H = a.H, W = a.W, D = a.D;
+  const unsigned step = gridDim.x * RUN_WARPS * IPW;
+
+  for (unsigned first = (blockIdx.x * RUN_WARPS + warp) * IPW; first < nitems; first += step) {
+    __syncwarp();
+    for (int e = lane; e < IPW * 9; e += 32) {
+      const unsigned item = first + e % IPW;
+      const int col = e / IPW;
+      int2 ent = make_int2(-1, 0);
+      if (item < nitems) {
+        const unsigned pix = item / (unsigned)nz;
+        const int c = (int)(pix % (unsigned)W), r = (int)(pix / (unsigned)W % (unsigned)H);
+        const int orow = r - 1 + col / 3, ocol = c - 1 + col % 3;
+        if (!oob(orow, H) && !oob(ocol, W)) {
+          const unsigned np = pix + (col / 3 - 1) * W + (col % 3 - 1);
+          ent = make_int2((int)(np * D), __ldg(a.base_plane + pix) - __ldg(a.base_plane + np));
+        }
+      }
+      tab[col * IPW + e % IPW] = ent;
+    }
+    __syncwarp();
+    const unsigned item = first + it;
+    const bool live = item < nitems;
+    const int pix = live ? (int)(item / (unsigned)nz) : 0;
+    const int z0 = live ? (int)(item % (unsigned)nz) * TZ : 0;             // first plane of the run
+
+    pk2 acc[TZ][NT / 2];
+#pragma unroll
+    for (int j = 0; j < TZ; ++j)
+#pragma unroll
+      for (int n = 0; n < NT / 2; ++n) acc[j][n] = 0ull;
+    float4 x[TZ + 2], y[TZ + 2];
+    auto request = [&](float4 (&v)[TZ + 2], int col) {
+      const int2 e = tab[col * IPW + it];
+      const int plane = z0 - 1 + e.y;
+      const float* p = src + ((long long)e.x + plane) * KCH;               // dereferenced for planes of the band only
+#pragma unroll
+      for (int r = 0; r < TZ + 2; ++r) {
+        v[r] = pad4;
+        if (e.x >= 0 && !oob(plane + r, D)) v[r] = __ldg(reinterpret_cast<const float4*>(p + r * KCH));
+      }
+    };
+    auto multiply = [&](const float4 (&v)[TZ + 2], int col) {
+      const float* wc = ws + (size_t)(col * 3 * LK + q) * WROW;
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        pk2 x2[TZ + 2];
+#pragma unroll
+        for (int r = 0; r < TZ + 2; ++r) {
+          const float s = kk == 0 ? v[r].x : kk == 1 ? v[r].y : kk == 2 ? v[r].z : v[r].w;
+          x2[r] = pk_make(s, s);
+        }
+#pragma unroll
+        for (int fz = 0; fz < 3; ++fz) {
+#pragma unroll
+          for (int n4 = 0; n4 < NT / 4; ++n4) {
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(wc + fz * LK * WROW + kk * NT + n4 * 4);
+#pragma unroll
+            for (int j = 0; j < TZ; ++j) {
+              pk_fma_to(acc[j][n4 * 2], x2[j + fz], w.x);
+              pk_fma_to(acc[j][n4 * 2 + 1], x2[j + fz], w.y);
+            }
+          }
+        }
+      }
+    };
+    request(x, 0);
+#pragma unroll 1
+    for (int col = 0; col < 8; col += 2) {   // two sets of rows in turn: one column's arithmetic covers the next one's loads
+      request(y, col + 1);
+      multiply(x, col);
+      request(x, col + 2);
+      multiply(y, col + 1);
+    }
+    multiply(x, 8);
+
+    // add the LK lanes' partial sums; lane q keeps values q*M/LK .. of the M = TZ*NT (plane, channel) sums
+    constexpr int M = TZ * NT;
+    float v[M];
+#pragma unroll
+    for (int j = 0; j < TZ; ++j)
+#pragma unroll
+      for (int n = 0; n < NT / 2; ++n) pk_split(acc[j][n], v[j * NT + 2 * n], v[j * NT + 2 * n + 1]);
+#pragma unroll
+    for (int s = LK / 2, half = M / 2; s >= 1; s >>= 1, half >>= 1) {
+      const bool hi = (q & s) != 0;
+#pragma unroll
+      for (int e = 0; e < M / 2; ++e) {
+        if (e < half) {
+          const float keep = hi ? v[e + half] : v[e];
+          const float send = hi ? v[e] : v[e + half];
+          v[e] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+        }
+      }
+    }
+    constexpr int MINE = M / LK, VW = MINE % 4 == 0 ? 4 : 2;
+    static_assert(MINE % 2 == 0, "vector stores");
+#pragma unroll
+    for (int e = 0; e < MINE; e += VW) {
+      const int at = q * MINE + e, z = z0 + at / NT;
+      float* o = dst + ((size_t)pix * D + z) * NCH + at % NT;
+      if (live && z < D) {
+        if constexpr (VW == 4) *reinterpret_cast<float4*>(o) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        else *reinterpret_cast<float2*>(o) = make_float2(v[e], v[e + 1]);
+      }
+    }
+  }
+}
+
+template <int KCH, int NCH, int TZ, bool FWD>
+int launch_tz(const ScArgs& a, cudaStream_t st) {
+  typedef RunCfg<KCH, NCH, TZ> Cf;
+  auto k = sc_run_kernel<KCH, NCH, TZ, FWD>;
+  if (int e = grant_smem(k, Cf::SMEM)) return e;
+  const int nz = (a.D + TZ - 1) / TZ;
+  const unsigned nitems = (unsigned)((long long)a.B * a.H * a.W * nz);     // at most as many as voxels
+  int per_sm = (int)((size_t)224 * 1024 / (Cf::SMEM + 1024));
+  if (per_sm > RUN_OCC) per_sm = RUN_OCC;
+  const unsigned split = NCH / Cf::NT;
+  const unsigned slots = 148u * per_sm / split, need = (nitems + RUN_WARPS * Cf::IPW - 1) / (RUN_WARPS * Cf::IPW);
+  k<<<dim3(need < slots ? need : slots, split), 32 * RUN_WARPS, Cf::SMEM, st>>>(a, nz, nitems);
+  return (int)cudaGetLastError();
+}
+template <int KCH, int NCH, bool FWD>
+int launch_run(const ScArgs& a, cudaStream_t st) {
+  // runs of four planes, of three where those leave fewer planes of the last run empty
+  if ((a.D + 2) / 3 * 3 < (a.D + 3) / 4 * 4 && KCH < 32) return launch_tz<KCH, NCH, KCH < 32 ? 3 : 4, FWD>(a, st);
+  return launch_tz<KCH, NCH, 4, FWD>(a, st);
+}
+
+}  // namespace
+
+// Runs that leave up to a third of their planes empty are still the faster ones (sc_tile.cu at 120x150x5, two runs of four planes:
+// 32 -> 32 channels 202 us there, 190 here, 32 -> 8 60 and 64).
+bool sc_run_supported(int dtype, const ScArgs& a, int gathered) {
+  auto ok = [](int c) { return c == 8 || c == 16 || c == 32; };
+  const int in4 = (a.D + 3) / 4 * 4, in3 = (a.D + 2) / 3 * 3, planes = gathered < 32 && in3 < in4 ? in3 : in4;
+  return dtype == 0 && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 && a.sr == 1 && a.sc == 1 &&
+         a.sd == 1 && ok(a.Cin) && ok(a.Cout) && a.nvox_in < (1LL << 31) - 4096 && 2 * planes <= 3 * a.D;
+}
+
+int sc_run_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {
+  const int in = dgrad ? a.Cout : a.Cin, out = dgrad ? a.Cin : a.Cout;
+  if (sc_band_f32_better(a, in, out)) return sc_band_f32_launch(a, dgrad, st);
+#define CHOP_CASE(K, N) if (in == K && out == N) return dgrad ? launch_run<K, N, false>(a, st) : launch_run<K, N, true>(a, st);
+  CHOP_CASE(8, 8) CHOP_CASE(8, 16) CHOP_CASE(8, 32) CHOP_CASE(16, 8) CHOP_CASE(16, 16) CHOP_CASE(16, 32) CHOP_CASE(32, 8)
+  CHOP_CASE(32, 16) CHOP_CASE(32, 32)
+#undef CHOP_CASE
+  return -4;
+}
+
+}  // namespace chop

@@ -101,12 +101,12 @@ __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, uint32_t* r) {
 // 91 / 110 / 127 us for 8 -> 16 channels on the CUDA cores and take 30 / 31 / 21 here, 32 -> 8 191 / 159 / 236 and 68 / 35 / 120.
 __host__ __device__ constexpr int pad16(int c) { return c < 16 ? 16 : c; }
 // COLS: the tiles in the order [filter column][filter row][depth tap], not the filter's [row][column][depth].
-template <int CR, int NR, bool DGRAD, bool COLS = false, int NTHR = 128>
+template <int CR, int NR, bool DGRAD, bool COLS = false>
 __device__ __forceinline__ void stage_filter_tiles(const unsigned short* flt, unsigned char* sB, int tid, uint32_t lbo,
                                                    uint32_t sbo, int tap_bytes) {
   constexpr int COUT = pad16(NR), KC = pad16(CR) / 8;
 #pragma unroll 2
-  for (int e = tid; e < 27 * COUT * KC; e += NTHR) {
+  for (int e = tid; e < 27 * COUT * KC; e += 128) {
     const int kg = e % KC, n = (e / KC) % COUT, t = e / (KC * COUT);
     uint4 w = make_uint4(0, 0, 0, 0);
     if (kg * 8 >= CR || n >= NR) {
