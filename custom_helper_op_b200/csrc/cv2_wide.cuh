@@ -5,45 +5,29 @@
 // bfloat16 per corner (half the loads, addresses and record reads per channel), blends with the four bilinear weights and
 // takes the products with the reference pixel at once, in pairs.  There is no cache and no test per plane: where every lane
 // sees the block's planes (the usual case) the loads of several planes are in flight together.
-// Bound: latency of the gathers behind the unpacking (32 of 128 instructions).  Four views, 1152x1536x8, C = 8, eight
-// groups: 567 -> 430 us (602 -> 438 with planes eight times as far apart); 576x768x32, C = 16, eight groups: 648 -> 571
-// (780 -> 602).
+// Bound: latency of the gathers behind the unpacking (32 of 128 instructions).  Four views, 576x768x32, C = 16, eight groups:
+// 648 -> 571 us (780 -> 602 with planes eight times as far apart).  Eight channels are cv2_vox.cuh's.
 //
 // Float32 features double the fetch, and with few groups per channel the cached form (a plane costs its GROUPS only) stays
 // ahead while the footprint rests (C = 32, eight groups, planes 1 apart: 251 us against 328).  Where it is chosen otherwise:
 // v2_wide_fwd.
 #pragma once
-#include "cv_packed.cuh"
+#include "cv2_vox.cuh"
 
 namespace chop {
-
-// A lane's eight consecutive channels of one texel, widened to pairs on use.
-template <typename T>
-struct Ch8;
-template <>
-struct Ch8<__nv_bfloat16> {
-  uint4 r;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { r = __ldg(reinterpret_cast<const uint4*>(p)); }
-  __device__ __forceinline__ pk2 get(int k) const {
-    const unsigned w = k == 0 ? r.x : k == 1 ? r.y : k == 2 ? r.z : r.w;
-    return pk_make(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-  }
-};
 
 template <int C, int SUB>
 struct V2Wide {
   static constexpr int LG = C / 8, G = 32 / LG;
-  static constexpr int PB = SUB == 4 ? 8 : 4;        // planes per block: at most 32 accumulator registers
-  static constexpr int BLOCKS = C == 8 ? 4 : 5;      // CTAs per SM: 128 registers measured better for one lane per pixel
+  static constexpr int PB = 4;                       // planes per block: at most 32 accumulator registers
+  static constexpr int BLOCKS = 5;                   // CTAs per SM
   static constexpr int PL = PB / LG;                 // planes that a lane projects
   // A lane owns whole pixels, so a small image has too few warps even with one block of planes each.  From so many on this is
   // the faster kernel; us here : with four channels per lane, four views (replayed from a graph):
-  //   C = 8, 8 / 4 groups  48x60x24  540 warps 7.3 : 5.9 / 7.1 : 5.7, 64x80x16  640 8.3 : 8.8 / 7.9 : 8.2
-  //   C = 8, 2 groups      96x120x16 720 warps 14.3 : 12.5, 64x80x48 960 14.9 : 13.9, 96x120x24 1080 13.8 : 19.2
   //   C = 16, 16 / 8       48x60x24 1080 warps 7.6 : 7.0 / 7.3 : 6.4, 64x80x16 1280 8.3 : 10.3 / 7.7 : 9.3
   //   C = 32, 32           48x60x8   720 warps 6.4 : 7.6 (nothing smaller measured)
-  static constexpr int MIN_WARPS = 148 * (SUB == 4 ? 7 : C == 16 ? 8 : 4);
-  static constexpr size_t smem_per_warp = LG == 1 ? 0 : (size_t)PB * G * 16;
+  static constexpr int MIN_WARPS = 148 * (C == 16 ? 8 : 4);
+  static constexpr size_t smem_per_warp = (size_t)PB * G * 16;
 };
 
 template <typename T, int C, int SUB>
@@ -53,7 +37,7 @@ __global__ void __launch_bounds__(128, V2Wide<C, SUB>::BLOCKS) cv2_fwd_wide(cons
   constexpr int LG = Cf::LG, G = Cf::G, PB = Cf::PB, PL = Cf::PL;
   constexpr int NG = 8 / SUB;              // groups per lane
   constexpr int GR = C / SUB;              // groups per voxel
-  constexpr int NA = SUB == 4 ? 2 : 4;     // paired accumulators per plane
+  constexpr int NA = 4;                    // paired accumulators per plane
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int li = lane & (LG - 1);
@@ -131,19 +115,13 @@ __global__ void __launch_bounds__(128, V2Wide<C, SUB>::BLOCKS) cv2_fwd_wide(cons
         used[p] += seen;
         all_seen &= seen;
       }
-      if constexpr (LG > 1) {
-        __syncwarp();
+      __syncwarp();
 #pragma unroll
-        for (int p = 0; p < PL; ++p) rec[(p * LG + li) * G] = make_float4(__int_as_float(tex[p]), dw[p], dh[p], 0.0f);
-        __syncwarp();
-      }
+      for (int p = 0; p < PL; ++p) rec[(p * LG + li) * G] = make_float4(__int_as_float(tex[p]), dw[p], dh[p], 0.0f);
+      __syncwarp();
       auto record = [&](int j, int& t, float& fw, float& fh) {
-        if constexpr (LG > 1) {
-          const float4 r = rec[j * G];
-          t = __float_as_int(r.x); fw = r.y; fh = r.z;
-        } else {
-          t = tex[j]; fw = dw[j]; fh = dh[j];
-        }
+        const float4 r = rec[j * G];
+        t = __float_as_int(r.x); fw = r.y; fh = r.z;
       };
       auto plane = [&](int j, int t, float fw, float fh) {
         Ch8<T> x00, x01, x10, x11;
@@ -158,8 +136,7 @@ __global__ void __launch_bounds__(128, V2Wide<C, SUB>::BLOCKS) cv2_fwd_wide(cons
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const pk2 s = pk_fma(p11, x11.get(k), pk_fma(p10, x10.get(k), pk_fma(p01, x01.get(k), pk_mul(p00, x00.get(k)))));
-          const int q = SUB == 4 ? k / 2 : k;
-          acc[j][q] = pk_fma(s, ref[k], acc[j][q]);   // sum_c sample*ref (v2:118-120)
+          acc[j][k] = pk_fma(s, ref[k], acc[j][k]);   // sum_c sample*ref (v2:118-120)
         }
       };
       if (__all_sync(0xffffffffu, all_seen)) {
@@ -188,7 +165,7 @@ __global__ void __launch_bounds__(128, V2Wide<C, SUB>::BLOCKS) cv2_fwd_wide(cons
     }
 #pragma unroll
     for (int j = 0; j < PB; ++j) {
-      const int u = LG > 1 ? __shfl_sync(0xffffffffu, used[j / LG], g * LG + j % LG) : used[j / LG];
+      const int u = __shfl_sync(0xffffffffu, used[j / LG], g * LG + j % LG);
       const float inv = u > 0 ? 1.0f / (float)u : 0.0f;   // v2:128-133
       float o[NG];
 #pragma unroll
@@ -230,18 +207,12 @@ inline int v2_wide_go(const CvArgs& a0, cudaStream_t st) {
 // pixels, so a warp's stores are 32-byte pieces a cost slab (D * groups floats) apart, and the more planes the wider apart.
 // Measured at 1, 2, 3, 4 and 6 views, 8 to 64 planes, depths 1 and 8 apart (the footprint rests / moves), us of this kernel
 // against four channels per lane:
-//   C = 8, 8 groups:   8 planes, 1 view 71 : 64 / 70 : 66, 2 views 84 : 92 / 84 : 98; 16 planes, 1 view 138 : 105 / 137 : 113,
-//                      2 views 164 : 159 / 165 : 174; 64 planes, 2 views 193 : 162 / 195 : 175, 3 views 219 : 209 / 223 : 229
-//   C = 8, 4 groups:   8 planes, 1 view 51 : 59 / 53 : 61; 16 planes, 1 view 102 : 99 / 102 : 106; 64 planes, 2 views
-//                      159 : 152 / 160 : 162 (80x100x48 13.0 : 14.5), 3 views 186 : 193 / 192 : 211; 2 groups the same within 5 %
 //   C = 16, 16 groups: 16 planes, 1 view 173 : 141 / 172 : 158, 2 views 223 : 225 / 227 : 260; 64 planes, 2 views
 //                      238 : 195 / 245 : 244, 3 views 283 : 256 / 291 : 322
 //   C = 16, 8 groups:  16 planes, 1 view 123 : 121 / 125 : 139; 32 planes, 1 view 74 : 64 / 74 : 71, 2 views 101 : 96 / 106 : 119
 //   C = 32, 32 groups: 16 planes, 1 view 215 : 223 / 225 : 279; 64 planes, 1 view 213 : 176 / 217 : 217, 2 views 291 : 266 / 303 : 358
 inline int v2_wide_views(int C, int sub, int D) {
-  if (C == 8 && sub > 1) return D <= (sub == 2 ? 12 : 8) ? 1 : 2;
   const int n = D <= 8 ? 1 : D <= 16 ? 2 : 3;
-  if (C == 8) return n < 2 ? 2 : n;
   return C == 16 && sub == 1 ? n : n > 1 ? n - 1 : 1;
 }
 
@@ -250,7 +221,6 @@ inline int v2_wide_fwd(const CvArgs& a, cudaStream_t st) {
   if (((reinterpret_cast<size_t>(a.ref) | reinterpret_cast<size_t>(a.src) | reinterpret_cast<size_t>(a.cost)) & 15) != 0) return -4;
   const int sub = a.C / a.G;
   if (a.N < v2_wide_views(a.C, sub, a.D)) return -4;
-  if (a.C == 8) return sub == 1 ? v2_wide_go<8, 1>(a, st) : sub == 2 ? v2_wide_go<8, 2>(a, st) : sub == 4 ? v2_wide_go<8, 4>(a, st) : -4;
   if (a.C == 16) return sub == 1 ? v2_wide_go<16, 1>(a, st) : sub == 2 ? v2_wide_go<16, 2>(a, st) : -4;
   if (a.C == 32 && sub == 1) return v2_wide_go<32, 1>(a, st);
   return -4;

@@ -25,6 +25,10 @@ int cv_fwd_bf16(const CvArgs& a, const CvPlan& p, cudaStream_t st) {
       default: break;
     }
   }
+  if (p.use_tuned && p.use_packed == 1 && p.kind == 2 && p.mode != 1 && p.cpl == 4) {
+    const int r = v2_vox_fwd<__nv_bfloat16>(a, p.mode == 2, st);   // eight channels: a lane per voxel
+    if (r != -4) return r;
+  }
   if (p.use_tuned && p.use_packed && p.kind == 2 && p.mode == 0 && p.cpl == 4) {
     const int r = v2_wide_fwd(a, st);   // eight channels per lane where that is the better kernel
     if (r != -4) return r;

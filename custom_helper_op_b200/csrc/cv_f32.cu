@@ -1,5 +1,6 @@
 // float32 features: channel slices of 1 or 4 per lane; compile-time-C kernels for the common
 // CostVolume MEAN configurations.
+#include "cv2_vox.cuh"
 #include "cv_launch.cuh"
 #include "cv_entry.h"
 
@@ -23,6 +24,10 @@ int cv_fwd_f32(const CvArgs& a, const CvPlan& p, cudaStream_t st) {
       case 64: return fwd_tuned_go<float, 64, 4, true>(a, st);
       default: break;
     }
+  }
+  if (p.use_tuned && p.use_packed == 1 && p.kind == 2 && p.mode != 1 && p.cpl == 4) {
+    const int r = v2_vox_fwd<float>(a, p.mode == 2, st);   // eight channels: a lane per voxel
+    if (r != -4) return r;
   }
   if (p.use_tuned && p.kind == 2 && p.mode != 1 && p.cpl == 4) {
     const int r = tuned2_dispatch<float>(false, p.mode == 2, a, st);

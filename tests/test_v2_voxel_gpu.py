@@ -1,0 +1,42 @@
+"""CostVolumeV2 forward with eight channels (a lane per voxel): both types, MEAN and MIN, groups of one, two and four channels, depth
+counts around the planes of a warp, ragged pixel counts, views that miss part of the volume, depth ranges, against the oracle and,
+for MIN, bit for bit.  The gradient's blocks of two and four planes on the same cases."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from custom_helper_op_b200.python.ops import custom_helper_ops as ops
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("G", [8, 4, 2])
+@pytest.mark.parametrize("shape", [(1, 1, 3, 5, 1), (2, 3, 9, 11, 4), (1, 2, 7, 13, 9), (3, 4, 5, 31, 16), (1, 5, 12, 10, 19), (1, 2, 2, 3, 20)])
+@pytest.mark.parametrize("reduce", ["MEAN", "MIN"])
+def test_forward_and_gradient(dtype, G, shape, reduce):
+    B, N, H, W, D = shape
+    c = helpers.make_case(2, 90 + G, B, N, H, W, 8, D, "random" if H > 7 else "rot_y", np.float32)
+    t = {k: torch.from_numpy(c[k]).to(dtype) for k in ("ref", "src")}
+    f = {k: t[k].float().numpy() for k in t}
+    want, mask = oracle.cost_fwd(2, f["ref"], f["src"], c["depth"], None, c["Rs"], c["Ts"], reduce, G, True, np.float32)
+    args = [t["ref"].cuda(), t["src"].cuda(), torch.from_numpy(c["depth"]).cuda(), None, torch.from_numpy(c["Rs"]).cuda(),
+            torch.from_numpy(c["Ts"]).cuda()]
+    got, m = ops.cost_forward(2, *args, reduce, G)
+    assert np.array_equal(m.cpu().numpy().reshape(mask.shape), mask)
+    if reduce == "MIN":
+        assert np.array_equal(got.cpu().numpy().reshape(want.shape), want)
+    else:
+        assert helpers.rel_err(got.cpu().numpy().reshape(want.shape), want) <= 1e-5
+    if D > 2:   # a depth range leaves the other planes alone
+        out = (torch.full_like(got, 7.0), torch.full_like(m, 7))
+        ops.cost_forward(2, *args, reduce, G, d_range=(1, D - 1), out=out)
+        assert torch.equal(out[0][..., 1:D - 1, :], got[..., 1:D - 1, :]) and torch.equal(out[1][..., 1:D - 1, :], m[..., 1:D - 1, :])
+        assert bool((out[0][..., [0, D - 1], :] == 7).all()) and bool((out[1][..., [0, D - 1], :] == 7).all())
+    cg = np.random.default_rng(3).standard_normal(want.shape).astype(np.float32)
+    grads = ops.cost_backward(2, *args, torch.from_numpy(cg).cuda(), m, reduce, G)
+    want_g = oracle.cost_bwd(2, f["ref"], f["src"], c["depth"], None, c["Rs"], c["Ts"], cg, mask, reduce, G, True, np.float32)
+    for g, w in zip(grads, want_g):
+        assert helpers.rel_err(g.cpu().numpy().reshape(w.shape), w) <= 1e-4
