@@ -166,10 +166,18 @@ inline int fwd2_min_tuned_go(const CvArgs& a, cudaStream_t st) {
   return (int)cudaGetLastError();
 }
 
+// Eight channels (two lanes per pixel) with two or one groups per lane: blocks of four planes instead of two, so that a footprint
+// that rests is flushed and fetched again half as often.  288x384x48, four views, planes 1 / 8 apart, us with two and with four:
+// two channels per group 334 / 397, 293 / 370, four 324 / 396, 265 / 360; eight planes 485 / 500, 355 / 414 (shared memory).  One
+// per group 374 / 434, 366 / 426, but 256 -> 290 with six views; MIN with two per group 239 -> 261 there; C = 16 spills (560 -> 808).
 template <typename T, int C, int SUB, bool RMIN>
-inline int bwd2_tuned_go(const CvArgs& a, cudaStream_t st) {
-  auto k = cv2_bwd_tuned<T, C, SUB, RMIN>;
-  const size_t spw = tuned2_bwd_smem_per_warp<T>(a.N, 32 / (C / 4));
+inline int bwd2_tuned_go(const CvArgs& a0, cudaStream_t st) {
+  constexpr int PL = C == 8 && (SUB == 4 || (SUB == 2 && !RMIN)) ? 2 : 1, PB = C / 4 * PL;
+  CvArgs a = a0;
+  a.chunk = (a.chunk + PB - 1) / PB * PB;
+  a.nchunks = (a.d_end - a.d_begin + a.chunk - 1) / a.chunk;
+  auto k = cv2_bwd_tuned<T, C, SUB, RMIN, PL>;
+  const size_t spw = tuned2_bwd_smem_per_warp(a.N, 32 / (C / 4), PL);
   const int warps = 4;
   const size_t smem = spw * warps;
   if (smem > 200 * 1024) return -4;

@@ -651,17 +651,18 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
             cur = rc.texel;
             const T* p00 = src_lane + (size_t)rc.texel * C;
             const T* p10 = p00 + row;
-            float t00[CPL], t01[CPL], t10[CPL], t11[CPL];
-            Vec<T, float, CPL>::load(p00, t00);
-            Vec<T, float, CPL>::load(p00 + C, t01);
-            Vec<T, float, CPL>::load(p10, t10);
-            Vec<T, float, CPL>::load(p10 + C, t11);
+            Tex4<T> t00, t01, t10, t11;
+            t00.load(p00);
+            t01.load(p00 + C);
+            t10.load(p10);
+            t11.load(p10 + C);
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
-              a0[k] = t00[k] - refv[k];
-              u[k] = t10[k] - t00[k];
-              v[k] = t01[k] - t00[k];
-              t1[k] = (t11[k] - t01[k]) - u[k];  // :447
+              const float c00 = t00.get(k), c01 = t01.get(k);
+              a0[k] = t00.minus(k, refv[k]);
+              u[k] = t10.minus(k, c00);
+              v[k] = c01 - c00;
+              t1[k] = t11.minus(k, c01) - u[k];  // :447
               acc[0][k] = acc[1][k] = acc[2][k] = acc[3][k] = 0.0f;
             }
           }
@@ -733,9 +734,8 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
 // per group SUB in {1,2,4} (a lane's four channels cover whole groups).  Same loop nest and footprint
 // caching as above.  Reference: cost_volume_kernels_gpu_v2.cu.cc:33-135 (forward), :349-479 (gradient).
 // ---------------------------------------------------------------------------------------------------
-template <typename T>
-__host__ __device__ inline size_t tuned2_bwd_smem_per_warp(int N, int G) {
-  return (size_t)N * G * sizeof(Coef<float>) + (size_t)N * 32 * (sizeof(ProjF<float>) + sizeof(RecG));
+__host__ __device__ inline size_t tuned2_bwd_smem_per_warp(int N, int G, int PL) {
+  return (size_t)N * G * sizeof(Coef<float>) + (size_t)N * PL * 32 * (sizeof(ProjF<float>) + sizeof(RecG));
 }
 
 // Forward: on a reload the corner differences are multiplied by the reference pixel and summed over each
@@ -775,8 +775,8 @@ __global__ void __launch_bounds__(256, 3) cv2_fwd_tuned(const CvArgs a, const in
   __syncwarp();
 
   const T* src_lane = static_cast<const T*>(a.src) + li * CPL;
-  float refv[CPL];
-  Vec<T, float, CPL>::load(static_cast<const T*>(a.ref) + pix * C + li * CPL, refv);
+  Tex4<T> refv;
+  refv.load(static_cast<const T*>(a.ref) + pix * C + li * CPL);
   const float* dgrid = static_cast<const float*>(a.depth) + pix * D;
   const size_t row = (size_t)a.Ws * C;
   const ProjF<float>* myrec = proj + g * LG;
@@ -830,11 +830,11 @@ __global__ void __launch_bounds__(256, 3) cv2_fwd_tuned(const CvArgs a, const in
           if (rc.texel >= 0) {
             const T* p00 = src_lane + (size_t)rc.texel * C;
             const T* p10 = p00 + row;
-            float t00[CPL], t01[CPL], t10[CPL], t11[CPL];
-            Vec<T, float, CPL>::load(p00, t00);
-            Vec<T, float, CPL>::load(p00 + C, t01);
-            Vec<T, float, CPL>::load(p10, t10);
-            Vec<T, float, CPL>::load(p10 + C, t11);
+            Tex4<T> t00, t01, t10, t11;
+            t00.load(p00);
+            t01.load(p00 + C);
+            t10.load(p10);
+            t11.load(p10 + C);
             // The correlation is linear in the sample, so the reference pixel is applied to the four CORNERS first
             // (one dot product per corner and group) and the bilinear differences are formed on the group sums:
             // 4 multiply-adds per channel + 4 subtractions per group instead of 8 operations per channel.
@@ -844,10 +844,10 @@ __global__ void __launch_bounds__(256, 3) cv2_fwd_tuned(const CvArgs a, const in
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
               const int q = k / SUB;
-              d00[q] = fmaf(t00[k], refv[k], d00[q]);
-              d01[q] = fmaf(t01[k], refv[k], d01[q]);
-              d10[q] = fmaf(t10[k], refv[k], d10[q]);
-              d11[q] = fmaf(t11[k], refv[k], d11[q]);
+              d00[q] = t00.times(k, refv, d00[q]);
+              d01[q] = t01.times(k, refv, d01[q]);
+              d10[q] = t10.times(k, refv, d10[q]);
+              d11[q] = t11.times(k, refv, d11[q]);
             }
 #pragma unroll
             for (int q = 0; q < NG; ++q) {
@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(256, 2) cv2_fwd_min_tuned(const CvArgs a, cons
 #endif
 // RMIN = true: `mask` holds the winning view per (voxel, group); only that view is differentiated, with
 // no division by the view count (v2:483-601); a voxel whose first group has no winner is skipped.
-template <typename T, int C, int SUB, bool RMIN = false>
+template <typename T, int C, int SUB, bool RMIN = false, int PL = 1>
 __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(const CvArgs a, const int warps, const size_t smem_per_warp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int CPL = 4;
@@ -1029,6 +1029,7 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
   constexpr int G = 32 / LG;
   constexpr int NG = CPL / SUB;
   constexpr int GR = C / SUB;
+  constexpr int PB = LG * PL;   // planes per block: PL per lane in phase A
   static_assert(LG * CPL == C && (LG & (LG - 1)) == 0 && LG <= 32 && NG * SUB == CPL, "unsupported C / SUB");
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
@@ -1050,7 +1051,7 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
   unsigned char* mine = smem_raw + (size_t)wib * smem_per_warp;
   Coef<float>* coef = reinterpret_cast<Coef<float>*>(mine);
   ProjF<float>* recA = reinterpret_cast<ProjF<float>*>(coef + N * G);  // aux = 1/(valid views)
-  RecG* recG = reinterpret_cast<RecG*>(recA + N * 32);
+  RecG* recG = reinterpret_cast<RecG*>(recA + N * PL * 32);
 
   stage_coefs<float>(a, coef, lane, G, pix0);
   __syncwarp();
@@ -1070,20 +1071,26 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
   // The lane's depth hypothesis and validity count / winner of plane dblk+li stream in from HBM: they are requested
   // one block ahead, so phase A does not start with an exposed DRAM round trip.
   const int mk_stride = RMIN ? GR : 1;
-  float depth_next = 0.0f;
-  int m_next = 0;
-  if (pvalid && dlo + li < dhi) {
-    depth_next = __ldg(dgrid + dlo + li);
-    m_next = __ldg(a.mask + (pix * D + dlo + li) * mk_stride);
+  float depth_next[PL];
+  int m_next[PL];
+#pragma unroll
+  for (int p = 0; p < PL; ++p) {
+    depth_next[p] = 0.0f;
+    m_next[p] = 0;
+    const int d = dlo + p * LG + li;
+    if (pvalid && d < dhi) {
+      depth_next[p] = __ldg(dgrid + d);
+      m_next[p] = __ldg(a.mask + (pix * D + d) * mk_stride);
+    }
   }
-  for (int dblk = dlo; dblk < dhi; dblk += LG, cg_lane += LG * GR, mk_lane += LG * GR) {
+  for (int dblk = dlo; dblk < dhi; dblk += PB, cg_lane += PB * GR, mk_lane += PB * GR) {
     __syncwarp();
     // the block's upstream gradient (and winners): one request per plane, all in flight together and shared by the
     // views, instead of a dependent load per (plane, view); requested before phase A, whose projections cover the latency
-    float cgall[LG][NG];
-    int mkall[RMIN ? LG : 1][NG];
+    float cgall[PB][NG];
+    int mkall[RMIN ? PB : 1][NG];
 #pragma unroll
-    for (int j = 0; j < LG; ++j) {
+    for (int j = 0; j < PB; ++j) {
 #pragma unroll
       for (int q = 0; q < NG; ++q) {
         cgall[j][q] = 0.0f;
@@ -1100,18 +1107,18 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
       }
     }
     // ---- phase A -----------------------------------------------------------------------------------------
-    const int dA = dblk + li;
-    const bool dvA = pvalid && dA < dhi;
-    {
-      float depth = 0.0f, scale = 0.0f;
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      const int dA = dblk + p * LG + li;
+      float scale = 0.0f;
       bool live = false;
-      const int m0 = m_next;
-      depth = depth_next;
-      if (pvalid && dA + LG < dhi) {
-        depth_next = __ldg(dgrid + dA + LG);
-        m_next = __ldg(a.mask + (pix * D + dA + LG) * mk_stride);
+      const int m0 = m_next[p];
+      const float depth = depth_next[p];
+      if (pvalid && dA + PB < dhi) {
+        depth_next[p] = __ldg(dgrid + dA + PB);
+        m_next[p] = __ldg(a.mask + (pix * D + dA + PB) * mk_stride);
       }
-      if (dvA) {
+      if (pvalid && dA < dhi) {
         if constexpr (RMIN) {
           live = m0 >= 0;                      // v2:495
           scale = 1.0f;                        // v2:583
@@ -1128,19 +1135,19 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
         r.aux = scale;
         q.gh = q.gw = 0.0f;
         if (live) r.texel = project<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw);
-        recA[n * 32 + lane] = r;
-        recG[n * 32 + lane] = q;
+        recA[(n * PL + p) * 32 + lane] = r;
+        recG[(n * PL + p) * 32 + lane] = q;
       }
     }
     __syncwarp();
 
     // ---- phase B -----------------------------------------------------------------------------------------
-    float dv[LG];
+    float dv[PB];
 #pragma unroll
-    for (int j = 0; j < LG; ++j) dv[j] = 0.0f;
+    for (int j = 0; j < PB; ++j) dv[j] = 0.0f;
     for (int n = 0; n < N; ++n) {
-      const ProjF<float>* rA = recA + n * 32 + g * LG;
-      const RecG* rGp = recG + n * 32 + g * LG;
+      const ProjF<float>* rA = recA + n * PL * 32 + g * LG;   // plane j: entry (j / LG) * 32 + j % LG
+      const RecG* rGp = recG + n * PL * 32 + g * LG;
       int cur = -1;
       float a0[CPL], u[CPL], v[CPL], t1[CPL];   // p00 and the corner differences of the footprint
       float T1R[NG], UR[NG], VR[NG], m[4][NG];
@@ -1167,34 +1174,35 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
         red_add<float, CPL>(gp + row + C, c11);
       };
 #pragma unroll
-      for (int j = 0; j < LG; ++j) {
-        const ProjF<float> rc = rA[j];
+      for (int j = 0; j < PB; ++j) {
+        const ProjF<float> rc = rA[(j / LG) * 32 + j % LG];
         if (rc.texel >= 0) {
           if (rc.texel != cur) {
             if (cur >= 0) flush();
             cur = rc.texel;
-            float t00[CPL], t01[CPL], t10[CPL], t11[CPL];
+            Tex4<T> t00, t01, t10, t11;
             const T* p00 = src_lane + (size_t)rc.texel * C;
             const T* p10 = p00 + row;
-            Vec<T, float, CPL>::load(p00, t00);
-            Vec<T, float, CPL>::load(p00 + C, t01);
-            Vec<T, float, CPL>::load(p10, t10);
-            Vec<T, float, CPL>::load(p10 + C, t11);
+            t00.load(p00);
+            t01.load(p00 + C);
+            t10.load(p10);
+            t11.load(p10 + C);
 #pragma unroll
             for (int q = 0; q < NG; ++q) T1R[q] = UR[q] = VR[q] = m[0][q] = m[1][q] = m[2][q] = m[3][q] = 0.0f;
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
               const int q = k / SUB;
-              a0[k] = t00[k];
-              u[k] = t10[k] - t00[k];
-              v[k] = t01[k] - t00[k];
-              t1[k] = (t11[k] - t01[k]) - u[k];
+              a0[k] = t00.get(k);
+              u[k] = t10.minus(k, a0[k]);
+              const float c01 = t01.get(k);
+              v[k] = c01 - a0[k];
+              t1[k] = t11.minus(k, c01) - u[k];
               T1R[q] = fmaf(t1[k], refv[k], T1R[q]);
               UR[q] = fmaf(u[k], refv[k], UR[q]);
               VR[q] = fmaf(v[k], refv[k], VR[q]);
             }
           }
-          const RecG rq = rGp[j];
+          const RecG rq = rGp[(j / LG) * 32 + j % LG];
           float cgv[NG];
 #pragma unroll
           for (int q = 0; q < NG; ++q) cgv[q] = cgall[j][q];
@@ -1222,18 +1230,23 @@ __global__ void __launch_bounds__(128, CHOP_V2_BWD_MIN_BLOCKS) cv2_bwd_tuned(con
       }
       if (cur >= 0) flush();
     }
-    // reduce-scatter the per-plane partials over the pixel's LG lanes: lane li keeps plane li
+    // reduce-scatter the per-plane partials over the pixel's LG lanes: lane li keeps the planes that it projected
 #pragma unroll
-    for (int s = LG / 2; s >= 1; s >>= 1) {
+    for (int p = 0; p < PL; ++p) {
+      float* part = dv + p * LG;
 #pragma unroll
-      for (int i = 0; i < s; ++i) {
-        const bool hi = (li & s) != 0;
-        const float keep = hi ? dv[i + s] : dv[i];
-        const float send = hi ? dv[i] : dv[i + s];
-        dv[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+      for (int s = LG / 2; s >= 1; s >>= 1) {
+#pragma unroll
+        for (int i = 0; i < s; ++i) {
+          const bool hi = (li & s) != 0;
+          const float keep = hi ? part[i + s] : part[i];
+          const float send = hi ? part[i] : part[i + s];
+          part[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+        }
       }
+      const int dA = dblk + p * LG + li;
+      if (pvalid && dA < dhi) dgrad[dA] = part[0];   // v2:477 (plain store; zero for a voxel no view saw)
     }
-    if (dvA) dgrad[dA] = dv[0];   // v2:477 (plain store; zero for a voxel no view saw)
   }
 
   if (pvalid) red_add<float, CPL>(static_cast<float*>(a.ref_grad) + pix * C + li * CPL, rg);
