@@ -40,6 +40,8 @@ int run_wgrad(int dtype, const ScArgs& a, int nparts, cudaStream_t st) {
     if (nparts > ntiles) nparts = (int)ntiles;
     return chop::sc_umma_wgrad_launch(a, nparts, st);
   }
+  if (chop::g_use_tile.load() == 1 && chop::sc_run_wgrad_supported(dtype, a) && al16(a.images) && al16(a.out_grad))
+    return chop::sc_run_wgrad_launch(a, nparts, st);
   if (chop::g_use_tile.load() && chop::sc_tile_supported(dtype, a) && al16(a.images) && al16(a.out_grad) &&
       al16(a.workspace))
     return chop::sc_tile_wgrad_launch(dtype, a, nparts, st);

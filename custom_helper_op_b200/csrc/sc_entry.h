@@ -28,6 +28,8 @@ int sc_tile_gather_launch(int dtype, const ScArgs& a, cudaStream_t st);
 // float32, 3x3x3, stride 1, by runs of planes (sc_run.cu) or on the tensor cores (sc_band.cu); the filter may lie at any address
 bool sc_run_supported(int dtype, const ScArgs& a, int gathered);
 int sc_run_launch(const ScArgs& a, bool dgrad, cudaStream_t st);
+bool sc_run_wgrad_supported(int dtype, const ScArgs& a);
+int sc_run_wgrad_launch(const ScArgs& a, int nparts, cudaStream_t st);
 // sums nparts slabs of taps*KC*NC + 1 floats; default_grad may be null
 int sc_slab_reduce(const float* part, int nparts, int taps, int KC, int NC, bool transposed, float* filter_grad,
                    float* default_grad, cudaStream_t st);

@@ -186,6 +186,199 @@ int launch_run(const ScArgs& a, cudaStream_t st) {
   return launch_tz<KCH, NCH, 4, FWD>(a, st);
 }
 
+// Filter gradient of the same convolution: dW[fr,fc,fz][k][n] = sum over voxels of gathered[k] * upstream[n].
+// A thread holds four gathered and eight upstream channels of the THREE depth taps of one filter column, 96 sums in pairs, and
+// walks the planes of a pixel: the neighbour's row of one plane meets the upstream rows of three, so a plane costs it one 16-byte
+// load of gathered values and two (warp-uniform but for the channels) of upstream ones for 48 paired multiply-adds, where a
+// thread per tap loads five for 32.  288 threads are 9 columns x the channel blocks x as many groups as that leaves room for, each
+// with pixels of its own; their sums are added in shared memory in a fixed order and sc_slab_reduce adds the CTAs'.
+// The upstream rows of the next pixels are copied while the present ones are multiplied.
+// Bound: issue and latency at three warps a scheduler (158 registers).  189x251x7, float32, 3x3x3, the filter gradient and its
+// reduction, us before (sc_tile.cu) and now: 16 -> 16 channels 215, 140; 8 -> 8 95, 48; 32 -> 32 670, 570.  Four upstream channels per
+// thread and two CTAs of nine warps 205, 288 threads 170.  Error against float64 (2-norm), 60x80: 16 -> 16 at 17 planes 2.39e-7
+// before, 2.3e-7 now; 32 -> 32 3.3e-7, 2.4e-7.
+constexpr int WG_THR = 384;   // twelve warps, three to a scheduler; 288 left one with three and three with two
+constexpr int WG_CHAIN = 64;    // planes after which a thread's sums go to its group's table, which keeps the chains of additions short
+template <int KCH, int NCH>
+struct WgRun {
+  static constexpr int QK = KCH / 4, QN = NCH / 8;    // channel blocks
+  static constexpr int TPG = 9 * QK * QN, GROUPS = WG_THR / TPG;
+  static constexpr int SUMS = 27 * KCH * NCH;
+  static constexpr size_t TABLE = (size_t)GROUPS * SUMS * 4;
+  // two buffers of upstream rows and (first voxel, shift) per pixel and column, behind the groups' tables
+  static size_t stage(int px, int D) { return (size_t)px * D * NCH * 4 + (size_t)px * 9 * sizeof(int2); }
+  static int pixels(int D) {                          // per stage: whole rounds of the groups, about 24 KB
+    int r = (int)(24 * 1024 / stage(GROUPS, D));
+    return GROUPS * (r < 1 ? 1 : r > 8 ? 8 : r);
+  }
+  static size_t smem(int D) { return TABLE + 2 * ((stage(pixels(D), D) + 15) / 16 * 16); }
+};
+
+template <int KCH, int NCH>
+__global__ void __launch_bounds__(WG_THR, 1) sc_wgrad_run_kernel(const __grid_constant__ ScArgs a, const int px, const int stage_bytes,
+                                                                 const unsigned pix_per_cta, const int chain_max) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef WgRun<KCH, NCH> Cf;
+  const int D = a.D, H = a.H, W = a.W, tid = threadIdx.x;
+  const unsigned npix = (unsigned)a.B * H * W;
+  const unsigned p0 = blockIdx.x * pix_per_cta, p1 = min(npix, p0 + pix_per_cta);
+  const float* og = static_cast<const float*>(a.out_grad);
+  auto rows_of = [&](int buf) { return reinterpret_cast<float*>(smem_raw + Cf::TABLE + (size_t)buf * stage_bytes); };
+  auto tab_of = [&](int buf) { return reinterpret_cast<int2*>(smem_raw + Cf::TABLE + (size_t)buf * stage_bytes + (size_t)px * D * NCH * 4); };
+  auto fetch = [&](unsigned first, int buf) {         // px pixels from `first` on
+    const int n = (int)min((unsigned)px, p1 - first);
+    float* rows = rows_of(buf);
+    const float* from = og + (size_t)first * D * NCH;
+    for (int e = tid * 4; e < n * D * NCH; e += WG_THR * 4)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(rows + e)), "l"(from + e) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    int2* tab = tab_of(buf);
+    for (int e = tid; e < n * 9; e += WG_THR) {
+      const unsigned pix = first + e / 9;
+      const int col = e % 9, c = (int)(pix % (unsigned)W), r = (int)(pix / (unsigned)W % (unsigned)H);
+      const int orow = r - 1 + col / 3, ocol = c - 1 + col % 3;
+      int2 ent = make_int2(-1, 0);
+      if (!oob(orow, H) && !oob(ocol, W)) {
+        const unsigned np = pix + (col / 3 - 1) * W + (col % 3 - 1);
+        ent = make_int2((int)(np * D), __ldg(a.base_plane + pix) - __ldg(a.base_plane + np));
+      }
+      tab[e] = ent;
+    }
+  };
+  // lanes: channel blocks fastest, so that a warp's loads of gathered rows are whole rows
+  const int group = tid / Cf::TPG, t = tid % Cf::TPG;
+  const int qk = t % Cf::QK, qn = t / Cf::QK % Cf::QN, col = t / (Cf::QK * Cf::QN);
+  const float pad = __ldg(static_cast<const float*>(a.default_value));
+  const float4 pad4 = make_float4(pad, pad, pad, pad);
+  const float* img = static_cast<const float*>(a.images) + qk * 4;
+  constexpr int NN = 8;
+  pk2 acc[3][4][NN / 2];
+#pragma unroll
+  for (int f = 0; f < 3; ++f)
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int n = 0; n < NN / 2; ++n) acc[f][k][n] = 0ull;
+
+  // table of a group: [3*4*NN/2 pairs][TPG threads]
+  pk2* mine = reinterpret_cast<pk2*>(smem_raw) + (size_t)group * (12 * NN / 2) * Cf::TPG + t;
+  bool written = false;
+  auto put = [&]() {
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int n = 0; n < NN / 2; ++n) {
+          pk2* o = mine + ((f * 4 + k) * (NN / 2) + n) * Cf::TPG;
+          *o = written ? pk_add(*o, acc[f][k][n]) : acc[f][k][n];
+          acc[f][k][n] = 0ull;
+        }
+    written = true;
+  };
+  const bool active = group < Cf::GROUPS;
+  int buf = 0, chain = 0;
+  if (p0 < p1) fetch(p0, 0);
+  for (unsigned first = p0; first < p1; first += px, buf ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                  // this stage has landed; the other one has been read
+    if (first + px < p1) fetch(first + px, buf ^ 1);
+    const int n = (int)min((unsigned)px, p1 - first);
+    for (int i = active ? group : n; i < n; i += Cf::GROUPS) {
+      if (chain >= chain_max) {
+        put();
+        chain = 0;
+      }
+      chain += D;
+      const int2 e = tab_of(buf)[i * 9 + col];
+      const ulonglong2* g = reinterpret_cast<const ulonglong2*>(rows_of(buf) + (size_t)i * D * NCH + qn * NN);
+      auto row = [&](int plane) {                     // gathered row of a plane of the neighbour, or padding
+        float4 v = pad4;
+        if (e.x >= 0 && !oob(plane, D)) v = __ldg(reinterpret_cast<const float4*>(img + (size_t)(e.x + plane) * KCH));
+        return v;
+      };
+      const int s = e.y;                              // plane z of the pixel is plane z + s of the neighbour
+      pk2 x[3][4];
+      auto splat = [](pk2 (&o)[4], const float4& v) {
+        o[0] = pk_make(v.x, v.x);
+        o[1] = pk_make(v.y, v.y);
+        o[2] = pk_make(v.z, v.z);
+        o[3] = pk_make(v.w, v.w);
+      };
+      auto plane = [&](const pk2 (&lo)[4], const pk2 (&mid)[4], const pk2 (&hi)[4], int z) {
+        pk2 gs[NN / 2];
+#pragma unroll
+        for (int n = 0; n < NN / 4; ++n) {
+          const ulonglong2 v = g[z * (NCH / 4) + n];
+          gs[2 * n] = v.x;
+          gs[2 * n + 1] = v.y;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int n = 0; n < NN / 2; ++n) {
+            pk_fma_to(acc[0][k][n], lo[k], gs[n]);
+            pk_fma_to(acc[1][k][n], mid[k], gs[n]);
+            pk_fma_to(acc[2][k][n], hi[k], gs[n]);
+          }
+      };
+      splat(x[0], row(s - 1));
+      splat(x[1], row(s));
+      float4 n0 = row(s + 1), n1 = row(s + 2), n2 = row(s + 3);   // requested three planes ahead
+      for (int z = 0; z < D; z += 3) {
+        splat(x[2], n0);
+        n0 = row(z + s + 4);
+        plane(x[0], x[1], x[2], z);
+        if (z + 1 < D) {
+          splat(x[0], n1);
+          n1 = row(z + s + 5);
+          plane(x[1], x[2], x[0], z + 1);
+        }
+        if (z + 2 < D) {
+          splat(x[1], n2);
+          n2 = row(z + s + 6);
+          plane(x[2], x[0], x[1], z + 2);
+        }
+      }
+    }
+  }
+  if (active) put();
+  __syncthreads();
+  // the groups' sums, in order
+  float* part = static_cast<float*>(a.workspace) + (size_t)blockIdx.x * (Cf::SUMS + 1);
+  const float* table = reinterpret_cast<const float*>(smem_raw);
+  for (int e = tid; e < Cf::SUMS; e += WG_THR) {
+    const int n = e % NCH, k = e / NCH % KCH, tap = e / (NCH * KCH);
+    const int pair = ((tap % 3) * 4 + k % 4) * (NN / 2) + n % NN / 2, th = (tap / 3 * Cf::QN + n / NN) * Cf::QK + k / 4;
+    float v = 0.f;
+    for (int gr = 0; gr < Cf::GROUPS; ++gr) v += table[(((size_t)gr * (12 * NN / 2) + pair) * Cf::TPG + th) * 2 + n % 2];
+    part[e] = v;
+  }
+  if (tid == 0) part[Cf::SUMS] = 0.f;                 // the default value's gradient: not asked for
+}
+
+template <int KCH, int NCH>
+int launch_wgrad(const ScArgs& a, int nparts, cudaStream_t st) {
+  typedef WgRun<KCH, NCH> Cf;
+  auto k = sc_wgrad_run_kernel<KCH, NCH>;
+  const int px = Cf::pixels(a.D);
+  const size_t smem = Cf::smem(a.D), stage = (Cf::stage(px, a.D) + 15) / 16 * 16;
+  if (int e = grant_smem(k, smem)) return e;
+  const unsigned npix = (unsigned)a.B * a.H * a.W;
+  if (nparts > 148) nparts = 148;                     // one CTA per SM
+  const unsigned rounds = (npix + Cf::GROUPS - 1) / Cf::GROUPS;   // whole rounds of the groups
+  if ((unsigned)nparts > rounds) nparts = (int)rounds;
+  const unsigned per = (rounds + nparts - 1) / nparts * Cf::GROUPS;
+  nparts = (int)((npix + per - 1) / per);             // every CTA owns at least one pixel and writes its slab
+  // a small problem has short chains anyway: half of a thread's planes (32 instead of 64 costs 12 us at 189x251x7)
+  const long long half = (long long)per / Cf::GROUPS * a.D / 2;
+  k<<<nparts, WG_THR, smem, st>>>(a, px, (int)stage, per, half < WG_CHAIN ? (int)half : WG_CHAIN);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return (int)e;
+  return sc_slab_reduce(static_cast<const float*>(a.workspace), nparts, 27, KCH, NCH, false, static_cast<float*>(a.filter_grad),
+                        static_cast<float*>(a.default_grad), st);
+}
+
 }  // namespace
 
 // Runs that leave up to a third of their planes empty are still the faster ones (sc_tile.cu at 120x150x5, two runs of four planes:
@@ -201,6 +394,20 @@ int sc_run_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {
   const int in = dgrad ? a.Cout : a.Cin, out = dgrad ? a.Cin : a.Cout;
   if (sc_band_f32_better(a, in, out)) return sc_band_f32_launch(a, dgrad, st);
 #define CHOP_CASE(K, N) if (in == K && out == N) return dgrad ? launch_run<K, N, false>(a, st) : launch_run<K, N, true>(a, st);
+  CHOP_CASE(8, 8) CHOP_CASE(8, 16) CHOP_CASE(8, 32) CHOP_CASE(16, 8) CHOP_CASE(16, 16) CHOP_CASE(16, 32) CHOP_CASE(32, 8)
+  CHOP_CASE(32, 16) CHOP_CASE(32, 32)
+#undef CHOP_CASE
+  return -4;
+}
+
+// Filter gradient; a.images and a.out_grad 16-byte aligned, nparts slabs of 27*Cin*Cout + 1 floats in the workspace.
+bool sc_run_wgrad_supported(int dtype, const ScArgs& a) {
+  auto ok = [](int c) { return c == 8 || c == 16 || c == 32; };
+  return dtype == 0 && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 && a.sr == 1 && a.sc == 1 &&
+         a.sd == 1 && ok(a.Cin) && ok(a.Cout) && !a.dynamic_default && a.D <= 64 && a.nvox_in < (1LL << 31) - 4096;
+}
+int sc_run_wgrad_launch(const ScArgs& a, int nparts, cudaStream_t st) {
+#define CHOP_CASE(K, N) if (a.Cin == K && a.Cout == N) return launch_wgrad<K, N>(a, nparts, st);
   CHOP_CASE(8, 8) CHOP_CASE(8, 16) CHOP_CASE(8, 32) CHOP_CASE(16, 8) CHOP_CASE(16, 16) CHOP_CASE(16, 32) CHOP_CASE(32, 8)
   CHOP_CASE(32, 16) CHOP_CASE(32, 32)
 #undef CHOP_CASE

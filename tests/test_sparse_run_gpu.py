@@ -29,12 +29,14 @@ def test_against_the_oracle(D, spread, chans):
     images, filters, bp, og = _case(D + spread, 2, 9, 21, D, Cin, Cout, spread)
     defv = 0.5
     want = oracle.sparse_conv3d_fwd(images, filters, defv, bp)
-    ig_w = oracle.sparse_conv3d_bwd(images, filters, defv, bp, og)[0]
+    ig_w, fg_w, _ = oracle.sparse_conv3d_bwd(images, filters, defv, bp, og)
     out = ops.sparse_conv3d_forward(cuda(images), cuda(filters), defv, cuda(bp))
-    ig = ops.sparse_conv3d_backward(cuda(images), cuda(filters), defv, cuda(bp), cuda(og))[0]
+    ig, fg, dg = ops.sparse_conv3d_backward(cuda(images), cuda(filters), defv, cuda(bp), cuda(og))
     # 27 * channels products of order one, summed in 24 bits: some units of 2^-24 times the root of the number of terms
     assert helpers.rel_err(out.cpu().numpy(), want) <= 3e-6
     assert helpers.rel_err(ig.cpu().numpy(), ig_w) <= 3e-6
+    # 2*9*21*D products: the root of their number times 2^-24, against the largest sum of as many
+    assert helpers.rel_err(fg.cpu().numpy(), fg_w) <= 3e-6 and float(dg) == 0.0
     coarse = og                                            # the transposed op at strides 1: gather form with the real default
     t_w = oracle.sparse_conv3d_transpose_fwd(coarse, filters, defv, bp, images.shape[1:4])
     t = ops.sparse_conv3d_transpose_forward(cuda(coarse), cuda(filters), defv, cuda(bp), images.shape[1:4])
