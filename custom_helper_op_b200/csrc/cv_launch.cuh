@@ -127,10 +127,14 @@ inline int agg_min_fwd_tuned_go(const CvArgs& a, cudaStream_t st) {
   return (int)cudaGetLastError();
 }
 
-template <typename T, int C, int CPL, bool AGG = false, bool RMIN = false>
-inline int bwd_tuned_go(const CvArgs& a, cudaStream_t st) {
-  auto k = cv_bwd_tuned<T, C, CPL, AGG, RMIN>;
-  const size_t spw = tuned_bwd_smem_per_warp<C>(a.N, 32 / (C / CPL), (RMIN && !AGG) ? 2 : 1);
+template <typename T, int C, int CPL, bool AGG, bool RMIN, int PL>
+inline int bwd_tuned_pl(const CvArgs& a0, cudaStream_t st) {
+  constexpr int PB = C / CPL * PL;
+  CvArgs a = a0;
+  a.chunk = (a.chunk + PB - 1) / PB * PB;
+  a.nchunks = (a.d_end - a.d_begin + a.chunk - 1) / a.chunk;
+  auto k = cv_bwd_tuned<T, C, CPL, AGG, RMIN, PL>;
+  const size_t spw = tuned_bwd_smem_per_warp<C>(a.N, 32 / (C / CPL), AGG ? 0 : RMIN ? 2 : 1, PL);
   const int warps = 4;
   const size_t smem = spw * warps;
   if (smem > 200 * 1024) return -4;
@@ -138,6 +142,19 @@ inline int bwd_tuned_go(const CvArgs& a, cudaStream_t st) {
   const long long items = (long long)a.npb * a.nchunks;
   k<<<(unsigned)((items + warps - 1) / warps), warps * 32, smem, st>>>(a, warps, spw);
   return (int)cudaGetLastError();
+}
+// Eight and sixteen channels have two and four lanes per pixel, and a block of as many planes, at whose end every footprint is flushed.
+// Blocks of twice the planes halve that while the records and the staged upstream slice of the 24 warps that registers allow still
+// fit into an SM's shared memory.  128x160x192, one / two views, us with short and with long blocks: CostVolume C = 8 113 / 163, 104 / 152,
+// C = 16 132 / 195, 127 / 179; CostAggregate C = 8 97 / 148, 87 / 129, C = 16 110 / 173, 101 / 153.  Where they do not fit: CostVolume, six
+// views, C = 16 300, 338; CostAggregate MIN, four views, C = 8 131, 143.  With winners staged too (CostVolume MIN) they lose: C = 16 223, 245.
+template <typename T, int C, int CPL, bool AGG = false, bool RMIN = false>
+inline int bwd_tuned_go(const CvArgs& a, cudaStream_t st) {
+  if constexpr (C <= 16 && (AGG || !RMIN)) {
+    if (24 * tuned_bwd_smem_per_warp<C>(a.N, 32 / (C / CPL), AGG ? 0 : 1, 2) <= (RMIN ? 180 : 216) * 1024)
+      return bwd_tuned_pl<T, C, CPL, AGG, RMIN, 2>(a, st);
+  }
+  return bwd_tuned_pl<T, C, CPL, AGG, RMIN, 1>(a, st);
 }
 
 template <typename T, int C, int SUB>

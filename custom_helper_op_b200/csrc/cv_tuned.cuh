@@ -439,21 +439,16 @@ __global__ void __launch_bounds__(256, 2) cv_agg_min_fwd_tuned(const CvArgs a, c
 #ifndef CHOP_BWD_MIN_BLOCKS
 #define CHOP_BWD_MIN_BLOCKS 6
 #endif
-#ifndef CHOP_BWD_CG_BUFS
-#define CHOP_BWD_CG_BUFS 1
-#endif
-constexpr int CG_BUFS = CHOP_BWD_CG_BUFS;  // 2: copy a block ahead into the other buffer; 1: copy after use
-
 struct alignas(8) RecG {
   float gh, gw;  // d(sample row)/d(depth), d(sample column)/d(depth)
 };
 
 // `staged` = per-channel tensors copied into shared memory ahead of use: cost_grad, and for MIN also
-// the arg-index tensor; each buffer holds G*LG*C values = 128*C bytes.
+// the arg-index tensor; each buffer holds G*LG*PL*C values = 128*C*PL bytes.
 template <int C>
-__host__ __device__ inline size_t tuned_bwd_smem_per_warp(int N, int G, int staged = 1) {
-  return (size_t)N * G * sizeof(Coef<float>) + (size_t)N * 32 * (sizeof(ProjF<float>) + sizeof(RecG)) +
-         (size_t)staged * CG_BUFS * 128 * C;
+__host__ __device__ inline size_t tuned_bwd_smem_per_warp(int N, int G, int staged, int PL) {
+  return (size_t)N * G * sizeof(Coef<float>) + (size_t)N * PL * 32 * (sizeof(ProjF<float>) + sizeof(RecG)) +
+         (size_t)staged * PL * 128 * C;
 }
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
@@ -488,11 +483,12 @@ __device__ __forceinline__ void flush_corners(float* gp, size_t row, int C, floa
 // RMIN = true is the MIN reduction: `mask` holds the winning view per (voxel, channel) (per voxel for
 // AGG) and only that view receives the gradient (cost_volume_kernels_gpu.cu.cc:472-577,
 // cost_aggregate_kernels_gpu.cu.cc:462-568); a voxel whose first channel has no winner is skipped (:484).
-template <typename T, int C, int CPL, bool AGG = false, bool RMIN = false>
+template <typename T, int C, int CPL, bool AGG = false, bool RMIN = false, int PL = 1>
 __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const CvArgs a, const int warps, const size_t smem_per_warp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int LG = C / CPL;
   constexpr int G = 32 / LG;
+  constexpr int PB = LG * PL;   // planes per block: PL per lane in phase A
   static_assert(CPL == 4, "the cost_grad staging copies 16 bytes per lane and plane");
   static_assert(LG * CPL == C && (LG & (LG - 1)) == 0 && LG <= 32, "C/CPL must be a power of two <= 32");
   const int lane = threadIdx.x & 31;
@@ -515,11 +511,11 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
   unsigned char* mine = smem_raw + (size_t)wib * smem_per_warp;
   Coef<float>* coef = reinterpret_cast<Coef<float>*>(mine);
   ProjF<float>* recA = reinterpret_cast<ProjF<float>*>(coef + N * G);  // aux = 2/(valid views)
-  RecG* recG = reinterpret_cast<RecG*>(recA + N * 32);
-  float* cgbuf = reinterpret_cast<float*>(recG + N * 32);             // [2][G][LG][C]
-  float* cg_mine = cgbuf + (g * LG) * C + li * CPL;                    // + buf*32*C + j*C
+  RecG* recG = reinterpret_cast<RecG*>(recA + N * PL * 32);
+  float* cgbuf = reinterpret_cast<float*>(recG + N * PL * 32);        // [G][PB][C]
+  float* cg_mine = cgbuf + (g * PB) * C + li * CPL;                    // + j*C
   constexpr bool STAGE_MASK = RMIN && !AGG;
-  constexpr int MK_OFF = CG_BUFS * 32 * C;                             // arg indices behind the cost_grad buffers
+  constexpr int MK_OFF = G * PB * C;                                   // arg indices behind the cost_grad buffers
 
   stage_coefs<float>(a, coef, lane, G, pix0);
 
@@ -540,7 +536,7 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
   // stage the first block's upstream gradient
   if constexpr (!AGG) {
 #pragma unroll
-    for (int j = 0; j < LG; ++j) {
+    for (int j = 0; j < PB; ++j) {
       if (dlo + j < dhi) {
         cp_async16(cg_mine + j * C, cg_src + j * C);
         if (STAGE_MASK) cp_async16(cg_mine + MK_OFF + j * C, mk_src + j * C);
@@ -556,45 +552,33 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
   // The lane's validity count / winning view of plane dblk+li streams in from HBM: it is requested one block ahead,
   // so phase A does not start with an exposed DRAM round trip.
   const int mk_stride = (RMIN && !AGG) ? C : 1;
-  int m_next = 0;
-  float ag_next = 0.0f;   // aggregate: the voxel's single upstream value, requested a block ahead as well
-  if (pvalid && dlo + li < dhi) {
-    m_next = __ldg(a.mask + (pix * D + dlo + li) * mk_stride);
-    if (AGG) ag_next = __ldg(static_cast<const float*>(a.cost_grad) + pix * D + dlo + li);
-  }
-  int buf = 0;
-  for (int dblk = dlo; dblk < dhi; dblk += LG, cg_src += LG * C, buf ^= (CG_BUFS - 1)) {
-    if (!AGG && CG_BUFS == 2) {
-      cp_async_wait_all();  // this block's slice has landed (each lane reads back only what it copied)
-      __syncwarp();         // and every lane is done with the other buffer and with the records
-      const int nxt = dblk + LG;
-      float* dst = cg_mine + (buf ^ 1) * 32 * C;
+  int m_next[PL];
+  float ag_next[PL];   // aggregate: the voxel's single upstream value, requested a block ahead as well
 #pragma unroll
-      for (int j = 0; j < LG; ++j) {
-        if (nxt + j < dhi) {
-          cp_async16(dst + j * C, cg_src + (LG + j) * C);
-          if (STAGE_MASK) cp_async16(dst + MK_OFF + j * C, mk_src + (nxt - dlo + j) * C);
-        } else {
-          *reinterpret_cast<float4*>(dst + j * C) = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (STAGE_MASK) *reinterpret_cast<int4*>(dst + MK_OFF + j * C) = make_int4(-1, -1, -1, -1);
-        }
-      }
-      cp_async_commit();
-    } else {
-      __syncwarp();
+  for (int p = 0; p < PL; ++p) {
+    m_next[p] = 0;
+    ag_next[p] = 0.0f;
+    const int d = dlo + p * LG + li;
+    if (pvalid && d < dhi) {
+      m_next[p] = __ldg(a.mask + (pix * D + d) * mk_stride);
+      if (AGG) ag_next[p] = __ldg(static_cast<const float*>(a.cost_grad) + pix * D + d);
     }
+  }
+  for (int dblk = dlo; dblk < dhi; dblk += PB, cg_src += PB * C) {
+    __syncwarp();
 
     // ---- phase A: lane (g, li) projects plane dblk+li of pixel g into every view ---------------------
-    {
-      const int d = dblk + li;
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      const int d = dblk + p * LG + li;
       const bool dv = pvalid && d < dhi;
       float depth = 0.0f, scale = 0.0f;
       bool live = false;
-      const int m0 = m_next;
-      const float ag0 = ag_next;
-      if (pvalid && d + LG < dhi) {
-        m_next = __ldg(a.mask + (pix * D + d + LG) * mk_stride);
-        if (AGG) ag_next = __ldg(static_cast<const float*>(a.cost_grad) + pix * D + d + LG);
+      const int m0 = m_next[p];
+      const float ag0 = ag_next[p];
+      if (pvalid && d + PB < dhi) {
+        m_next[p] = __ldg(a.mask + (pix * D + d + PB) * mk_stride);
+        if (AGG) ag_next[p] = __ldg(static_cast<const float*>(a.cost_grad) + pix * D + d + PB);
       }
       if (dv) {
         depth = xadd(base, offs[d]);
@@ -623,18 +607,18 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
         // aggregate MIN: only the winning view of the voxel is differentiated
         if (live && (!(RMIN && AGG) || m0 == n))
           r.texel = project<float, true>(coef[n * G + g], depth, a, r.dh, r.dw, q.gh, q.gw);
-        recA[n * 32 + lane] = r;
-        recG[n * 32 + lane] = q;
+        recA[(n * PL + p) * 32 + lane] = r;
+        recG[(n * PL + p) * 32 + lane] = q;
       }
     }
-    if (!AGG && CG_BUFS == 1) cp_async_wait_all();  // the slice requested at the end of the previous block
+    if (!AGG) cp_async_wait_all();  // the slice requested at the end of the previous block
     __syncwarp();
 
     // ---- phase B ---------------------------------------------------------------------------------------
-    const float* cgb = cg_mine + buf * 32 * C;
+    const float* cgb = cg_mine;
     for (int n = 0; n < N; ++n) {
-      const ProjF<float>* rA = recA + n * 32 + g * LG;
-      const RecG* rGp = recG + n * 32 + g * LG;
+      const ProjF<float>* rA = recA + n * PL * 32 + g * LG;   // plane j: entry (j / LG) * 32 + j % LG
+      const RecG* rGp = recG + n * PL * 32 + g * LG;
       int cur = -1;
       float a0[CPL], u[CPL], v[CPL], t1[CPL], acc[4][CPL];
 #pragma unroll
@@ -643,8 +627,8 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
         acc[0][k] = acc[1][k] = acc[2][k] = acc[3][k] = 0.0f;
       }
 #pragma unroll
-      for (int j = 0; j < LG; ++j) {
-        const ProjF<float> rc = rA[j];
+      for (int j = 0; j < PB; ++j) {
+        const ProjF<float> rc = rA[(j / LG) * 32 + j % LG];
         if (rc.texel >= 0) {
           if (rc.texel != cur) {
             if (cur >= 0) flush_corners<CPL>(sg_lane + (size_t)cur * C, row, C, acc, rg);
@@ -666,7 +650,7 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
               acc[0][k] = acc[1][k] = acc[2][k] = acc[3][k] = 0.0f;
             }
           }
-          const RecG rq = rGp[j];
+          const RecG rq = rGp[(j / LG) * 32 + j % LG];
           float cgs[4];
           if constexpr (AGG) {
             cgs[0] = cgs[1] = cgs[2] = cgs[3] = rc.aux;
@@ -705,13 +689,13 @@ __global__ void __launch_bounds__(128, CHOP_BWD_MIN_BLOCKS) cv_bwd_tuned(const C
       }
       if (cur >= 0) flush_corners<CPL>(sg_lane + (size_t)cur * C, row, C, acc, rg);
     }
-    if (!AGG && CG_BUFS == 1) {
-      // single buffer: each lane has finished reading its own slots, request the next block's slice now
-      const int nxt = dblk + LG;
+    if (!AGG) {
+      // each lane has finished reading its own slots, request the next block's slice now
+      const int nxt = dblk + PB;
 #pragma unroll
-      for (int j = 0; j < LG; ++j) {
+      for (int j = 0; j < PB; ++j) {
         if (nxt + j < dhi) {
-          cp_async16(cg_mine + j * C, cg_src + (LG + j) * C);
+          cp_async16(cg_mine + j * C, cg_src + (PB + j) * C);
           if (STAGE_MASK) cp_async16(cg_mine + MK_OFF + j * C, mk_src + (nxt - dlo + j) * C);
         } else {
           *reinterpret_cast<float4*>(cg_mine + j * C) = make_float4(0.f, 0.f, 0.f, 0.f);
