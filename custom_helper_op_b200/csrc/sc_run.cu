@@ -400,11 +400,21 @@ int sc_run_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {
   return -4;
 }
 
-// Filter gradient; a.images and a.out_grad 16-byte aligned, nparts slabs of 27*Cin*Cout + 1 floats in the workspace.
+namespace {
+size_t wgrad_run_smem(int k, int n, int D) {
+#define CHOP_CASE(K, N) if (k == K && n == N) return WgRun<K, N>::smem(D);
+  CHOP_CASE(8, 8) CHOP_CASE(8, 16) CHOP_CASE(8, 32) CHOP_CASE(16, 8) CHOP_CASE(16, 16) CHOP_CASE(16, 32) CHOP_CASE(32, 8)
+  CHOP_CASE(32, 16) CHOP_CASE(32, 32)
+#undef CHOP_CASE
+  return (size_t)-1;   // other channel counts
+}
+}  // namespace
+// Filter gradient; a.images and a.out_grad 16-byte aligned, nparts slabs of 27*Cin*Cout + 1 floats in the workspace.  Bands whose
+// stages do not fit beside the groups' tables (8 -> 8 channels: more than 57 planes) take sc_tile.cu's.
 bool sc_run_wgrad_supported(int dtype, const ScArgs& a) {
-  auto ok = [](int c) { return c == 8 || c == 16 || c == 32; };
   return dtype == 0 && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 && a.sr == 1 && a.sc == 1 &&
-         a.sd == 1 && ok(a.Cin) && ok(a.Cout) && !a.dynamic_default && a.D <= 64 && a.nvox_in < (1LL << 31) - 4096;
+         a.sd == 1 && !a.dynamic_default && a.D <= 64 && wgrad_run_smem(a.Cin, a.Cout, a.D) <= 220 * 1024 &&
+         a.nvox_in < (1LL << 31) - 4096;
 }
 int sc_run_wgrad_launch(const ScArgs& a, int nparts, cudaStream_t st) {
 #define CHOP_CASE(K, N) if (a.Cin == K && a.Cout == N) return launch_wgrad<K, N>(a, nparts, st);

@@ -22,7 +22,7 @@ def _case(seed, B, H, W, D, Cin, Cout, spread):
 cuda = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to("cuda")
 
 
-@pytest.mark.parametrize("D,spread", [(1, 2), (3, 0), (4, 9), (5, 60), (7, 7), (7, 8), (10, 4), (11, 19), (11, 300), (24, 6), (25, 3)])
+@pytest.mark.parametrize("D,spread", [(1, 2), (3, 0), (4, 9), (5, 60), (7, 7), (7, 8), (10, 4), (11, 19), (11, 300), (24, 6), (25, 3), (64, 2)])
 @pytest.mark.parametrize("chans", [(16, 16), (16, 32), (32, 16), (8, 16), (32, 8), (8, 8)])
 def test_against_the_oracle(D, spread, chans):
     Cin, Cout = chans
