@@ -41,6 +41,12 @@ int sc_band_f32_launch(const ScArgs& a, bool dgrad, cudaStream_t st);   // float
 int sc_band_timeouts();
 int sc_band_publish_mirror(int* dptr);
 int sc_band_clear_timeouts();
+// strided gather form with every coarse voxel staged once (sc_up.cu)
+bool sc_up_supported(const ScArgs& a);
+int sc_up_launch(const ScArgs& a, cudaStream_t st);
+int sc_up_timeouts();
+int sc_up_publish_mirror(int* dptr);
+int sc_up_clear_timeouts();
 int sc_umma_timeouts();
 int sc_umma_watch();
 int sc_umma_note_timeout_for_test(int on);

@@ -36,7 +36,7 @@ namespace chop {
 namespace {
 
 __global__ void note_timeout_kernel() { note_timeout(); }
-std::atomic<int> g_umma_rows{1};   // tuning knob "umma_rows": 0 = always the per-tap gather, 2 = never sc_band.cu
+std::atomic<int> g_umma_rows{1};   // tuning knob "umma_rows": 0 = always the per-tap gather, 2 = never sc_band.cu and sc_up.cu
 
 // ---- tap geometry (3x3x3, dilation 1) -----------------------------------------------------------------------
 // The tile's voxels are OUTPUT voxels of the (strided) convolution, grid [B,oH,oW,oD]; a tap reads the input grid
@@ -1339,6 +1339,7 @@ int launch(const ScArgs& a, long long nvox, cudaStream_t st) {
   // otherwise at stride 1, for bands of at most 126 planes: the shifted-row kernel
   if (s1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_rows<CIN, COUT, DGRAD>(a, st);
   if constexpr (DGRAD) {
+    if (!s1 && g_umma_rows.load() == 1 && sc_up_supported(a)) return sc_up_launch(a, st);   // 256x320x9: 43 -> 32 us, see there
     if (!s1) return launch_class<CIN, COUT>(a, st);
   }
   auto k = s1 ? sc_umma_kernel<CIN, COUT, DGRAD, true> : sc_umma_kernel<CIN, COUT, DGRAD, DGRAD>;
@@ -1408,8 +1409,8 @@ int sc_umma_twgrad_launch(const ScArgs& a, int nparts, cudaStream_t st) {
 void sc_umma_set_rows(int on) { g_umma_rows = on; }
 
 int sc_umma_timeouts() {
-  const int here = timeouts_here(), band = sc_band_timeouts();
-  return here < 0 || band < 0 ? -1 : here + band;
+  const int here = timeouts_here(), band = sc_band_timeouts(), up = sc_up_timeouts();
+  return here < 0 || band < 0 || up < 0 ? -1 : here + band + up;
 }
 
 namespace {
@@ -1436,7 +1437,7 @@ int sc_umma_watch() {
   if (!((g_watch_devs >> dev) & 1ull)) {
     int* dptr = nullptr;
     if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&dptr), g_watch_host, 0) != cudaSuccess ||
-        publish_mirror_here(dptr) != cudaSuccess || sc_band_publish_mirror(dptr) != 0) {
+        publish_mirror_here(dptr) != cudaSuccess || sc_band_publish_mirror(dptr) != 0 || sc_up_publish_mirror(dptr) != 0) {
       cudaGetLastError();
       return -1;
     }
@@ -1452,7 +1453,7 @@ int sc_umma_note_timeout_for_test(int on) {
     note_timeout_kernel<<<1, 1>>>();
     return (int)cudaGetLastError();
   }
-  if (clear_timeouts_here() != cudaSuccess || sc_band_clear_timeouts() != 0) return (int)cudaGetLastError();
+  if (clear_timeouts_here() != cudaSuccess || sc_band_clear_timeouts() != 0 || sc_up_clear_timeouts() != 0) return (int)cudaGetLastError();
   std::lock_guard<std::mutex> lk(g_watch_mu);
   if (g_watch_host) *const_cast<volatile int*>(g_watch_host) = 0;
   return 0;

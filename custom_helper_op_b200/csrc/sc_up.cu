@@ -1,0 +1,322 @@
+// Strided gather form on the tensor cores with every coarse voxel staged once: the transposed convolution and the image gradient
+// of the strided one, 3x3x3, strides 2 along rows and columns and 1 or 2 along depth, bfloat16, float32 accumulation, 8 or 16
+// produced channels.
+//
+// Row r and column c of a fine voxel decide which filter columns exist there: (fr, fc) belongs to class (fr != 1, fc != 1) of
+// (r mod 2, c mod 2) and reads the coarse pixel (r/2 + (fr == 2), c/2 + (fc == 2)).  So the four fine pixels over one coarse pixel
+// read the 2x2 coarse pixels from there on, and the nine columns are spread over the four.  A tile is PT coarse pixels of a row;
+// the 2 x (PT+1) around them are staged once, as windows of RP absolute coarse planes (as in sc_band.cu), and each of the four
+// offsets is ONE operand for all classes that use it: the accumulators of the classes (1,0), (1,1), (0,1), (0,0) lie side by side, so the
+// offsets (0,0), (1,0), (0,1) and (1,1) are MMAs over four, two, two and one of them, each three depth taps wide.
+// Depth: accumulator row zc holds, per tap fz, the product with coarse plane zc.  At depth stride 2 the fine plane 2*zc is tap 1 of
+// row zc, 2*zc + 1 is tap 0 of row zc plus tap 2 of row zc + 1; at depth stride 1 rows z-1, z, z+1 add up.
+// What a tap reads that does not exist (default_value, zero in gradients) is a constant per class and parity, added at the end.
+// Base planes that do not fit the window take further passes.
+// Bound: the epilogue (48 accumulator columns per class and row) and a tile's chain of staging, MMAs and epilogue at two CTAs of
+// eight warps an SM.  Transposed forward, 256x320x9, bfloat16, strides (2,2,2), us with a gather per tap and class
+// (sc_umma_class_kernel) and here: 16 <- 16 channels 43, 32; 16 <- 32 80, 37; 8 <- 8 38, 27; at 17 planes 66, 36; strides (2,2,1) 45, 37;
+// 60x75x12 16, 12.  With 32 produced channels the accumulators do not fit twice: those stay there.
+#include "sc_entry.h"
+#include "sc_umma_common.cuh"
+#include "smem_grant.h"
+
+namespace chop {
+namespace {
+
+template <int CR, int NR, int RP> struct UpGeo {
+  static constexpr int PT = 128 / RP;                 // coarse pixels of a tile
+  static constexpr int PW = PT + 1, NPIX = 2 * PW;    // staged coarse pixels
+  static constexpr int ROWS = NPIX * RP, NRB = (ROWS + 7) / 8 * 8 + 4;
+  static constexpr int N3 = 3 * pad16(NR), COLS = 4 * N3;
+  static constexpr int FILTER = 27 * pad16(NR) * pad16(CR) * 2;
+  static constexpr size_t SMEM = (size_t)FILTER + (size_t)(pad16(CR) / 8) * NRB * 16 + 1024;
+  static constexpr int CTAS = 2;                      // tensor memory: 256 columns each
+  static_assert(COLS <= 256 && 4 * PT <= 32, "tile");
+};
+
+// Tiles of the flipped, channel-swapped filter (stage_filter_tiles) in the order in which the operands use them: per offset
+// (di, dj) the classes side by side, three depth taps each.  Slot of filter column (fr, fc):
+//   (0,0): classes (1,0) fr 0 fc 1 | (1,1) 0 0 | (0,1) 1 0 | (0,0) 1 1;  (1,0): 2 1 | 2 0;  (0,1): 0 2 | 1 2;  (1,1): 2 2
+__device__ __forceinline__ int up_slot(int fr, int fc) {
+  const int at[9] = {1, 0, 6, 2, 3, 7, 5, 4, 8};      // [fr*3 + fc]
+  return at[fr * 3 + fc];
+}
+
+template <int CR, int NR, int RP, int SD>
+__global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int ntiles, const int tiles_w) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  typedef UpGeo<CR, NR, RP> G;
+  constexpr int PT = G::PT, PW = G::PW, NPIX = G::NPIX, NRB = G::NRB, N3 = G::N3;
+  constexpr int CIN = pad16(CR), COUT = pad16(NR), KC = CIN / 8, KR = CR / 8;
+  __shared__ __align__(8) uint64_t mbar_s;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int2 coarse_s[3][NPIX];                    // first voxel (-1: outside the image), first absolute coarse plane
+  __shared__ int2 fine_s[3][4 * PT];                    // per fine pixel [coarse pixel][class]: first voxel (-1: none), base plane
+  __shared__ float pad_s[4][2][NR];                     // class, parity: what the taps that do not exist add
+  constexpr uint32_t B_LBO = 128, B_SBO = KC * 128;
+  constexpr uint32_t A_LBO = NRB * 16, A_SBO = 128;
+  constexpr int B_TAP_BYTES = COUT * CIN * 2;
+  unsigned char* sB = smem;
+  unsigned char* sX = smem + G::FILTER;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.out_grad);
+  __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.images_grad);
+  const int H = a.H, W = a.W, D = a.D, oD = a.oD;
+
+  if (KR < KC)   // the padding channels stay zero
+    for (int e = tid; e < G::ROWS; e += 256) *reinterpret_cast<uint4*>(sX + A_LBO + e * 16) = make_uint4(0, 0, 0, 0);
+  if (tid < 32) {
+    uint32_t slot = smem_u32(&tmem_base_s), ncols = 256;
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&mbar_s)), "r"(1) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  unsigned d16 = 0;
+  if (!a.pad_zero) d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
+  const unsigned d32 = d16 | (d16 << 16);
+  const uint4 padv = make_uint4(d32, d32, d32, d32);
+  const bool padded = (d16 & 0x7fffu) != 0;
+
+  // this thread's entry of a tile's tables: a coarse pixel (tid < NPIX) or a fine one (tid - 64 < 4*PT)
+  auto entry = [&](int tile) {
+    int2 e = make_int2(-1, 0);
+    if (tile >= ntiles) return e;
+    const int tw = tile % tiles_w, t = tile / tiles_w, i = t % a.oH, b = t / a.oH;
+    if (tid < NPIX) {
+      const int ci = i + tid / PW, cj = tw * PT + tid % PW;
+      if (ci < a.oH && cj < a.oW) {
+        const int bp = __ldg(a.base_plane + (b * H + 2 * ci) * W + 2 * cj);
+        e = make_int2(((b * a.oH + ci) * a.oW + cj) * oD, (bp + SD - 1) / SD);   // as in sc_tap_t
+      }
+    } else if (tid >= 64 && tid < 64 + 4 * PT) {
+      const int f = tid - 64, q = f / 4, cls = f % 4;   // classes in the accumulators' order
+      const int r = 2 * i + (cls < 2), c = 2 * (tw * PT + q) + (cls == 1 || cls == 2);
+      if (r < H && c < W) {
+        const int pix = (b * H + r) * W + c;
+        e = make_int2(pix * D, __ldg(a.base_plane + pix));
+      }
+    }
+    return e;
+  };
+  auto keep = [&](int buf, const int2& e) {
+    if (tid < NPIX) coarse_s[buf][tid] = e;
+    else if (tid >= 64 && tid < 64 + 4 * PT) fine_s[buf][tid - 64] = e;
+  };
+  struct Step {   // one staging and its MMAs: a pass over a tile; the same in every thread
+    int tile, z0;
+    unsigned now, left;   // fine pixels of this pass, still to do
+  };
+  auto floor_sd = [](int x) { return SD == 1 ? x : x >> 1; };
+  auto window = [&](Step& s, const int2& e) {   // lane i: fine pixel i
+    const int lo = floor_sd(e.y - 1), hi = floor_sd(e.y + D);   // coarse planes that its taps read
+    s.z0 = __reduce_min_sync(0xffffffffu, (s.left >> lane) & 1u ? lo : 0x7fffffff);
+    s.now = __ballot_sync(0xffffffffu, ((s.left >> lane) & 1u) && (unsigned)hi - (unsigned)s.z0 < (unsigned)RP);
+    if (s.now == 0) s.now = s.left;   // base planes at the ends of the integers: the passes end all the same
+    s.left &= ~s.now;
+  };
+  auto fine_entry = [&](int buf) { return lane < 4 * PT ? fine_s[buf][lane] : make_int2(-1, 0); };
+  auto open = [&](Step& s, int buf) {
+    const int2 e = fine_entry(buf);
+    s.left = __ballot_sync(0xffffffffu, e.x >= 0);
+    window(s, e);
+  };
+  constexpr int NI = (G::ROWS * KR + 255) / 256, RSTEP = 256 / KR;
+  const int chunk = tid % KR, row0 = tid / KR;
+  uint4 val[NI];
+  auto request = [&](const Step& s, int buf) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int row = row0 + i * RSTEP;
+      val[i] = padv;
+      if ((i + 1) * RSTEP > G::ROWS && row >= G::ROWS) continue;
+      const int2 e = coarse_s[buf][row / RP];
+      const int plane = row % RP + s.z0 - e.y;
+      if (e.x >= 0 && !oob(plane, oD)) val[i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(e.x + plane) * CR) + chunk);
+    }
+  };
+
+  Step cur, nxt;
+  cur.tile = blockIdx.x;
+  int2 ahead = entry(cur.tile);
+  keep(0, ahead);
+  __syncthreads();
+  open(cur, 0);
+  request(cur, 0);
+  ahead = entry(cur.tile + (int)gridDim.x);
+  // filter tiles: offset order; the loop of stage_filter_tiles with slots of its own
+  for (int e = tid; e < 27 * COUT * KC; e += 256) {
+    const int kg = e % KC, n = (e / KC) % COUT, t = e / (KC * COUT);
+    uint4 w = make_uint4(0, 0, 0, 0);
+    if (kg * 8 < CR && n < NR) w = __ldg(reinterpret_cast<const uint4*>(static_cast<const unsigned short*>(a.filters) + ((size_t)(26 - t) * NR + n) * CR + kg * 8));
+    *reinterpret_cast<uint4*>(sB + (up_slot(t / 9, t / 3 % 3) * 3 + t % 3) * B_TAP_BYTES + (n / 8) * B_SBO + kg * B_LBO + (n % 8) * 16) = w;
+  }
+  for (int e = tid; e < 8 * NR; e += 256) {
+    const int n = e % NR, par = e / NR % 2, cls = e / NR / 2, pr = cls < 2, pc = cls == 1 || cls == 2;
+    float sum = 0.f;
+    if (padded) {
+      for (int t = 0; t < 27; ++t) {
+        const int fr = t / 9, fc = t / 3 % 3, fz = t % 3;
+        if ((fr != 1) == pr && (fc != 1) == pc && (SD == 1 || (fz != 1) == par)) continue;   // the tap exists
+        for (int k = 0; k < CR; ++k) sum += __bfloat162float(static_cast<const __nv_bfloat16*>(a.filters)[((size_t)(26 - t) * NR + n) * CR + k]);
+      }
+    }
+    pad_s[cls][par][n] = __uint_as_float(d16 << 16) * sum;
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  const uint32_t mbar = smem_u32(&mbar_s);
+  auto idesc = [](int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n * N3 >> 3) << 17) | ((128u >> 4) << 24); };
+  const uint64_t da0 = umma_desc(smem_u32(sX), A_LBO, A_SBO);
+  const uint64_t db0 = umma_desc(smem_u32(sB), B_LBO, B_SBO);
+  uint32_t phase = 0;
+  int buf = 0;
+  auto next = [](int b) { return b == 2 ? 0 : b + 1; };
+
+  while (true) {
+    const bool again = cur.left != 0;
+    // the next step's tables; their buffer was last read two steps ago, before the barrier behind the last staging
+    if (again) keep(next(buf), tid < NPIX ? coarse_s[buf][tid] : tid >= 64 && tid < 64 + 4 * PT ? fine_s[buf][tid - 64] : make_int2(0, 0));
+    else keep(next(buf), ahead);
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if ((i + 1) * RSTEP <= G::ROWS || row0 + i * RSTEP < G::ROWS)
+        *reinterpret_cast<uint4*>(sX + chunk * A_LBO + (row0 + i * RSTEP) * 16) = val[i];
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int k16 = 0; k16 < CIN / 16; ++k16) {
+        const uint64_t da = umma_desc_advance(da0, k16 * 2 * A_LBO), db = umma_desc_advance(db0, k16 * 2 * B_LBO);
+        auto slot = [&](int s) { return umma_desc_advance(db, s * 3 * B_TAP_BYTES); };
+        umma_bf16(tmem, da, slot(0), idesc(4), k16 != 0 ? 1u : 0u);                                        // offset (0,0): all classes
+        umma_bf16(tmem, umma_desc_advance(da, PW * RP * 16), slot(4), idesc(2), 1u);                       // (1,0): (1,0), (1,1)
+        umma_bf16(tmem + N3, umma_desc_advance(da, RP * 16), slot(6), idesc(2), 1u);                       // (0,1): (1,1), (0,1)
+        umma_bf16(tmem + N3, umma_desc_advance(da, (PW + 1) * RP * 16), slot(8), idesc(1), 1u);            // (1,1): (1,1)
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+    }
+    // ---- while they run: the next step's pixels and rows ---------------------------------------------------------
+    nxt = cur;
+    bool go = true;
+    if (!again) {
+      nxt.tile = cur.tile + (int)gridDim.x;
+      go = nxt.tile < ntiles;
+      if (go) open(nxt, next(buf));
+    } else {
+      window(nxt, fine_entry(next(buf)));
+    }
+    if (go) {
+      request(nxt, next(buf));
+      if (!again) ahead = entry(nxt.tile + (int)gridDim.x);
+    }
+    bool done = true;
+    if (tid < 32) done = mbar_wait(mbar, phase);
+    phase ^= 1;
+    if (!__syncthreads_and(done)) {
+      if (tid == 0) note_timeout();
+      break;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    // ---- epilogue: two classes per half of the warps ---------------------------------------------------------------
+    const int m = tid & 127, q = m / RP, w = m % RP;
+#pragma unroll 1
+    for (int cls = tid / 128 * 2; cls < tid / 128 * 2 + 2; ++cls) {
+      const int2 e = fine_s[buf][q * 4 + cls];
+      const bool mine = (cur.now >> (q * 4 + cls)) & 1u;
+      uint32_t t[3][NR];
+      const uint32_t col = tmem + ((uint32_t)(m / 32 * 32) << 16) + cls * N3;
+#pragma unroll
+      for (int fz = 0; fz < 3; ++fz) tmem_ld<NR>(col + fz * COUT, t[fz]);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      uint32_t h[2][NR / 2];
+#pragma unroll
+      for (int k = 0; k < NR; k += 2) {
+        float s[2][2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float t0 = __uint_as_float(t[0][k + i]), t1 = __uint_as_float(t[1][k + i]);
+          const float above = __uint_as_float(__shfl_down_sync(0xffffffffu, t[2][k + i], 1));
+          if (SD == 1) {
+            s[0][i] = __shfl_up_sync(0xffffffffu, t0, 1) + t1 + above;
+            s[1][i] = 0.f;
+          } else {
+            s[0][i] = t1;
+            s[1][i] = t0 + above;
+          }
+          if (padded) {
+            s[0][i] += pad_s[cls][0][k + i];
+            s[1][i] += pad_s[cls][1][k + i];
+          }
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const __nv_bfloat162 b2 = __floats2bfloat162_rn(s[p][0], s[p][1]);
+          h[p][k / 2] = *reinterpret_cast<const uint32_t*>(&b2);
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < SD; ++p) {
+        const int d = (w + cur.z0) * SD + p - e.y;
+        if (!mine || oob(d, D)) continue;
+        uint4* o = reinterpret_cast<uint4*>(dst + (size_t)(e.x + d) * NR);
+#pragma unroll
+        for (int k = 0; k < NR / 8; ++k) o[k] = make_uint4(h[p][4 * k], h[p][4 * k + 1], h[p][4 * k + 2], h[p][4 * k + 3]);
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (!go) break;
+    cur = nxt;
+    buf = next(buf);
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (tid < 32) {
+    uint32_t ncols = 256;
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+  }
+}
+
+template <int CIN, int COUT, int RP, int SD>
+int launch_up(const ScArgs& a, cudaStream_t st) {
+  typedef UpGeo<CIN, COUT, RP> G;
+  auto k = sc_up_kernel<CIN, COUT, RP, SD>;
+  if (int e = grant_smem(k, G::SMEM)) return e;
+  const int tw = (a.oW + G::PT - 1) / G::PT;
+  const long long ntiles = (long long)a.B * a.oH * tw;
+  constexpr long long slots = 148LL * G::CTAS;
+  k<<<(unsigned)(ntiles < slots ? ntiles : slots), 256, G::SMEM, st>>>(a, (int)ntiles, tw);
+  return (int)cudaGetLastError();
+}
+
+}  // namespace
+
+// 3x3x3, dilation 1 and 31-bit voxel counts are the caller's conditions (sc_umma_supported)
+bool sc_up_supported(const ScArgs& a) {
+  if (a.sr != 2 || a.sc != 2 || a.sd > 2 || a.Cin > 16) return false;
+  return a.D <= 24;
+}
+int sc_up_launch(const ScArgs& a, cudaStream_t st) {
+#define CHOP_CASE(I, O)                                                              \
+  if (a.Cout == I && a.Cin == O) {                                                   \
+    if (a.sd == 2) return launch_up<I, O, 16, 2>(a, st);                             \
+    return a.D <= 10 ? launch_up<I, O, 16, 1>(a, st) : launch_up<I, O, 32, 1>(a, st); \
+  }
+  CHOP_CASE(8, 8) CHOP_CASE(16, 8) CHOP_CASE(32, 8) CHOP_CASE(8, 16) CHOP_CASE(16, 16) CHOP_CASE(32, 16)
+#undef CHOP_CASE
+  return -4;
+}
+int sc_up_timeouts() { return timeouts_here(); }
+int sc_up_publish_mirror(int* dptr) { return (int)publish_mirror_here(dptr); }
+int sc_up_clear_timeouts() { return (int)clear_timeouts_here(); }
+
+}  // namespace chop
