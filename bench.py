@@ -673,7 +673,7 @@ def sparse_conv_main(args):
            "config": {"workload": "c4_sparse_conv: SparseConv3DFast fwd+bwd, B=%d, %dx%d, band of %d planes, 3x3x3, %d->%d, bf16/fp32-acc"
                                   % (B, H, W, D, Cin, Cout), "l2": "flushed between steps (256 MB write)"},
            "gpu_launches": 4 * K, "umma_timeouts": _lib.lib().chop_umma_timeouts(),
-           "roofline": {"bound": "hbm", "kernel": "sc_umma_rows_kernel (forward)", "achieved": fwd_b / (fwd_ms * 1e-3) / 1e9, "peak": peak,
+           "roofline": {"bound": "hbm", "kernel": "sc_band_kernel (forward)", "achieved": fwd_b / (fwd_ms * 1e-3) / 1e9, "peak": peak,
                         "peak_source": peak_kind, "unit": "GB/s", "frac": fwd_b / (fwd_ms * 1e-3) / 1e9 / peak,
                         "traffic": (rec_f or {}).get("dram_bytes"),
                         # sm__pipe_tensor_cycles_active of the recorded ncu captures (null once sc_umma.cu has changed)
