@@ -13,7 +13,7 @@
 
 namespace chop {
 std::atomic<int> g_use_umma{1};  // tuning knob "umma": 0 forces the generic kernels
-std::atomic<int> g_use_tile{1};  // tuning knob "tile": 0 = never the register-tiled float32 kernels, 2 = never those of sc_run.cu and sc_band.cu
+std::atomic<int> g_use_tile{1};  // tuning knob "tile": 0 = never the register-tiled float32 kernels, 2 = never those of sc_run.cu, sc_band.cu and sc_up.cu
 }
 
 namespace {
@@ -54,6 +54,8 @@ int run_dgrad(int dtype, const ScArgs& in, cudaStream_t st) {
     return chop::sc_umma_dgrad_launch(a, st);
   if (chop::g_use_tile.load() == 1 && chop::sc_run_supported(dtype, a, a.Cout) && al16(a.out_grad) && al16(a.images_grad))
     return chop::sc_run_launch(a, true, st);
+  if (chop::g_use_tile.load() == 1 && chop::sc_up_f32_supported(dtype, a) && al16(a.out_grad) && al16(a.images_grad))
+    return chop::sc_up_f32_launch(a, st);
   if (chop::g_use_tile.load() && chop::sc_tile_supported(dtype, a) && al16(a.out_grad) && al16(a.images_grad) && al16(a.filters))
     return chop::sc_tile_gather_launch(dtype, a, st);
   return chop::sc_dgrad_simt_launch(dtype, a, st);
@@ -183,6 +185,8 @@ int chop_sparse_conv3d_transpose_fwd(const chop_sc_desc* d, const void* images, 
     return chop::sc_umma_dgrad_launch(a, st);
   if (chop::g_use_tile.load() == 1 && chop::sc_run_supported(d->dtype, a, a.Cout) && al16(a.out_grad) && al16(a.images_grad))
     return chop::sc_run_launch(a, true, st);
+  if (chop::g_use_tile.load() == 1 && chop::sc_up_f32_supported(d->dtype, a) && al16(a.out_grad) && al16(a.images_grad))
+    return chop::sc_up_f32_launch(a, st);
   if (chop::g_use_tile.load() && chop::sc_tile_supported(d->dtype, a) && al16(a.out_grad) && al16(a.images_grad) && al16(a.filters))
     return chop::sc_tile_gather_launch(d->dtype, a, st);
   return chop::sc_tconv_simt_launch(d->dtype, a, st);

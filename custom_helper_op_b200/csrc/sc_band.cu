@@ -64,34 +64,6 @@ template <typename T, int CR, int NR, int RP> struct BandGeo {
   static_assert(PT * RP == 128 && 32 % RP == 0 && ROWS % 8 == 0 && NPIX <= 128 && R * PT <= 32 && COLS <= 256 && (P == 1 || R == 1), "tile");
 };
 
-// Eight float32 values as three bfloat16 pieces each, by truncation: x = x1 + x2 + x3 exactly (8 + 8 + 8 significant bits).
-__device__ __forceinline__ void split3(const float (&v)[8], unsigned (&p)[3][4]) {
-#pragma unroll
-  for (int i = 0; i < 8; i += 2) {
-    unsigned hi[3][2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      float r = v[i + j];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        hi[q][j] = __float_as_uint(r) & 0xffff0000u;
-        if (q < 2) r = __fsub_rn(r, __uint_as_float(hi[q][j]));
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) p[q][i / 2] = __byte_perm(hi[q][0], hi[q][1], 0x7632);
-  }
-}
-// Largest magnitude, as bits.  Values of which it is not finite, or not zero and below 2^-50, are not for the pieces: an
-// infinity times a zero piece is not a number, and products of low pieces would fall below the normal range.
-__device__ __forceinline__ unsigned top_bits(const float (&v)[8]) {
-  unsigned m = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
-  return m;
-}
-__device__ __forceinline__ bool not_for_pieces(unsigned top) { return top >= 0x7f800000u || (top != 0 && top < 0x26800000u); }
-
 // The filter in three pieces: tile [filter column][filter row][piece][depth tap], each as in stage_filter_tiles; channels n0 ..
 // n0 + NR - 1 of NF produced ones.  Returns the largest magnitude that this thread has seen.
 template <int CR, int NR, int NF, bool DGRAD>
@@ -541,8 +513,8 @@ bool sc_band_better(const ScArgs& a, int cin, int cout) {
 
 // float32, where this beats sc_run_kernel and is no less exact.  189x251x7, us there and here: 16 -> 16 127, 88; 16 -> 32 238, 166;
 // 16 -> 8 79, 84; 8 -> 8 49, 70; 8 -> 16 73, 74; 256x320x9 254, 140; 493, 268; 155, 134; 87, 112; 134, 117; 60x75x9, 16 -> 16 29, 30.
-// 2-norm of the error against float64 over that of the result: 16 gathered channels 1.77e-7 here, 1.80 to 1.92e-7 there; 32, whose
-// chains are twice as long, 3.0e-7, so they stay there.
+// 2-norm of the error against float64 over that of the result: 16 gathered channels 1.38e-7 here, 1.80 to 1.92e-7 there; 32, whose
+// chains are twice as long, 3.0e-7 with the pieces cut off (not rounded), so they stay there.
 bool sc_band_f32_better(const ScArgs& a, int cin, int cout) { return cin == 16 && cout >= 16 && a.D >= 5 && a.D <= 24; }
 
 int sc_band_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {

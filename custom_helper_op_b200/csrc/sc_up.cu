@@ -1,6 +1,6 @@
 // Strided gather form on the tensor cores with every coarse voxel staged once: the transposed convolution and the image gradient
-// of the strided one, 3x3x3, strides 2 along rows and columns and 1 or 2 along depth, bfloat16, float32 accumulation, 8 or 16
-// produced channels.
+// of the strided one, 3x3x3, strides 2 along rows and columns and 1 or 2 along depth, bfloat16 and float32 (in three pieces, as in
+// sc_band.cu), float32 accumulation, 8 or 16 produced channels.
 //
 // Row r and column c of a fine voxel decide which filter columns exist there: (fr, fc) belongs to class (fr != 1, fc != 1) of
 // (r mod 2, c mod 2) and reads the coarse pixel (r/2 + (fr == 2), c/2 + (fc == 2)).  So the four fine pixels over one coarse pixel
@@ -23,14 +23,17 @@
 namespace chop {
 namespace {
 
-template <int CR, int NR, int RP> struct UpGeo {
+// T: bfloat16, all four classes in one CTA; float32, in three bfloat16 pieces as in sc_band.cu, two of the classes (blockIdx.y), each
+// with an accumulator for x1*w1 and one for the five small products.
+template <typename T, int CR, int NR, int RP> struct UpGeo {
+  static constexpr int P = sizeof(T) == 2 ? 1 : 3, NCLS = P == 1 ? 4 : 2;
   static constexpr int PT = 128 / RP;                 // coarse pixels of a tile
   static constexpr int PW = PT + 1, NPIX = 2 * PW;    // staged coarse pixels
   static constexpr int ROWS = NPIX * RP, NRB = (ROWS + 7) / 8 * 8 + 4;
   static constexpr int N3 = 3 * pad16(NR), COLS = 4 * N3;
-  static constexpr int FILTER = 27 * pad16(NR) * pad16(CR) * 2;
-  static constexpr size_t SMEM = (size_t)FILTER + (size_t)(pad16(CR) / 8) * NRB * 16 + 1024;
-  static constexpr int CTAS = 2;                      // tensor memory: 256 columns each
+  static constexpr int PIECE = 27 * pad16(NR) * pad16(CR) * 2;   // bytes of the filter's tiles
+  static constexpr size_t SMEM = (size_t)P * PIECE + (size_t)P * (pad16(CR) / 8) * NRB * 16 + 1024;
+  static constexpr int CTAS = SMEM > 110 * 1024 ? 1 : 2;   // tensor memory: 256 columns each
   static_assert(COLS <= 256 && 4 * PT <= 32, "tile");
 };
 
@@ -42,29 +45,52 @@ __device__ __forceinline__ int up_slot(int fr, int fc) {
   return at[fr * 3 + fc];
 }
 
-template <int CR, int NR, int RP, int SD>
-__global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int ntiles, const int tiles_w) {
+// The sums of the fine pixels `todo` (coarse pixel*4 + class) of a tile by plain multiply-adds: values that are not for the pieces.
+template <int CR, int NR>
+__device__ __noinline__ void up_plain(const ScArgs& a, int b, int i, int j0, unsigned todo, float pad) {
+  const float* src = static_cast<const float*>(a.out_grad);
+  const float* flt = static_cast<const float*>(a.filters);
+  for (; todo; todo &= todo - 1) {
+    const int f = __ffs(todo) - 1, cls = f % 4, r = 2 * i + (cls < 2), c = 2 * (j0 + f / 4) + (cls == 1 || cls == 2);
+    for (int e = threadIdx.x; e < a.D * NR; e += 256) {
+      const int n = e % NR, dz = e / NR;
+      float s = 0.f;
+      for (int t = 0; t < 27; ++t) {
+        const long long v = sc_tap_t(a, b, r, c, dz, t / 9, t / 3 % 3, t % 3);
+        if (v < 0 && pad == 0.f) continue;
+        for (int k = 0; k < CR; ++k) s = fmaf(v < 0 ? pad : __ldg(src + v * CR + k), __ldg(flt + ((size_t)(26 - t) * NR + n) * CR + k), s);
+      }
+      static_cast<float*>(a.images_grad)[(((size_t)(b * a.H + r) * a.W + c) * a.D + dz) * NR + n] = s;
+    }
+  }
+}
+
+template <typename T, int CR, int NR, int RP, int SD>
+__global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kernel(const ScArgs a, const int ntiles, const int tiles_w) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  typedef UpGeo<CR, NR, RP> G;
-  constexpr int PT = G::PT, PW = G::PW, NPIX = G::NPIX, NRB = G::NRB, N3 = G::N3;
+  typedef UpGeo<T, CR, NR, RP> G;
+  constexpr int PT = G::PT, PW = G::PW, NPIX = G::NPIX, NRB = G::NRB, N3 = G::N3, P = G::P, NCLS = G::NCLS;
   constexpr int CIN = pad16(CR), COUT = pad16(NR), KC = CIN / 8, KR = CR / 8;
   __shared__ __align__(8) uint64_t mbar_s;
   __shared__ uint32_t tmem_base_s;
   __shared__ int2 coarse_s[3][NPIX];                    // first voxel (-1: outside the image), first absolute coarse plane
   __shared__ int2 fine_s[3][4 * PT];                    // per fine pixel [coarse pixel][class]: first voxel (-1: none), base plane
+  __shared__ unsigned top_s[4];                         // float32: largest magnitude of a step, three steps in turn; the filter's
   __shared__ float pad_s[4][2][NR];                     // class, parity: what the taps that do not exist add
   constexpr uint32_t B_LBO = 128, B_SBO = KC * 128;
   constexpr uint32_t A_LBO = NRB * 16, A_SBO = 128;
   constexpr int B_TAP_BYTES = COUT * CIN * 2;
   unsigned char* sB = smem;
-  unsigned char* sX = smem + G::FILTER;
+  unsigned char* sX = smem + P * G::PIECE;              // [piece][K-chunk][row]
+  const int half = P == 1 ? 0 : blockIdx.y;             // float32: classes 2*half, 2*half + 1
   const int tid = threadIdx.x, lane = tid & 31;
-  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.out_grad);
-  __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.images_grad);
+  const T* src = static_cast<const T*>(a.out_grad);
+  T* dst = static_cast<T*>(a.images_grad);
   const int H = a.H, W = a.W, D = a.D, oD = a.oD;
 
   if (KR < KC)   // the padding channels stay zero
-    for (int e = tid; e < G::ROWS; e += 256) *reinterpret_cast<uint4*>(sX + A_LBO + e * 16) = make_uint4(0, 0, 0, 0);
+    for (int e = tid; e < P * G::ROWS; e += 256)
+      *reinterpret_cast<uint4*>(sX + (e / G::ROWS * KC + 1) * A_LBO + e % G::ROWS * 16) = make_uint4(0, 0, 0, 0);
   if (tid < 32) {
     uint32_t slot = smem_u32(&tmem_base_s), ncols = 256;
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(ncols) : "memory");
@@ -74,11 +100,21 @@ __global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&mbar_s)), "r"(1) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  unsigned d16 = 0;
-  if (!a.pad_zero) d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
-  const unsigned d32 = d16 | (d16 << 16);
-  const uint4 padv = make_uint4(d32, d32, d32, d32);
-  const bool padded = (d16 & 0x7fffu) != 0;
+  float padf = 0.f;
+  uint4 padv = make_uint4(0, 0, 0, 0);                  // 16 bytes of padding values
+  if (!a.pad_zero) {
+    unsigned d32;
+    if constexpr (P == 1) {
+      const unsigned d16 = __ldg(static_cast<const unsigned short*>(a.default_value));
+      padf = __uint_as_float(d16 << 16);
+      d32 = d16 | (d16 << 16);
+    } else {
+      padf = __ldg(static_cast<const float*>(a.default_value));
+      d32 = __float_as_uint(padf);
+    }
+    padv = make_uint4(d32, d32, d32, d32);
+  }
+  const bool padded = padf != 0.f;                      // also where it is not a number
 
   // this thread's entry of a tile's tables: a coarse pixel (tid < NPIX) or a fine one (tid - 64 < 4*PT)
   auto entry = [&](int tile) {
@@ -120,21 +156,26 @@ __global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int
   auto fine_entry = [&](int buf) { return lane < 4 * PT ? fine_s[buf][lane] : make_int2(-1, 0); };
   auto open = [&](Step& s, int buf) {
     const int2 e = fine_entry(buf);
-    s.left = __ballot_sync(0xffffffffu, e.x >= 0);
+    s.left = __ballot_sync(0xffffffffu, e.x >= 0 && (P == 1 || lane % 4 / 2 == half));
     window(s, e);
   };
   constexpr int NI = (G::ROWS * KR + 255) / 256, RSTEP = 256 / KR;
   const int chunk = tid % KR, row0 = tid / KR;
-  uint4 val[NI];
+  constexpr int VEC = (int)sizeof(T) / 2;               // 16-byte words of a chunk of eight channels
+  uint4 val[NI][VEC];
   auto request = [&](const Step& s, int buf) {
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int row = row0 + i * RSTEP;
-      val[i] = padv;
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) val[i][k] = padv;
       if ((i + 1) * RSTEP > G::ROWS && row >= G::ROWS) continue;
       const int2 e = coarse_s[buf][row / RP];
       const int plane = row % RP + s.z0 - e.y;
-      if (e.x >= 0 && !oob(plane, oD)) val[i] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(e.x + plane) * CR) + chunk);
+      if (e.x >= 0 && !oob(plane, oD)) {
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) val[i][k] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(e.x + plane) * CR) + chunk * VEC + k);
+      }
     }
   };
 
@@ -147,11 +188,33 @@ __global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int
   request(cur, 0);
   ahead = entry(cur.tile + (int)gridDim.x);
   // filter tiles: offset order; the loop of stage_filter_tiles with slots of its own
+  unsigned top = 0;
   for (int e = tid; e < 27 * COUT * KC; e += 256) {
     const int kg = e % KC, n = (e / KC) % COUT, t = e / (KC * COUT);
-    uint4 w = make_uint4(0, 0, 0, 0);
-    if (kg * 8 < CR && n < NR) w = __ldg(reinterpret_cast<const uint4*>(static_cast<const unsigned short*>(a.filters) + ((size_t)(26 - t) * NR + n) * CR + kg * 8));
-    *reinterpret_cast<uint4*>(sB + (up_slot(t / 9, t / 3 % 3) * 3 + t % 3) * B_TAP_BYTES + (n / 8) * B_SBO + kg * B_LBO + (n % 8) * 16) = w;
+    unsigned char* o = sB + (up_slot(t / 9, t / 3 % 3) * 3 + t % 3) * B_TAP_BYTES + (n / 8) * B_SBO + kg * B_LBO + (n % 8) * 16;
+    const T* from = static_cast<const T*>(a.filters) + ((size_t)(26 - t) * NR + n) * CR + kg * 8;
+    const bool is = kg * 8 < CR && n < NR;
+    if constexpr (P == 1) {
+      *reinterpret_cast<uint4*>(o) = is ? __ldg(reinterpret_cast<const uint4*>(from)) : make_uint4(0, 0, 0, 0);
+    } else {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = is ? __ldg(from + i) : 0.f;
+      top = max(top, top_bits(v));
+      unsigned p[3][4];
+      split3(v, p);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(o + q * G::PIECE) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+    }
+  }
+  bool plain_filter = false, plain = false;
+  if constexpr (P > 1) {
+    if (tid < 4) top_s[tid] = 0;
+    __syncthreads();
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) atomicMax(&top_s[3], top);
+    __syncthreads();
+    plain_filter = not_for_pieces(top_s[3]);
   }
   for (int e = tid; e < 8 * NR; e += 256) {
     const int n = e % NR, par = e / NR % 2, cls = e / NR / 2, pr = cls < 2, pc = cls == 1 || cls == 2;
@@ -160,10 +223,10 @@ __global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int
       for (int t = 0; t < 27; ++t) {
         const int fr = t / 9, fc = t / 3 % 3, fz = t % 3;
         if ((fr != 1) == pr && (fc != 1) == pc && (SD == 1 || (fz != 1) == par)) continue;   // the tap exists
-        for (int k = 0; k < CR; ++k) sum += __bfloat162float(static_cast<const __nv_bfloat16*>(a.filters)[((size_t)(26 - t) * NR + n) * CR + k]);
+        for (int k = 0; k < CR; ++k) sum += ScIo<T>::ld(static_cast<const T*>(a.filters) + ((size_t)(26 - t) * NR + n) * CR + k);
       }
     }
-    pad_s[cls][par][n] = __uint_as_float(d16 << 16) * sum;
+    pad_s[cls][par][n] = padf * sum;
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -183,19 +246,61 @@ __global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int
     // the next step's tables; their buffer was last read two steps ago, before the barrier behind the last staging
     if (again) keep(next(buf), tid < NPIX ? coarse_s[buf][tid] : tid >= 64 && tid < 64 + 4 * PT ? fine_s[buf][tid - 64] : make_int2(0, 0));
     else keep(next(buf), ahead);
+    top = 0;
 #pragma unroll
-    for (int i = 0; i < NI; ++i)
-      if ((i + 1) * RSTEP <= G::ROWS || row0 + i * RSTEP < G::ROWS)
-        *reinterpret_cast<uint4*>(sX + chunk * A_LBO + (row0 + i * RSTEP) * 16) = val[i];
+    for (int i = 0; i < NI; ++i) {
+      if ((i + 1) * RSTEP > G::ROWS && row0 + i * RSTEP >= G::ROWS) continue;
+      unsigned char* o = sX + chunk * A_LBO + (row0 + i * RSTEP) * 16;
+      if constexpr (P == 1) {
+        *reinterpret_cast<uint4*>(o) = val[i][0];
+      } else {
+        const uint4 lo = val[i][0], hi = val[i][VEC - 1];
+        const float v[8] = {__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(lo.w),
+                            __uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z), __uint_as_float(hi.w)};
+        top = max(top, top_bits(v));
+        unsigned p[3][4];
+        split3(v, p);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(o + q * KC * A_LBO) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+      }
+    }
+    if constexpr (P > 1) {
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0) atomicMax(&top_s[buf], top);
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (P > 1) {
+      plain = plain_filter || not_for_pieces(top_s[buf]);
+      if (tid == 0) top_s[next(next(buf))] = 0;         // read in the last step, written two steps on
+    }
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int k16 = 0; k16 < CIN / 16; ++k16) {
         const uint64_t da = umma_desc_advance(da0, k16 * 2 * A_LBO), db = umma_desc_advance(db0, k16 * 2 * B_LBO);
         auto slot = [&](int s) { return umma_desc_advance(db, s * 3 * B_TAP_BYTES); };
+        if constexpr (P > 1) {
+          // pieces (p, q): x1*w1 | x1*w2, x2*w1, x1*w3, x2*w2, x3*w1
+          constexpr int PQ[6][2] = {{0, 0}, {0, 1}, {1, 0}, {0, 2}, {1, 1}, {2, 0}};
+#pragma unroll
+          for (int c = 0; c < 6; ++c) {
+            const uint64_t dx = umma_desc_advance(da, PQ[c][0] * KC * A_LBO);
+            auto piece = [&](int s) { return umma_desc_advance(slot(s), PQ[c][1] * G::PIECE); };
+            const uint32_t acc = tmem + (c == 0 ? 0 : NCLS * N3);
+            const uint32_t add = k16 != 0 || c > 1 ? 1u : 0u;
+            umma_bf16(acc, dx, piece(half == 0 ? 0 : 2), idesc(2), add);
+            if (half == 0) {
+              umma_bf16(acc, umma_desc_advance(dx, PW * RP * 16), piece(4), idesc(2), 1u);
+              umma_bf16(acc + N3, umma_desc_advance(dx, RP * 16), piece(6), idesc(1), 1u);
+              umma_bf16(acc + N3, umma_desc_advance(dx, (PW + 1) * RP * 16), piece(8), idesc(1), 1u);
+            } else {
+              umma_bf16(acc, umma_desc_advance(dx, RP * 16), piece(7), idesc(1), 1u);
+            }
+          }
+          continue;
+        }
         umma_bf16(tmem, da, slot(0), idesc(4), k16 != 0 ? 1u : 0u);                                        // offset (0,0): all classes
         umma_bf16(tmem, umma_desc_advance(da, PW * RP * 16), slot(4), idesc(2), 1u);                       // (1,0): (1,0), (1,1)
         umma_bf16(tmem + N3, umma_desc_advance(da, RP * 16), slot(6), idesc(2), 1u);                       // (0,1): (1,1), (0,1)
@@ -226,50 +331,73 @@ __global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    // ---- epilogue: two classes per half of the warps ---------------------------------------------------------------
+    // ---- epilogue: the classes are dealt out to the two halves of the warps --------------------------------------
+    constexpr int NE = P == 1 ? NR : 8;                 // channels at a time
     const int m = tid & 127, q = m / RP, w = m % RP;
-#pragma unroll 1
-    for (int cls = tid / 128 * 2; cls < tid / 128 * 2 + 2; ++cls) {
-      const int2 e = fine_s[buf][q * 4 + cls];
-      const bool mine = (cur.now >> (q * 4 + cls)) & 1u;
-      uint32_t t[3][NR];
-      const uint32_t col = tmem + ((uint32_t)(m / 32 * 32) << 16) + cls * N3;
-#pragma unroll
-      for (int fz = 0; fz < 3; ++fz) tmem_ld<NR>(col + fz * COUT, t[fz]);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      uint32_t h[2][NR / 2];
-#pragma unroll
-      for (int k = 0; k < NR; k += 2) {
-        float s[2][2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float t0 = __uint_as_float(t[0][k + i]), t1 = __uint_as_float(t[1][k + i]);
-          const float above = __uint_as_float(__shfl_down_sync(0xffffffffu, t[2][k + i], 1));
-          if (SD == 1) {
-            s[0][i] = __shfl_up_sync(0xffffffffu, t0, 1) + t1 + above;
-            s[1][i] = 0.f;
-          } else {
-            s[0][i] = t1;
-            s[1][i] = t0 + above;
-          }
-          if (padded) {
-            s[0][i] += pad_s[cls][0][k + i];
-            s[1][i] += pad_s[cls][1][k + i];
-          }
-        }
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          const __nv_bfloat162 b2 = __floats2bfloat162_rn(s[p][0], s[p][1]);
-          h[p][k / 2] = *reinterpret_cast<const uint32_t*>(&b2);
-        }
+    if (P > 1 && plain) {
+      if constexpr (P > 1) {
+        const int t = cur.tile / tiles_w;
+        up_plain<CR, NR>(a, t / a.oH, t % a.oH, cur.tile % tiles_w * PT, cur.now, padf);
       }
+    } else {
+#pragma unroll 1
+      for (int l = tid / 128 * (NCLS / 2); l < (tid / 128 + 1) * (NCLS / 2); ++l) {
+        const int cls = P == 1 ? l : half * 2 + l;
+        const int2 e = fine_s[buf][q * 4 + cls];
+        const bool mine = (cur.now >> (q * 4 + cls)) & 1u;
+#pragma unroll 1
+        for (int c0 = 0; c0 < NR; c0 += NE) {
+          uint32_t t[P == 1 ? 1 : 2][3][NE];
+          const uint32_t col = tmem + ((uint32_t)(m / 32 * 32) << 16) + l * N3 + c0;
 #pragma unroll
-      for (int p = 0; p < SD; ++p) {
-        const int d = (w + cur.z0) * SD + p - e.y;
-        if (!mine || oob(d, D)) continue;
-        uint4* o = reinterpret_cast<uint4*>(dst + (size_t)(e.x + d) * NR);
+          for (int g = 0; g < (P == 1 ? 1 : 2); ++g)
 #pragma unroll
-        for (int k = 0; k < NR / 8; ++k) o[k] = make_uint4(h[p][4 * k], h[p][4 * k + 1], h[p][4 * k + 2], h[p][4 * k + 3]);
+            for (int fz = 0; fz < 3; ++fz) tmem_ld<NE>(col + g * NCLS * N3 + fz * COUT, t[g][fz]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          float s[2][NE];
+#pragma unroll
+          for (int k = 0; k < NE; ++k) {
+            float f[3];
+#pragma unroll
+            for (int fz = 0; fz < 3; ++fz) {
+              f[fz] = __uint_as_float(t[0][fz][k]);
+              if constexpr (P > 1) f[fz] += __uint_as_float(t[1][fz][k]);
+            }
+            const float above = __shfl_down_sync(0xffffffffu, f[2], 1);
+            if (SD == 1) {
+              s[0][k] = __shfl_up_sync(0xffffffffu, f[0], 1) + f[1] + above;
+              s[1][k] = 0.f;
+            } else {
+              s[0][k] = f[1];
+              s[1][k] = f[0] + above;
+            }
+            if (padded) {
+              s[0][k] += pad_s[cls][0][c0 + k];
+              s[1][k] += pad_s[cls][1][c0 + k];
+            }
+          }
+#pragma unroll
+          for (int p = 0; p < SD; ++p) {
+            const int d = (w + cur.z0) * SD + p - e.y;
+            if (!mine || oob(d, D)) continue;
+            T* o = dst + (size_t)(e.x + d) * NR + c0;
+            if constexpr (P == 1) {
+#pragma unroll
+              for (int k = 0; k < NE; k += 8) {
+                uint32_t h[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const __nv_bfloat162 b2 = __floats2bfloat162_rn(s[p][k + 2 * i], s[p][k + 2 * i + 1]);
+                  h[i] = *reinterpret_cast<const uint32_t*>(&b2);
+                }
+                *reinterpret_cast<uint4*>(o + k) = make_uint4(h[0], h[1], h[2], h[3]);
+              }
+            } else {
+#pragma unroll
+              for (int k = 0; k < NE; k += 4) *reinterpret_cast<float4*>(o + k) = make_float4(s[p][k], s[p][k + 1], s[p][k + 2], s[p][k + 3]);
+            }
+          }
+        }
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -286,33 +414,48 @@ __global__ void __launch_bounds__(256, 2) sc_up_kernel(const ScArgs a, const int
   }
 }
 
-template <int CIN, int COUT, int RP, int SD>
+template <typename T, int CIN, int COUT, int RP, int SD>
 int launch_up(const ScArgs& a, cudaStream_t st) {
-  typedef UpGeo<CIN, COUT, RP> G;
-  auto k = sc_up_kernel<CIN, COUT, RP, SD>;
+  typedef UpGeo<T, CIN, COUT, RP> G;
+  auto k = sc_up_kernel<T, CIN, COUT, RP, SD>;
   if (int e = grant_smem(k, G::SMEM)) return e;
   const int tw = (a.oW + G::PT - 1) / G::PT;
   const long long ntiles = (long long)a.B * a.oH * tw;
-  constexpr long long slots = 148LL * G::CTAS;
-  k<<<(unsigned)(ntiles < slots ? ntiles : slots), 256, G::SMEM, st>>>(a, (int)ntiles, tw);
+  constexpr long long slots = 148LL * G::CTAS * G::NCLS / 4;
+  k<<<dim3((unsigned)(ntiles < slots ? ntiles : slots), 4 / G::NCLS), 256, G::SMEM, st>>>(a, (int)ntiles, tw);
   return (int)cudaGetLastError();
+}
+template <typename T, int CIN, int COUT>
+int launch_depth(const ScArgs& a, cudaStream_t st) {
+  if (a.sd == 2) return launch_up<T, CIN, COUT, 16, 2>(a, st);
+  return a.D <= 10 ? launch_up<T, CIN, COUT, 16, 1>(a, st) : launch_up<T, CIN, COUT, 32, 1>(a, st);
 }
 
 }  // namespace
 
-// 3x3x3, dilation 1 and 31-bit voxel counts are the caller's conditions (sc_umma_supported)
-bool sc_up_supported(const ScArgs& a) {
-  if (a.sr != 2 || a.sc != 2 || a.sd > 2 || a.Cin > 16) return false;
-  return a.D <= 24;
-}
+// 3x3x3, dilation 1 and 31-bit voxel counts are the caller's conditions
+bool sc_up_supported(const ScArgs& a) { return a.sr == 2 && a.sc == 2 && a.sd <= 2 && a.Cin <= 16 && a.D <= 24; }
 int sc_up_launch(const ScArgs& a, cudaStream_t st) {
-#define CHOP_CASE(I, O)                                                              \
-  if (a.Cout == I && a.Cin == O) {                                                   \
-    if (a.sd == 2) return launch_up<I, O, 16, 2>(a, st);                             \
-    return a.D <= 10 ? launch_up<I, O, 16, 1>(a, st) : launch_up<I, O, 32, 1>(a, st); \
-  }
+#define CHOP_CASE(I, O) if (a.Cout == I && a.Cin == O) return launch_depth<__nv_bfloat16, I, O>(a, st);
   CHOP_CASE(8, 8) CHOP_CASE(16, 8) CHOP_CASE(32, 8) CHOP_CASE(8, 16) CHOP_CASE(16, 16) CHOP_CASE(32, 16)
 #undef CHOP_CASE
+  return -4;
+}
+// float32, where this is faster than sc_tile.cu and no less exact.  Transposed forward, us there and here (produced < gathered):
+// strides (2,2,2), 256x320x9 16<16 165, 83; 8<16 104, 72; 16<8 102, 78; 8<8 82, 68; at 17 planes 279, 92; 168, 74; 161, 89; 125, 72;
+// (2,2,1) 189x251x7 16<16 90, 70; 8<16 59, 64; 16<8 57, 64; 8<8 47, 58.  2-norm of the error against float64: (2,2,2) 16 gathered channels
+// 8.6e-8 there, 6.2e-8 here, 8 8.0e-8, 4.7e-8; 32 8.9e-8, 9.5e-8 (and at depth stride 1 slower), so those stay there.
+bool sc_up_f32_supported(int dtype, const ScArgs& a) {
+  return dtype == 0 && sc_up_supported(a) && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 &&
+         (a.Cin == 8 || a.Cin == 16) && (a.Cout == 16 || (a.Cout == 8 && a.sd == 2)) && (a.sd == 2 || a.Cin == 16) &&
+         a.nvox_in < (1LL << 31) - 4096;
+}
+int sc_up_f32_launch(const ScArgs& a, cudaStream_t st) {
+  if (a.Cout == 16 && a.Cin == 16) return launch_depth<float, 16, 16>(a, st);
+  if (a.sd != 2) return -4;
+  if (a.Cout == 8 && a.Cin == 8) return launch_up<float, 8, 8, 16, 2>(a, st);
+  if (a.Cout == 16 && a.Cin == 8) return launch_up<float, 16, 8, 16, 2>(a, st);
+  if (a.Cout == 8 && a.Cin == 16) return launch_up<float, 8, 16, 16, 2>(a, st);
   return -4;
 }
 int sc_up_timeouts() { return timeouts_here(); }
