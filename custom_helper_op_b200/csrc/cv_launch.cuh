@@ -148,9 +148,10 @@ inline int bwd_tuned_pl(const CvArgs& a0, cudaStream_t st) {
 // fit into an SM's shared memory.  128x160x192, one / two views, us with short and with long blocks: CostVolume C = 8 113 / 163, 104 / 152,
 // C = 16 132 / 195, 127 / 179; CostAggregate C = 8 97 / 148, 87 / 129, C = 16 110 / 173, 101 / 153.  Where they do not fit: CostVolume, six
 // views, C = 16 300, 338; CostAggregate MIN, four views, C = 8 131, 143.  With winners staged too (CostVolume MIN) they lose: C = 16 223, 245.
+// CostVolume C = 16 in bfloat16 keeps short ones: three items of 139x174, two views, short and long, 36 planes 260, 265; 64 381, 384; 68 397, 410.
 template <typename T, int C, int CPL, bool AGG = false, bool RMIN = false>
 inline int bwd_tuned_go(const CvArgs& a, cudaStream_t st) {
-  if constexpr (C <= 16 && (AGG || !RMIN)) {
+  if constexpr (C <= 16 && (AGG || !RMIN) && (AGG || C == 8 || sizeof(T) == 4)) {
     if (24 * tuned_bwd_smem_per_warp<C>(a.N, 32 / (C / CPL), AGG ? 0 : 1, 2) <= (RMIN ? 180 : 216) * 1024)
       return bwd_tuned_pl<T, C, CPL, AGG, RMIN, 2>(a, st);
   }
