@@ -405,10 +405,10 @@ struct ScArgs {
   std::array<int64_t, 5> out_shape;
 };
 
-// Before a tensor-core (bfloat16) call: raise if a kernel of an EARLIER call gave up a bounded wait on its MMA barrier.
-// Reads one int of pinned host memory (chop_umma_watch); only the first call per device synchronises.
+// Before a call that may take tensor-core kernels (bfloat16 and float32): raise if a kernel of an EARLIER call gave up a bounded
+// wait on its MMA barrier.  Reads one int of pinned host memory (chop_umma_watch); only the first call per device does more.
 void umma_watch(at::ScalarType dt) {
-  if (dt != at::kBFloat16) return;
+  if (dt != at::kBFloat16 && dt != at::kFloat) return;
   const int n = chop_umma_watch();
   if (n > 0)
     throw std::runtime_error("custom_helper_op: " + std::to_string(n) +

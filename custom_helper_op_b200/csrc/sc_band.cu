@@ -533,7 +533,7 @@ int sc_band_f32_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {
 #undef CHOP_CASE
 
 int sc_band_timeouts() { return timeouts_here(); }
-int sc_band_publish_mirror(int* dptr) { return (int)publish_mirror_here(dptr); }
+int sc_band_publish_mirror(int* dptr, cudaStream_t st) { return (int)publish_mirror_here(dptr, st); }
 int sc_band_clear_timeouts() { return (int)clear_timeouts_here(); }
 
 }  // namespace chop

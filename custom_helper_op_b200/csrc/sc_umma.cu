@@ -1420,11 +1420,18 @@ unsigned long long g_watch_devs = 0;  // devices that know its address (bit = de
 }  // namespace
 
 // Number of abandoned waits seen through the host-visible mirror; -1 if it cannot be set up.  The first call per
-// device allocates (once per process) and publishes the mirror - that call synchronises; later calls read host memory.
+// device allocates (once per process) and publishes the mirror, on a stream of its own and with this thread's capture mode
+// relaxed: a program may make its first call while a stream is being captured.  Later calls read host memory.
 int sc_umma_watch() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
   std::lock_guard<std::mutex> lk(g_watch_mu);
+  if (g_watch_host && ((g_watch_devs >> dev) & 1ull)) return *const_cast<volatile int*>(g_watch_host);
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
   if (!g_watch_host) {
     int* h = nullptr;
     if (cudaHostAlloc(reinterpret_cast<void**>(&h), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
@@ -1434,15 +1441,17 @@ int sc_umma_watch() {
     *h = 0;
     g_watch_host = h;
   }
-  if (!((g_watch_devs >> dev) & 1ull)) {
-    int* dptr = nullptr;
-    if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&dptr), g_watch_host, 0) != cudaSuccess ||
-        publish_mirror_here(dptr) != cudaSuccess || sc_band_publish_mirror(dptr) != 0 || sc_up_publish_mirror(dptr) != 0) {
-      cudaGetLastError();
-      return -1;
-    }
-    g_watch_devs |= 1ull << dev;
+  int* dptr = nullptr;
+  cudaStream_t st = nullptr;
+  bool ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
+  ok = ok && cudaHostGetDevicePointer(reinterpret_cast<void**>(&dptr), g_watch_host, 0) == cudaSuccess &&
+       publish_mirror_here(dptr, st) == cudaSuccess && sc_band_publish_mirror(dptr, st) == 0 && sc_up_publish_mirror(dptr, st) == 0;
+  if (st) cudaStreamDestroy(st);
+  if (!ok) {
+    cudaGetLastError();
+    return -1;
   }
+  g_watch_devs |= 1ull << dev;
   return *const_cast<volatile int*>(g_watch_host);
 }
 

@@ -26,7 +26,10 @@ inline int timeouts_here() {
   int v = -1;
   return cudaMemcpyFromSymbol(&v, g_umma_timeouts, sizeof(int)) == cudaSuccess ? v : -1;
 }
-inline cudaError_t publish_mirror_here(int* dptr) { return cudaMemcpyToSymbol(g_umma_host_mirror, &dptr, sizeof(dptr)); }
+inline cudaError_t publish_mirror_here(int* dptr, cudaStream_t st) {   // the stream is waited for: a capture elsewhere goes on
+  const cudaError_t e = cudaMemcpyToSymbolAsync(g_umma_host_mirror, &dptr, sizeof(dptr), 0, cudaMemcpyHostToDevice, st);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+}
 inline cudaError_t clear_timeouts_here() {
   const int zero = 0;
   return cudaMemcpyToSymbol(g_umma_timeouts, &zero, sizeof(int));

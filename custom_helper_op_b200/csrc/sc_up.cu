@@ -459,7 +459,7 @@ int sc_up_f32_launch(const ScArgs& a, cudaStream_t st) {
   return -4;
 }
 int sc_up_timeouts() { return timeouts_here(); }
-int sc_up_publish_mirror(int* dptr) { return (int)publish_mirror_here(dptr); }
+int sc_up_publish_mirror(int* dptr, cudaStream_t st) { return (int)publish_mirror_here(dptr, st); }
 int sc_up_clear_timeouts() { return (int)clear_timeouts_here(); }
 
 }  // namespace chop

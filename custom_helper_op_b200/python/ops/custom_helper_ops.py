@@ -306,10 +306,10 @@ def _scalar(value, like):
 
 
 def _umma_watch(images):
-    """Before a tensor-core (bfloat16) manifold-convolution call: raise if a kernel of an EARLIER call gave up a
-    bounded wait on its MMA barrier - the outputs of the calls since the last check are then incomplete.  Reads one
-    int of pinned host memory (chop_umma_watch); only the first call per device synchronises."""
-    if images.dtype != torch.bfloat16:
+    """Before a manifold-convolution call that may take tensor-core kernels (bfloat16 and float32): raise if a kernel of
+    an EARLIER call gave up a bounded wait on its MMA barrier - the outputs of the calls since the last check are then
+    incomplete.  Reads one int of pinned host memory (chop_umma_watch); only the first call per device does more."""
+    if images.dtype not in (torch.bfloat16, torch.float32):
         return
     with torch.cuda.device(images.device):
         n = _lib.lib().chop_umma_watch()

@@ -255,7 +255,8 @@ CHOP_API int chop_umma_timeouts(void);
 /* The same count without touching the device, for hosts that must not synchronise (a framework op, a serving loop):
  * the kernels also bump a mapped, pinned host int once this function has published it to the current device.  The
  * first call in a process allocates that int (4 bytes, cudaHostAlloc) and the first call per device copies its address
- * to the device - those calls synchronise; every later call only reads host memory.  Give-ups on a device before its
+ * to the device, on a stream of its own that it waits for (also while another stream is being captured); every later call
+ * only reads host memory.  Give-ups on a device before its
  * first call are not in the count, and a bump becomes visible when the kernel that made it has written it through,
  * at the latest when that kernel ends: a caller polls before its NEXT call, or after its own synchronisation point.
  * No compute entry point calls this by itself (they allocate nothing).  -1 if the mirror cannot be set up. */

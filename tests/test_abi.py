@@ -91,9 +91,10 @@ def test_tuning_knobs_are_inert_without_the_opt_in():
 
 
 def test_wrappers_refuse_to_run_after_a_reported_give_up(monkeypatch):
-    """Host logic of the non-synchronising check: the bf16 manifold-convolution wrappers read chop_umma_watch()
-    before launching and raise when it reports abandoned waits; other dtypes do not look.  (A fake library stands
-    in: without a device the real entry point answers -1, 'no mirror', which the wrappers ignore.)"""
+    """Host logic of the non-synchronising check: the bfloat16 and float32 manifold-convolution wrappers, whose kernels
+    wait for MMAs, read chop_umma_watch() before launching and raise when it reports abandoned waits; float64 does not
+    look.  (A fake library stands in: without a device the real entry point answers -1, 'no mirror', which the wrappers
+    ignore.)"""
     import contextlib
     import types
     import torch
@@ -105,11 +106,14 @@ def test_wrappers_refuse_to_run_after_a_reported_give_up(monkeypatch):
     monkeypatch.setattr(torch.cuda, "device", lambda dev: contextlib.nullcontext())
     bf16 = types.SimpleNamespace(dtype=torch.bfloat16, device=torch.device("cuda", 0))
     f32 = types.SimpleNamespace(dtype=torch.float32, device=torch.device("cuda", 0))
+    f64 = types.SimpleNamespace(dtype=torch.float64, device=torch.device("cuda", 0))
     ops._umma_watch(bf16)
     for n in (-1, 0):
         count["n"] = n
         ops._umma_watch(bf16)
+        ops._umma_watch(f32)
     count["n"] = 2
-    ops._umma_watch(f32)
-    with pytest.raises(RuntimeError, match="2 tensor-core convolution wait"):
-        ops._umma_watch(bf16)
+    ops._umma_watch(f64)
+    for images in (bf16, f32):
+        with pytest.raises(RuntimeError, match="2 tensor-core convolution wait"):
+            ops._umma_watch(images)

@@ -83,3 +83,32 @@ def test_manifold_convolution_step_replays_from_a_graph():
     assert torch.equal(got[0], want_out)
     for x, y in zip(got[1:], want_grads):
         assert helpers.rel_err(x.float().cpu().numpy(), y.float().cpu().numpy()) <= 1e-6
+
+
+def test_a_first_float32_convolution_may_be_captured():
+    """A process whose very first convolution is a captured float32 one: setting up the record of abandoned waits neither
+    spoils the capture nor is left out by it."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from custom_helper_op_b200 import _lib
+from custom_helper_op_b200.python.ops import custom_helper_ops as ops
+g = torch.Generator(device="cuda").manual_seed(1)
+x = torch.randn((1, 9, 21, 7, 16), generator=g, device="cuda")
+f = torch.randn((3, 3, 3, 16, 16), generator=g, device="cuda")
+z = torch.zeros((), device="cuda")
+b = torch.zeros((1, 9, 21, 1), dtype=torch.int32, device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    y = ops.sparse_conv3d_fast(x, f, z, b)
+x.normal_(generator=g)
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(y, ops.sparse_conv3d_fast(x, f, z, b))
+assert _lib.lib().chop_umma_watch() == 0
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stdout + out.stderr

@@ -242,8 +242,8 @@ def test_autograd_wrapper():
 def test_a_give_up_reaches_the_host_without_a_synchronising_poll():
     """The bookkeeping a tensor-core kernel performs when a bounded wait runs out, exercised without any wait: a
     one-thread kernel bumps the device counter and its pinned host mirror (test knob "note_timeout").  The host sees
-    the count through chop_umma_watch() - a plain read of host memory - and the bf16 wrappers refuse to run until
-    the counters are cleared."""
+    the count through chop_umma_watch() - a plain read of host memory - and the wrappers of both types that have
+    tensor-core kernels refuse to run until the counters are cleared."""
     from custom_helper_op_b200 import _lib
     from custom_helper_op_b200.python.ops import custom_helper_ops as ops
     L = _lib.lib()
@@ -256,9 +256,13 @@ def test_a_give_up_reaches_the_host_without_a_synchronising_poll():
         _lib.set_tuning("note_timeout", 1)
         torch.cuda.synchronize()
         assert L.chop_umma_watch() == 1 and L.chop_umma_timeouts() == 1
-        with pytest.raises(RuntimeError, match="timed out"):
-            ops.sparse_conv3d_forward(*args)
-        ops.sparse_conv3d_forward(args[0].float(), args[1].float(), args[2], args[3])   # float32: no tensor-core kernel, no check
+        for dt in (torch.bfloat16, torch.float32):
+            a = (args[0].to(dt), args[1].to(dt), args[2], args[3])
+            with pytest.raises(RuntimeError, match="timed out"):
+                ops.sparse_conv3d_forward(*a)
+            with pytest.raises(RuntimeError, match="timed out"):   # the differentiable op and its native node
+                ops.sparse_conv3d_fast(*a)
+        ops.sparse_conv3d_forward(args[0].double(), args[1].double(), args[2], args[3])   # float64: no tensor-core kernel, no check
     finally:
         _lib.set_tuning("note_timeout", 0)
     assert L.chop_umma_watch() == 0 and L.chop_umma_timeouts() == 0
