@@ -22,7 +22,7 @@
 // Tiles of four rows with 256 threads: 45; of one row: 49; windows that do not divide 32 rows (25 for 17 planes): 108.
 //
 // float32: a value is the exact sum of three bfloat16 pieces, x = x1 + x2 + x3, and x*w the sum of the six products
-// x1w1, x1w2, x2w1, x1w3, x2w2, x3w1 (what is left out is below 2^-24 of it).  Steps whose values are not finite or all tiny are
+// x1w1, x1w2, x2w1, x1w3, x2w2, x3w1 (what is left out is below 2^-24 of it).  Steps that the pieces cannot hold (pieces_fit) are
 // computed by plain multiply-adds (band_plain).  189x251x7, 16 -> 16 channels: 150 us with a thread per four voxels (sc_tile.cu),
 // 127 in runs of planes (sc_run.cu), 88 here; 16 -> 32 334, 238, 166.  Bound: 79 % of the shared-memory data pipe (operands 38,
 // load-store 41) at eight warps an SM; with a quarter of the MMAs 72 us, without the loads 90, without splitting 85.  Three
@@ -257,14 +257,14 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
   open(cur, tab_s[0]);
   request(cur, tab_s[0]);
   ahead = entry(cur.tile + (int)gridDim.x);             // of the tile after the present one
-  bool plain_filter = false;
+  unsigned w_top = 0;                                   // float32: the filter's largest magnitude
   if constexpr (P == 1) {
     stage_filter_tiles<CR, NR, DGRAD, true>(static_cast<const unsigned short*>(a.filters), sB, tid, B_LBO, B_SBO, B_TAP_BYTES);
   } else {
     const unsigned top = __reduce_max_sync(0xffffffffu, stage_filter_pieces<CR, NR, NF, DGRAD>(static_cast<const float*>(a.filters), n0, sB, tid, B_LBO, B_SBO, B_TAP_BYTES));
     if (lane == 0) top_s[warp] = top;
     __syncthreads();
-    plain_filter = not_for_pieces(max(max(top_s[0], top_s[1]), max(top_s[2], top_s[3])));
+    w_top = max(max(top_s[0], top_s[1]), max(top_s[2], top_s[3]));
     __syncthreads();
     if (tid < 3) top_s[tid] = 0;
   }
@@ -318,8 +318,8 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if constexpr (P > 1) {
-      if (cur.sub < 0 || cur.sub % G::GROUPS == 0) plain = plain_filter;
-      plain = plain || not_for_pieces(top_s[buf]);
+      if (cur.sub < 0 || cur.sub % G::GROUPS == 0) plain = false;
+      plain = plain || !pieces_fit<CR>(top_s[buf], w_top);
       if (tid == 0) top_s[next(next(buf))] = 0;         // read in the last step, written two steps on
     }
     if (tid == 0) {

@@ -126,8 +126,8 @@ __device__ __forceinline__ void stage_filter_tiles(const unsigned short* flt, un
   }
 }
 
-// Eight float32 values as three bfloat16 pieces each, every piece the nearest to what is left: x = x1 + x2 + x3 exactly (the
-// remainders have 15 and 6 significant bits).  Cut off instead of rounded, all pieces of a value have its sign and the products
+// Eight float32 values as three bfloat16 pieces each, every piece the nearest to what is left: x = x1 + x2 + x3, exactly from
+// |x| = 2^-109 on (the remainders have 15 and 6 significant bits; below, x3 is rounded to a multiple of 2^-133).  Cut off instead of rounded, all pieces of a value have its sign and the products
 // that are left out add up: 2-norm error of the transposed forward, strides (2,2,2), 16 channels, 1.02e-7.
 __device__ __forceinline__ void split3(const float (&v)[8], unsigned (&p)[3][4]) {
 #pragma unroll
@@ -144,15 +144,28 @@ __device__ __forceinline__ void split3(const float (&v)[8], unsigned (&p)[3][4])
     }
   }
 }
-// Largest magnitude, as bits.  Values of which it is not finite, rounds to an infinity, or is not zero and below 2^-50, are not for the pieces: an
-// infinity times a zero piece is not a number, and products of low pieces would fall below the normal range.
+// Largest magnitude, as bits.
 __device__ __forceinline__ unsigned top_bits(const float (&v)[8]) {
   unsigned m = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
   return m;
 }
-__device__ __forceinline__ bool not_for_pieces(unsigned top) { return top >= 0x7f7f0000u || (top != 0 && top < 0x26800000u); }
+// Whether sums of 27*CR products x*w can be made of pieces; x: largest magnitude of a step's values (top_bits), w: of the filter.
+//   * Finite, and not rounded to an infinity: that times a zero piece is not a number.
+//   * No sum of so many products, rounded up to the next power of two, can pass the largest float: x1*w1 and the small products are
+//     added up apart, so an overflow would be an infinity too early, or two of them with different signs.
+//   * Neither x nor w nor their product below 2^-100, so that the third pieces (2^-17 of the value) and what they are multiplied to are
+//     normal numbers.  Smaller values beside these lose bits below 2^-133, the end of bfloat16's subnormal numbers.
+template <int CR>
+__device__ __forceinline__ bool pieces_fit(unsigned x, unsigned w) {
+  constexpr int LOG = CR == 8 ? 8 : CR == 16 ? 9 : 10;  // 27*CR <= 2^LOG
+  constexpr unsigned INF = 0x7f7f0000u;
+  if (x >= INF || w >= INF) return false;
+  if (x == 0 || w == 0) return true;
+  const int ex = (int)(x >> 23) - 127, ew = (int)(w >> 23) - 127;   // the values are below 2^(e + 1)
+  return ex >= -100 && ew >= -100 && ex + ew >= -100 && ex + ew + 2 + LOG <= 127;
+}
 
 }  // namespace
 }  // namespace chop

@@ -207,14 +207,15 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
       for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(o + q * G::PIECE) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
     }
   }
-  bool plain_filter = false, plain = false;
+  unsigned w_top = 0;                                   // float32: the filter's largest magnitude
+  bool plain = false;
   if constexpr (P > 1) {
     if (tid < 4) top_s[tid] = 0;
     __syncthreads();
     top = __reduce_max_sync(0xffffffffu, top);
     if (lane == 0) atomicMax(&top_s[3], top);
     __syncthreads();
-    plain_filter = not_for_pieces(top_s[3]);
+    w_top = top_s[3];
   }
   for (int e = tid; e < 8 * NR; e += 256) {
     const int n = e % NR, par = e / NR % 2, cls = e / NR / 2, pr = cls < 2, pc = cls == 1 || cls == 2;
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if constexpr (P > 1) {
-      plain = plain_filter || not_for_pieces(top_s[buf]);
+      plain = !pieces_fit<CR>(top_s[buf], w_top);
       if (tid == 0) top_s[next(next(buf))] = 0;         // read in the last step, written two steps on
     }
     if (tid == 0) {
