@@ -167,5 +167,26 @@ __device__ __forceinline__ bool pieces_fit(unsigned x, unsigned w) {
   return ex >= -100 && ew >= -100 && ex + ew >= -100 && ex + ew + 2 + LOG <= 127;
 }
 
+// For sums that the pieces cannot hold: s[j] += x . (the weights of produced channel j), four gathered and four produced channels.
+// The filter may lie at any address.  w: FWD weight [0][0] of rows of NF produced channels, otherwise of rows of CR gathered ones.
+__device__ __forceinline__ float4 ld4_any(const float* p, bool aligned) {
+  return aligned ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+template <bool FWD>
+__device__ __forceinline__ void plain_fma(float (&s)[4], const float4& x, const float* w, int pitch, bool aligned) {
+  const float4 a = ld4_any(w, aligned), b = ld4_any(w + pitch, aligned), c = ld4_any(w + 2 * pitch, aligned), d = ld4_any(w + 3 * pitch, aligned);
+  if (FWD) {
+    s[0] = fmaf(x.w, d.x, fmaf(x.z, c.x, fmaf(x.y, b.x, fmaf(x.x, a.x, s[0]))));
+    s[1] = fmaf(x.w, d.y, fmaf(x.z, c.y, fmaf(x.y, b.y, fmaf(x.x, a.y, s[1]))));
+    s[2] = fmaf(x.w, d.z, fmaf(x.z, c.z, fmaf(x.y, b.z, fmaf(x.x, a.z, s[2]))));
+    s[3] = fmaf(x.w, d.w, fmaf(x.z, c.w, fmaf(x.y, b.w, fmaf(x.x, a.w, s[3]))));
+  } else {
+    s[0] = fmaf(x.w, a.w, fmaf(x.z, a.z, fmaf(x.y, a.y, fmaf(x.x, a.x, s[0]))));
+    s[1] = fmaf(x.w, b.w, fmaf(x.z, b.z, fmaf(x.y, b.y, fmaf(x.x, b.x, s[1]))));
+    s[2] = fmaf(x.w, c.w, fmaf(x.z, c.z, fmaf(x.y, c.y, fmaf(x.x, c.x, s[2]))));
+    s[3] = fmaf(x.w, d.w, fmaf(x.z, d.z, fmaf(x.y, d.y, fmaf(x.x, d.x, s[3]))));
+  }
+}
+
 }  // namespace
 }  // namespace chop

@@ -46,22 +46,32 @@ __device__ __forceinline__ int up_slot(int fr, int fc) {
 }
 
 // The sums of the fine pixels `todo` (coarse pixel*4 + class) of a tile by plain multiply-adds: values that are not for the pieces.
-template <int CR, int NR>
-__device__ __noinline__ void up_plain(const ScArgs& a, int b, int i, int j0, unsigned todo, float pad) {
+// coarse, fine: the tile's tables; skip: as in band_plain.
+template <int CR, int NR, int SD, int PW>
+__device__ __noinline__ void up_plain(const ScArgs& a, const int2* coarse, const int2* fine, unsigned todo, float pad, bool skip) {
   const float* src = static_cast<const float*>(a.out_grad);
   const float* flt = static_cast<const float*>(a.filters);
-  for (; todo; todo &= todo - 1) {
-    const int f = __ffs(todo) - 1, cls = f % 4, r = 2 * i + (cls < 2), c = 2 * (j0 + f / 4) + (cls == 1 || cls == 2);
-    for (int e = threadIdx.x; e < a.D * NR; e += 256) {
-      const int n = e % NR, dz = e / NR;
-      float s = 0.f;
-      for (int t = 0; t < 27; ++t) {
-        const long long v = sc_tap_t(a, b, r, c, dz, t / 9, t / 3 % 3, t % 3);
-        if (v < 0 && pad == 0.f) continue;
-        for (int k = 0; k < CR; ++k) s = fmaf(v < 0 ? pad : __ldg(src + v * CR + k), __ldg(flt + ((size_t)(26 - t) * NR + n) * CR + k), s);
-      }
-      static_cast<float*>(a.images_grad)[(((size_t)(b * a.H + r) * a.W + c) * a.D + dz) * NR + n] = s;
+  const bool aligned = (reinterpret_cast<size_t>(flt) & 15) == 0;
+  const float4 pad4 = make_float4(pad, pad, pad, pad);
+  constexpr int N4 = NR / 4;
+  for (int e = threadIdx.x; e < 4 * (PW - 1) * a.D * N4; e += 256) {
+    const int n = e % N4 * 4, d = e / N4 % a.D, f = e / N4 / a.D;
+    if (!((todo >> f) & 1u)) continue;
+    const int2 o = fine[f];
+    const bool pr = f % 4 < 2, pc = f % 4 == 1 || f % 4 == 2;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int t = 0; t < 27; ++t) {
+      const int fr = t / 9, fc = t / 3 % 3, od = d + o.y - 1 + t % 3;
+      const int2 c = coarse[(fr == 2 ? PW : 0) + f / 4 + (fc == 2)];
+      const int plane = (SD == 1 ? od : od >> 1) - c.y;
+      const bool in = (fr != 1) == pr && (fc != 1) == pc && (SD == 1 || (od & 1) == 0) && c.x >= 0 && !oob(plane, a.oD);
+      if (!in && skip) continue;
+      const float4* x = reinterpret_cast<const float4*>(src + (size_t)(in ? c.x + plane : 0) * CR);
+      const float* w = flt + ((size_t)(26 - t) * NR + n) * CR;
+#pragma unroll 1
+      for (int k = 0; k < CR; k += 4) plain_fma<false>(s, in ? __ldg(x + k / 4) : pad4, w + k, CR, aligned);
     }
+    *reinterpret_cast<float4*>(static_cast<float*>(a.images_grad) + ((size_t)o.x + d) * NR + n) = make_float4(s[0], s[1], s[2], s[3]);
   }
 }
 
@@ -336,10 +346,7 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
     constexpr int NE = P == 1 ? NR : 8;                 // channels at a time
     const int m = tid & 127, q = m / RP, w = m % RP;
     if (P > 1 && plain) {
-      if constexpr (P > 1) {
-        const int t = cur.tile / tiles_w;
-        up_plain<CR, NR>(a, t / a.oH, t % a.oH, cur.tile % tiles_w * PT, cur.now, padf);
-      }
+      if constexpr (P > 1) up_plain<CR, NR, SD, PW>(a, coarse_s[buf], fine_s[buf], cur.now, padf, a.pad_zero || (!padded && w_top < 0x7f800000u));
     } else {
 #pragma unroll 1
       for (int l = tid / 128 * (NCLS / 2); l < (tid / 128 + 1) * (NCLS / 2); ++l) {

@@ -79,3 +79,48 @@ def test_small_values_beside_ordinary_ones(form):
     # and products below 2^-126 that the tensor core may round to a multiple of 2^-149: K of them and their sums
     bound = K * 2.0 ** -24 * terms + 2.0 ** -133 * np.abs(ws).astype(np.float64).sum(0) + 8 * K * 2.0 ** -149
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max(1)
+
+
+@pytest.mark.parametrize("spread", [3, 60])       # base planes that fit a window, and that do not
+@pytest.mark.parametrize("default", [0.0, 0.75])
+@pytest.mark.parametrize("form", FORMS)
+def test_values_that_are_no_numbers(form, default, spread):
+    """Infinities and NaN in either operand, against the kernels with a thread per output: where results are not finite, and the rest.
+    A tap that is padding multiplies the default value in the forward forms, also a zero, and adds nothing in the gradients."""
+    op, strides, K, N = form
+    H, W, D = SIZE
+    rng = np.random.default_rng(spread)
+    rnd = lambda *s: rng.standard_normal(s).astype(np.float32)
+    coarse = [-(-n // s) for n, s in zip(SIZE, strides)]
+    images, filters = rnd(1, *coarse, K), rnd(*((3, 3, 3, K, N) if op == "conv" else (3, 3, 3, N, K)))
+    bp = torch.from_numpy(rng.integers(0, spread + 1, (1, H, W, 1)).astype(np.int32)).cuda()
+    fine = torch.zeros((1, H, W, D, N), device="cuda")
+    bad_images, bad_filters, tiny = images.copy(), filters.copy(), images.copy()
+    for a, at in ((bad_images, (0, 2, 3, 1)), (bad_filters, (0, 2, 1))):
+        a[at + (3,) * (5 - len(at))] = np.inf
+        a[(0, 1, 2, 2, 5)[:len(a.shape)] if a is bad_images else (2, 0, 1, 5, 4)] = np.nan
+    tiny *= np.float32(2.0 ** -110)               # a step of these is computed without pieces
+    tiny[0, :, 10:] = images[0, :, 10:]           # beside steps that are not
+
+    def run(i, f):
+        i, f = torch.from_numpy(i).cuda(), torch.from_numpy(f).cuda()
+        if op == "conv":
+            return [ops.sparse_conv3d_forward(i, f, default, bp, strides).cpu().numpy()]
+        return [ops.sparse_conv3d_transpose_forward(i, f, default, bp, SIZE, strides).cpu().numpy(),
+                ops.sparse_conv3d_backward(fine, f, default, bp, i, strides)[0].cpu().numpy()]
+
+    for i, f in ((bad_images, filters), (images, bad_filters), (tiny, filters)):
+        got = run(i, f)
+        _lib.set_tuning("tile", 0)
+        try:
+            want = run(i, f)
+        finally:
+            _lib.set_tuning("tile", 1)
+        for g, w in zip(got, want):
+            assert np.array_equal(np.isnan(g), np.isnan(w)) and np.array_equal(np.isposinf(g), np.isposinf(w))
+            assert np.array_equal(np.isneginf(g), np.isneginf(w))
+            ok = np.isfinite(w)
+            assert np.isfinite(w).any() and (np.abs(g[ok] - w[ok]) <= 3e-6 * np.abs(w[ok]).max()).all()
+            if i is tiny and default == 0.0:      # and the voxels that see small values alone, relative to themselves
+                small = np.abs(w) < 2.0 ** -90
+                assert small.any() and (np.abs(g[small] - w[small]) <= 3e-6 * np.abs(w[small]).max()).all()
