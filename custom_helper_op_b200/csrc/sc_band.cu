@@ -13,18 +13,24 @@
 //     filter row fr of output row hr - fr, and the output rows' accumulators lie side by side, last row first.
 //   * A pixel's D planes and one on either side must lie in the window: base_plane may vary by RP-2-D over the tile.  A tile
 //     that varies more takes a second pass with the window moved; one that would need a third is "rough" (a random base
-//     plane, not a depth map) and stages its filter columns one by one, each pixel's rows shifted as in sc_umma_rows_kernel.
+//     plane, not a depth map) and stages its filter columns one by one, each pixel's rows shifted as in sc_umma_rows_kernel, as many
+//     columns a step as shared memory holds beside the other CTAs (all nine of 8 or 16 bfloat16 channels, five otherwise).
 //
 // Base planes of 64 planes over the image (two sinusoid periods), D = 9: 1.00 passes a tile at 256x320 pixels, 1.4 at 100x125.
 // Bound: the shared-memory data pipe (56 % load-store, of which half is the epilogue's tensor-memory reads and shuffles; 35 %
 // MMA operands) and, with four CTAs an SM, a tile's chain of staging, MMAs and epilogue.  256x320x9, 3x3x3, bfloat16, us:
 // 16 -> 16 channels 59 -> 41, 8 -> 8 51 -> 33, 32 -> 32 213 -> 100, 32 -> 16 129 -> 74; at 17 planes 97 -> 72, 344 -> 182.
 // Tiles of four rows with 256 threads: 45; of one row: 49; windows that do not divide 32 rows (25 for 17 planes): 108.
+// Base planes that vary: smooth / smooth with up to eight planes of noise on it / random, us of sc_umma_rows_kernel | with the window's
+// rows as the rough tile's buffer | here: 256x320x9 16 -> 16 57 / 56 / 53 | 37 / 96 / 94 | 36 / 65 / 59; 8 -> 8 51 / 50 / 50 | 34 / 73 / 71 |
+// 33 / 52 / 49; 32 -> 32 210 / 210 / 198 | 98 / 255 / 250 | 84 / 182 / 176; 16 -> 32 76 / 74 / 70 | 64 / 126 / 123 | 59 / 91 / 84; objects in
+// front of a background, sharp edges: 16 -> 16 57 | 49 | 44.  float32 189x251x7 16 -> 16, sc_tile.cu first, which leaves out taps that no voxel
+// of a warp has: 138 / 135 / 61 | 81 / 157 / 182 | 75 / 144 / 143.
 //
 // float32: a value is the exact sum of three bfloat16 pieces, x = x1 + x2 + x3, and x*w the sum of the six products
 // x1w1, x1w2, x2w1, x1w3, x2w2, x3w1 (what is left out is below 2^-24 of it).  Steps that the pieces cannot hold (pieces_fit) are
 // computed by plain multiply-adds (band_plain).  189x251x7, 16 -> 16 channels: 150 us with a thread per four voxels (sc_tile.cu),
-// 127 in runs of planes (sc_run.cu), 88 here; 16 -> 32 334, 238, 166.  Bound: 79 % of the shared-memory data pipe (operands 38,
+// 127 in runs of planes (sc_run.cu), 80 here; 16 -> 32 334, 238, 150.  Bound: 79 % of the shared-memory data pipe (operands 38,
 // load-store 41) at eight warps an SM; with a quarter of the MMAs 72 us, without the loads 90, without splitting 85.  Three
 // groups of four warps around one filter 92 us, a thread per four channels instead of eight 99.
 #include "sc_entry.h"
@@ -52,15 +58,21 @@ template <typename T, int CR, int NR, int RP> struct BandGeo {
   static constexpr int R = BandType<T>::rows(CR, NR); // MMA blocks of a tile
   static constexpr int PW = PT + 2, NPIX = (R + 2) * PW;
   static constexpr int ROWS = NPIX * RP;              // staged rows
-  static constexpr int NRB = ROWS + 4;                // K-chunk stride 64 bytes off a multiple of 128 (bank conflicts)
-  static constexpr int CG = ROWS / 128;               // filter columns per step of a rough tile
-  static constexpr int GROUPS = (9 + CG - 1) / CG;
   static constexpr int FILTER = P * 27 * pad16(NR) * pad16(CR) * 2;
-  static constexpr size_t SMEM = (size_t)FILTER + (size_t)P * (pad16(CR) / 8) * NRB * 16 + 1024;
+  static constexpr int ROW = P * (pad16(CR) / 8) * 16;   // bytes of a staged row
   static constexpr int COLS = R * P * 3 * pad16(NR);  // accumulators
   static constexpr uint32_t TMEM = COLS <= 64 ? 64 : COLS <= 128 ? 128 : 256;
-  static constexpr int BY_SMEM = (int)((size_t)224 * 1024 / (SMEM + 2048)), BY_TMEM = 512 / TMEM;
+  // CTAs that an SM holds with the window alone; the filter columns per step of a rough tile fill what that leaves of shared memory
+  static constexpr int PER_SM = 224 * 1024;
+  static constexpr int BY_SMEM = PER_SM / (FILTER + (ROWS + 4) * ROW + 3072), BY_TMEM = 512 / TMEM;
   static constexpr int CTAS = BY_SMEM < 1 ? 1 : BY_SMEM < BY_TMEM ? BY_SMEM : BY_TMEM;
+  static constexpr int FIT = (PER_SM / CTAS - FILTER - 3072 - 4 * ROW) / (128 * ROW);
+  static constexpr int GROUPS = FIT >= 9 ? 1 : FIT >= 5 ? 2 : 3;   // steps per image row of a rough tile
+  static constexpr int CG = (9 + GROUPS - 1) / GROUPS;
+  static constexpr int SROWS = CG * 128 > ROWS ? CG * 128 : ROWS;
+  static constexpr int NRB = SROWS + 4;               // K-chunk stride 64 bytes off a multiple of 128 (bank conflicts)
+  static constexpr size_t SMEM = (size_t)FILTER + (size_t)NRB * ROW + 1024;
+  static_assert(FIT >= 3, "rough tiles");
   static_assert(PT * RP == 128 && 32 % RP == 0 && ROWS % 8 == 0 && NPIX <= 128 && R * PT <= 32 && COLS <= 256 && (P == 1 || R == 1), "tile");
 };
 
@@ -148,8 +160,8 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
   T* dst = static_cast<T*>(DGRAD ? a.images_grad : a.output) + n0;
 
   if (KR < KC)   // the padding channels stay zero
-    for (int e = tid; e < P * G::ROWS; e += 128)
-      *reinterpret_cast<uint4*>(sX + (e / G::ROWS * KC + 1) * A_LBO + e % G::ROWS * 16) = make_uint4(0, 0, 0, 0);
+    for (int e = tid; e < P * G::SROWS; e += 128)
+      *reinterpret_cast<uint4*>(sX + (e / G::SROWS * KC + 1) * A_LBO + e % G::SROWS * 16) = make_uint4(0, 0, 0, 0);
   constexpr uint32_t TCOLS = G::TMEM;
   if (warp == 0) {
     uint32_t slot = smem_u32(&tmem_base_s), ncols = TCOLS;
@@ -226,24 +238,47 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
   constexpr int VEC = (int)sizeof(T) / 2;               // 16-byte words of a chunk
   const int chunk = tid % KR, row0 = tid / KR;
   uint4 val[NI][VEC];
+  // A rough tile's step: rows of CG filter columns, UC of them at a time in `val`.  Column c is staged in rows c*128 .., RPC chunks
+  // of it by a thread, all of the same window row.
+  constexpr int RPC = 128 / RSTEP, UC = NI / RPC;
+  static_assert(RSTEP % RP == 0 && UC >= 1, "rough tiles");
+  auto request_columns = [&](const Step& s, const int2* tab, int c0) {
+    const int2* at = tab + s.sub / G::GROUPS * PW + row0 / RP;
+    const int first = s.sub % G::GROUPS * CG;
+    int from[RPC];
+#pragma unroll
+    for (int j = 0; j < RPC; ++j) from[j] = row0 % RP - 1 + at[PW + 1 + j * (RSTEP / RP)].y;
+#pragma unroll
+    for (int u = 0; u < UC; ++u) {
+      const int col = first + c0 + u;
+      if (c0 + u >= CG || col >= 9) continue;
+#pragma unroll
+      for (int j = 0; j < RPC; ++j) {
+        const int2 e = at[col / 3 * PW + col % 3 + j * (RSTEP / RP)];
+        const int plane = from[j] - e.y;
+        const bool in = e.x >= 0 && !oob(plane, D);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) {
+          val[u * RPC + j][k] = padv;
+          if (in) val[u * RPC + j][k] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(e.x + plane) * CR) + chunk * VEC + k);
+        }
+      }
+    }
+  };
   // The chunks of a row are fetched by neighbouring lanes, a pixel's planes by the lanes behind: consecutive addresses.
   auto request = [&](const Step& s, const int2* tab) {
+    if (s.sub >= 0) {
+      request_columns(s, tab, 0);
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int row = row0 + i * RSTEP;
       int2 e = make_int2(-1, 0);
       int plane = 0;
-      if ((i + 1) * RSTEP > G::ROWS && row >= G::ROWS) {   // a last, partial round
-      } else if (s.sub < 0) {
+      if ((i + 1) * RSTEP <= G::ROWS || row < G::ROWS) {   // a last, partial round
         e = tab[row / RP];
         plane = row % RP + s.z0 - e.y;
-      } else {
-        const int blk = s.sub / G::GROUPS, col = (s.sub % G::GROUPS) * CG + row / 128, q = row % 128 / RP;
-        if (col < 9) {
-          const int2 o = tab[(blk + 1) * PW + q + 1];
-          e = tab[(blk + col / 3) * PW + q + col % 3];
-          plane = row % RP - 1 + o.y - e.y;
-        }
       }
       const bool in = e.x >= 0 && !oob(plane, D);
 #pragma unroll
@@ -288,8 +323,8 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
 
   unsigned top = 0;
   bool plain = false;                                   // float32: this step's values are not for the pieces
-  auto store = [&](int i) {
-    unsigned char* o = sX + chunk * A_LBO + (row0 + i * RSTEP) * 16;
+  auto store = [&](int i, int row) {
+    unsigned char* o = sX + chunk * A_LBO + row * 16;
     if constexpr (P == 1) {
       *reinterpret_cast<uint4*>(o) = val[i][0];
     } else {
@@ -311,10 +346,20 @@ sc_band_kernel(const ScArgs a, const int ntiles, const int tiles_w, const int ti
     // the table of the next step; its buffer was last read two steps ago, before the barrier behind the last staging
     if (tid < NPIX) tab_s[next(buf)][tid] = again ? tab_s[buf][tid] : ahead;
     top = 0;
+    if (cur.sub < 0) {
 #pragma unroll
-    for (int i = 0; i < NI; ++i)
-      if ((i + 1) * RSTEP <= G::ROWS || row0 + i * RSTEP < G::ROWS)
-        store(i);
+      for (int i = 0; i < NI; ++i)
+        if ((i + 1) * RSTEP <= G::ROWS || row0 + i * RSTEP < G::ROWS)
+          store(i, row0 + i * RSTEP);
+    } else {
+#pragma unroll 1
+      for (int c0 = 0; c0 < CG; c0 += UC) {
+        if (c0 > 0) request_columns(cur, tab_s[buf], c0);
+#pragma unroll
+        for (int i = 0; i < UC * RPC; ++i)
+          if (c0 + i / RPC < CG && cur.sub % G::GROUPS * CG + c0 + i / RPC < 9) store(i, row0 + c0 * 128 + i * RSTEP);
+      }
+    }
     if constexpr (P > 1) {
       top = __reduce_max_sync(0xffffffffu, top);
       if (lane == 0) atomicMax(&top_s[buf], top);
