@@ -11,11 +11,18 @@
 // Depth: accumulator row zc holds, per tap fz, the product with coarse plane zc.  At depth stride 2 the fine plane 2*zc is tap 1 of
 // row zc, 2*zc + 1 is tap 0 of row zc plus tap 2 of row zc + 1; at depth stride 1 rows z-1, z, z+1 add up.
 // What a tap reads that does not exist (default_value, zero in gradients) is a constant per class and parity, added at the end.
-// Base planes that do not fit the window take further passes.
+// Base planes that do not fit the window take further passes, with the window moved.  A tile that would need a fifth is "rough" (no depth
+// map) and left for the end: there the operand of each of its nine (offset, class) pairs - filter columns - is staged by itself, every
+// fine pixel's rows from the first coarse plane that its own taps read, SL columns at a time.
 // Bound: the epilogue (48 accumulator columns per class and row) and a tile's chain of staging, MMAs and epilogue at two CTAs of
 // eight warps an SM.  Transposed forward, 256x320x9, bfloat16, strides (2,2,2), us with a gather per tap and class
 // (sc_umma_class_kernel) and here: 16 <- 16 channels 43, 32; 16 <- 32 80, 37; 8 <- 8 38, 27; at 17 planes 66, 36; strides (2,2,1) 45, 37;
 // 60x75x12 16, 12.  With 32 produced channels the accumulators do not fit twice: those stay there.
+// Base planes that vary: smooth / smooth with up to eight planes of noise on it / random, us of the gather | here with one pass more for
+// every pixel that does not fit | with rough tiles.  256x320x9, bfloat16: (2,2,2) 16 <- 16 40 / 40 / 38 | 34 / 36 / 387 | 35 / 37 / 55, 16 <- 32
+// 74 / 67 / 65 | 33 / 38 / 496 | 33 / 38 / 84; (2,2,1) 16 <- 16 41 / 40 / 38 | 31 / 63 / 439 | 32 / 64 / 51; float32 (sc_tile.cu, which leaves out
+// taps that no voxel of a warp has) (2,2,2) 16 <- 16 155 / 153 / 100 | 76 / 79 / 766 | 77 / 80 / 163.  Two passes and no more: noise
+// (2,2,1) 53, but objects with sharp edges in front of a background 40 instead of 37 (36 before, 41 the gather).
 #include "sc_entry.h"
 #include "sc_umma_common.cuh"
 #include "smem_grant.h"
@@ -29,7 +36,10 @@ template <typename T, int CR, int NR, int RP> struct UpGeo {
   static constexpr int P = sizeof(T) == 2 ? 1 : 3, NCLS = P == 1 ? 4 : 2;
   static constexpr int PT = 128 / RP;                 // coarse pixels of a tile
   static constexpr int PW = PT + 1, NPIX = 2 * PW;    // staged coarse pixels
-  static constexpr int ROWS = NPIX * RP, NRB = (ROWS + 7) / 8 * 8 + 4;
+  static constexpr int ROWS = NPIX * RP;
+  // filter columns that a rough tile stages at once, of nine; float32 has six (classes 0 and 1) or three
+  static constexpr int SL = P == 1 ? (CR <= 16 ? 9 : 5) : 3;
+  static constexpr int SROWS = ROWS > SL * 128 ? ROWS : SL * 128, NRB = (SROWS + 7) / 8 * 8 + 4;
   static constexpr int N3 = 3 * pad16(NR), COLS = 4 * N3;
   static constexpr int PIECE = 27 * pad16(NR) * pad16(CR) * 2;   // bytes of the filter's tiles
   static constexpr size_t SMEM = (size_t)P * PIECE + (size_t)P * (pad16(CR) / 8) * NRB * 16 + 1024;
@@ -37,6 +47,15 @@ template <typename T, int CR, int NR, int RP> struct UpGeo {
   static_assert(COLS <= 256 && 4 * PT <= 32, "tile");
 };
 
+// The columns of classes 2*half and 2*half + 1 by slot (half < 0: of all); the class of a slot and the coarse pixel that it reads.
+__device__ __forceinline__ int up_column(int half, int i) {
+  if (half < 0) return i;
+  if (half > 0) return i < 2 ? 2 + i : 7;
+  return i < 2 ? i : i < 5 ? 2 + i : 8;
+}
+__device__ __forceinline__ int up_class(int slot) { return slot < 4 ? slot : slot == 4 ? 0 : slot == 7 ? 2 : 1; }
+__device__ __forceinline__ int up_below(int slot) { return slot == 4 || slot == 5 || slot == 8; }
+__device__ __forceinline__ int up_right(int slot) { return slot >= 6; }
 // Tiles of the flipped, channel-swapped filter (stage_filter_tiles) in the order in which the operands use them: per offset
 // (di, dj) the classes side by side, three depth taps each.  Slot of filter column (fr, fc):
 //   (0,0): classes (1,0) fr 0 fc 1 | (1,1) 0 0 | (0,1) 1 0 | (0,0) 1 1;  (1,0): 2 1 | 2 0;  (0,1): 0 2 | 1 2;  (1,1): 2 2
@@ -86,6 +105,7 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
   __shared__ int2 coarse_s[3][NPIX];                    // first voxel (-1: outside the image), first absolute coarse plane
   __shared__ int2 fine_s[3][4 * PT];                    // per fine pixel [coarse pixel][class]: first voxel (-1: none), base plane
   __shared__ unsigned top_s[4];                         // float32: largest magnitude of a step, three steps in turn; the filter's
+  __shared__ unsigned rough_s[2];                       // rough tiles: a bit each, the last for all from the 64th on
   __shared__ float pad_s[4][2][NR];                     // class, parity: what the taps that do not exist add
   constexpr uint32_t B_LBO = 128, B_SBO = KC * 128;
   constexpr uint32_t A_LBO = NRB * 16, A_SBO = 128;
@@ -99,8 +119,8 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
   const int H = a.H, W = a.W, D = a.D, oD = a.oD;
 
   if (KR < KC)   // the padding channels stay zero
-    for (int e = tid; e < P * G::ROWS; e += 256)
-      *reinterpret_cast<uint4*>(sX + (e / G::ROWS * KC + 1) * A_LBO + e % G::ROWS * 16) = make_uint4(0, 0, 0, 0);
+    for (int e = tid; e < P * G::SROWS; e += 256)
+      *reinterpret_cast<uint4*>(sX + (e / G::SROWS * KC + 1) * A_LBO + e % G::SROWS * 16) = make_uint4(0, 0, 0, 0);
   if (tid < 32) {
     uint32_t slot = smem_u32(&tmem_base_s), ncols = 256;
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(ncols) : "memory");
@@ -164,10 +184,17 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
     s.left &= ~s.now;
   };
   auto fine_entry = [&](int buf) { return lane < 4 * PT ? fine_s[buf][lane] : make_int2(-1, 0); };
-  auto open = [&](Step& s, int buf) {
+  auto open = [&](Step& s, int buf) -> unsigned {       // the fine pixels of a rough tile, which gets none here; otherwise zero
     const int2 e = fine_entry(buf);
     s.left = __ballot_sync(0xffffffffu, e.x >= 0 && (P == 1 || lane % 4 / 2 == half));
+    const unsigned all = s.left;
     window(s, e);
+    if (s.left == 0) return 0;
+    Step t = s;
+    for (int pass = 1; pass < 4 && t.left != 0; ++pass) window(t, e);
+    if (t.left == 0) return 0;
+    s.now = s.left = 0;
+    return all;
   };
   constexpr int NI = (G::ROWS * KR + 255) / 256, RSTEP = 256 / KR;
   const int chunk = tid % KR, row0 = tid / KR;
@@ -194,7 +221,12 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
   int2 ahead = entry(cur.tile);
   keep(0, ahead);
   __syncthreads();
-  open(cur, 0);
+  auto mark = [&](int tile) {                           // a rough tile of this CTA, by their order
+    const int turn = min((tile - (int)blockIdx.x) / (int)gridDim.x, 63);
+    if (tid == 0) rough_s[turn / 32] |= 1u << (turn % 32);
+  };
+  if (tid == 0) rough_s[0] = rough_s[1] = 0;
+  if (open(cur, 0) != 0) mark(cur.tile);
   request(cur, 0);
   ahead = entry(cur.tile + (int)gridDim.x);
   // filter tiles: offset order; the loop of stage_filter_tiles with slots of its own
@@ -252,6 +284,92 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
   int buf = 0;
   auto next = [](int b) { return b == 2 ? 0 : b + 1; };
 
+  auto put = [&](int row, const uint4 (&v)[VEC]) -> unsigned {   // this thread's chunk of a row; float32: its largest magnitude
+    unsigned char* o = sX + chunk * A_LBO + row * 16;
+    if constexpr (P == 1) {
+      *reinterpret_cast<uint4*>(o) = v[0];
+      return 0;
+    } else {
+      const uint4 lo = v[0], hi = v[VEC - 1];
+      const float x[8] = {__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(lo.w),
+                          __uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z), __uint_as_float(hi.w)};
+      unsigned p[3][4];
+      split3(x, p);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(o + q * KC * A_LBO) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+      return top_bits(x);
+    }
+  };
+  // epilogue of the fine pixels `now`, whose windows begin at first(entry): the classes are dealt out to the two halves of the warps
+  auto finish = [&](unsigned now, int buf, auto first) {
+    if (now == 0) return;
+    constexpr int NE = P == 1 ? NR : 8;                 // channels at a time
+    const int m = tid & 127, q = m / RP, w = m % RP;
+    if (P > 1 && plain) {
+      if constexpr (P > 1) up_plain<CR, NR, SD, PW>(a, coarse_s[buf], fine_s[buf], now, padf, a.pad_zero || (!padded && w_top < 0x7f800000u));
+    } else {
+#pragma unroll 1
+      for (int l = tid / 128 * (NCLS / 2); l < (tid / 128 + 1) * (NCLS / 2); ++l) {
+        const int cls = P == 1 ? l : half * 2 + l;
+        const int2 e = fine_s[buf][q * 4 + cls];
+        const bool mine = (now >> (q * 4 + cls)) & 1u;
+#pragma unroll 1
+        for (int c0 = 0; c0 < NR; c0 += NE) {
+          uint32_t t[P == 1 ? 1 : 2][3][NE];
+          const uint32_t col = tmem + ((uint32_t)(m / 32 * 32) << 16) + l * N3 + c0;
+#pragma unroll
+          for (int g = 0; g < (P == 1 ? 1 : 2); ++g)
+#pragma unroll
+            for (int fz = 0; fz < 3; ++fz) tmem_ld<NE>(col + g * NCLS * N3 + fz * COUT, t[g][fz]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          float s[2][NE];
+#pragma unroll
+          for (int k = 0; k < NE; ++k) {
+            float f[3];
+#pragma unroll
+            for (int fz = 0; fz < 3; ++fz) {
+              f[fz] = __uint_as_float(t[0][fz][k]);
+              if constexpr (P > 1) f[fz] += __uint_as_float(t[1][fz][k]);
+            }
+            const float above = __shfl_down_sync(0xffffffffu, f[2], 1);
+            if (SD == 1) {
+              s[0][k] = __shfl_up_sync(0xffffffffu, f[0], 1) + f[1] + above;
+              s[1][k] = 0.f;
+            } else {
+              s[0][k] = f[1];
+              s[1][k] = f[0] + above;
+            }
+            if (padded) {
+              s[0][k] += pad_s[cls][0][c0 + k];
+              s[1][k] += pad_s[cls][1][c0 + k];
+            }
+          }
+#pragma unroll
+          for (int p = 0; p < SD; ++p) {
+            const int d = (w + first(e)) * SD + p - e.y;
+            if (!mine || oob(d, D)) continue;
+            T* o = dst + (size_t)(e.x + d) * NR + c0;
+            if constexpr (P == 1) {
+#pragma unroll
+              for (int k = 0; k < NE; k += 8) {
+                uint32_t h[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const __nv_bfloat162 b2 = __floats2bfloat162_rn(s[p][k + 2 * i], s[p][k + 2 * i + 1]);
+                  h[i] = *reinterpret_cast<const uint32_t*>(&b2);
+                }
+                *reinterpret_cast<uint4*>(o + k) = make_uint4(h[0], h[1], h[2], h[3]);
+              }
+            } else {
+#pragma unroll
+              for (int k = 0; k < NE; k += 4) *reinterpret_cast<float4*>(o + k) = make_float4(s[p][k], s[p][k + 1], s[p][k + 2], s[p][k + 3]);
+            }
+          }
+        }
+      }
+    }
+  };
+
   while (true) {
     const bool again = cur.left != 0;
     // the next step's tables; their buffer was last read two steps ago, before the barrier behind the last staging
@@ -261,19 +379,7 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       if ((i + 1) * RSTEP > G::ROWS && row0 + i * RSTEP >= G::ROWS) continue;
-      unsigned char* o = sX + chunk * A_LBO + (row0 + i * RSTEP) * 16;
-      if constexpr (P == 1) {
-        *reinterpret_cast<uint4*>(o) = val[i][0];
-      } else {
-        const uint4 lo = val[i][0], hi = val[i][VEC - 1];
-        const float v[8] = {__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(lo.w),
-                            __uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z), __uint_as_float(hi.w)};
-        top = max(top, top_bits(v));
-        unsigned p[3][4];
-        split3(v, p);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(o + q * KC * A_LBO) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
-      }
+      top = max(top, put(row0 + i * RSTEP, val[i]));
     }
     if constexpr (P > 1) {
       top = __reduce_max_sync(0xffffffffu, top);
@@ -325,7 +431,7 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
     if (!again) {
       nxt.tile = cur.tile + (int)gridDim.x;
       go = nxt.tile < ntiles;
-      if (go) open(nxt, next(buf));
+      if (go && open(nxt, next(buf)) != 0) mark(nxt.tile);
     } else {
       window(nxt, fine_entry(next(buf)));
     }
@@ -338,80 +444,89 @@ __global__ void __launch_bounds__(256, (UpGeo<T, CR, NR, RP>::CTAS)) sc_up_kerne
     phase ^= 1;
     if (!__syncthreads_and(done)) {
       if (tid == 0) note_timeout();
+      if (tid == 0) rough_s[0] = rough_s[1] = 0;
       break;
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    // ---- epilogue: the classes are dealt out to the two halves of the warps --------------------------------------
-    constexpr int NE = P == 1 ? NR : 8;                 // channels at a time
-    const int m = tid & 127, q = m / RP, w = m % RP;
-    if (P > 1 && plain) {
-      if constexpr (P > 1) up_plain<CR, NR, SD, PW>(a, coarse_s[buf], fine_s[buf], cur.now, padf, a.pad_zero || (!padded && w_top < 0x7f800000u));
-    } else {
-#pragma unroll 1
-      for (int l = tid / 128 * (NCLS / 2); l < (tid / 128 + 1) * (NCLS / 2); ++l) {
-        const int cls = P == 1 ? l : half * 2 + l;
-        const int2 e = fine_s[buf][q * 4 + cls];
-        const bool mine = (cur.now >> (q * 4 + cls)) & 1u;
-#pragma unroll 1
-        for (int c0 = 0; c0 < NR; c0 += NE) {
-          uint32_t t[P == 1 ? 1 : 2][3][NE];
-          const uint32_t col = tmem + ((uint32_t)(m / 32 * 32) << 16) + l * N3 + c0;
-#pragma unroll
-          for (int g = 0; g < (P == 1 ? 1 : 2); ++g)
-#pragma unroll
-            for (int fz = 0; fz < 3; ++fz) tmem_ld<NE>(col + g * NCLS * N3 + fz * COUT, t[g][fz]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          float s[2][NE];
-#pragma unroll
-          for (int k = 0; k < NE; ++k) {
-            float f[3];
-#pragma unroll
-            for (int fz = 0; fz < 3; ++fz) {
-              f[fz] = __uint_as_float(t[0][fz][k]);
-              if constexpr (P > 1) f[fz] += __uint_as_float(t[1][fz][k]);
-            }
-            const float above = __shfl_down_sync(0xffffffffu, f[2], 1);
-            if (SD == 1) {
-              s[0][k] = __shfl_up_sync(0xffffffffu, f[0], 1) + f[1] + above;
-              s[1][k] = 0.f;
-            } else {
-              s[0][k] = f[1];
-              s[1][k] = f[0] + above;
-            }
-            if (padded) {
-              s[0][k] += pad_s[cls][0][c0 + k];
-              s[1][k] += pad_s[cls][1][c0 + k];
-            }
-          }
-#pragma unroll
-          for (int p = 0; p < SD; ++p) {
-            const int d = (w + cur.z0) * SD + p - e.y;
-            if (!mine || oob(d, D)) continue;
-            T* o = dst + (size_t)(e.x + d) * NR + c0;
-            if constexpr (P == 1) {
-#pragma unroll
-              for (int k = 0; k < NE; k += 8) {
-                uint32_t h[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const __nv_bfloat162 b2 = __floats2bfloat162_rn(s[p][k + 2 * i], s[p][k + 2 * i + 1]);
-                  h[i] = *reinterpret_cast<const uint32_t*>(&b2);
-                }
-                *reinterpret_cast<uint4*>(o + k) = make_uint4(h[0], h[1], h[2], h[3]);
-              }
-            } else {
-#pragma unroll
-              for (int k = 0; k < NE; k += 4) *reinterpret_cast<float4*>(o + k) = make_float4(s[p][k], s[p][k + 1], s[p][k + 2], s[p][k + 3]);
-            }
-          }
-        }
-      }
-    }
+    finish(cur.now, buf, [&](const int2&) { return cur.z0; });
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     if (!go) break;
     cur = nxt;
     buf = next(buf);
+  }
+
+  __syncthreads();
+  if ((rough_s[0] | rough_s[1]) != 0) {
+    const int columns = P == 1 ? 9 : half == 0 ? 6 : 3;
+    bool ok = true;
+    int turn = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, turn += turn < 63) {
+      if (!((rough_s[turn / 32] >> (turn % 32)) & 1u)) continue;
+      __syncthreads();                                  // the tables and the largest magnitude have been read
+      keep(0, entry(tile));
+      if (tid == 0) top_s[0] = 0;
+      __syncthreads();
+      Step s;
+      const unsigned now = open(s, 0);
+      if (now == 0) continue;
+      for (int c0 = 0; ok && c0 < columns; c0 += G::SL) {
+        const int n = min(G::SL, columns - c0);
+        unsigned most = 0;
+        for (int row = row0; row < n * 128; row += RSTEP) {
+          const int slot = up_column(P == 1 ? -1 : half, c0 + row / 128), q = row % 128 / RP;
+          const int2 f = fine_s[0][q * 4 + up_class(slot)], e = coarse_s[0][up_below(slot) * PW + q + up_right(slot)];
+          const int plane = floor_sd(f.y - 1) + row % RP - e.y;
+          const bool in = f.x >= 0 && e.x >= 0 && !oob(plane, oD);
+          uint4 v[VEC];
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) {
+            v[k] = padv;
+            if (in) v[k] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(e.x + plane) * CR) + chunk * VEC + k);
+          }
+          most = max(most, put(row, v));
+        }
+        if constexpr (P > 1) {
+          most = __reduce_max_sync(0xffffffffu, most);
+          if (lane == 0) atomicMax(&top_s[0], most);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          for (int i = 0; i < n; ++i) {                 // columns 0 .. 3 are the first of their classes
+            const int slot = up_column(P == 1 ? -1 : half, c0 + i);
+            const uint32_t acc = tmem + (up_class(slot) - (P == 1 ? 0 : 2 * half)) * N3;
+#pragma unroll
+            for (int k16 = 0; k16 < CIN / 16; ++k16) {
+              const uint64_t dx = umma_desc_advance(da0, i * 128 * 16 + k16 * 2 * A_LBO);
+              const uint64_t dw = umma_desc_advance(db0, slot * 3 * B_TAP_BYTES + k16 * 2 * B_LBO);
+              const uint32_t add = slot >= 4 || k16 != 0 ? 1u : 0u;
+              umma_bf16(acc, dx, dw, idesc(1), add);
+              if constexpr (P > 1) {
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+#pragma unroll
+                  for (int r = p == 0 ? 1 : 0; r < 3 - p; ++r)
+                    umma_bf16(acc + NCLS * N3, umma_desc_advance(dx, p * KC * A_LBO), umma_desc_advance(dw, r * G::PIECE), idesc(1), p == 0 && r == 1 ? add : 1u);
+              }
+            }
+          }
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+        }
+        bool done = true;
+        if (tid < 32) done = mbar_wait(mbar, phase);
+        phase ^= 1;
+        ok = __syncthreads_and(done);
+        if (!ok && tid == 0) note_timeout();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      if (!ok) break;
+      if constexpr (P > 1) plain = !pieces_fit<CR>(top_s[0], w_top);
+      finish(now, 0, [&](const int2& e) { return floor_sd(e.y - 1); });
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
