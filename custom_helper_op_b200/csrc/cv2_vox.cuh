@@ -8,7 +8,7 @@
 // Bound: L1 (gather) and the widening.  Four views, planes 1 / 8 apart, us before and now:
 //   bfloat16 MEAN, 8 groups  1152x1536x8 437 / 442, 371 / 447; 288x384x48 193 / 198, 138 / 144; 2 groups 385 / 407, 332 / 352; 166 / 176, 127 / 131
 //   bfloat16 MIN,  8 groups  1152x1536x8 632 / 662, 527 / 529; 2 groups 554 / 582, 403 / 404
-//   float32  MEAN, 8 groups  288x384x48 205 / 223, 158 / 207; 1152x1536x8 598 / 634, 526 / 683 (the one place where it is slower)
+//   float32  MEAN, 8 groups  288x384x48 205 / 223, 158 / 207; 1152x1536x8 569 / 613, 516 / 610; where it is the slower one: v2_vox_fwd
 // PB = 4 against 2, bfloat16, 8 groups: 378 / 450 and 400 / 428 at 1152x1536x8, 143 / 146 and 157 / 157 at 288x384x48; 2 groups 335 / 410
 // and 336 / 353; float32 at 288x384x64, one view 104 and 135 (eight planes: 774 and 683).  Eight planes of four pixels 383 / 561.
 // Two or four voxels per lane (the cameras fetched once for them): 406 / 550, 454 / 631.  With 16 and 32 channels (two and four
@@ -19,11 +19,12 @@
 
 namespace chop {
 
-// A lane's eight consecutive channels of one texel, widened to pairs on use.
-template <typename T>
+// A lane's eight consecutive channels of one texel, widened to pairs on use.  WIDE: 32 bytes in one load where the type has as many
+// (two 16-byte loads of a warp's texels touch every line twice), which need addresses that are multiples of 32.
+template <typename T, bool WIDE = false>
 struct Ch8;
-template <>
-struct Ch8<__nv_bfloat16> {
+template <bool WIDE>
+struct Ch8<__nv_bfloat16, WIDE> {
   uint4 r;
   __device__ __forceinline__ void load(const __nv_bfloat16* p) { r = __ldg(reinterpret_cast<const uint4*>(p)); }
   __device__ __forceinline__ unsigned word(int k) const { return k == 0 ? r.x : k == 1 ? r.y : k == 2 ? r.z : r.w; }
@@ -33,12 +34,16 @@ struct Ch8<__nv_bfloat16> {
     return pk_make(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
   }
 };
-template <>
-struct Ch8<float> {
+template <bool WIDE>
+struct Ch8<float, WIDE> {
   pk2 r[4];
   __device__ __forceinline__ void load(const float* p) {
-    PkLoad<float>::ld(p, r[0], r[1]);
-    PkLoad<float>::ld(p + 4, r[2], r[3]);
+    if constexpr (WIDE) {
+      asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r[0]), "=l"(r[1]), "=l"(r[2]), "=l"(r[3]) : "l"(p));
+    } else {
+      PkLoad<float>::ld(p, r[0], r[1]);
+      PkLoad<float>::ld(p + 4, r[2], r[3]);
+    }
   }
   __device__ __forceinline__ pk2 get(int k) const { return r[k]; }
   __device__ __forceinline__ float one(int k) const {
@@ -53,6 +58,10 @@ __device__ __forceinline__ float dot2_bf16(unsigned a, unsigned b, float acc) { 
 // PB planes by 32/PB neighbouring pixels per warp: a lane is a voxel.
 constexpr int VOX_CTAS = 10;   // 128-thread CTAs per SM, 48 registers
 constexpr int VOX_MIN_CTAS = 8;
+// 32-byte loads: everywhere but in MIN with one channel per group, whose 64 registers do not hold their aligned groups (1152x1536x8, four
+// views, planes 1 / 8 apart: 581 / 717 us without, 686 / 790 with)
+template <int SUB, bool MIN>
+constexpr bool VOX_WIDE = !(MIN && SUB == 1);
 
 template <typename T, int SUB, int PB, bool MIN>
 __global__ void __launch_bounds__(128, MIN ? VOX_MIN_CTAS : VOX_CTAS) cv2_fwd_vox(const CvArgs a, const unsigned nitems, const unsigned ndb) {
@@ -76,7 +85,8 @@ __global__ void __launch_bounds__(128, MIN ? VOX_MIN_CTAS : VOX_CTAS) cv2_fwd_vo
   }
   const size_t pix = (size_t)b * hw + p;
   const float depth = __ldcs(static_cast<const float*>(a.depth) + pix * a.D + d);
-  Ch8<T> ref;
+  constexpr bool WIDE = VOX_WIDE<SUB, MIN>;
+  Ch8<T, WIDE> ref;
   ref.load(static_cast<const T*>(a.ref) + pix * C);
   pk2 acc[NA];
 #pragma unroll
@@ -106,7 +116,7 @@ __global__ void __launch_bounds__(128, MIN ? VOX_MIN_CTAS : VOX_CTAS) cv2_fwd_vo
     float dh, dw, gh, gw;
     const bool seen = project_rcp<false>(cf, depth, a, fh, fw, dh, dw, gh, gw);
     auto add = [&]() {
-      Ch8<T> x00, x01, x10, x11;
+      Ch8<T, WIDE> x00, x01, x10, x11;
       const T* q = src + (size_t)((fh - FLOOR_BIAS + a.Hs * (n + N * b)) * a.Ws + (fw - FLOOR_BIAS)) * C;
       x00.load(q);
       x01.load(q + C);
@@ -134,7 +144,7 @@ __global__ void __launch_bounds__(128, MIN ? VOX_MIN_CTAS : VOX_CTAS) cv2_fwd_vo
       bilinear_weights_fast(dh, dw, w00, w01, w11, w10);
       const pk2 p00 = pk_make(w00, w00), p01 = pk_make(w01, w01), p10 = pk_make(w10, w10), p11 = pk_make(w11, w11);
       if constexpr (DOT) {
-        auto dots = [&](const Ch8<T>& t) {           // both groups' products with the reference pixel
+        auto dots = [&](const Ch8<T, WIDE>& t) {           // both groups' products with the reference pixel
           return pk_make(dot2_bf16(t.word(1), ref.word(1), dot2_bf16(t.word(0), ref.word(0), 0.0f)),
                          dot2_bf16(t.word(3), ref.word(3), dot2_bf16(t.word(2), ref.word(2), 0.0f)));
         };
@@ -191,20 +201,32 @@ inline int v2_vox_go(const CvArgs& a, cudaStream_t st) {
   cv2_fwd_vox<T, SUB, PB, MIN><<<dim3((unsigned)((items + 3) / 4), a.B), 128, 0, st>>>(a, (unsigned)items, (unsigned)ndb);
   return (int)cudaGetLastError();
 }
-// C = 8, 16-byte aligned features, cost and mask; -4: not one of the cases
+// C = 8, aligned features (float32 MEAN, and MIN with two or four channels per group: to 32 bytes), cost and mask; -4: not one of the cases.
+// us at 1152x1536x8 / 576x768x16 (12 where noted), planes 1, 3 and 8 apart, kernels before (two lanes per pixel) against this one:
+//   float32 MEAN 8 groups, 1 view  225 229 239 : 239 237 243 / 108 110 116 : 98 98 102 (12: 83 84 88 : 90 90 93)
+//                          4 views 569 591 613 : 516 548 610 / 273 284 296 : 262 266 296 with two planes, 237 258 317 with four
+//                2 groups, 4 views 494 516 539 : 440 468 514 / 247 258 273 : 225 233 261 (16-byte loads 446 504 594 / 229 243 286)
+//   float32 MIN  8 groups, 1 view  274 281 291 : 300 306 321 / 133 135 141 : 120 119 124; 4 views 629 654 680 : 581 639 717 / 305 315 329 : 241 268 360
+//   bfloat16 MEAN 8 groups, 4 views 426 428 428 : 364 399 463 with four planes, 383 391 419 with two / 221 224 224 : 177 181 217, 190 192 204
+//   bfloat16 MIN 8 groups, 1 view  261 265 273 : 294 286 280 / 123 125 129 : 123 120 118 (12: 100 101 104 : 108 106 107)
+// How far a plane moves a footprint is not known here: four planes where they lie close by in most uses of so many planes and views.
 template <typename T>
 inline int v2_vox_fwd(const CvArgs& a, bool min, cudaStream_t st) {
-  if (a.C != 8 || ((reinterpret_cast<size_t>(a.ref) | reinterpret_cast<size_t>(a.src) | reinterpret_cast<size_t>(a.cost) |
-                    reinterpret_cast<size_t>(a.mask)) & 15) != 0)
-    return -4;
   const int sub = a.C / a.G;
+  const size_t feat = sizeof(T) == 4 && !(min && sub == 1) ? 31 : 15;
+  if (a.C != 8 || ((reinterpret_cast<size_t>(a.ref) | reinterpret_cast<size_t>(a.src)) & feat) != 0 ||
+      ((reinterpret_cast<size_t>(a.cost) | reinterpret_cast<size_t>(a.mask)) & 15) != 0)
+    return -4;
   const int nd = a.d_end - a.d_begin;
   if (min) {
-    if (sub == 1) return nd >= 16 ? v2_vox_go<T, 1, 4, true>(a, st) : v2_vox_go<T, 1, 2, true>(a, st);
+    if (sub == 1) return nd >= 16 ? v2_vox_go<T, 1, 4, true>(a, st) : a.N > 1 ? v2_vox_go<T, 1, 2, true>(a, st) : -4;
     return sub == 2 ? v2_vox_go<T, 2, 2, true>(a, st) : sub == 4 ? v2_vox_go<T, 4, 2, true>(a, st) : -4;
   }
-  if (sub == 1 && nd % 4 == 0 && (sizeof(T) == 2 || nd >= 16)) return v2_vox_go<T, 1, 4, false>(a, st);
-  if (sub == 1) return v2_vox_go<T, 1, 2, false>(a, st);
+  if (sub == 1) {
+    const bool four = sizeof(T) == 2 || (nd >= 16 && (a.N <= 2 || nd >= 32));
+    if (nd % 4 == 0 && four) return v2_vox_go<T, 1, 4, false>(a, st);
+    return sizeof(T) == 2 || a.N > 1 ? v2_vox_go<T, 1, 2, false>(a, st) : -4;
+  }
   return sub == 2 ? v2_vox_go<T, 2, 2, false>(a, st) : sub == 4 ? v2_vox_go<T, 4, 2, false>(a, st) : -4;
 }
 

@@ -40,3 +40,30 @@ def test_forward_and_gradient(dtype, G, shape, reduce):
     want_g = oracle.cost_bwd(2, f["ref"], f["src"], c["depth"], None, c["Rs"], c["Ts"], cg, mask, reduce, G, True, np.float32)
     for g, w in zip(grads, want_g):
         assert helpers.rel_err(g.cpu().numpy().reshape(w.shape), w) <= 1e-4
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("G", [8, 2])
+@pytest.mark.parametrize("N,D", [(1, 8), (1, 16), (1, 18), (3, 16), (3, 32), (4, 24)])   # both sides of the choice of kernel and of planes
+@pytest.mark.parametrize("reduce", ["MEAN", "MIN"])
+@pytest.mark.parametrize("shift", [0, 16])   # bytes by which the features miss a 32-byte boundary
+def test_choice_of_kernel(dtype, G, N, D, reduce, shift):
+    c = helpers.make_case(2, 17, 1, N, 6, 9, 8, D, "random", np.float32)
+    t = {k: torch.from_numpy(c[k]).to(dtype) for k in ("ref", "src")}
+    f = {k: t[k].float().numpy() for k in t}
+    want, mask = oracle.cost_fwd(2, f["ref"], f["src"], c["depth"], None, c["Rs"], c["Ts"], reduce, G, True, np.float32)
+
+    def place(x):
+        room = torch.empty(x.numel() + 32, dtype=x.dtype, device="cuda")
+        n = shift // x.element_size()
+        return room[n:n + x.numel()].view(x.shape).copy_(x)
+
+    cuda = lambda k: torch.from_numpy(c[k]).cuda()
+    ref, src = place(t["ref"]), place(t["src"])
+    assert ref.data_ptr() % 32 == shift
+    got, m = ops.cost_forward(2, ref, src, cuda("depth"), None, cuda("Rs"), cuda("Ts"), reduce, G)
+    assert np.array_equal(m.cpu().numpy().reshape(mask.shape), mask)
+    if reduce == "MIN":
+        assert np.array_equal(got.cpu().numpy().reshape(want.shape), want)
+    else:
+        assert helpers.rel_err(got.cpu().numpy().reshape(want.shape), want) <= 1e-5
