@@ -33,7 +33,8 @@ import numpy as np  # noqa: E402
 
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "dram_traffic.json")
 KERNEL_SOURCES = ("cv_packed.cuh", "cv_tuned.cuh", "cv_project.cuh", "chop_common.cuh", "cv_launch.cuh")
-CONV_SOURCES = ("sc_umma.cu", "sc_common.cuh", "sc_abi.cu")
+CONV_FWD_KERNEL = "sc_band_kernel"
+CONV_SOURCES = ("sc_band.cu", "sc_umma.cu", "sc_umma_common.cuh", "sc_common.cuh", "sc_entry.h", "sc_abi.cu")
 
 
 def cost_volume_config(workload, shard, B, N, C, H, W, D):
@@ -54,16 +55,16 @@ def kernel_source_digest(names=KERNEL_SOURCES):
     return h.hexdigest()
 
 
-def recorded_counters(workload, which, names=KERNEL_SOURCES):
+def recorded_counters(workload, which, names=KERNEL_SOURCES, kernel=""):
     """The ncu figures of one kernel of a workload, as written into profiles/dram_traffic.json when the capture was
     summarised (dram_bytes = dram__bytes_read.sum + dram__bytes_write.sum per launch; tensor_pipe_util where it
-    applies).  None if there is no record, or if the kernel sources have changed since (a stale figure is worse
-    than none)."""
+    applies).  None if there is no record, if the kernel sources have changed since (a stale figure is worse than none),
+    or if the record is of a kernel whose name does not begin with `kernel`."""
     try:
         rec = json.load(open(TRAFFIC_FILE))[workload]
         if rec.get("source_sha1") != kernel_source_digest(names):
             return None
-        return rec[which]
+        return rec[which] if rec[which]["kernel"].startswith(kernel) else None
     except Exception:
         return None
 
@@ -665,18 +666,18 @@ def sparse_conv_main(args):
     except Exception:
         pass
     ms = fwd_ms + bwd_ms
-    rec_f = recorded_counters("c4_sparse_conv", "fwd", CONV_SOURCES)
-    rec_w = recorded_counters("c4_sparse_conv", "wgrad", CONV_SOURCES)
+    rec_f = recorded_counters("c4_sparse_conv", "fwd", CONV_SOURCES, CONV_FWD_KERNEL)
+    rec_w = recorded_counters("c4_sparse_conv", "wgrad", CONV_SOURCES, "sc_umma_wgrad_rows_kernel")
     out = {"metric": "sparse_conv3d_fwd_bwd_voxels_per_s", "value": nvox / (ms * 1e-3), "unit": "voxels/s", "n_gpus": 1,
            "steps": K, "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
            "vs_baseline": None, "dtype": "bf16", "data": "synthetic",
            "config": {"workload": "c4_sparse_conv: SparseConv3DFast fwd+bwd, B=%d, %dx%d, band of %d planes, 3x3x3, %d->%d, bf16/fp32-acc"
                                   % (B, H, W, D, Cin, Cout), "l2": "flushed between steps (256 MB write)"},
            "gpu_launches": 4 * K, "umma_timeouts": _lib.lib().chop_umma_timeouts(),
-           "roofline": {"bound": "hbm", "kernel": "sc_band_kernel (forward)", "achieved": fwd_b / (fwd_ms * 1e-3) / 1e9, "peak": peak,
+           "roofline": {"bound": "hbm", "kernel": CONV_FWD_KERNEL + " (forward)", "achieved": fwd_b / (fwd_ms * 1e-3) / 1e9, "peak": peak,
                         "peak_source": peak_kind, "unit": "GB/s", "frac": fwd_b / (fwd_ms * 1e-3) / 1e9 / peak,
                         "traffic": (rec_f or {}).get("dram_bytes"),
-                        # sm__pipe_tensor_cycles_active of the recorded ncu captures (null once sc_umma.cu has changed)
+                        # sm__pipe_tensor_cycles_active of the recorded ncu captures (null once a file of CONV_SOURCES has changed)
                         "tensor_pipe_util": None if rec_f is None else {"fwd": rec_f.get("tensor_pipe_util"),
                                                                         "wgrad": (rec_w or {}).get("tensor_pipe_util")},
                         "fwd": {"ms": fwd_ms, "algorithmic_bytes": fwd_b, "tflops": flops_fwd / (fwd_ms * 1e-3) / 1e12,

@@ -38,6 +38,27 @@ def test_reference_arm_line():
     assert d["config"] == bench.cost_volume_config("c1_mvsnet", "batch", 1, 2, 32, 128, 160, 192)
 
 
+def test_recorded_counters_are_of_the_code_and_kernel_that_is_reported(tmp_path, monkeypatch):
+    import bench
+    src = os.path.join(ROOT, "custom_helper_op_b200", "csrc")
+    assert any(bench.CONV_FWD_KERNEL + "(" in open(os.path.join(src, n)).read() for n in bench.CONV_SOURCES)
+    used = [ln.split('"')[1] for n in bench.CONV_SOURCES for ln in open(os.path.join(src, n)) if ln.startswith('#include "')]
+    assert not [n for n in used if n.startswith("sc_") and n not in bench.CONV_SOURCES]
+    record = {"c4_sparse_conv": {"source_sha1": bench.kernel_source_digest(bench.CONV_SOURCES),
+                                 "fwd": {"kernel": bench.CONV_FWD_KERNEL + "<16, 16, 0>", "dram_bytes": 1}}}
+    path = tmp_path / "traffic.json"
+    monkeypatch.setattr(bench, "TRAFFIC_FILE", str(path))
+    look = lambda: bench.recorded_counters("c4_sparse_conv", "fwd", bench.CONV_SOURCES, bench.CONV_FWD_KERNEL)
+    path.write_text(json.dumps(record))
+    assert look()["dram_bytes"] == 1
+    record["c4_sparse_conv"]["fwd"]["kernel"] = "sc_umma_rows_kernel<16, 16, 0>"   # another kernel's figures
+    path.write_text(json.dumps(record))
+    assert look() is None
+    record["c4_sparse_conv"].update(source_sha1="0" * 40, fwd={"kernel": bench.CONV_FWD_KERNEL, "dram_bytes": 1})   # other code's
+    path.write_text(json.dumps(record))
+    assert look() is None
+
+
 @pytest.mark.gpu
 def test_cuda_arm_line():
     import bench
