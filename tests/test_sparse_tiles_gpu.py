@@ -1,0 +1,66 @@
+"""The convolutions that stage windows of planes, at sizes where every CTA takes many tiles: all channel pairs of the bfloat16 stride-1
+form, base planes that change from one tile to the next.  Against the kernels with a thread per output."""
+import numpy as np
+import pytest
+import torch
+
+from custom_helper_op_b200 import _lib
+from custom_helper_op_b200.python.ops import custom_helper_ops as ops
+
+pytestmark = pytest.mark.gpu
+CHANNELS = (8, 16, 32)
+
+
+def _bases(kind, B, H, W, slack, seed=0):
+    """smooth: one window a tile.  passes: up to one plane more than a window holds.  mixed: smooth, with rough patches."""
+    rng = np.random.default_rng(seed)
+    r, c = np.indices((H, W))
+    smooth = np.round(30 + 20 * np.sin(2 * np.pi * (r / H + 0.3)) * np.cos(2 * np.pi * c / W)).astype(np.int64)
+    if kind == "passes":
+        smooth = smooth * 0 + rng.integers(0, slack + 2, (H, W))
+    if kind == "mixed":
+        patch = np.kron(rng.random((H // 7 + 1, W // 11 + 1)) < 0.2, np.ones((7, 11), bool))[:H, :W]
+        smooth = np.where(patch, rng.integers(-40, 2000, (H, W)), smooth)
+    return torch.from_numpy(np.broadcast_to(smooth[None, :, :, None], (B, H, W, 1)).astype(np.int32).copy()).cuda()
+
+
+def _both(run):
+    """run() with the default kernels, and with a thread per output."""
+    got = run()
+    for knob in ("umma", "tile"):
+        _lib.set_tuning(knob, 0)
+    try:
+        want = run()
+    finally:
+        for knob in ("umma", "tile"):
+            _lib.set_tuning(knob, 1)
+    assert _lib.lib().chop_umma_timeouts() == 0
+    return list(zip(got, want))
+
+
+def _compare(got, want, taps):
+    """Both sides round sums of `taps` products: float32 in 24 bits at every addition, 2^-24 of the largest partial sum each (which the
+    largest result stands for), results in bfloat16 to one unit in the last place of eight bits apart."""
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[torch.isinf(got)], want[torch.isinf(want)])
+    ok = torch.isfinite(want)
+    g, w = got[ok].double(), want[ok].double()
+    if got.dtype == torch.bfloat16:
+        bound = 2.0 ** -7 * w.abs() + taps * 2.0 ** -24 * w.abs().max()
+    else:
+        bound = 3e-6 * w.abs().max()          # the root of the number of terms, some units of 2^-24
+    assert w.numel() > 0 and bool(((g - w).abs() <= bound).all()), float(((g - w).abs() / bound).max())
+
+
+@pytest.mark.parametrize("D,kind", [(9, "passes"), (9, "mixed"), (17, "passes"), (17, "mixed")])
+@pytest.mark.parametrize("cout", CHANNELS)
+@pytest.mark.parametrize("cin", CHANNELS)
+def test_bfloat16_stride_1_all_channel_pairs(cin, cout, D, kind):
+    B, H, W = (1, 141, 163) if D == 9 else (2, 67, 83)        # 3 to 20 tiles a CTA, none of which divides the image
+    g = torch.Generator(device="cuda").manual_seed(cin + cout + D)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()
+    images, filters, og = rnd(B, H, W, D, cin), rnd(3, 3, 3, cin, cout) * 0.25, rnd(B, H, W, D, cout)
+    bp = _bases(kind, B, H, W, (16 if D <= 10 else 32) - 2 - D)
+    run = lambda: (ops.sparse_conv3d_forward(images, filters, 0.75, bp), ops.sparse_conv3d_backward(images, filters, 0.75, bp, og)[0])
+    for (got, want), k in zip(_both(run), (cin, cout)):
+        _compare(got, want, 27 * k)
