@@ -1,5 +1,6 @@
 """The convolutions that stage windows of planes, at sizes where every CTA takes many tiles: all channel pairs of the bfloat16 stride-1
-form, base planes that change from one tile to the next.  Against the kernels with a thread per output."""
+form, the float32 stride-1 and transposed forms, base planes and values that change from one tile to the next.  Against the kernels
+with a thread per output."""
 import numpy as np
 import pytest
 import torch
@@ -64,3 +65,57 @@ def test_bfloat16_stride_1_all_channel_pairs(cin, cout, D, kind):
     run = lambda: (ops.sparse_conv3d_forward(images, filters, 0.75, bp), ops.sparse_conv3d_backward(images, filters, 0.75, bp, og)[0])
     for (got, want), k in zip(_both(run), (cin, cout)):
         _compare(got, want, 27 * k)
+
+
+def _spoil(x, g):
+    """Tiles that float32 computes without pieces between tiles in pieces: blocks of pixels of values near 2^-110, single voxels that are
+    no numbers."""
+    B, H, W, D, C = x.shape
+    block = torch.rand((B, H // 9 + 1, W // 23 + 1), generator=g, device="cuda") < 0.25
+    block = block.repeat_interleave(9, 1).repeat_interleave(23, 2)[:, :H, :W]
+    x = torch.where(block[..., None, None], x * 2.0 ** -110, x)
+    for i, v in enumerate((float("inf"), float("-inf"), float("nan"))):
+        at = torch.randint(0, B * H * W * D, (12,), generator=g, device="cuda")
+        x.view(-1, C)[at, i] = v
+    return x
+
+
+@pytest.mark.parametrize("values", ["ordinary", "spoilt"])
+@pytest.mark.parametrize("kind", ["smooth", "mixed"])
+@pytest.mark.parametrize("D", [7, 13])
+@pytest.mark.parametrize("chans", [(16, 16), (16, 32), (32, 16), (8, 8)])
+def test_float32_stride_1(chans, D, kind, values):
+    cin, cout = chans
+    B, H, W = 1, 101, 163                                     # 7 and more tiles a CTA
+    g = torch.Generator(device="cuda").manual_seed(cin + cout + D)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    images, filters, og = rnd(B, H, W, D, cin), rnd(3, 3, 3, cin, cout), rnd(B, H, W, D, cout)
+    if values == "spoilt":
+        images, og = _spoil(images, g), _spoil(og, g)
+    bp = _bases(kind, B, H, W, 0)
+
+    def run():                                                # the backward's gather form with no padding, and with one
+        return (ops.sparse_conv3d_forward(images, filters, 0.75, bp), ops.sparse_conv3d_backward(images, filters, 0.75, bp, og)[0],
+                ops.sparse_conv3d_transpose_forward(og, filters, 0.75, bp, (H, W, D)))
+    for (got, want), k in zip(_both(run), (cin, cout, cout)):
+        _compare(got, want, 27 * k)
+
+
+@pytest.mark.parametrize("values", ["ordinary", "spoilt"])
+@pytest.mark.parametrize("kind", ["smooth", "mixed"])
+@pytest.mark.parametrize("strides,chans", [((2, 2, 2), (8, 8)), ((2, 2, 2), (8, 16)), ((2, 2, 2), (16, 8)), ((2, 2, 2), (16, 16)),
+                                           ((2, 2, 1), (16, 16))])
+def test_float32_transposed(strides, chans, kind, values):
+    cin, cout = chans                                         # produced, gathered
+    H, W, D = 129, 163, 9                                     # 7 and more tiles a CTA
+    g = torch.Generator(device="cuda").manual_seed(cin + cout)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    coarse = [-(-n // s) for n, s in zip((H, W, D), strides)]
+    images, filters, fine = rnd(1, *coarse, cout), rnd(3, 3, 3, cin, cout), rnd(1, H, W, D, cin)
+    if values == "spoilt":
+        images = _spoil(images, g)
+    bp = _bases(kind, 1, H, W, 0)
+    run = lambda: (ops.sparse_conv3d_transpose_forward(images, filters, 0.75, bp, (H, W, D), strides),
+                   ops.sparse_conv3d_backward(fine, filters, 0.75, bp, images, strides)[0])
+    for got, want in _both(run):
+        _compare(got, want, 27 * cout)
