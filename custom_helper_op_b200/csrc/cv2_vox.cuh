@@ -5,10 +5,11 @@
 // from the next lane's: 32 lines a request, half of all that the L1 looked up.  Here the lanes of a warp are PB consecutive planes
 // of 32/PB neighbouring pixels: stores are whole runs of a slab, the corners of neighbouring pixels and planes share their
 // lines, a lane holds one voxel's sums (48 registers, 40 warps an SM) and nothing passes through shared memory.
-// Bound: L1 (gather) and the widening.  Four views, planes 1 / 8 apart, us before and now:
-//   bfloat16 MEAN, 8 groups  1152x1536x8 437 / 442, 371 / 447; 288x384x48 193 / 198, 138 / 144; 2 groups 385 / 407, 332 / 352; 166 / 176, 127 / 131
-//   bfloat16 MIN,  8 groups  1152x1536x8 632 / 662, 527 / 529; 2 groups 554 / 582, 403 / 404
-//   float32  MEAN, 8 groups  288x384x48 205 / 223, 158 / 207; 1152x1536x8 569 / 613, 516 / 610; where it is the slower one: v2_vox_fwd
+// Bound: issue (77 % of the slots at 1152x1536x8, bfloat16 MEAN; widening and paired blends) and the L1 behind it (68 % of its data pipe, four
+// gathers per voxel and view; a warp waits for them half of the time).  Four views, planes 1 / 8 apart, us before and now:
+//   bfloat16 MEAN, 8 groups  1152x1536x8 419 / 425, 364 / 408; 288x384x48 184 / 189, 131 / 134
+//   bfloat16 MIN,  8 groups  1152x1536x8 607 / 645, 530 / 515; 288x384x48 213 / 227, 176 / 174
+//   float32  MEAN, 8 groups  288x384x48 193 / 212, 144 / 184; 1152x1536x8 561 / 612, 514 / 560; where it is the slower one: v2_vox_fwd
 // PB = 4 against 2, bfloat16, 8 groups: 378 / 450 and 400 / 428 at 1152x1536x8, 143 / 146 and 157 / 157 at 288x384x48; 2 groups 335 / 410
 // and 336 / 353; float32 at 288x384x64, one view 104 and 135 (eight planes: 774 and 683).  Eight planes of four pixels 383 / 561.
 // Two or four voxels per lane (the cameras fetched once for them): 406 / 550, 454 / 631.  With 16 and 32 channels (two and four
@@ -58,12 +59,7 @@ __device__ __forceinline__ float dot2_bf16(unsigned a, unsigned b, float acc) { 
 // PB planes by 32/PB neighbouring pixels per warp: a lane is a voxel.
 constexpr int VOX_CTAS = 10;   // 128-thread CTAs per SM, 48 registers
 constexpr int VOX_MIN_CTAS = 8;
-// 32-byte loads: everywhere but in MIN with one channel per group, whose 64 registers do not hold their aligned groups (1152x1536x8, four
-// views, planes 1 / 8 apart: 581 / 717 us without, 686 / 790 with)
-template <int SUB, bool MIN>
-constexpr bool VOX_WIDE = !(MIN && SUB == 1);
-
-template <typename T, int SUB, int PB, bool MIN>
+template <typename T, int SUB, int PB, bool MIN, bool WIDE>
 __global__ void __launch_bounds__(128, MIN ? VOX_MIN_CTAS : VOX_CTAS) cv2_fwd_vox(const CvArgs a, const unsigned nitems, const unsigned ndb) {
   constexpr int C = 8, PX = 32 / PB;
   constexpr int NG = C / SUB;                        // groups per voxel
@@ -85,7 +81,6 @@ __global__ void __launch_bounds__(128, MIN ? VOX_MIN_CTAS : VOX_CTAS) cv2_fwd_vo
   }
   const size_t pix = (size_t)b * hw + p;
   const float depth = __ldcs(static_cast<const float*>(a.depth) + pix * a.D + d);
-  constexpr bool WIDE = VOX_WIDE<SUB, MIN>;
   Ch8<T, WIDE> ref;
   ref.load(static_cast<const T*>(a.ref) + pix * C);
   pk2 acc[NA];
@@ -193,41 +188,54 @@ __global__ void __launch_bounds__(128, MIN ? VOX_MIN_CTAS : VOX_CTAS) cv2_fwd_vo
   store_stream<float, NG>(static_cast<float*>(a.cost) + v * NG, o);
 }
 
-template <typename T, int SUB, int PB, bool MIN>
+template <typename T, int SUB, int PB, bool MIN, bool WIDE = false>
 inline int v2_vox_go(const CvArgs& a, cudaStream_t st) {
+  constexpr bool W = WIDE && sizeof(T) == 4;
+  if (((reinterpret_cast<size_t>(a.ref) | reinterpret_cast<size_t>(a.src)) & (W ? 31 : 15)) != 0) return -4;
   const int px = 32 / PB, ndb = (a.d_end - a.d_begin + PB - 1) / PB;
   const long long items = ((long long)a.H * a.W + px - 1) / px * ndb;
   if (items >= (1LL << 31) - 4 || a.B > 65535) return -4;
-  cv2_fwd_vox<T, SUB, PB, MIN><<<dim3((unsigned)((items + 3) / 4), a.B), 128, 0, st>>>(a, (unsigned)items, (unsigned)ndb);
+  cv2_fwd_vox<T, SUB, PB, MIN, W><<<dim3((unsigned)((items + 3) / 4), a.B), 128, 0, st>>>(a, (unsigned)items, (unsigned)ndb);
   return (int)cudaGetLastError();
 }
-// C = 8, aligned features (float32 MEAN, and MIN with two or four channels per group: to 32 bytes), cost and mask; -4: not one of the cases.
-// us at 1152x1536x8 / 576x768x16 (12 where noted), planes 1, 3 and 8 apart, kernels before (two lanes per pixel) against this one:
-//   float32 MEAN 8 groups, 1 view  225 229 239 : 239 237 243 / 108 110 116 : 98 98 102 (12: 83 84 88 : 90 90 93)
-//                          4 views 569 591 613 : 516 548 610 / 273 284 296 : 262 266 296 with two planes, 237 258 317 with four
-//                2 groups, 4 views 494 516 539 : 440 468 514 / 247 258 273 : 225 233 261 (16-byte loads 446 504 594 / 229 243 286)
-//   float32 MIN  8 groups, 1 view  274 281 291 : 300 306 321 / 133 135 141 : 120 119 124; 4 views 629 654 680 : 581 639 717 / 305 315 329 : 241 268 360
-//   bfloat16 MEAN 8 groups, 4 views 426 428 428 : 364 399 463 with four planes, 383 391 419 with two / 221 224 224 : 177 181 217, 190 192 204
-//   bfloat16 MIN 8 groups, 1 view  261 265 273 : 294 286 280 / 123 125 129 : 123 120 118 (12: 100 101 104 : 108 106 107)
-// How far a plane moves a footprint is not known here: four planes where they lie close by in most uses of so many planes and views.
+// C = 8, aligned features, cost and mask; -4: not one of the cases, or one where two lanes per pixel (cv_tuned.cuh) are the faster kernel.
+// us of that kernel against this one, on the inputs of an inference program (smooth depths, cameras around the scene), planes 1 / 8 apart:
+//   * Four planes a warp, MEAN and MIN with one channel per group, from 16 planes on where few lanes idle.  576x768x16, float32 MEAN,
+//     1 view 108 / 118 : 89 / 110, 4 views 270 / 294 : 212 / 294 (two planes 261 / 276); MIN 301 / 327 : 242 / 303.  1152x1536x8 bfloat16
+//     MEAN 421 / 425 : 367 / 409 (two planes, elsewhere measured: 383 / 419).
+//   * One channel per group, one view, planes that four do not divide or fewer than 16: float32 MEAN 576x768x18 106 / 114 : 116 / 129,
+//     x19 113 / 121 : 136 / 149, 1152x1536x8 234 / 247 : 227 / 263; MIN 576x768x18 129 / 142 : 151 / 162, bfloat16 122 / 130 : 147 / 147.
+//   * Two views, the same: MIN 1152x1536x9 403 / 429 : 445 / 475, bfloat16 399 / 413 : 431 / 414; 576x768x18 191 / 207 : 204 / 215, but
+//     288x384x50 132 / 139 : 128 / 132.  float32 MEAN 576x768x19 179 / 192 : 187 / 206, 1152x1536x9 376 / 398 : 363 / 407, x18 no difference.
+//   * 32-byte loads where they were the faster ones: with four channels per group (288x384x48, 4 views, 8 planes apart 186 -> 176), in MIN
+//     with two and four (1152x1536x8 606 -> 506), and with one and two in MEAN where the source features are larger than L2, so that a line
+//     fetched twice is the dearer thing: 1152x1536x8, 4 views, 16 bytes 496 / 627, 32 bytes 518 / 561 (two lanes per pixel 563 / 614), two
+//     channels per group 457 / 582, 483 / 517 (524 / 577); smaller 288x384x48 144 / 184, 164 / 187; two 164 / 187, 175 / 183.
+//     In MIN with one channel per group the 64 registers do not hold their aligned groups (581 -> 686).
+// What is left: MEAN and MIN with one channel per group and planes 8 apart lose up to 7 % where they gain as much or more at 1 apart
+// (float32, 4 views, MIN 576x768x19 335 / 358 : 310 / 383, MEAN 576x768x32 530 / 583 : 409 / 597).
 template <typename T>
 inline int v2_vox_fwd(const CvArgs& a, bool min, cudaStream_t st) {
-  const int sub = a.C / a.G;
-  const size_t feat = sizeof(T) == 4 && !(min && sub == 1) ? 31 : 15;
-  if (a.C != 8 || ((reinterpret_cast<size_t>(a.ref) | reinterpret_cast<size_t>(a.src)) & feat) != 0 ||
-      ((reinterpret_cast<size_t>(a.cost) | reinterpret_cast<size_t>(a.mask)) & 15) != 0)
-    return -4;
-  const int nd = a.d_end - a.d_begin;
+  if (a.C != 8 || ((reinterpret_cast<size_t>(a.cost) | reinterpret_cast<size_t>(a.mask)) & 15) != 0) return -4;
+  const int sub = a.C / a.G, nd = a.d_end - a.d_begin;
+  const int nd4 = (nd + 3) / 4 * 4;
   if (min) {
-    if (sub == 1) return nd >= 16 ? v2_vox_go<T, 1, 4, true>(a, st) : a.N > 1 ? v2_vox_go<T, 1, 2, true>(a, st) : -4;
-    return sub == 2 ? v2_vox_go<T, 2, 2, true>(a, st) : sub == 4 ? v2_vox_go<T, 4, 2, true>(a, st) : -4;
+    if (sub == 1) {
+      if (nd >= 16 && nd == nd4) return v2_vox_go<T, 1, 4, true>(a, st);
+      if (a.N == 1 || (a.N == 2 && nd != nd4 && nd < 32)) return -4;
+      return nd >= 16 && 16 * nd4 <= 17 * nd ? v2_vox_go<T, 1, 4, true>(a, st) : v2_vox_go<T, 1, 2, true>(a, st);
+    }
+    return sub == 2 ? v2_vox_go<T, 2, 2, true, true>(a, st) : sub == 4 ? v2_vox_go<T, 4, 2, true, true>(a, st) : -4;
   }
+  const bool far = sizeof(T) == 4 && (long long)a.N * a.Hs * a.Ws * 32 > 126LL << 20 &&
+                   ((reinterpret_cast<size_t>(a.ref) | reinterpret_cast<size_t>(a.src)) & 31) == 0;
   if (sub == 1) {
-    const bool four = sizeof(T) == 2 || (nd >= 16 && (a.N <= 2 || nd >= 32));
-    if (nd % 4 == 0 && four) return v2_vox_go<T, 1, 4, false>(a, st);
-    return sizeof(T) == 2 || a.N > 1 ? v2_vox_go<T, 1, 2, false>(a, st) : -4;
+    if (nd == nd4 && (sizeof(T) == 2 || nd >= 16)) return v2_vox_go<T, 1, 4, false>(a, st);
+    if (sizeof(T) == 4 && (a.N == 1 || (a.N == 2 && nd % 2 != 0))) return -4;
+    return far ? v2_vox_go<T, 1, 2, false, true>(a, st) : v2_vox_go<T, 1, 2, false>(a, st);
   }
-  return sub == 2 ? v2_vox_go<T, 2, 2, false>(a, st) : sub == 4 ? v2_vox_go<T, 4, 2, false>(a, st) : -4;
+  if (sub == 2) return far ? v2_vox_go<T, 2, 2, false, true>(a, st) : v2_vox_go<T, 2, 2, false>(a, st);
+  return sub == 4 ? v2_vox_go<T, 4, 2, false, true>(a, st) : -4;
 }
 
 }  // namespace chop

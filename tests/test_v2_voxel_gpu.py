@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import oracle
+from custom_helper_op_b200 import synth
 from custom_helper_op_b200.python.ops import custom_helper_ops as ops
 from tests import helpers
 
@@ -44,7 +45,8 @@ def test_forward_and_gradient(dtype, G, shape, reduce):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("G", [8, 2])
-@pytest.mark.parametrize("N,D", [(1, 8), (1, 16), (1, 18), (3, 16), (3, 32), (4, 24)])   # both sides of the choice of kernel and of planes
+@pytest.mark.parametrize("N,D", [(1, 8), (1, 16), (1, 18), (2, 17), (2, 18), (2, 34), (3, 16), (3, 18), (3, 19), (3, 32), (4, 24)])   # both sides of
+                         # the choice of kernel and of planes
 @pytest.mark.parametrize("reduce", ["MEAN", "MIN"])
 @pytest.mark.parametrize("shift", [0, 16])   # bytes by which the features miss a 32-byte boundary
 def test_choice_of_kernel(dtype, G, N, D, reduce, shift):
@@ -67,3 +69,24 @@ def test_choice_of_kernel(dtype, G, N, D, reduce, shift):
         assert np.array_equal(got.cpu().numpy().reshape(want.shape), want)
     else:
         assert helpers.rel_err(got.cpu().numpy().reshape(want.shape), want) <= 1e-5
+
+
+@pytest.mark.parametrize("G", [8, 4])
+def test_features_larger_than_l2(G):
+    """Source features of more than 126 MB are read in 32-byte loads where their addresses allow it, otherwise as smaller ones are."""
+    N, H, W, D = 4, 1000, 1100, 4
+    g = torch.Generator(device="cuda").manual_seed(G)
+    Rs, Ts = (torch.from_numpy(x).to("cuda", torch.float32) for x in synth.random_cameras(np.random.default_rng(1), 1, N, H, W))
+    depth = 600.0 + 200.0 * torch.rand((1, H, W, D), generator=g, device="cuda")
+    room = torch.randn((N + 1) * H * W * 8 + 8, generator=g, device="cuda")
+
+    def run(shift):
+        x = torch.empty_like(room)
+        x[shift:shift + room.numel() - 8] = room[:-8]
+        ref = x[shift:shift + H * W * 8].view(1, H, W, 8)
+        src = x[shift + H * W * 8:shift + room.numel() - 8].view(1, N, H, W, 8)
+        assert src.data_ptr() % 32 == shift * 4
+        return ops.cost_forward(2, ref, src, depth, None, Rs, Ts, "MEAN", G)
+
+    (a, ma), (b, mb) = run(0), run(4)
+    assert torch.equal(ma, mb) and int(ma.max()) == N and torch.equal(a, b)
