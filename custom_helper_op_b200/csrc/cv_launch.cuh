@@ -143,16 +143,24 @@ inline int bwd_tuned_pl(const CvArgs& a0, cudaStream_t st) {
   k<<<(unsigned)((items + warps - 1) / warps), warps * 32, smem, st>>>(a, warps, spw);
   return (int)cudaGetLastError();
 }
+// Planes of a pixel that all its chunks walk through in blocks of PB.
+inline int planes_walked(const CvArgs& a, int PB) {
+  const int n = a.d_end - a.d_begin, chunk = (a.chunk + PB - 1) / PB * PB;
+  return n / chunk * chunk + (n % chunk + PB - 1) / PB * PB;
+}
 // Eight and sixteen channels have two and four lanes per pixel, and a block of as many planes, at whose end every footprint is flushed.
 // Blocks of twice the planes halve that while the records and the staged upstream slice of the 24 warps that registers allow still
 // fit into an SM's shared memory.  128x160x192, one / two views, us with short and with long blocks: CostVolume C = 8 113 / 163, 104 / 152,
 // C = 16 132 / 195, 127 / 179; CostAggregate C = 8 97 / 148, 87 / 129, C = 16 110 / 173, 101 / 153.  Where they do not fit: CostVolume, six
 // views, C = 16 300, 338; CostAggregate MIN, four views, C = 8 131, 143.  With winners staged too (CostVolume MIN) they lose: C = 16 223, 245.
 // CostVolume C = 16 in bfloat16 keeps short ones: three items of 139x174, two views, short and long, 36 planes 260, 265; 64 381, 384; 68 397, 410.
+// Few planes that long blocks do not divide: 200x260, float32, two views, CostVolume C = 16 17 planes 82.9, 85.7, 25 107.5, 109.6, 36 123.9,
+// 123.8; C = 8 17 planes, one view 30.1, 31.2; CostAggregate C = 16 17 planes 80.3, 81.8, 25 101.4, 101.3; C = 8 96x120x17 17.8, 19.1.
 template <typename T, int C, int CPL, bool AGG = false, bool RMIN = false>
 inline int bwd_tuned_go(const CvArgs& a, cudaStream_t st) {
   if constexpr (C <= 16 && (AGG || !RMIN) && (AGG || C == 8 || sizeof(T) == 4)) {
-    if (24 * tuned_bwd_smem_per_warp<C>(a.N, 32 / (C / CPL), AGG ? 0 : 1, 2) <= (RMIN ? 180 : 216) * 1024)
+    if (10 * planes_walked(a, C / CPL * 2) <= 11 * planes_walked(a, C / CPL) &&
+        24 * tuned_bwd_smem_per_warp<C>(a.N, 32 / (C / CPL), AGG ? 0 : 1, 2) <= (RMIN ? 180 : 216) * 1024)
       return bwd_tuned_pl<T, C, CPL, AGG, RMIN, 2>(a, st);
   }
   return bwd_tuned_pl<T, C, CPL, AGG, RMIN, 1>(a, st);
