@@ -17,9 +17,10 @@
 //     columns a step as shared memory holds beside the other CTAs (all nine of 8 or 16 bfloat16 channels, five otherwise).
 //
 // Base planes of 64 planes over the image (two sinusoid periods), D = 9: 1.00 passes a tile at 256x320 pixels, 1.4 at 100x125.
-// Bound: the shared-memory data pipe (56 % load-store, of which half is the epilogue's tensor-memory reads and shuffles; 35 %
-// MMA operands) and, with four CTAs an SM, a tile's chain of staging, MMAs and epilogue.  256x320x9, 3x3x3, bfloat16, us:
-// 16 -> 16 channels 59 -> 41, 8 -> 8 51 -> 33, 32 -> 32 213 -> 100, 32 -> 16 129 -> 74; at 17 planes 97 -> 72, 344 -> 182.
+// Bound: the shared-memory data pipe (58 % load-store, of which half is the epilogue's tensor-memory reads and shuffles; 32 %
+// MMA operands) and, with four CTAs an SM, a tile's chain of staging, MMAs and epilogue.  256x320x9, 3x3x3, bfloat16, us of
+// sc_umma_rows_kernel and here, replayed from a graph: 16 -> 16 channels 54, 36, 8 -> 8 47, 27, 32 -> 32 208, 87, 32 -> 16 123, 62; at 17 planes
+// 92, 65, 338, 152.
 // Tiles of four rows with 256 threads: 45; of one row: 49; windows that do not divide 32 rows (25 for 17 planes): 108.
 // Base planes that vary: smooth / smooth with up to eight planes of noise on it / random, us of sc_umma_rows_kernel | with the window's
 // rows as the rough tile's buffer | here: 256x320x9 16 -> 16 57 / 56 / 53 | 37 / 96 / 94 | 36 / 65 / 59; 8 -> 8 51 / 50 / 50 | 34 / 73 / 71 |
@@ -29,9 +30,9 @@
 //
 // float32: a value is the exact sum of three bfloat16 pieces, x = x1 + x2 + x3, and x*w the sum of the six products
 // x1w1, x1w2, x2w1, x1w3, x2w2, x3w1 (what is left out is below 2^-24 of it).  Steps that the pieces cannot hold (pieces_fit) are
-// computed by plain multiply-adds (band_plain).  189x251x7, 16 -> 16 channels: 150 us with a thread per four voxels (sc_tile.cu),
-// 127 in runs of planes (sc_run.cu), 80 here; 16 -> 32 334, 238, 150.  Bound: 79 % of the shared-memory data pipe (operands 38,
-// load-store 41) at eight warps an SM; with a quarter of the MMAs 72 us, without the loads 90, without splitting 85.  Three
+// computed by plain multiply-adds (band_plain).  189x251x7, 16 -> 16 channels: 135 us with a thread per four voxels (sc_tile.cu),
+// 127 in runs of planes (sc_run.cu), 71 here; 16 -> 32 320, 238, 140.  Bound: 84 % of the shared-memory data pipe (operands 39,
+// load-store 45) at eight warps an SM; when it took 88 us, 72 with a quarter of the MMAs, 90 without the loads, 85 without splitting.  Three
 // groups of four warps around one filter 92 us, a thread per four channels instead of eight 99.
 #include "sc_entry.h"
 #include "sc_umma_common.cuh"
@@ -562,9 +563,11 @@ bool sc_band_better(const ScArgs& a, int cin, int cout) {
 }
 
 // float32, where this beats sc_run_kernel and is no less exact.  189x251x7, us there and here: 16 -> 16 127, 88; 16 -> 32 238, 166;
-// 16 -> 8 79, 84; 8 -> 8 49, 70; 8 -> 16 73, 74; 256x320x9 254, 140; 493, 268; 155, 134; 87, 112; 134, 117; 60x75x9, 16 -> 16 29, 30.
-// 2-norm of the error against float64 over that of the result: 16 gathered channels 1.38e-7 here, 1.80 to 1.92e-7 there; 32, whose
-// chains are twice as long, 3.0e-7 with the pieces cut off (not rounded), so they stay there.
+// 16 -> 8 79, 84; 8 -> 8 49, 70; 8 -> 16 73, 74; 256x320x9 254, 140; 493, 268; 155, 134; 87, 112; 134, 117; 60x75x9, 16 -> 16 29, 30
+// (when these were compared; 16 -> 16 and 16 -> 32 now 71, 139 and 135, 239).
+// 2-norm of the error against float64 over that of the result: 16 gathered channels 1.31 to 1.38e-7 here, 1.80 to 1.92e-7 there.  32, whose
+// chains are twice as long, 2.5 to 2.6e-7 here and 1.85 to 1.90e-7 there: less exact, so they stay there, although 256x320x9 32 -> 32
+// would take 625 us instead of 1134, 32 -> 16 314 instead of 575.
 bool sc_band_f32_better(const ScArgs& a, int cin, int cout) { return cin == 16 && cout >= 16 && a.D >= 5 && a.D <= 24; }
 
 int sc_band_launch(const ScArgs& a, bool dgrad, cudaStream_t st) {

@@ -193,12 +193,14 @@ int launch_run(const ScArgs& a, cudaStream_t st) {
 // thread per tap loads five for 32.  288 threads are 9 columns x the channel blocks x as many groups as that leaves room for, each
 // with pixels of its own; their sums are added in shared memory in a fixed order and sc_slab_reduce adds the CTAs'.
 // The upstream rows of the next pixels are copied while the present ones are multiplied.
-// Bound: issue and latency at three warps a scheduler (158 registers).  189x251x7, float32, 3x3x3, the filter gradient and its
+// Bound: issue and latency at three warps a scheduler (158 registers: issue 51 %, FMA pipe 58 %, stalls on dependent arithmetic, on the
+// gathered rows and on the FMA pipe in equal parts).  189x251x7, float32, 3x3x3, the filter gradient and its
 // reduction, us before (sc_tile.cu) and now: 16 -> 16 channels 215, 140; 8 -> 8 95, 48; 32 -> 32 670, 570.  Four upstream channels per
-// thread and two CTAs of nine warps 205, 288 threads 170.  Error against float64 (2-norm), 60x80: 16 -> 16 at 17 planes 2.39e-7
-// before, 2.3e-7 now; 32 -> 32 3.3e-7, 2.4e-7.
+// thread and two CTAs of nine warps 205, 288 threads 170.  Error against float64 (2-norm), 60x80x17: 16 -> 16 channels 2.39e-7
+// before, 1.87e-7 now; 32 -> 32 3.11e-7, 1.93e-7; 256x320x17 8.5e-7, 2.1e-7; 1.20e-6, 2.8e-7.
 constexpr int WG_THR = 384;   // twelve warps, three to a scheduler; 288 left one with three and three with two
 constexpr int WG_CHAIN = 64;    // planes after which a thread's sums go to its group's table, which keeps the chains of additions short
+                                // (fewer where a thread has fewer than 128: half of them)
 template <int KCH, int NCH>
 struct WgRun {
   static constexpr int QK = KCH / 4, QN = NCH / 8;    // channel blocks

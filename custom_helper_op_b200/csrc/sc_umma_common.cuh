@@ -1,6 +1,6 @@
-// What the tensor-core convolution kernels of sc_umma.cu and sc_band.cu share: descriptors, tcgen05 wrappers, the bounded
-// wait and its bookkeeping, the filter tiles.  Everything has internal linkage: each of the two files has its own counter
-// of abandoned waits, which sc_umma.cu adds up.
+// What the tensor-core convolution kernels of sc_umma.cu, sc_band.cu and sc_up.cu share: descriptors, tcgen05 wrappers, the bounded
+// wait and its bookkeeping, the filter tiles, the three pieces of a float32.  Everything has internal linkage: each of the three
+// files has its own counter of abandoned waits, which sc_umma.cu adds up.
 #pragma once
 #include <cuda_bf16.h>
 

@@ -14,10 +14,11 @@
 // Base planes that do not fit the window take further passes, with the window moved.  A tile that would need a fifth is "rough" (no depth
 // map) and left for the end: there the operand of each of its nine (offset, class) pairs - filter columns - is staged by itself, every
 // fine pixel's rows from the first coarse plane that its own taps read, SL columns at a time.
-// Bound: the epilogue (48 accumulator columns per class and row) and a tile's chain of staging, MMAs and epilogue at two CTAs of
-// eight warps an SM.  Transposed forward, 256x320x9, bfloat16, strides (2,2,2), us with a gather per tap and class
-// (sc_umma_class_kernel) and here: 16 <- 16 channels 43, 32; 16 <- 32 80, 37; 8 <- 8 38, 27; at 17 planes 66, 36; strides (2,2,1) 45, 37;
-// 60x75x12 16, 12.  With 32 produced channels the accumulators do not fit twice: those stay there.
+// Bound: a tile's chain of staging, MMAs and epilogue (48 accumulator columns per class and row) at two CTAs of eight warps an SM: no pipe
+// is above half (bfloat16 16 <- 16: load-store data 43 %, issue 44 %, operands 7 %; float32 43, 40, 22), the largest stall is the barrier
+// (2.1 and 3.6 of 8 and 9 cycles an instruction).  Transposed forward, 256x320x9, bfloat16, strides (2,2,2), us with a gather
+// per tap and class (sc_umma_class_kernel) and here, replayed from a graph: 16 <- 16 channels 37, 26; 16 <- 32 71, 30; 8 <- 8 32, 21; at 17
+// planes 60, 29; strides (2,2,1) 39, 31; 60x75x12 11, 7.  With 32 produced channels the accumulators do not fit twice: those stay there.
 // Base planes that vary: smooth / smooth with up to eight planes of noise on it / random, us of the gather | here with one pass more for
 // every pixel that does not fit | with rough tiles.  256x320x9, bfloat16: (2,2,2) 16 <- 16 40 / 40 / 38 | 34 / 36 / 387 | 35 / 37 / 55, 16 <- 32
 // 74 / 67 / 65 | 33 / 38 / 496 | 33 / 38 / 84; (2,2,1) 16 <- 16 41 / 40 / 38 | 31 / 63 / 439 | 32 / 64 / 51; float32 (sc_tile.cu, which leaves out
@@ -565,8 +566,9 @@ int sc_up_launch(const ScArgs& a, cudaStream_t st) {
   return -4;
 }
 // float32, where this is faster than sc_tile.cu and no less exact.  Transposed forward, us there and here (produced < gathered):
-// strides (2,2,2), 256x320x9 16<16 165, 83; 8<16 104, 72; 16<8 102, 78; 8<8 82, 68; at 17 planes 279, 92; 168, 74; 161, 89; 125, 72;
-// (2,2,1) 189x251x7 16<16 90, 70; 8<16 59, 64; 16<8 57, 64; 8<8 47, 58.  2-norm of the error against float64: (2,2,2) 16 gathered channels
+// strides (2,2,2), 256x320x9 16<16 152, 73; 8<16 96, 62; 16<8 94, 68; 8<8 74, 60; at 17 planes 269, 87; 168, 74; 161, 89; 125, 72;
+// (2,2,1) 189x251x7 16<16 79, 46; 8<16 59, 64; 16<8 57, 64; 8<8 47, 58.  (At 17 planes and depth stride 1 but for 16<16 called one by one, the
+// others replayed from a graph.)  2-norm of the error against float64: (2,2,2) 16 gathered channels
 // 8.6e-8 there, 6.2e-8 here, 8 8.0e-8, 4.7e-8; 32 8.9e-8, 9.5e-8 (and at depth stride 1 slower), so those stay there.
 bool sc_up_f32_supported(int dtype, const ScArgs& a) {
   return dtype == 0 && sc_up_supported(a) && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 &&

@@ -281,10 +281,11 @@ CHOP_API int chop_version(void);
 
 /* Tuning knobs for experiments: "fwd_chunk", "bwd_chunk" (depth planes per warp work item, 0 =
  * heuristic), "bwd_views" (source views per backward pass, 0 = heuristic), "tuned" (1 = use the compile-time-C
- * kernels where one exists, 0 = always the generic kernels), "umma" (1 = tensor-core manifold convolution
- * where supported, 0 = always the generic kernels), "umma_rows" (1 = the stride-1 tensor-core forward / image
- * gradient stages one copy per neighbour pixel, 0 = one per tap), "tile" (1 = register-tiled float32 manifold
- * convolution kernels where supported, 0 = the one-thread-per-element kernels), "packed" (1 = the packed-pair CostVolume
+ * kernels where one exists, 0 = always the generic kernels), "umma" (1 = bfloat16 manifold convolution on the tensor
+ * cores where supported, 0 = never), "umma_rows" (bfloat16 on the tensor cores: 1 = windows of planes where every voxel is staged once,
+ * for strides 1 and the transposed forms, and the kernels below elsewhere; 2 = never windows: at strides 1 one staged copy per
+ * neighbour pixel; 0 = one per tap), "tile" (float32 manifold convolution: 1 = runs and windows of planes, the latter on the tensor cores, and
+ * register-tiled kernels, where supported; 2 = register-tiled kernels only; 0 = one thread per output), "packed" (1 = the packed-pair CostVolume
  * MEAN kernels where one exists, 0 = the previous compile-time-C kernels), "fa_stage" (1 = FeatureAggregateGrad copies
  * its upstream tensor into shared memory a block of planes ahead where the channel count allows, 0 = never), "note_timeout" (1 = launch a one-thread
  * kernel that performs the bookkeeping of an abandoned tensor-core wait, without any wait; 0 = clear the counter of
