@@ -42,7 +42,7 @@ int sc_band_timeouts();
 int sc_band_publish_mirror(int* dptr, cudaStream_t st);
 int sc_band_clear_timeouts();
 // strided gather form with every coarse voxel staged once (sc_up.cu)
-bool sc_up_supported(const ScArgs& a);
+bool sc_up_supported(int dtype, const ScArgs& a);
 int sc_up_launch(const ScArgs& a, cudaStream_t st);
 bool sc_up_f32_supported(int dtype, const ScArgs& a);   // float32, in three bfloat16 pieces; the filter may lie at any address
 int sc_up_f32_launch(const ScArgs& a, cudaStream_t st);

@@ -1339,7 +1339,7 @@ int launch(const ScArgs& a, long long nvox, cudaStream_t st) {
   // otherwise at stride 1, for bands of at most 126 planes: the shifted-row kernel
   if (s1 && a.D + 2 <= 128 && g_umma_rows.load()) return launch_rows<CIN, COUT, DGRAD>(a, st);
   if constexpr (DGRAD) {
-    if (!s1 && g_umma_rows.load() == 1 && sc_up_supported(a)) return sc_up_launch(a, st);   // 256x320x9: 37 -> 26 us, see there
+    if (!s1 && g_umma_rows.load() == 1 && sc_up_supported(2, a)) return sc_up_launch(a, st);   // 256x320x9: 37 -> 26 us, see there
     if (!s1) return launch_class<CIN, COUT>(a, st);
   }
   auto k = s1 ? sc_umma_kernel<CIN, COUT, DGRAD, true> : sc_umma_kernel<CIN, COUT, DGRAD, DGRAD>;

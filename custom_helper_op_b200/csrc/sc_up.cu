@@ -557,8 +557,21 @@ int launch_depth(const ScArgs& a, cudaStream_t st) {
 
 }  // namespace
 
-// 3x3x3, dilation 1 and 31-bit voxel counts are the caller's conditions
-bool sc_up_supported(const ScArgs& a) { return a.sr == 2 && a.sc == 2 && a.sd <= 2 && a.Cin <= 16 && a.D <= 24; }
+// 3x3x3, dilation 1 and 31-bit voxel counts are the caller's conditions.  Bands of few planes leave most of a window's 16 rows empty; there the
+// gather is the faster kernel (us of it and of this one, replayed from a graph):
+//   * bfloat16, 16 produced channels, fewer than four planes on large images: 180x230x3 16 <- 16 15.0, 15.9; five planes 18.6, 16.1; 146x180x3
+//     14.0, 11.9.  At depth stride 1 fewer than nine planes on very small ones (a tile of eight pixels takes as long as its four
+//     classes): 48x60x6 8.2, 9.2, 9 planes 9.4, 9.2; 96x130x6 13.2, 11.2; stride 2 8.2, 6.8.
+//   * float32 with eight channels on either side, fewer than five planes (eight on both: six) on large images: 180x230x3 8 <- 8 26.5, 35.9, 8 <- 16
+//     30.6, 36.3, 16 <- 8 32.2, 39.6, 16 <- 16 43.5, 41.0; five planes 34.3, 35.7, 39.7, 36.5, 41.2, 39.9; 146x180x3
+//     23.9, 24.5, 26.6, 25.8, 28.1, 27.0.
+bool sc_up_supported(int dtype, const ScArgs& a) {
+  if (a.sr != 2 || a.sc != 2 || a.sd > 2 || a.Cin > 16 || a.D > 24) return false;
+  const long long pixels = (long long)a.B * a.H * a.W;
+  if (dtype == 0) return pixels < 34000 || a.Cin + a.Cout == 32 || a.D >= (a.Cin + a.Cout == 16 ? 6 : 5);
+  if (a.Cin < 16) return true;
+  return pixels >= 34000 ? a.D >= 4 || a.Cout > 16 : pixels >= 6000 || a.sd == 2 || a.D >= 9;
+}
 int sc_up_launch(const ScArgs& a, cudaStream_t st) {
 #define CHOP_CASE(I, O) if (a.Cout == I && a.Cin == O) return launch_depth<__nv_bfloat16, I, O>(a, st);
   CHOP_CASE(8, 8) CHOP_CASE(16, 8) CHOP_CASE(32, 8) CHOP_CASE(8, 16) CHOP_CASE(16, 16) CHOP_CASE(32, 16)
@@ -571,7 +584,7 @@ int sc_up_launch(const ScArgs& a, cudaStream_t st) {
 // others replayed from a graph.)  2-norm of the error against float64: (2,2,2) 16 gathered channels
 // 8.6e-8 there, 6.2e-8 here, 8 8.0e-8, 4.7e-8; 32 8.9e-8, 9.5e-8 (and at depth stride 1 slower), so those stay there.
 bool sc_up_f32_supported(int dtype, const ScArgs& a) {
-  return dtype == 0 && sc_up_supported(a) && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 &&
+  return dtype == 0 && sc_up_supported(dtype, a) && a.fh == 3 && a.fw == 3 && a.fd == 3 && a.dr == 1 && a.dc == 1 && a.dd == 1 &&
          (a.Cin == 8 || a.Cin == 16) && (a.Cout == 16 || (a.Cout == 8 && a.sd == 2)) && (a.sd == 2 || a.Cin == 16) &&
          a.nvox_in < (1LL << 31) - 4096;
 }

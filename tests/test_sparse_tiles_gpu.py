@@ -119,3 +119,21 @@ def test_float32_transposed(strides, chans, kind, values):
                    ops.sparse_conv3d_backward(fine, filters, 0.75, bp, images, strides)[0])
     for got, want in _both(run):
         _compare(got, want, 27 * cout)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("strides", [(2, 2, 2), (2, 2, 1)])
+@pytest.mark.parametrize("size,D", [((60, 99), 3), ((60, 99), 8), ((60, 99), 9), ((60, 101), 8), ((183, 184), 3), ((185, 184), 3), ((185, 184), 4),
+                                    ((185, 184), 5), ((185, 184), 6)])
+@pytest.mark.parametrize("chans", [(8, 8), (8, 16), (16, 8), (16, 16), (16, 32)])
+def test_transposed_around_the_choice_of_kernel(dtype, strides, size, D, chans):
+    """Few planes, on both sides of the image sizes from which the gather per tap takes over."""
+    cin, cout = chans
+    H, W = size
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(dtype)
+    images, filters = rnd(1, *(-(-n // s) for n, s in zip((H, W, D), strides)), cout), rnd(3, 3, 3, cin, cout) * 0.25
+    bp = _bases("mixed", 1, H, W, 0)
+    run = lambda: (ops.sparse_conv3d_transpose_forward(images, filters, 0.75, bp, (H, W, D), strides),)
+    for got, want in _both(run):
+        _compare(got, want, 27 * cout)
